@@ -1,13 +1,15 @@
-"""build.py: compiles libtkd.so (the CUDA kernels and their C-ABI) for sm_100a, in the tree, with nvcc.
+"""build.py: compiles libtkd.so (the CUDA kernels and their C-ABI) for sm_100a and tkd_host.so (the Python layer's
+native launch path over it), in the tree, with nvcc and g++.
 
     python tensix-kernels_b200/build.py [--verbose]
 
-The library sits beside its sources (csrc/libtkd.so); the Python layer loads it with ctypes and refuses to work
-without it. nvcc cross-compiles: no GPU is needed to build.
+Both sit beside their sources (csrc/); the Python layer loads them and refuses to work without them. nvcc
+cross-compiles: no GPU is needed to build.
 """
 
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -18,14 +20,30 @@ SOURCES = ["tkd_api.cu", "tkd_pack.cu", "tkd_stream.cu", "tkd_stream_bfp8.cu", "
 LIB = CSRC / "libtkd.so"
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
 OBJ = CSRC / "build"
+HOST = CSRC / "tkd_host.so"
+
+
+def _older(target, deps):
+    return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in deps)
 
 
 def stale():
-    if not LIB.exists():
-        return True
-    t = LIB.stat().st_mtime
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.h")) + [CSRC.parents[1] / "include" / "tkd.h"]
-    return any(d.stat().st_mtime > t for d in deps)
+    header = CSRC.parents[1] / "include" / "tkd.h"
+    return _older(LIB, [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *CSRC.glob("*.h"), header])
+
+
+def build_host(verbose=False, force=False):
+    """tkd_host.so, the extension module over libtkd.so (which it finds beside itself) and torch's C++ libraries."""
+    if not force and not _older(HOST, [CSRC / "tkd_host.cpp", CSRC.parents[1] / "include" / "tkd.h", LIB]):
+        return HOST
+    import torch
+
+    at = Path(torch.__file__).parent
+    inc = [sysconfig.get_paths()["include"], at / "include", at / "include/torch/csrc/api/include", "/usr/local/cuda/include"]
+    _run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          *(f"-I{i}" for i in inc), "-o", str(HOST), str(CSRC / "tkd_host.cpp"), f"-L{at / 'lib'}", "-lc10", "-lc10_cuda",
+          "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", f"-L{CSRC}", "-l:libtkd.so", "-Wl,-rpath,$ORIGIN"], verbose)
+    return HOST
 
 
 def _run(cmd, verbose):
@@ -33,12 +51,14 @@ def _run(cmd, verbose):
     if verbose or r.returncode:
         sys.stderr.write(r.stdout + r.stderr)
     if r.returncode:
-        raise RuntimeError("nvcc failed building libtkd.so: " + " ".join(cmd))
+        raise RuntimeError("the build failed: " + " ".join(cmd))
 
 
 def build(verbose=False, force=False, defines=(), lib=LIB):
-    """Compile the sources (one nvcc per file, side by side) and link them. defines: extra -D flags (experiments)."""
+    """Compile the sources (one nvcc per file, side by side) and link them, then the host module. defines: extra -D flags
+    (experiments: the library alone)."""
     if not force and not defines and not stale():
+        build_host(verbose)
         return lib
     OBJ.mkdir(exist_ok=True)
     extra = [*(["-Xptxas", "-v"] if verbose else []), *[f"-D{d}" for d in defines]]
@@ -47,6 +67,8 @@ def build(verbose=False, force=False, defines=(), lib=LIB):
         list(pool.map(lambda so: _run(["nvcc", *FLAGS, *extra, "-c", "-o", str(so[1]), str(CSRC / so[0])], verbose),
                       zip(SOURCES, objs)))
     _run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", str(lib), *map(str, objs)], verbose)
+    if lib == LIB:
+        build_host(verbose, force)
     return lib
 
 

@@ -175,6 +175,7 @@ class Weight(Tensor):
         self.fmt = FMT[dtype] if fmt is None else fmt
         self.wide = self.fmt != FMT[dtype]
         self.serial = next(Weight._serials)
+        self.calls = {}  # dense_reader.linear's described calls on this weight
         sp = memory_config.shard_spec
         self._npad = sp.shape[1] * sp.banks if sp else _pad(n)
 
@@ -300,6 +301,7 @@ def deallocate(t):
     if isinstance(t, Weight):
         t.emax = None
         t._bf16_twin = None
+        t.calls.clear()
 
 
 def reshape(t, shape):

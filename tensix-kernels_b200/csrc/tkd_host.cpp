@@ -1,0 +1,99 @@
+// tkd_host.cpp: the Python side's launch path in native code (module tkd_host, used by dense_reader/linear.py and
+// moe/moe8.py): a call described once is launched again with other tensors.
+//
+// What bounds a small decode call is not its kernel (about 5 us) but the host: one launch through ctypes, with the
+// output allocated by torch.empty and the stream asked from Python, took 29 us for one token through a [4096, 2048]
+// bfloat8_b weight. Here the same steps (the output's allocation, the current stream, the descriptor's addresses, the
+// launch) are one call into C++ on a copy of the caller's descriptor, so nothing shared between threads is written.
+//
+// libtkd.so stays free of torch types (include/tkd.h is its whole interface); this module is a client of it.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/tkd.h"
+
+namespace {
+
+// A tensor argument, or null for None.
+const at::Tensor* tensor_or_null(PyObject* o) { return o == Py_None ? nullptr : &THPVariable_Unpack(o); }
+
+bool all_tensors(PyObject* const* args, std::initializer_list<int> need, std::initializer_list<int> may) {
+    for (int i : need)
+        if (!THPVariable_Check(args[i])) return false;
+    for (int i : may)
+        if (args[i] != Py_None && !THPVariable_Check(args[i])) return false;
+    return true;
+}
+
+PyObject* type_error(const char* what) {
+    PyErr_SetString(PyExc_TypeError, what);
+    return nullptr;
+}
+
+// The error of libtkd's code `rc` as the Python layer raises it.
+PyObject* tkd_error(int rc, const char* what) {
+    PyObject* mod = PyImport_ImportModule("dense_reader._tkd");
+    if (!mod) return nullptr;
+    PyObject* r = PyObject_CallMethod(mod, "check", "is", rc, what);
+    Py_XDECREF(r);
+    Py_DECREF(mod);
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, what);
+    return nullptr;
+}
+
+// matmul(descriptor's address, x, out or None, residual or None, workspace, row0) -> the output tensor.
+// The descriptor (a TkdMatmul kept by the caller) with this call's tensors: rows row0 .. row0 + m of x, out and residual.
+// out None: a new [1, 1, m, ldo] tensor of the descriptor's type.
+PyObject* host_matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 6 || !all_tensors(args, {1, 4}, {2, 3}))
+        return type_error("tkd_host.matmul: descriptor, x, out, residual, workspace, row0");
+    const auto* desc = static_cast<const TkdMatmul*>(PyLong_AsVoidPtr(args[0]));
+    const int64_t row0 = PyLong_AsLongLong(args[5]);
+    if (PyErr_Occurred()) return nullptr;
+    try {
+        const at::Tensor& x = THPVariable_Unpack(args[1]);
+        const at::Tensor *out = tensor_or_null(args[2]), *res = tensor_or_null(args[3]);
+        const at::Tensor& ws = THPVariable_Unpack(args[4]);
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != x.get_device()) guard.set_index(x.get_device());
+        TkdMatmul a = *desc;
+        at::Tensor made;
+        const bool f32 = a.out_dtype == TKD_DT_F32;
+        if (!out) {
+            const int64_t shape[4] = {1, 1, a.m, a.ldo};
+            made = at::detail::empty_cuda(shape, f32 ? at::kFloat : at::kBFloat16, x.device(), std::nullopt);
+            out = &made;
+        }
+        a.x = static_cast<const char*>(x.data_ptr()) + row0 * a.ldx * 2;
+        a.out = static_cast<char*>(out->data_ptr()) + row0 * a.ldo * (f32 ? 4 : 2);
+        a.residual = res ? static_cast<const char*>(res->data_ptr()) + row0 * a.ldr * (a.residual_dtype == TKD_DT_F32 ? 4 : 2) : nullptr;
+        a.workspace = ws.data_ptr();
+        a.workspace_bytes = (uint64_t)ws.nbytes();
+        void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
+        int rc;
+        Py_BEGIN_ALLOW_THREADS rc = tkd_matmul(&a, stream);
+        Py_END_ALLOW_THREADS if (rc) return tkd_error(rc, "tkd_matmul");
+        if (made.defined()) return THPVariable_Wrap(std::move(made));
+        Py_INCREF(args[2]);
+        return args[2];
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+PyMethodDef methods[] = {
+    {"matmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(host_matmul)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "tkd_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_tkd_host() { return PyModule_Create(&module_def); }

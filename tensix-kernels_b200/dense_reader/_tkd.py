@@ -5,6 +5,7 @@ non-zero code raises.
 """
 
 import ctypes
+import importlib.util
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parents[1]
@@ -111,6 +112,23 @@ def lib():
                                    f" is {L.tkd_struct_bytes(which)} bytes there, {ctypes.sizeof(mirror)} here): rebuild")
         _lib = L
     return _lib
+
+
+HOST_PATH = PKG / "csrc" / "tkd_host.so"
+_host = None
+
+
+def host():
+    """The native launch path over the library (csrc/tkd_host.cpp); a RuntimeError naming the build step when missing."""
+    global _host
+    if _host is None:
+        lib()  # (checks the library the module links to)
+        if not HOST_PATH.exists():
+            raise RuntimeError(f"dense_reader: {HOST_PATH} is missing; build it with `python {PKG / 'build.py'}`")
+        spec = importlib.util.spec_from_file_location("tkd_host", HOST_PATH)
+        _host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_host)
+    return _host
 
 
 class TkdError(RuntimeError):

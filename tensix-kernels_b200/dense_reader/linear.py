@@ -62,7 +62,7 @@ GLU_ROWS = True
 CONFIGS = ({"cores_per_bank": 2, "split": True, "rows": True},)
 # the top-k result tensor as bfloat16 (the same bytes as the uint32 words; False: uint32)  (linear.py:77-78)
 RECORDS_BF16 = False
-# launch descriptors cached by everything that shapes them (a hit only rewrites the tensors' addresses)  (:79-80)
+# calls kept with their weight by everything that shapes them (a hit only takes the tensors' addresses)  (:79-80)
 CACHE = True
 # a line per planned shape on stdout  (:81-82)
 LOG = False
@@ -77,9 +77,9 @@ _TENSIX_OPTS = {"cores_per_bank", "split", "rows", "xs", "kb", "kw", "sbw", "nos
 _OPTS = _TENSIX_OPTS | {"glu", "glu_act", "residual", "residual_mode", "out32", "blocks", "max_banks", "col_scales", "ks",
                         "max_ctas", "exchange", "hadamard"}
 
-_CALLS = {}      # whole calls by the identity of their arguments (a hit goes straight to the library)
+_CALLS = {}      # matmul_host's calls by the identity of their arguments (a hit goes straight to the library)
 _CALLS_MAX = 256
-_LAUNCHES = {}   # the launch cache: key -> (TkdMatmul, keep-alive)
+_WEIGHT_CALLS = 64  # described calls kept with a weight, at most
 _CHOICE = {}     # the plan cache
 _WORKSPACE = {}  # device id -> zeroed uint8 tensor
 _STATUS = {}     # device id -> int32 status word
@@ -396,20 +396,27 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
     as slices of 32, each reading the weights once."""
     call_key = None
     if CACHE:
-        # The same call again (the same tensor objects and options): everything was checked and described the first
-        # time; only the addresses are looked at again. The entry keeps its arguments alive, so their ids stay theirs.
-        call_key = _call_key(x, w, scale, topk, out, col0, w_up, max_banks, opts)
-        hit = _CALLS.get(call_key)
-        if hit is not None and hit["ws_key"][1] != WORKSPACE_SLOT:
-            hit = None
-        if hit is not None and _replay(hit):
-            return hit["y"]
-    launched = []
+        # A call described before on this weight, whatever its tensors' addresses: everything was checked then.
+        first, call_key = _call_key(x, w, scale, topk, out, col0, w_up, max_banks, fidelity, opts)
+        call = first.calls.get(call_key) if call_key is not None else None
+        if call is not None and call.fits(x, out):
+            y = call.run(x, out, opts.get("residual"))
+            return out if out is not None else ttnn.Tensor(y, call.out_dtype, ttnn.TILE_LAYOUT, call.device, memory_config)
+    y, call = _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0, w_up, max_banks, opts)
+    if call_key is not None and call.exchange is None:
+        if len(first.calls) >= _WEIGHT_CALLS:
+            first.calls.clear()
+        first.calls[call_key] = call
+    return y
+
+
+def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0, w_up, max_banks, opts):
+    """matmul's call checked, described and run once: (its output, the _Call that runs it again)."""
     device = x.device()
     unknown = set(opts) - _OPTS
     if unknown:
         raise TypeError(f"dense_reader.matmul: unknown options {sorted(unknown)}")
-    opts_in = dict(opts)
+    opts = dict(opts)
     if not isinstance(w, (list, tuple)):
         check_banks(w, max_banks)
     elif is_block_list(w):
@@ -497,28 +504,103 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
     slices = choose(device, x, w, full_sync, **opts)
     if segs:
         _block_kw_check(device, x, blocks_all, full_sync, opts, slices)
+    launches, need = [], 0
     for m0, _ in slices:
-        launched.append(_launch(x, blocks_all, scale, col_scales, y, m0, min(32, M - m0), topk, act, residual, glu,
-                                out32, opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, exchange, hadamard))
-    if call_key is not None and out is not None:
-        # (only calls that write into a given output: a fresh output per call cannot be replayed)
-        if len(_CALLS) >= _CALLS_MAX:
-            _CALLS.clear()
-        ws = _WORKSPACE.get(_ws_key(device))
-        _CALLS[call_key] = {
-            "y": y, "launches": launched, "device": device, "ws": ws, "ws_key": _ws_key(device), "exchange": exchange,
-            "keep": (x, w, scale, out, w_up, topk, opts_in),
-            "ptrs": (_raw(x).data_ptr(), _raw(y).data_ptr()),
-            "topk": None if topk is None else tuple(sorted((k, id(v)) for k, v in topk.items())),
-        }
-    return y
+        a, n = _describe_rows(x, blocks_all, scale, col_scales, y, min(32, M - m0), topk, act, residual, glu, out32,
+                              opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, hadamard)
+        launches.append((m0, a))
+        need = max(need, n)
+    scales = col_scales if isinstance(col_scales, (tuple, list)) else (col_scales,)
+    others = [t for g, u, _ in blocks_all for t in (g, u)][1:]
+    call = _Call(device, launches, need, (scale, col_scales, *scales, hadamard, topk and topk["r"], *others), y.dtype, exchange)
+    call.run(x, y, residual)
+    return y, call
 
 
-def _call_key(x, w, scale, topk, out, col0, w_up, max_banks, opts):
-    # (the entry keeps its arguments alive, so their ids stay theirs; ttnn.deallocate starts a new epoch, which retires
-    # every entry made before it)
-    return (ttnn.EPOCH, id(x), id(w), id(scale), id(out), id(w_up), id(topk), col0, max_banks, KS, MAX_CTAS, TOPK_UNIT, WORKSPACE_SLOT,
-            tuple((k, tuple(map(id, v)) if type(v) is tuple else id(v)) for k, v in opts.items()))
+_PLAIN = {int, bool, str, type(None)}
+
+
+def _call_key(x, w, scale, topk, out, col0, w_up, max_banks, fidelity, opts):
+    """(the weight a call is kept with, what else shapes it). Objects are named by their identities: the kept call keeps
+    them alive, so the identities stay theirs."""
+    if type(w) is list or type(w) is tuple:
+        try:
+            wk = tuple([(id(e[0]) if type(e[0]) is not tuple and type(e[0]) is not list else tuple(map(id, e[0])), e[1]) for e in w])
+            first = w[0][0]
+            if type(first) is tuple or type(first) is list:
+                first = first[0]
+        except (TypeError, IndexError):
+            return None, None  # (not a block list: the full path says so)
+    else:
+        first, wk = w, None
+    if type(first) is not ttnn.Weight:
+        return None, None
+    ok = ()
+    if opts:
+        ok = tuple([(k, v if type(v) in _PLAIN else tuple(map(id, v)) if type(v) is tuple else
+                     (v.t.shape, id(v.dtype)) if k == "residual" and type(v) is ttnn.Tensor else id(v)) for k, v in opts.items()])
+    tk = None
+    if topk is not None:
+        tk = (id(topk["r"]), topk["k"], topk["rows"], topk["slot0"], topk["base"], topk["n"], topk.get("write_y", False), TOPK_UNIT)
+    return first, (x.t.shape, None if out is None else out.t.shape, wk, id(scale), id(w_up), col0, max_banks, fidelity, ok, tk,
+                   KS, MAX_CTAS, dev.MAX_BANKS)
+
+
+class _Call:
+    """A described call on a weight: the launches' descriptors (first row, TkdMatmul), run again on other activations,
+    outputs and residuals of the same shapes. It keeps what it names but the weight it is kept with."""
+
+    __slots__ = ("device", "launches", "need", "single", "keep", "out_dtype", "exchange", "epoch", "where", "launch")
+
+    def __init__(self, device, launches, need, keep, out_dtype, exchange):
+        self.device, self.launches, self.need, self.keep = device, launches, need, keep
+        self.out_dtype, self.exchange = out_dtype, exchange
+        self.single = ctypes.addressof(launches[0][1]) if len(launches) == 1 and exchange is None else None
+        self.launch = _tkd.host().matmul
+        self.epoch = ttnn.EPOCH
+        self.where = [(t, t.t.data_ptr()) for t in keep if isinstance(t, ttnn.Tensor)]
+
+    def fits(self, x, out):
+        """Whether this call's tensors are of the kind described, and nothing it names was freed or moved since."""
+        if self.epoch != ttnn.EPOCH:
+            if any(t.t is None or t.t.data_ptr() != at for t, at in self.where):
+                return False
+            self.epoch = ttnn.EPOCH
+        return (x.dtype is ttnn.bfloat16 and x._device is self.device and x._mc.memory_layout is ttnn.TensorMemoryLayout.INTERLEAVED
+                and (out is None or out.dtype is self.out_dtype))
+
+    def run(self, x, out, residual):
+        """Launch: the output's torch tensor (a new one where out is None)."""
+        res = None if residual is None else residual.t
+        if self.single is not None:
+            return self.launch(self.single, x.t, None if out is None else out.t, res, _workspace(self.device, self.need), 0)
+        device = self.device
+        if out is None:
+            a = self.launches[0][1]
+            y = torch.empty(1, 1, x.t.shape[-2], a.ldo, dtype=ttnn._TORCH[self.out_dtype], device=device.torch)
+        else:
+            y = out.t
+        for row0, a in self.launches:
+            if self.exchange is None:
+                self.launch(ctypes.addressof(a), x.t, y, res, _workspace(self.device, self.need), row0)
+                continue
+            with torch.cuda.device(device.torch):
+                a = self.bound(x.t, y, res, row0)
+                _tkd.check(_tkd.lib().tkd_matmul(ctypes.byref(a), torch.cuda.current_stream().cuda_stream), "tkd_matmul")
+                self.exchange.after_launch(status_word(device))
+        return y
+
+    def bound(self, xt, yt, rt, row0=0):
+        """A copy of row slice row0's descriptor with these tensors' addresses."""
+        a = _tkd.TkdMatmul.from_buffer_copy(next(a for r, a in self.launches if r == row0))
+        a.x = xt.data_ptr() + row0 * a.ldx * 2
+        a.out = yt.data_ptr() + row0 * a.ldo * yt.element_size()
+        a.residual = rt.data_ptr() + row0 * a.ldr * rt.element_size() if rt is not None else None
+        ws = _workspace(self.device, self.need)
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        if self.exchange is not None:
+            self.exchange.fill(a, a.out, a.records)
+        return a
 
 
 def matmul_host(x_host, out_host, x, w, scale, *, topk=None, out=None, col0=0, w_up=None, max_banks=None, stream=None,
@@ -529,50 +611,34 @@ def matmul_host(x_host, out_host, x, w, scale, *, topk=None, out=None, col0=0, w
     (tkd_matmul_host) instead of three framework calls. The other arguments are matmul's; up to 32 rows. The first call with a given set of tensors goes
     through matmul itself (which checks everything and also launches once)."""
     assert out is not None and CACHE, "dense_reader.matmul_host: needs out= and the launch cache"
-    key = _call_key(x, w, scale, topk, out, col0, w_up, max_banks, opts)
+    key = (ttnn.EPOCH, id(x), id(w), id(scale), id(out), id(w_up), id(topk), col0, max_banks, KS, MAX_CTAS, TOPK_UNIT, WORKSPACE_SLOT,
+           tuple((k, tuple(map(id, v)) if type(v) is tuple else id(v)) for k, v in opts.items()))
+    ws = _WORKSPACE.get(_ws_key(x.device()))
     hit = _CALLS.get(key)
-    if hit is None:
-        if stream is None:
-            matmul(x, w, scale, topk=topk, out=out, col0=col0, w_up=w_up, max_banks=max_banks, **opts)
-        else:
-            with torch.cuda.stream(stream):
-                matmul(x, w, scale, topk=topk, out=out, col0=col0, w_up=w_up, max_banks=max_banks, **opts)
-        hit = _CALLS[key]
-    assert len(hit["launches"]) == 1, "dense_reader.matmul_host: one launch (up to 32 rows)"
-    assert hit["exchange"] is None or hit["exchange"].side is None, (
-        "dense_reader.matmul_host: the result is copied out by the same call, so an exchange must complete inside the kernel")
+    if hit is None or hit["ws"] is not ws:
+        with torch.cuda.stream(stream):  # (None: the current stream)
+            _, call = _described(x, w, scale, None, "hifi2", False, topk, out, col0, w_up, max_banks, opts)
+        assert len(call.launches) == 1, "dense_reader.matmul_host: one launch (up to 32 rows)"
+        assert call.exchange is None or call.exchange.side is None, (
+            "dense_reader.matmul_host: the result is copied out by the same call, so an exchange must complete inside the kernel")
+        if len(_CALLS) >= _CALLS_MAX:
+            _CALLS.clear()
+        res = opts.get("residual")
+        hit = _CALLS[key] = {
+            "a": call.bound(x.t, out.t, None if res is None else res.t), "ws": _WORKSPACE.get(_ws_key(x.device())), "call": call,
+            # (the arguments stay alive, so their ids stay theirs; ttnn.deallocate starts a new epoch, which retires
+            # every entry made before it)
+            "keep": (x, w, scale, out, w_up, topk, dict(opts)),
+        }
     sp = torch.cuda.current_stream().cuda_stream if stream is None else stream.cuda_stream
-    rc = _tkd.lib().tkd_matmul_host(ctypes.byref(hit["launches"][0]), x_host.data_ptr(), out_host.data_ptr(), sp)
+    rc = _tkd.lib().tkd_matmul_host(ctypes.byref(hit["a"]), x_host.data_ptr(), out_host.data_ptr(), sp)
     if rc:
         _tkd.check(rc, "tkd_matmul_host")
     return out
 
 
-def _replay(hit):
-    """Launch a cached call again; False when something under it has moved (then the full path runs)."""
-    x, _, _, _, _, topk, _ = hit["keep"]
-    device = hit["device"]
-    if (_raw(x).data_ptr(), _raw(hit["y"]).data_ptr()) != hit["ptrs"] or _WORKSPACE.get(hit["ws_key"]) is not hit["ws"]:
-        return False
-    if torch.cuda.current_device() != device.id:
-        return False
-    if topk is not None and tuple(sorted((k, id(v)) for k, v in topk.items())) != hit["topk"]:
-        return False
-    fn = _tkd.lib().tkd_matmul
-    stream = torch.cuda.current_stream().cuda_stream
-    for a in hit["launches"]:
-        rc = fn(ctypes.byref(a), stream)
-        if rc:
-            _tkd.check(rc, "tkd_matmul")
-        if hit["exchange"] is not None:
-            hit["exchange"].after_launch(status_word(device))
-    return True
-
-
-def _launch(x, entries, scale, col_scales, y, m0, m, topk, act, residual, glu, out32, ks=0, max_ctas=0, exchange=None,
-            hadamard=None):
-    """One launch of the stream kernel: rows m0 .. m0 + m of x into the same rows of y. The descriptor is cached by
-    everything that shapes it; a hit only rewrites the activation, output and residual addresses.
+def _describe_rows(x, entries, scale, col_scales, y, m, topk, act, residual, glu, out32, ks=0, max_ctas=0, hadamard=None):
+    """(the descriptor of one launch over m rows of x, without its tensors' addresses; the workspace it needs).
     (linear.py:828-1070)"""
     device = x.device()
     w, w_up, _ = entries[0]
@@ -594,47 +660,14 @@ def _launch(x, entries, scale, col_scales, y, m0, m, topk, act, residual, glu, o
         assert sc.dtype == torch.float32 and sc.is_cuda and sc.numel() >= w.n, "dense_reader: col_scales: float32 [N] on the device"
         scale_dt = _tkd.DT_F32
     res_dt = _tkd.DT_NONE if residual is None else (_tkd.DT_F32 if residual.dtype == ttnn.float32 else _tkd.DT_BF16)
-    xt, yt = _raw(x), _raw(y)
-    rt = _raw(residual) if residual is not None else None
-    key = None
-    if CACHE:
-        tk = None if topk is None else (_raw(topk["r"]).data_ptr(), topk["k"], topk["rows"], topk["slot0"], topk["base"],
-                                        topk["n"], bool(topk.get("write_y", False)), TOPK_UNIT)
-        key = (
-            # (weights by their serial numbers, never by address: a freed weight's memory may come back as another
-            # weight's stream, a serial does not come back)
-            ttnn.EPOCH, tuple((g.serial, u.serial if u is not None else 0, c0) for g, u, c0 in entries),
-            m, tuple(xt.shape), tuple(yt.shape), epi, act, sc.data_ptr() if sc is not None else 0,
-            sc_up.data_ptr() if sc_up is not None else 0, scale_dt, res_dt, tk, ks, max_ctas, device.id, id(exchange),
-            _raw(hadamard).data_ptr() if hadamard is not None else 0,
-        )
-    hit = _LAUNCHES.get(key) if key is not None else None
-    if hit is None:
-        blocks = [(g, u, c0 * TILE) for g, u, c0 in entries]
-        a = _describe(xt, m, blocks, epi, act, sc, sc_up, scale_dt, rt, res_dt, yt, topk, ks, max_ctas)
-        need = ctypes.c_uint64(0)
-        _tkd.check(_tkd.lib().tkd_matmul_workspace(ctypes.byref(a), ctypes.byref(need)), "tkd_matmul_workspace")
-        a.hadamard = _raw(hadamard).data_ptr() if hadamard is not None else None
-        hit = (a, need.value, (sc, sc_up, exchange, hadamard))
-        if key is not None:
-            _LAUNCHES[key] = hit
-    a, need, _ = hit
-    ws = _workspace(device, need)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    blocks = [(g, u, c0 * TILE) for g, u, c0 in entries]
+    a = _describe(_raw(x), m, blocks, epi, act, sc, sc_up, scale_dt, None if residual is None else _raw(residual), res_dt, _raw(y),
+                  topk, ks, max_ctas)
+    need = ctypes.c_uint64(0)
+    _tkd.check(_tkd.lib().tkd_matmul_workspace(ctypes.byref(a), ctypes.byref(need)), "tkd_matmul_workspace")
+    a.hadamard = _raw(hadamard).data_ptr() if hadamard is not None else None
     a.status = status_word(device).data_ptr()
-    esz_x, esz_y = xt.element_size(), yt.element_size()
-    a.x = xt.data_ptr() + m0 * xt.shape[-1] * esz_x
-    a.out = yt.data_ptr() + m0 * yt.shape[-1] * esz_y
-    a.residual = rt.data_ptr() + m0 * rt.shape[-1] * rt.element_size() if rt is not None else None
-    if exchange is not None:
-        exchange.fill(a, a.out, a.records)
-    with torch.cuda.device(device.torch):
-        _tkd.check(_tkd.lib().tkd_matmul(ctypes.byref(a), torch.cuda.current_stream().cuda_stream), "tkd_matmul")
-        if exchange is not None:
-            exchange.after_launch(status_word(device))
-    done = _tkd.TkdMatmul()
-    ctypes.pointer(done)[0] = a  # (a copy: the cached descriptor is rewritten by the next row slice or call)
-    return done
+    return a, need.value
 
 
 # --- top-k records ----------------------------------------------------------------------------------------------------
@@ -702,6 +735,9 @@ def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **o
     (applied after the matmul), "swiglu" or "geglu" (w is interleave_glu's weight with scale None, the output N / 2
     wide; or w is (gate, up), the output N wide). out_dtype ttnn.float32: out32. A block list for w: plain weights with
     activation None, (gate, up) pairs with "swiglu" or "geglu". opts go to matmul. (linear.py:1073-1124)"""
+    if (activation is None and out_dtype is None and type(w) is ttnn.Weight and x.t.dim() == 4
+            and x._mc.memory_layout is ttnn.TensorMemoryLayout.INTERLEAVED):
+        return matmul(x, w, scale, memory_config=memory_config, **opts)
     shape = list(x.shape)
     glu_kinds = {"swiglu": 0, "geglu": 1}
     if out_dtype not in (None, ttnn.bfloat16):

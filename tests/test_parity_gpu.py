@@ -492,3 +492,39 @@ def test_pack_then_matmul_in_stream_order(device):
     _tkd.check(L.tkd_matmul(ctypes.byref(c), st), "tkd_matmul")  # ... and after a synchronisation
     torch.cuda.synchronize()
     assert torch.equal(outs[1], outs[2]) and not torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("m,out32", [(1, False), (5, True), (70, False)])
+def test_kept_calls_take_new_tensors(device, m, out32):
+    """A call kept with its weight runs again on other activations, residuals and outputs (given or new), on another stream,
+    and not once a tensor it names was freed: every result is what a call described anew gives, bit for bit."""
+    g = torch.Generator().manual_seed(95 + m)
+    k, n = 512, 160
+    tw, ts = linear.native_weight(device, torch.randn(n, k, generator=g) * 0.02, ttnn.bfloat8_b, col_scale=True)
+    rdt = ttnn.float32 if out32 else ttnn.bfloat16
+
+    def call(x, r, out=None, scale=None):
+        opts = {"out32": out32, "residual": r} if scale is None else {}
+        return host(linear.matmul(x, tw, scale, out=out, **opts))
+
+    side = torch.cuda.Stream()
+    for rnd in range(3):
+        x = dev_x(device, torch.randn(m, k, generator=g))
+        r = ttnn.from_torch(torch.randn(1, 1, m, n, generator=g), dtype=rdt, layout=ttnn.TILE_LAYOUT, device=device)
+        out = ttnn.allocate_tensor_on_device([1, 1, m, n], rdt, ttnn.TILE_LAYOUT, device)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side if rnd == 1 else torch.cuda.current_stream()):
+            got = [call(x, r), call(x, r, out), call(x, None, scale=ts)]
+            torch.cuda.synchronize()
+        linear.CACHE = False
+        try:
+            want = [call(x, r), call(x, r, out), call(x, None, scale=ts)]
+        finally:
+            linear.CACHE = True
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), rnd
+    assert len(tw.calls) == 3
+    ttnn.deallocate(ts)
+    with pytest.raises(Exception):
+        call(x, None, scale=ts)
+    assert torch.equal(call(x, r), want[0])
+    linear.check_status(device)
