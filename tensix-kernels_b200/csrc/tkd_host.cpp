@@ -88,8 +88,77 @@ PyObject* host_matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
 }
 
+// moe(descriptor's address, x, ids, routing weights (gate_up) or None (down), workspace (down) or None) -> the output:
+// bf16 [1, 1, 1, ldo], or with by_union [1, 1, 32, ldo] with zeros in the rows past the descriptor's.
+PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 5 || !all_tensors(args, {1, 2}, {3, 4})) return type_error("tkd_host.moe: descriptor, x, ids, w, workspace");
+    const auto* desc = static_cast<const TkdMoe*>(PyLong_AsVoidPtr(args[0]));
+    if (PyErr_Occurred()) return nullptr;
+    try {
+        const at::Tensor &x = THPVariable_Unpack(args[1]), &ids = THPVariable_Unpack(args[2]);
+        const at::Tensor *w = tensor_or_null(args[3]), *ws = tensor_or_null(args[4]);
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != x.get_device()) guard.set_index(x.get_device());
+        TkdMoe a = *desc;
+        const int64_t shape[4] = {1, 1, a.by_union ? 32 : 1, a.ldo};
+        at::Tensor out = at::detail::empty_cuda(shape, at::kBFloat16, x.device(), std::nullopt);
+        cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
+        a.x = x.data_ptr(), a.ldx = x.stride(-2);
+        a.ids = ids.data_ptr(), a.ld_ids = ids.stride(-2);
+        if (w) a.route_w = w->data_ptr(), a.ld_w = w->stride(-2);
+        if (ws) a.workspace = ws->data_ptr(), a.workspace_bytes = (uint64_t)ws->nbytes();
+        a.out = out.data_ptr();
+        if (a.by_union && a.rows < 32) {
+            const cudaError_t e = cudaMemsetAsync(static_cast<char*>(a.out) + (size_t)a.rows * a.ldo * 2, 0, (size_t)(32 - a.rows) * a.ldo * 2, stream);
+            if (e != cudaSuccess) return tkd_error(TKD_ERR_CUDA + (int)e, "cudaMemsetAsync");
+        }
+        int rc;
+        Py_BEGIN_ALLOW_THREADS rc = w ? tkd_moe_gate_up(&a, stream) : tkd_moe_down(&a, stream);
+        Py_END_ALLOW_THREADS if (rc) return tkd_error(rc, w ? "tkd_moe_gate_up" : "tkd_moe_down");
+        return THPVariable_Wrap(std::move(out));
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+// route(logits, ids, w, bias or None, shared or None, (rows, experts, k, kind, scale, norm, groups, groups kept, has slot, slot,
+// 32-bit ids)): the router's picks into ids and w (and the shared expert's gate).
+PyObject* host_route(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 6 || !all_tensors(args, {0, 1, 2}, {3, 4})) return type_error("tkd_host.route: logits, ids, w, bias, shared, settings");
+    int rows, experts, k, kind, norm, ng, tg, has_slot, ids32;
+    unsigned slot;
+    double scale;
+    if (!PyArg_ParseTuple(args[5], "iiiidiiiiIi", &rows, &experts, &k, &kind, &scale, &norm, &ng, &tg, &has_slot, &slot, &ids32)) return nullptr;
+    try {
+        const at::Tensor &logits = THPVariable_Unpack(args[0]), &ids = THPVariable_Unpack(args[1]), &w = THPVariable_Unpack(args[2]);
+        const at::Tensor *bias = tensor_or_null(args[3]), *shared = tensor_or_null(args[4]);
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != logits.get_device()) guard.set_index(logits.get_device());
+        void* stream = c10::cuda::getCurrentCUDAStream(logits.get_device()).stream();
+        const int64_t ld = logits.stride(-2), ld_ids = ids.stride(-2), ld_w = w.stride(-2), ld_sh = shared ? shared->stride(-2) : 0;
+        const float* lp = static_cast<const float*>(logits.data_ptr());
+        const float* bp = bias ? static_cast<const float*>(bias->data_ptr()) : nullptr;
+        void *ip = ids.data_ptr(), *wp = w.data_ptr(), *sp = shared ? shared->data_ptr() : nullptr;
+        int rc;
+        Py_BEGIN_ALLOW_THREADS rc = tkd_moe_route(lp, ld, rows, experts, k, kind, bp, scale, norm, ng, tg, has_slot, slot, ip, ids32, ld_ids, wp,
+                                                  ld_w, sp, ld_sh, stream);
+        Py_END_ALLOW_THREADS if (rc) return tkd_error(rc, "tkd_moe_route");
+        Py_RETURN_NONE;
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyMethodDef fast(const char* name) {
+    return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(F)), METH_FASTCALL, nullptr};
+}
 PyMethodDef methods[] = {
-    {"matmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(host_matmul)), METH_FASTCALL, nullptr},
+    fast<host_matmul>("matmul"),
+    fast<host_moe>("moe"),
+    fast<host_route>("route"),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "tkd_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -248,7 +248,7 @@ def _layer(device, E, H, I, banks, cpb, arrays, kblock=False):
         "gu": u8(arrays["gu"]), "gu_emax": arrays["gu_emax"], "dn": u8(arrays["dn"]), "dn_emax": arrays["dn_emax"],
         "gu_bias": arrays["bias"] is not None, "gu_bias_t": arrays["bias"], "kblock": bool(kblock), "fmt": fmt,
         "bytes": sum(arrays[n].numel() for n in ("gu", "gu_emax", "dn", "dn_emax") if arrays[n] is not None),
-        "_device": device, "_ws": {},
+        "_device": device, "_ws": {}, "_ops": {},
     }
 
 
@@ -425,66 +425,66 @@ def _ids_args(ids, w, rows, k, ids32):
         assert w.dtype == ttnn.bfloat16 and w.shape[-1] >= k and w.shape[-2] >= rows, (w.dtype, w.shape)
 
 
-def _fill(a, P, what, x, ids, w, rows, k, ids32, by_union, slots, out):
-    H, I = P["H"], P["I"]
+class _Op:
+    """One of the layer's ops described for its shapes and settings (a TkdMoe without its tensors' addresses): kept with the
+    layer and run again on other tensors of those shapes."""
+
+    __slots__ = ("a", "address", "weights", "ids_dtype", "need", "launch")
+
+    def __init__(self, P, gu, rows, k, ids32, by_union, slots, act):
+        H, I = P["H"], P["I"]
+        a = self.a = _tkd.TkdMoe()
+        em = P["gu_emax"] if gu else P["dn_emax"]
+        weights = (P["gu"] if gu else P["dn"]).t
+        a.w, a.emax, a.fmt, a.expert_bytes = weights.data_ptr(), None if em is None else em.data_ptr(), P["fmt"], weights.shape[1]
+        a.experts, a.k_in, a.n = P["E"], (H if gu else I), (2 * I if gu else H)
+        a.rows, a.ids32, a.k, a.by_union, a.slots, a.ldo = rows, int(ids32), k, int(by_union), slots, slots * I if gu else H
+        if gu:
+            a.act, a.bias = ACTS[act], P["gu_bias_t"].data_ptr() if P["gu_bias"] else None
+        need = ctypes.c_uint64(0)
+        if not gu:
+            _tkd.check(_tkd.lib().tkd_moe_workspace(ctypes.byref(a), ctypes.byref(need)), "tkd_moe_workspace")
+        self.need, self.address, self.weights = need.value, ctypes.addressof(a), weights.data_ptr()
+        self.ids_dtype, self.launch = (ttnn.uint32 if ids32 else ttnn.uint16), _tkd.host().moe
+
+
+def _op(P, what, x, ids, w, rows, k, ids32, by_union, act=None):
+    """The described op, its arguments checked the first time they come in these shapes."""
     gu = what == "gu"
-    em = P["gu_emax"] if gu else P["dn_emax"]
-    a.w, a.emax, a.fmt = (P["gu"] if gu else P["dn"]).t.data_ptr(), (None if em is None else em.data_ptr()), P["fmt"]
-    a.expert_bytes = (P["gu"] if gu else P["dn"]).t.shape[1]
-    a.experts, a.k_in, a.n = P["E"], (H if gu else I), (2 * I if gu else H)
-    a.rows, a.x, a.ldx = rows, x.t.data_ptr(), x.t.stride(-2)
-    a.ids, a.ids32, a.k, a.ld_ids = ids.t.data_ptr(), int(ids32), k, ids.t.stride(-2)
-    if w is not None:
-        a.route_w, a.ld_w = w.t.data_ptr(), w.t.stride(-2)
-    a.by_union, a.slots = int(by_union), slots
-    a.out, a.ldo = out.data_ptr(), out.stride(-2)
+    key = (what, x.t.shape, ids.t.shape, None if w is None else w.t.shape, rows, k, ids32, by_union, act)
+    op = P["_ops"].get(key)
+    if (op is not None and x.dtype is ttnn.bfloat16 and ids.dtype is op.ids_dtype and (w is None or w.dtype is ttnn.bfloat16)
+            and P["gu" if gu else "dn"].t.data_ptr() == op.weights):
+        return op
+    assert 1 <= k <= 16, k
+    H, I = P["H"], P["I"]
+    slots = u_max(P, rows, k) if by_union else k
+    if gu:
+        assert act in ACTS, f"moe8: act {act!r}"
+        assert x.dtype == ttnn.bfloat16 and x.shape[-1] == H and x.shape[-2] >= rows, (x.dtype, x.shape)
+    else:
+        assert x.dtype == ttnn.bfloat16 and x.shape[-1] >= slots * I and x.shape[-2] >= rows, (x.dtype, x.shape)
+    _ids_args(ids, w, rows, k, ids32)
+    if len(P["_ops"]) >= 64:
+        P["_ops"].clear()
+    op = P["_ops"][key] = _Op(P, gu, rows, k, ids32, by_union, slots, act)
+    return op
 
 
 def _gate_up(x, P, ids, w, k, rows, ids32, by_union, act, memory_config):
-    assert act in ACTS, f"moe8: act {act!r}"
-    assert 1 <= k <= 16, k
-    device = x.device()
-    H, I = P["H"], P["I"]
-    assert x.dtype == ttnn.bfloat16 and x.shape[-1] == H and x.shape[-2] >= rows, (x.dtype, x.shape)
-    _ids_args(ids, w, rows, k, ids32)
-    slots = u_max(P, rows, k) if by_union else k
-    with torch.cuda.device(device.torch):
-        if by_union:
-            out = torch.zeros(1, 1, TILE, slots * I, dtype=torch.bfloat16, device=device.torch)
-        else:
-            out = torch.empty(1, 1, 1, slots * I, dtype=torch.bfloat16, device=device.torch)
-        a = _tkd.TkdMoe()
-        _fill(a, P, "gu", x, ids, w, rows, k, ids32, by_union, slots, out)
-        a.act = ACTS[act]
-        a.bias = P["gu_bias_t"].data_ptr() if P["gu_bias"] else None
-        _tkd.check(_tkd.lib().tkd_moe_gate_up(ctypes.byref(a), torch.cuda.current_stream().cuda_stream), "tkd_moe_gate_up")
-    return ttnn.Tensor(out, ttnn.bfloat16, ttnn.TILE_LAYOUT, device, memory_config or ttnn.DRAM_MEMORY_CONFIG)
+    op = _op(P, "gu", x, ids, w, rows, k, ids32, by_union, act)
+    out = op.launch(op.address, x.t, ids.t, w.t, None)
+    return ttnn.Tensor(out, ttnn.bfloat16, ttnn.TILE_LAYOUT, x._device, memory_config)
 
 
 def _down(h, P, ids, k, rows, ids32, by_union, memory_config):
-    assert 1 <= k <= 16, k
-    device = h.device()
-    H, I = P["H"], P["I"]
-    slots = u_max(P, rows, k) if by_union else k
-    assert h.dtype == ttnn.bfloat16 and h.shape[-1] >= slots * I and h.shape[-2] >= rows, (h.dtype, h.shape)
-    _ids_args(ids, None, rows, k, ids32)
-    L = _tkd.lib()
-    with torch.cuda.device(device.torch):
-        if by_union:
-            out = torch.zeros(1, 1, TILE, H, dtype=torch.bfloat16, device=device.torch)
-        else:
-            out = torch.empty(1, 1, 1, H, dtype=torch.bfloat16, device=device.torch)
-        a = _tkd.TkdMoe()
-        _fill(a, P, "dn", h, ids, None, rows, k, ids32, by_union, slots, out)
-        need = ctypes.c_uint64(0)
-        _tkd.check(L.tkd_moe_workspace(ctypes.byref(a), ctypes.byref(need)), "tkd_moe_workspace")
-        ws = P["_ws"].get("dn")
-        if ws is None or ws.numel() < need.value:
-            # (zeroed once: the kernel returns its counters to zero; calls on one layer run in stream order)
-            ws = P["_ws"]["dn"] = torch.zeros(need.value, dtype=torch.uint8, device=device.torch)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        _tkd.check(L.tkd_moe_down(ctypes.byref(a), torch.cuda.current_stream().cuda_stream), "tkd_moe_down")
-    return ttnn.Tensor(out, ttnn.bfloat16, ttnn.TILE_LAYOUT, device, memory_config or ttnn.DRAM_MEMORY_CONFIG)
+    op = _op(P, "dn", h, ids, None, rows, k, ids32, by_union)
+    ws = P["_ws"].get("dn")
+    if ws is None or ws.numel() < op.need:
+        # (zeroed once: the kernel returns its counters to zero; calls on one layer run in stream order)
+        ws = P["_ws"]["dn"] = torch.zeros(op.need, dtype=torch.uint8, device=h._device.torch)
+    out = op.launch(op.address, h.t, ids.t, None, ws)
+    return ttnn.Tensor(out, ttnn.bfloat16, ttnn.TILE_LAYOUT, h._device, memory_config)
 
 
 def gate_up(x, P, ids, w, k, *, ids32=False, kw=8, fidelity="hifi2", memory_config=None, cpb=None, loaders=None, act="silu"):
@@ -539,6 +539,25 @@ def route(logits, ids, w, k, *, kind="softmax", bias=None, ids32=False, experts=
     own sigmoid). shared: a [1, 1, R, 1] bf16 that gets sigmoid(logits[:, E]). scale: every weight times it (0 < scale <
     4). groups=(n_group, topk_group): the sigmoid kind with a bias; a group's score the sum of its two largest keys, the
     topk_group best groups kept. slot: that id as slot k of every row at weight 1.0 (ids and w hold k + 1). Returns w."""
+    key = (logits.t.shape, ids.t.shape, w.t.shape, k, kind, None if bias is None else bias.t.shape, ids32, experts,
+           None if shared is None else shared.t.shape, scale, norm, groups and tuple(groups), slot)
+    settings = _ROUTES.get(key)
+    if (settings is None or logits.dtype is not ttnn.float32 or ids.dtype is not (ttnn.uint32 if ids32 else ttnn.uint16)
+            or w.dtype is not ttnn.bfloat16 or (bias is not None and bias.dtype is not ttnn.float32)
+            or (shared is not None and shared.dtype is not ttnn.bfloat16)):
+        settings = _route_settings(logits, ids, w, k, kind, bias, ids32, experts, shared, scale, norm, groups, slot)
+        if len(_ROUTES) >= 256:
+            _ROUTES.clear()
+        _ROUTES[key] = settings
+    _tkd.host().route(logits.t, ids.t, w.t, bias.t if settings[3] == 1 else None, None if shared is None else shared.t, settings)
+    return w
+
+
+_ROUTES = {}  # the settings of routes checked before, by shapes and options
+
+
+def _route_settings(logits, ids, w, k, kind, bias, ids32, experts, shared, scale, norm, groups, slot):
+    """route's arguments checked, as the native call takes them."""
     assert kind in ("softmax", "sigmoid"), f"moe8.route: kind {kind!r}"
     R, W = logits.shape[-2], logits.shape[-1]
     E = experts or W
@@ -562,16 +581,7 @@ def route(logits, ids, w, k, *, kind="softmax", bias=None, ids32=False, experts=
     if shared is not None:
         assert shared.dtype == ttnn.bfloat16 and shared.shape[-2] >= R, (shared.dtype, shared.shape)
     kcode = 0 if kind == "softmax" else (1 if sig else 2)
-    device = logits.device()
-    with torch.cuda.device(device.torch):
-        _tkd.check(
-            _tkd.lib().tkd_moe_route(
-                logits.t.data_ptr(), logits.t.stride(-2), R, E, k, kcode, bias.t.data_ptr() if sig else None, float(scale),
-                int(bool(norm)), ng, tg, int(slot is not None), int(slot or 0), ids.t.data_ptr(), int(ids32), ids.t.stride(-2),
-                w.t.data_ptr(), w.t.stride(-2), shared.t.data_ptr() if shared is not None else None,
-                shared.t.stride(-2) if shared is not None else 0, torch.cuda.current_stream().cuda_stream),
-            "tkd_moe_route")
-    return w
+    return (R, E, k, kcode, float(scale), int(bool(norm)), ng, tg, int(slot is not None), int(slot or 0), int(ids32))
 
 
 def route_reference(logits, k, kind="softmax", bias=None, scale=1.0, norm=True, groups=None, slot=None):
