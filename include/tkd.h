@@ -80,6 +80,15 @@ int tkd_quantise(int fmt, const float* src, int orient, int64_t k, int64_t n, co
  * multiple of 32), emax and info unused (NULL). The weight is code * scale exactly; tkd_unpack returns that. */
 int tkd_pack(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* codes, void* packed, uint8_t* emax,
              int32_t* info, void* stream);
+/* tkd_quantise and tkd_pack in one pass over the source, with the same result (TKD_FMT_BFP8, BFP4 or BF16). src: orient 0
+ * [n, k] with ld elements a row (16-byte aligned rows), orient 1 [k, n] with ld elements a row; k a multiple of 32.
+ * col_div: as tkd_quantise's. col_scale (or NULL; not with col_div): the columns are divided by c = their largest
+ * magnitude, at least 1e-8, rounded up to bf16, and c is written to col_scale [n] (bf16): native_weight's col_scale
+ * (dense_reader/linear.py:144-156). info: one int32 the device can write, in device or in pinned host memory, zeroed by
+ * the caller; set to 1 when the weight is wide (see tkd_pack). TKD_ERR_UNSUPPORTED: a k past 200 K inputs (use the two
+ * calls). */
+int tkd_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, const float* col_div, void* col_scale,
+                    void* packed, uint8_t* emax, int32_t* info, void* stream);
 /* tkd_quantise's block-float numbers (TKD_FMT_BFP8 or BFP4) as bf16 bits [K, npad] (uint16), the canonical form
  * tkd_pack takes for TKD_FMT_BF16: every such number is a bf16 value exactly, subnormals included. */
 int tkd_dequantise_bf16(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* codes, void* out_bf16, void* stream);

@@ -233,6 +233,18 @@ int tkd_pack(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* cod
                                          static_cast<cudaStream_t>(stream)));
 }
 
+int tkd_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, const float* col_div, void* col_scale,
+                    void* packed, uint8_t* emax, int32_t* info, void* stream) {
+    if (!fmt_ok(fmt) || fmt == TKD_INT4 || !src || !packed || k < 32 || k % 32 || n < 1 || (orient != 0 && orient != 1) ||
+        ld < (orient ? n : k) || (col_div && col_scale) || (has_emax(fmt) && (!emax || !info)))
+        return TKD_ERR_BAD_ARG;
+    if (orient == 0 && (ld % 4 || reinterpret_cast<uintptr_t>(src) & 15)) return TKD_ERR_BAD_ARG;
+    if (reinterpret_cast<uintptr_t>(packed) & 15) return TKD_ERR_BAD_ARG;
+    if (k > 200 * 1024) return TKD_ERR_UNSUPPORTED;  // (a byte a k in shared memory)
+    return launch_err(tkd_launch_pack_weight(fmt, src, orient, ld, k, n, tkd_padded_cols(n), col_div, static_cast<uint16_t*>(col_scale),
+                                             packed, emax, info, static_cast<cudaStream_t>(stream)));
+}
+
 int tkd_dequantise_bf16(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* codes, void* out_bf16, void* stream) {
     if ((fmt != TKD_BFP8 && fmt != TKD_BFP4) || !exps || !codes || !out_bf16 || k < 1 || n < 1) return TKD_ERR_BAD_ARG;
     return launch_err(tkd_launch_dequantise_bf16(fmt, k, tkd_padded_cols(n), exps, codes, out_bf16,

@@ -10,10 +10,14 @@
 //      tiles hold, before any re-layout; what the parity tests compare bit for bit);
 //   2. tkd_emax_kernel: per group of 16 columns the largest exponent of a row with a non-zero code (a block a group);
 //   3. tkd_permute_kernel: canonical -> stream, one thread per 32-bit word of the stream.
+// tkd_pack_weight_kernel does all three at once and is what a weight's loading runs; the passes serve callers that hold the
+// canonical numbers (int4 and ternary codes, K-block experts), and a K too long for its shared memory.
 // tkd_unpack_kernel is the inverse (stream -> float32 [K, Npad]), used for the weight's read-back.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "tkd_internal.h"
 #include "tkd_layout.h"
@@ -232,7 +236,221 @@ __global__ void tkd_unpack_kernel(int fmt, int64_t K, int64_t npad, const uint8_
     out[idx] = v;
 }
 
+// The three passes above in one, for float32 -> stream at load time: a CTA owns a group of 16 columns and all of K, and a
+// warp takes a super-atom at a time. A lane loads exactly the numbers whose codes it will write (8 consecutive k of columns
+// g and g + 8 per block of 32 k: the fragment layout of tkd_layout.h), the shared exponents of its 8 k come from three
+// shuffles over the lanes of the same k, and its 16 bytes of codes go straight to the stream. Only the exponents wait for
+// the group's largest: a byte a k in shared memory, written as the stream's words at the end. A row of the group holds a
+// non-zero code exactly when its shared exponent is not zero (the largest value's implicit bit survives the rounding).
+// SCALE 1: the columns are divided by col_div first; 2: by their largest magnitude rounded up to bf16 (native_weight's
+// col_scale), found by a first walk over the CTA's 16 columns, whose second reading then comes from L2, and written out.
+// Bound: HBM. [14336, 4096] float32 to bfloat4_b (235 MB in, 33 MB out): tkd_quantise, the emax and the permute pass 410 us
+// together (1 byte a weight of codes written and read back, uncoalesced loads of the [N, K] matrix).
+constexpr int kPackThreads = 256, kPackWarps = kPackThreads / 32;
+
+// |v|'s bits rounded up to bf16, as a float (linear.bf16_ceil), of at least 1e-8
+__device__ __forceinline__ float pack_col_scale(uint32_t bits) {
+    const float a = __uint_as_float(bits), s = a < 1e-8f ? 1e-8f : a;  // (a NaN stays)
+    const float down = __bfloat162float(__float2bfloat16_rn(s));
+    return down >= s ? down : __uint_as_float(__float_as_uint(down) + 0x10000u);
+}
+
+// One value's code in place: sign at bit 15, the magnitude from bit `p` (0 for 7 bits, 4 for 3), by the rule of
+// tkd_quantise_kernel. Rounding to nearest even is one addition: half less one, plus the kept part's last bit.
+template <int FMT>
+__device__ __forceinline__ uint32_t pack_code(uint32_t bits, uint32_t shared) {
+    constexpr int mb = FMT == TKD_BFP8 ? 7 : 3, shift = 24 - mb, p = FMT == TKD_BFP8 ? 0 : 4;
+    const uint32_t e = (bits >> 23) & 0xFFu;
+    uint32_t m = ((bits & 0x7FFFFFu) | 0x800000u) >> min(shared - e, 31u);
+    m = (m + ((1u << (shift - 1)) - 1u) + ((m >> shift) & 1u)) >> shift;
+    m = e ? min(m, (1u << mb) - 1u) : 0u;
+    return m ? ((bits >> 16) & 0x8000u) | (m << p) : 0u;
+}
+
+template <int FMT, int ORIENT, int SCALE>
+__global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const float* __restrict__ src, int64_t ld, int K, int64_t N,
+                                                                       const float* __restrict__ col_div,
+                                                                       uint16_t* __restrict__ scale_out, uint8_t* __restrict__ stream,
+                                                                       uint8_t* __restrict__ emax, int* info) {
+    constexpr int KSA = FMT == TKD_BFP4 ? 64 : 32, XB = KSA / 32, EB = FMT == TKD_BFP8 ? 32 : FMT == TKD_BFP4 ? 64 : 0;
+    extern __shared__ __align__(16) uint8_t exps[];  // the shared exponent of every k (not for bf16)
+    __shared__ uint32_t cmax[kPackWarps][16];
+    __shared__ float cdiv[16];
+    __shared__ int shi[kPackWarps], slo[kPackWarps];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int64_t grp = blockIdx.x, n0 = grp * 16 + g, n1 = n0 + 8;
+    const bool in0 = n0 < N, in1 = n1 < N;
+    const int nsa = (K + KSA - 1) / KSA;
+    // 8 consecutive k of one column
+    auto load8 = [&](float (&v)[8], int64_t n, bool in, int k) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = 0.f;
+        if (!in || k >= K) return;
+        if constexpr (ORIENT == 0) {
+            const float4* s = reinterpret_cast<const float4*>(src + n * ld + k);
+            const float4 a = __ldg(s), b = __ldg(s + 1);
+            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(src + (int64_t)(k + i) * ld + n);
+        }
+    };
+    float d0 = 1.f, d1 = 1.f;
+    if constexpr (SCALE == 1) {
+        if (in0) d0 = col_div[n0];
+        if (in1) d1 = col_div[n1];
+    } else if constexpr (SCALE == 2) {
+        uint32_t m0 = 0, m1 = 0;
+#pragma unroll 2
+        for (int b = warp; b < K / 32; b += kPackWarps) {
+            float v0[8], v1[8];
+            load8(v0, n0, in0, 32 * b + 8 * t);
+            load8(v1, n1, in1, 32 * b + 8 * t);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)  // (magnitudes order as their bits do, a NaN above all)
+                m0 = max(m0, __float_as_uint(v0[i]) & 0x7FFFFFFFu), m1 = max(m1, __float_as_uint(v1[i]) & 0x7FFFFFFFu);
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            m0 = max(m0, __shfl_xor_sync(0xFFFFFFFFu, m0, o));
+            m1 = max(m1, __shfl_xor_sync(0xFFFFFFFFu, m1, o));
+        }
+        if (t == 0) cmax[warp][g] = m0, cmax[warp][g + 8] = m1;
+        __syncthreads();
+        if (tid < 16) {
+            uint32_t m = 0;
+#pragma unroll
+            for (int w = 0; w < kPackWarps; ++w) m = max(m, cmax[w][tid]);
+            const float c = pack_col_scale(m);
+            cdiv[tid] = c;
+            if (grp * 16 + tid < N) scale_out[grp * 16 + tid] = __bfloat16_as_ushort(__float2bfloat16_rn(c));
+        }
+        __syncthreads();
+        d0 = cdiv[g], d1 = cdiv[g + 8];
+    }
+    uint32_t hi = 0, lo = 255;
+    for (int sa = warp; sa < nsa; sa += kPackWarps) {
+        uint8_t* dst = stream + tkd_sa_offset(FMT, K, grp, sa) + EB + lane * 16;
+        float v[2][XB][8];
+#pragma unroll
+        for (int q = 0; q < XB; ++q) {
+            load8(v[0][q], n0, in0, sa * KSA + 32 * q + 8 * t);
+            load8(v[1][q], n1, in1, sa * KSA + 32 * q + 8 * t);
+        }
+        if constexpr (SCALE != 0) {
+#pragma unroll
+            for (int q = 0; q < XB; ++q)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[0][q][i] = __fdiv_rn(v[0][q][i], d0), v[1][q][i] = __fdiv_rn(v[1][q][i], d1);
+        }
+        uint32_t words[4];
+#pragma unroll
+        for (int q = 0; q < XB; ++q) {
+            if constexpr (FMT == TKD_BF16) {
+                uint32_t b[2][4];  // the column's pairs of k
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        b[c][i] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v[c][q][2 * i])) |
+                                  ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v[c][q][2 * i + 1])) << 16);
+#pragma unroll
+                for (int jj = 0; jj < 2; ++jj)
+                    *reinterpret_cast<uint4*>(dst + 512 * jj) = make_uint4(b[0][2 * jj], b[1][2 * jj], b[0][2 * jj + 1], b[1][2 * jj + 1]);
+            } else {
+                uint32_t sh[8];
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    // two k's exponents to a word, their maxima over the 16 columns
+                    uint32_t w[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        w[j] = max((__float_as_uint(v[0][q][i + j]) >> 23) & 0xFFu, (__float_as_uint(v[1][q][i + j]) >> 23) & 0xFFu);
+                    uint32_t both = w[0] | (w[1] << 16);
+#pragma unroll
+                    for (int o = 4; o < 32; o <<= 1) both = __vmaxu2(both, __shfl_xor_sync(0xFFFFFFFFu, both, o));
+                    sh[i] = both & 0xFFFFu, sh[i + 1] = both >> 16;
+                }
+                if (g == 0) {
+                    uint32_t* ex = reinterpret_cast<uint32_t*>(exps + sa * KSA + 32 * q + 8 * t);
+                    ex[0] = sh[0] | (sh[1] << 8) | (sh[2] << 16) | (sh[3] << 24);
+                    ex[1] = sh[4] | (sh[5] << 8) | (sh[6] << 16) | (sh[7] << 24);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) hi = max(hi, sh[i]), lo = min(lo, sh[i] ? sh[i] : 255u);
+                uint32_t r[2][4];  // (column g or g + 8, pair of k): a fragment register
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        r[c][i] = pack_code<FMT>(__float_as_uint(v[c][q][2 * i]), sh[2 * i]) |
+                                  (pack_code<FMT>(__float_as_uint(v[c][q][2 * i + 1]), sh[2 * i + 1]) << 16);
+                if constexpr (FMT == TKD_BFP8) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) words[i] = r[0][i] | tkd_rotl(r[1][i], 8);
+                } else {
+#pragma unroll
+                    for (int jj = 0; jj < 2; ++jj)
+                        words[2 * q + jj] = r[0][2 * jj] | (r[1][2 * jj] >> 4) | tkd_rotl(r[0][2 * jj + 1] | (r[1][2 * jj + 1] >> 4), 8);
+                }
+            }
+        }
+        if constexpr (FMT != TKD_BF16) *reinterpret_cast<uint4*>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
+    }
+    if constexpr (FMT != TKD_BF16) {
+        hi = __reduce_max_sync(0xFFFFFFFFu, hi), lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+        if (lane == 0) shi[warp] = (int)hi, slo[warp] = (int)lo;
+        __syncthreads();
+        int top = 0, low = 255;
+#pragma unroll
+        for (int w = 0; w < kPackWarps; ++w) top = max(top, shi[w]), low = min(low, slo[w]);
+        if (tid == 0) {
+            emax[grp] = (uint8_t)top;
+            if (low <= top && top - low > TKD_ESPREAD) *static_cast<volatile int*>(info) = 1;
+        }
+        // the exponent words: word (t, j) of a super-atom covers k = 32 (j / 2) + 8 t + 4 (j % 2) .. + 3
+        constexpr int PT = 2 * XB, PW = 4 * PT;
+        for (int i = tid; i < nsa * PW; i += kPackThreads) {
+            const int sa = i / PW, wi = i % PW, wt = wi / PT, j = wi % PT;
+            const uint32_t e4 = *reinterpret_cast<const uint32_t*>(exps + sa * KSA + 32 * (j >> 1) + 8 * wt + 4 * (j & 1));
+            uint32_t word = 0;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int sh = (int)((e4 >> (8 * r)) & 0xFFu);
+                const int e = sh ? max(tkd_ezero(FMT), sh - top + tkd_ebias(FMT)) : tkd_ezero(FMT);
+                word |= tkd_exp_bits(FMT, (uint32_t)e, r);
+            }
+            *reinterpret_cast<uint32_t*>(stream + tkd_sa_offset(FMT, K, grp, sa) + wi * 4) = word;
+        }
+    }
+}
+
+template <int FMT, int ORIENT>
+int launch_pack_weight(const float* src, int64_t ld, int64_t K, int64_t N, int64_t npad, const float* col_div, uint16_t* scale_out,
+                       void* packed, uint8_t* emax, int* info, cudaStream_t st) {
+    const size_t smem = FMT == TKD_BF16 ? 0 : (size_t)(K + 63) / 64 * 64;
+    auto kern = scale_out ? tkd_pack_weight_kernel<FMT, ORIENT, 2>
+                          : col_div ? tkd_pack_weight_kernel<FMT, ORIENT, 1> : tkd_pack_weight_kernel<FMT, ORIENT, 0>;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    kern<<<(unsigned)(npad / 16), kPackThreads, smem, st>>>(src, ld, (int)K, N, col_div, scale_out, static_cast<uint8_t*>(packed), emax, info);
+    return (int)cudaGetLastError();
+}
+
 }  // namespace
+
+int tkd_launch_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t K, int64_t N, int64_t npad, const float* col_div,
+                           uint16_t* scale_out, void* packed, uint8_t* emax, int* info, cudaStream_t st) {
+    auto go = [&](auto f) {
+        constexpr int F = decltype(f)::value;
+        return orient == 0 ? launch_pack_weight<F, 0>(src, ld, K, N, npad, col_div, scale_out, packed, emax, info, st)
+                           : launch_pack_weight<F, 1>(src, ld, K, N, npad, col_div, scale_out, packed, emax, info, st);
+    };
+    return fmt == TKD_BFP8 ? go(std::integral_constant<int, TKD_BFP8>{}) : fmt == TKD_BFP4 ? go(std::integral_constant<int, TKD_BFP4>{})
+                                                                                           : go(std::integral_constant<int, TKD_BF16>{});
+}
 
 int tkd_launch_quantise(int fmt, const float* src, int orient, int64_t K, int64_t N, int64_t npad,
                         const float* col_div, uint8_t* exps, void* codes, cudaStream_t st) {

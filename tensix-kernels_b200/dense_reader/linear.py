@@ -124,12 +124,12 @@ def native_weight(device, t, dtype, col_scale=False, sharded=True, max_banks=Non
     The weight is quantised and packed on the GPU (libtkd); `sharded` / `max_banks` only set what its memory config
     reports (width-sharded over the device's banks, or interleaved)."""
     assert dtype in NATIVE_TILES, f"dense_reader: weights are bfloat8_b, bfloat4_b or bfloat16, not {dtype}"
-    t = t.float()
-    c = bf16_ceil(t.abs().amax(dim=1).clamp(min=1e-8)) if col_scale else torch.ones(t.shape[0])
     n, k = t.shape
+    c = torch.empty(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch) if col_scale else \
+        torch.ones(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch)
     mc = sharded_memcfg(device, k, n, max_banks=max_banks) if sharded else ttnn.DRAM_MEMORY_CONFIG
-    w = ttnn.pack_weight(device, t, dtype, 0, col_div=c if col_scale else None, memory_config=mc)
-    return w, scale_tensor(device, c)
+    w = ttnn.pack_weight(device, t, dtype, 0, memory_config=mc, col_scale=c if col_scale else None)
+    return w, ttnn.Tensor(c, ttnn.bfloat16, ttnn.TILE_LAYOUT, device, ttnn.DRAM_MEMORY_CONFIG)
 
 
 def block_float(t, dtype):

@@ -124,8 +124,8 @@ def _glu_order(m, I):
 
 
 def _pack_experts(device, mats, what):
-    """[E, K, N] float -> (streams uint8 [E, bytes], emax uint8 [E, N_pad / 16]) on the device: tkd_quantise and tkd_pack
-    of each expert into its slice."""
+    """[E, K, N] float -> (streams uint8 [E, bytes], emax uint8 [E, N_pad / 16]) on the device: tkd_pack_weight of each
+    expert into its slice."""
     L = _tkd.lib()
     E, k, n = mats.shape
     npad = L.tkd_padded_cols(n)
@@ -135,15 +135,11 @@ def _pack_experts(device, mats, what):
     with torch.cuda.device(device.torch):
         streams = torch.empty(E, nbytes, dtype=torch.uint8, device=device.torch)
         emax = torch.empty(E, npad // 16, dtype=torch.uint8, device=device.torch)
-        exps = torch.empty(k * (npad // 16), dtype=torch.uint8, device=device.torch)
-        codes = torch.empty(k * npad, dtype=torch.uint8, device=device.torch)
         info = torch.zeros(1, dtype=torch.int32, device=device.torch)
         for e in range(E):
             src = mats[e].to(device.torch, torch.float32).contiguous()
-            _tkd.check(L.tkd_quantise(_tkd.FMT_BFP4, src.data_ptr(), 1, k, n, None, exps.data_ptr(), codes.data_ptr(), st),
-                       "tkd_quantise")
-            _tkd.check(L.tkd_pack(_tkd.FMT_BFP4, k, n, exps.data_ptr(), codes.data_ptr(), streams[e].data_ptr(),
-                                  emax[e].data_ptr(), info.data_ptr(), st), "tkd_pack")
+            _tkd.check(L.tkd_pack_weight(_tkd.FMT_BFP4, src.data_ptr(), 1, n, k, n, None, None, streams[e].data_ptr(), emax[e].data_ptr(),
+                                         info.data_ptr(), st), "tkd_pack_weight")
         torch.cuda.current_stream().synchronize()  # (the ops read the weights ahead of nothing, but src is a temporary)
         if int(info.item()) & 1:
             raise ValueError(f"moe8: an expert's {what} weight has exponents inside a group of 16 columns more than 48"

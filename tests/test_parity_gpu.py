@@ -528,3 +528,32 @@ def test_kept_calls_take_new_tensors(device, m, out32):
         call(x, None, scale=ts)
     assert torch.equal(call(x, r), want[0])
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
+@pytest.mark.parametrize("k,n", [(32, 1), (96, 40), (544, 130), (4096, 272)])
+def test_packing_in_one_pass_equals_the_passes(device, fmt, k, n):
+    """tkd_pack_weight against tkd_quantise and tkd_pack, bytes and scales: K inside a super-atom and a chunk, N inside a group
+    and a panel, zero rows and denormals, both orientations (one with a wider leading dimension), with and without the
+    columns' own scales (against bf16_ceil's on the host)."""
+    from dense_reader import _tkd
+
+    g = torch.Generator().manual_seed(k + n)
+    w = torch.randn(n, k, generator=g) * 0.02 * torch.exp2(torch.randint(-6, 7, (n, 1), generator=g).float())
+    w[:, 1] = 0
+    w[:, 3] = 1e-41
+    w[0, 0] = 0.0 if n > 1 else w[0, 0]
+    wide = torch.zeros(k, n + 5)
+    wide[:, :n] = w.T
+    for scaled in (False, True):
+        c = linear.bf16_ceil(w.abs().amax(dim=1).clamp(min=1e-8))
+        div = c.to(device.torch) if scaled else None
+        want, emax, f = ttnn._pack_in_passes(device, w.to(device.torch), _tkd.__dict__["FMT_" + fmt.upper()], 0, k, n, div)
+        cs = torch.zeros(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch) if scaled else None
+        got = [ttnn.pack_weight(device, w, DT[fmt], 0, col_scale=cs), ttnn.pack_weight(device, w, DT[fmt], 0, col_div=div),
+               ttnn.pack_weight(device, wide.to(device.torch)[:, :n], DT[fmt], 1, col_div=div)]
+        for t in got:
+            assert t.fmt == f and torch.equal(t.t, want)
+            assert emax is None or torch.equal(t.emax, emax)
+        if scaled:
+            assert torch.equal(cs.float().cpu().reshape(-1), c)
