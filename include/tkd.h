@@ -85,7 +85,7 @@ int tkd_pack(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* cod
  * col_div: as tkd_quantise's. col_scale (or NULL; not with col_div): the columns are divided by c = their largest
  * magnitude, at least 1e-8, rounded up to bf16, and c is written to col_scale [n] (bf16): native_weight's col_scale
  * (dense_reader/linear.py:144-156). info: one int32 the device can write, in device or in pinned host memory, zeroed by
- * the caller; set to 1 when the weight is wide (see tkd_pack). TKD_ERR_UNSUPPORTED: a k past 200 K inputs (use the two
+ * the caller; set to 1 when the weight is wide (see tkd_pack). TKD_ERR_UNSUPPORTED: a k past 102400 inputs (use the two
  * calls). */
 int tkd_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, const float* col_div, void* col_scale,
                     void* packed, uint8_t* emax, int32_t* info, void* stream);

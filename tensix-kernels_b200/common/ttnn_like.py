@@ -14,7 +14,6 @@ read (csrc/tkd_layout.h), made on the GPU by libtkd's packer.
 import enum
 import itertools
 import math
-import threading
 
 import torch
 
@@ -193,53 +192,40 @@ def _stream_ptr():
     return torch.cuda.current_stream().cuda_stream
 
 
-_LOCAL = threading.local()
-
-
-def _wide_word():
-    """This thread's int32 in pinned host memory that a packing kernel sets when its weight is wide (read once the stream
-    has been waited for: no copy back)."""
-    word = getattr(_LOCAL, "wide", None)
-    if word is None:
-        word = _LOCAL.wide = torch.zeros(1, dtype=torch.int32).pin_memory()
-    word.zero_()
-    return word
-
-
-def pack_weight(device, wt, dtype, orient, col_div=None, memory_config=None, col_scale=None):
+def pack_weight(device, wt, dtype, orient, col_div=None, memory_config=None):
     """A float matrix (orient 0: [N, K] as torch's [out, in]; 1: [K, N]) -> Weight, on the GPU in one launch
-    (tkd_pack_weight). col_div: divisors of the columns; col_scale: a bf16 [1, 1, 1, N] tensor for the columns' own (their
-    largest magnitudes rounded up)."""
-    L = _tkd.lib()
+    (tkd_pack_weight). col_div: divisors of the columns."""
+    return _packed(device, wt, dtype, orient, col_div, memory_config, False)[0]
+
+
+def pack_weight_scaled(device, wt, dtype, memory_config=None):
+    """(Weight, bf16 [1, 1, 1, N]) of a [N, K] matrix whose columns are first divided by their own scales, their largest
+    magnitudes rounded up."""
+    return _packed(device, wt, dtype, 0, None, memory_config, True)
+
+
+def _packed(device, wt, dtype, orient, col_div, memory_config, own):
     fmt = FMT[dtype]
     src = wt.to(device.torch, torch.float32)
-    if src.stride(1) != 1 or src.stride(0) < src.shape[1] or (orient == 0 and (src.stride(0) % 4 or src.data_ptr() % 16)):
+    ld, width = src.stride(0), src.shape[1]
+    if src.stride(1) != 1 or ld < width or (orient == 0 and (ld % 4 or src.data_ptr() % 16)):
         src = src.clone(memory_format=torch.contiguous_format)
-    n, k = (src.shape[0], src.shape[1]) if orient == 0 else (src.shape[1], src.shape[0])
+    n, k = (src.shape[0], width) if orient == 0 else (width, src.shape[0])
     assert k % TILE == 0, f"K {k} is not a multiple of 32"
-    npad = L.tkd_padded_cols(n)
-    with torch.cuda.device(device.torch):
-        div = None if col_div is None else col_div.to(device.torch, torch.float32).contiguous()
-        stream = torch.empty(L.tkd_packed_bytes(fmt, k, n), dtype=torch.uint8, device=device.torch)
-        emax = None if fmt == _tkd.FMT_BF16 else torch.empty(npad // 16, dtype=torch.uint8, device=device.torch)
-        wide = _wide_word()
-        rc = L.tkd_pack_weight(fmt, src.data_ptr(), orient, src.stride(0), k, n, None if div is None else div.data_ptr(),
-                               None if col_scale is None else col_scale.data_ptr(), stream.data_ptr(),
-                               None if emax is None else emax.data_ptr(), wide.data_ptr(), _stream_ptr())
-        if rc != _tkd.ERR_UNSUPPORTED:
-            _tkd.check(rc, "tkd_pack_weight")
-            # (waited for whatever the format: launches read weights ahead of stream order)
-            torch.cuda.current_stream().synchronize()
-            if not int(wide):
-                return Weight(stream, emax, k, n, dtype, device, memory_config or DRAM_MEMORY_CONFIG, fmt=fmt)
-        elif col_scale is not None:
-            top = src.abs().amax(dim=1 - orient).clamp(min=1e-8)
-            down = top.to(torch.bfloat16).float()
-            col_scale.copy_(torch.where(down >= top, down, (down.view(torch.int32) + (1 << 16)).view(torch.float32)).reshape(col_scale.shape))
-        if col_scale is not None:
-            div = col_scale.float().reshape(-1)
-        stream, emax, fmt = _pack_in_passes(device, src.contiguous(), fmt, orient, k, n, div)
-    return Weight(stream, emax, k, n, dtype, device, memory_config or DRAM_MEMORY_CONFIG, fmt=fmt)
+    div = None if col_div is None else col_div.to(device.torch, torch.float32).contiguous()
+    stream, emax, scale, state = _tkd.host().pack(fmt, src, orient, div, own)
+    if state:
+        # (a wide weight, or a K past what one pass takes)
+        with torch.cuda.device(device.torch):
+            if own:
+                if state == 2:
+                    top = src.abs().amax(dim=1).clamp(min=1e-8)
+                    down = top.to(torch.bfloat16).float()
+                    up = (down.view(torch.int32) + (1 << 16)).view(torch.float32)
+                    scale = torch.where(down >= top, down, up).to(torch.bfloat16).reshape(1, 1, 1, n)
+                div = scale.float().reshape(-1)
+            stream, emax, fmt = _pack_in_passes(device, src.contiguous(), fmt, orient, k, n, div)
+    return Weight(stream, emax, k, n, dtype, device, memory_config or DRAM_MEMORY_CONFIG, fmt=fmt), scale
 
 
 def _pack_in_passes(device, src, fmt, orient, k, n, div):

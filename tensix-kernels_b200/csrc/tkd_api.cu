@@ -240,7 +240,7 @@ int tkd_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k
         return TKD_ERR_BAD_ARG;
     if (orient == 0 && (ld % 4 || reinterpret_cast<uintptr_t>(src) & 15)) return TKD_ERR_BAD_ARG;
     if (reinterpret_cast<uintptr_t>(packed) & 15) return TKD_ERR_BAD_ARG;
-    if (k > 200 * 1024) return TKD_ERR_UNSUPPORTED;  // (a byte a k in shared memory)
+    if (k > 100 * 1024) return TKD_ERR_UNSUPPORTED;  // (two bytes a k in shared memory)
     return launch_err(tkd_launch_pack_weight(fmt, src, orient, ld, k, n, tkd_padded_cols(n), col_div, static_cast<uint16_t*>(col_scale),
                                              packed, emax, info, static_cast<cudaStream_t>(stream)));
 }

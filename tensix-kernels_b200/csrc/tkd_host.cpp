@@ -151,6 +151,60 @@ PyObject* host_route(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
 }
 
+// This thread's int in pinned host memory, which a packing kernel sets when its weight is wide: read after the stream has been
+// waited for, with nothing copied back.
+struct WideWord {
+    int* p = nullptr;
+    int* get() {
+        if (!p && cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocPortable) != cudaSuccess) p = nullptr;
+        return p;
+    }
+    ~WideWord() {
+        if (p) (void)cudaFreeHost(p);
+    }
+};
+
+// pack(format, float32 matrix, orientation, divisors or None, own scales) -> (stream, emax or None, scales or None, state):
+// tkd_pack_weight into new tensors, waited for (launches read weights ahead of stream order). state 0: done; 1: the weight
+// is wide; 2: this K is not taken (then nothing was packed).
+PyObject* host_pack(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 5 || !all_tensors(args, {1}, {3})) return type_error("tkd_host.pack: format, matrix, orientation, divisors, own scales");
+    const int fmt = (int)PyLong_AsLong(args[0]), orient = (int)PyLong_AsLong(args[2]), own = PyObject_IsTrue(args[4]);
+    if (PyErr_Occurred()) return nullptr;
+    static thread_local WideWord word;
+    try {
+        const at::Tensor& src = THPVariable_Unpack(args[1]);
+        const at::Tensor* div = tensor_or_null(args[3]);
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != src.get_device()) guard.set_index(src.get_device());
+        const int64_t cols = src.size(orient ? 1 : 0), k = src.size(orient ? 0 : 1);
+        int* wide = word.get();
+        if (!wide) return tkd_error(TKD_ERR_CUDA + (int)cudaGetLastError(), "cudaHostAlloc");
+        *wide = 0;
+        auto bytes = [&](int64_t b) { return at::detail::empty_cuda({b}, at::kByte, src.device(), std::nullopt); };
+        at::Tensor stream = bytes(tkd_packed_bytes(fmt, k, cols)), emax, scales;
+        if (fmt != TKD_FMT_BF16) emax = bytes(tkd_padded_cols(cols) / 16);
+        if (own) scales = at::detail::empty_cuda({1, 1, 1, cols}, at::kBFloat16, src.device(), std::nullopt);
+        cudaStream_t st = c10::cuda::getCurrentCUDAStream(src.get_device()).stream();
+        int rc;
+        cudaError_t e = cudaSuccess;
+        Py_BEGIN_ALLOW_THREADS rc = tkd_pack_weight(fmt, static_cast<const float*>(src.data_ptr()), orient, src.stride(0), k, cols,
+                                                    div ? static_cast<const float*>(div->data_ptr()) : nullptr, own ? scales.data_ptr() : nullptr,
+                                                    stream.data_ptr(), emax.defined() ? static_cast<uint8_t*>(emax.data_ptr()) : nullptr, wide, st);
+        if (!rc) e = cudaStreamSynchronize(st);
+        Py_END_ALLOW_THREADS if (rc && rc != TKD_ERR_UNSUPPORTED) return tkd_error(rc, "tkd_pack_weight");
+        if (e != cudaSuccess) return tkd_error(TKD_ERR_CUDA + (int)e, "tkd_pack_weight");
+        auto wrap = [](at::Tensor& t) -> PyObject* {
+            if (t.defined()) return THPVariable_Wrap(std::move(t));
+            Py_RETURN_NONE;
+        };
+        return Py_BuildValue("NNNi", wrap(stream), wrap(emax), wrap(scales), rc ? 2 : *static_cast<volatile int*>(wide) ? 1 : 0);
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyMethodDef fast(const char* name) {
     return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(F)), METH_FASTCALL, nullptr};
@@ -159,6 +213,7 @@ PyMethodDef methods[] = {
     fast<host_matmul>("matmul"),
     fast<host_moe>("moe"),
     fast<host_route>("route"),
+    fast<host_pack>("pack"),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "tkd_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

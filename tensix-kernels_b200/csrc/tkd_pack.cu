@@ -240,13 +240,16 @@ __global__ void tkd_unpack_kernel(int fmt, int64_t K, int64_t npad, const uint8_
 // warp takes a super-atom at a time. A lane loads exactly the numbers whose codes it will write (8 consecutive k of columns
 // g and g + 8 per block of 32 k: the fragment layout of tkd_layout.h), the shared exponents of its 8 k come from three
 // shuffles over the lanes of the same k, and its 16 bytes of codes go straight to the stream. Only the exponents wait for
-// the group's largest: a byte a k in shared memory, written as the stream's words at the end. A row of the group holds a
+// the group's largest: two bytes a k in shared memory, written as the stream's words at the end. A row of the group holds a
 // non-zero code exactly when its shared exponent is not zero (the largest value's implicit bit survives the rounding).
 // SCALE 1: the columns are divided by col_div first; 2: by their largest magnitude rounded up to bf16 (native_weight's
 // col_scale), found by a first walk over the CTA's 16 columns, whose second reading then comes from L2, and written out.
 // Bound: HBM. [14336, 4096] float32 to bfloat4_b (235 MB in, 33 MB out): tkd_quantise, the emax and the permute pass 410 us
-// together (1 byte a weight of codes written and read back, uncoalesced loads of the [N, K] matrix).
-constexpr int kPackThreads = 256, kPackWarps = kPackThreads / 32;
+// together (1 byte a weight of codes written and read back, uncoalesced loads of the [N, K] matrix); here 54 us without
+// column scales (5.0 TB/s), 88 with its own.
+// threads of a CTA: with the columns' own scales two large CTAs an SM (77 MB of the matrix between the two readings: it stays
+// in the 126 MB L2), else as many as fit
+__host__ __device__ constexpr int pack_threads(int scale) { return scale == 2 ? 512 : 256; }
 
 // |v|'s bits rounded up to bf16, as a float (linear.bf16_ceil), of at least 1e-8
 __device__ __forceinline__ float pack_col_scale(uint32_t bits) {
@@ -267,13 +270,35 @@ __device__ __forceinline__ uint32_t pack_code(uint32_t bits, uint32_t shared) {
     return m ? ((bits >> 16) & 0x8000u) | (m << p) : 0u;
 }
 
+// The codes of two values (k even in the low half) in floating point, six instructions a value instead of sixteen on the
+// half-rate integer pipe: y = |v| / the code's unit (s, a power of two, so exact); the alignment's truncation is y - 2^mb
+// rounded down (its last place is the one the rule keeps, and a y of 2^(mb - 1) or more, not shifted, is exact); adding
+// 1.5 * 2^23 + 2^mb rounds that to the nearest integer, ties to even, in the sum's low bits. Denormals are flushed to the
+// rule's zero. For shared exponents of 8 to 254, or 0.
+template <int FMT>
+__device__ __forceinline__ uint32_t pack_pair(float v0, float v1, float s0, float s1) {
+    constexpr float top = FMT == TKD_BFP8 ? 128.f : 8.f;
+    float z[2];
+    const float v[2] = {v0, v1}, s[2] = {s0, s1};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        float y;
+        asm("{\n\t.reg .f32 a;\n\tabs.ftz.f32 a, %1;\n\tmul.ftz.f32 %0, a, %2;\n\t}" : "=f"(y) : "f"(v[i]), "f"(s[i]));
+        z[i] = __fadd_rn(__fadd_rd(fminf(y, top - 1.f), -top), 12582912.f + top);
+    }
+    const uint32_t m = __byte_perm(__float_as_uint(z[0]), __float_as_uint(z[1]), 0x5410);
+    const uint32_t sign = __byte_perm(__float_as_uint(v0), __float_as_uint(v1), 0x7632) & (m + 0x7FFF7FFFu) & 0x80008000u;
+    return FMT == TKD_BFP8 ? m | sign : m * 16u + sign;
+}
+
 template <int FMT, int ORIENT, int SCALE>
-__global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const float* __restrict__ src, int64_t ld, int K, int64_t N,
+__global__ void __launch_bounds__(pack_threads(SCALE)) tkd_pack_weight_kernel(const float* __restrict__ src, int64_t ld, int K, int64_t N,
                                                                        const float* __restrict__ col_div,
                                                                        uint16_t* __restrict__ scale_out, uint8_t* __restrict__ stream,
                                                                        uint8_t* __restrict__ emax, int* info) {
     constexpr int KSA = FMT == TKD_BFP4 ? 64 : 32, XB = KSA / 32, EB = FMT == TKD_BFP8 ? 32 : FMT == TKD_BFP4 ? 64 : 0;
-    extern __shared__ __align__(16) uint8_t exps[];  // the shared exponent of every k (not for bf16)
+    constexpr int kPackThreads = pack_threads(SCALE), kPackWarps = kPackThreads / 32;
+    extern __shared__ __align__(16) uint8_t exps[];  // the shared exponent of every k, 16 bits each, from bit 7 (not for bf16)
     __shared__ uint32_t cmax[kPackWarps][16];
     __shared__ float cdiv[16];
     __shared__ int shi[kPackWarps], slo[kPackWarps];
@@ -295,13 +320,14 @@ __global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const flo
             for (int i = 0; i < 8; ++i) v[i] = __ldg(src + (int64_t)(k + i) * ld + n);
         }
     };
-    float d0 = 1.f, d1 = 1.f;
+    float d0 = 1.f, d1 = 1.f, r0 = 1.f, r1 = 1.f;
+    bool slow = SCALE == 1;  // divide by the division
     if constexpr (SCALE == 1) {
         if (in0) d0 = col_div[n0];
         if (in1) d1 = col_div[n1];
     } else if constexpr (SCALE == 2) {
         uint32_t m0 = 0, m1 = 0;
-#pragma unroll 2
+#pragma unroll 4
         for (int b = warp; b < K / 32; b += kPackWarps) {
             float v0[8], v1[8];
             load8(v0, n0, in0, 32 * b + 8 * t);
@@ -327,8 +353,9 @@ __global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const flo
         }
         __syncthreads();
         d0 = cdiv[g], d1 = cdiv[g + 8];
+        r0 = __frcp_rn(d0), r1 = __frcp_rn(d1);
+        slow = __any_sync(0xFFFFFFFFu, !(d0 < 0x1p60f) || !(d1 < 0x1p60f));
     }
-    uint32_t hi = 0, lo = 255;
     for (int sa = warp; sa < nsa; sa += kPackWarps) {
         uint8_t* dst = stream + tkd_sa_offset(FMT, K, grp, sa) + EB + lane * 16;
         float v[2][XB][8];
@@ -338,10 +365,23 @@ __global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const flo
             load8(v[1][q], n1, in1, sa * KSA + 32 * q + 8 * t);
         }
         if constexpr (SCALE != 0) {
+            // (own scales) v / d correctly rounded from the correctly rounded reciprocal r: q = v r, then q + (v - q d) r
+            // (P. Markstein, IBM J. Res. Dev. 34, 1990; a bf16 divisor is not the exceptional one whose significand bits are
+            // all set). It needs v - q d exact: a block whose largest quotients lie near the denormals is divided again below.
+            if (SCALE == 2 && FMT != TKD_BF16 && !slow) {
 #pragma unroll
-            for (int q = 0; q < XB; ++q)
+                for (int q = 0; q < XB; ++q)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[0][q][i] = __fdiv_rn(v[0][q][i], d0), v[1][q][i] = __fdiv_rn(v[1][q][i], d1);
+                    for (int i = 0; i < 8; ++i) {
+                        const float x = v[0][q][i] * r0, y = v[1][q][i] * r1;
+                        v[0][q][i] = fmaf(fmaf(-x, d0, v[0][q][i]), r0, x), v[1][q][i] = fmaf(fmaf(-y, d1, v[1][q][i]), r1, y);
+                    }
+            } else {
+#pragma unroll
+                for (int q = 0; q < XB; ++q)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[0][q][i] = __fdiv_rn(v[0][q][i], d0), v[1][q][i] = __fdiv_rn(v[1][q][i], d1);
+            }
         }
         uint32_t words[4];
 #pragma unroll
@@ -358,33 +398,54 @@ __global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const flo
                 for (int jj = 0; jj < 2; ++jj)
                     *reinterpret_cast<uint4*>(dst + 512 * jj) = make_uint4(b[0][2 * jj], b[1][2 * jj], b[0][2 * jj + 1], b[1][2 * jj + 1]);
             } else {
-                uint32_t sh[8];
+                // the largest upper halves (exponent and seven bits) of the 16 columns at each k, two k to a word
+                uint32_t both[4];
+                auto maxima = [&]() {
+                    uint32_t odd = 0;
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    // two k's exponents to a word, their maxima over the 16 columns
-                    uint32_t w[2];
+                    for (int i = 0; i < 4; ++i) {
+                        uint32_t w[2];
 #pragma unroll
-                    for (int j = 0; j < 2; ++j)
-                        w[j] = max((__float_as_uint(v[0][q][i + j]) >> 23) & 0xFFu, (__float_as_uint(v[1][q][i + j]) >> 23) & 0xFFu);
-                    uint32_t both = w[0] | (w[1] << 16);
+                        for (int c = 0; c < 2; ++c)
+                            w[c] = __byte_perm(__float_as_uint(v[c][q][2 * i]), __float_as_uint(v[c][q][2 * i + 1]), 0x7632) & 0x7FFF7FFFu;
+                        both[i] = __vmaxu2(w[0], w[1]);
 #pragma unroll
-                    for (int o = 4; o < 32; o <<= 1) both = __vmaxu2(both, __shfl_xor_sync(0xFFFFFFFFu, both, o));
-                    sh[i] = both & 0xFFFFu, sh[i + 1] = both >> 16;
+                        for (int o = 4; o < 32; o <<= 1) both[i] = __vmaxu2(both[i], __shfl_xor_sync(0xFFFFFFFFu, both[i], o));
+                        both[i] &= 0x7F807F80u;
+                        // an exponent of 1 to 7, or of 255, leaves pack_pair's scale outside the normal numbers; (own scales)
+                        // one below 100 may come of a quotient that was not exact
+                        const uint32_t e0 = both[i] & 0xFFFFu, e1 = both[i] >> 16, low = SCALE == 2 ? 100u << 7 : 8u << 7;
+                        const uint32_t from = SCALE == 2 ? 0u : 1u;
+                        odd |= (e0 - from < low - from) | (e1 - from < low - from) | (e0 == 0x7F80u) | (e1 == 0x7F80u);
+                    }
+                    return __any_sync(0xFFFFFFFFu, odd) != 0;
+                };
+                bool odd = maxima();
+                if (SCALE == 2 && odd && !slow) {
+                    load8(v[0][q], n0, in0, sa * KSA + 32 * q + 8 * t);
+                    load8(v[1][q], n1, in1, sa * KSA + 32 * q + 8 * t);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[0][q][i] = __fdiv_rn(v[0][q][i], d0), v[1][q][i] = __fdiv_rn(v[1][q][i], d1);
+                    (void)maxima();
                 }
-                if (g == 0) {
-                    uint32_t* ex = reinterpret_cast<uint32_t*>(exps + sa * KSA + 32 * q + 8 * t);
-                    ex[0] = sh[0] | (sh[1] << 8) | (sh[2] << 16) | (sh[3] << 24);
-                    ex[1] = sh[4] | (sh[5] << 8) | (sh[6] << 16) | (sh[7] << 24);
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) hi = max(hi, sh[i]), lo = min(lo, sh[i] ? sh[i] : 255u);
+                if (g == 0) *reinterpret_cast<uint4*>(exps + (sa * KSA + 32 * q + 8 * t) * 2) = make_uint4(both[0], both[1], both[2], both[3]);
                 uint32_t r[2][4];  // (column g or g + 8, pair of k): a fragment register
+                if (!odd) {
+                    constexpr uint32_t unit = (uint32_t)(253 + (FMT == TKD_BFP8 ? 7 : 3)) << 23;
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
+                    for (int i = 0; i < 4; ++i) {
+                        const float s0 = __uint_as_float(unit - (both[i] << 16)), s1 = __uint_as_float(unit - (both[i] & 0xFFFF0000u));
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        r[c][i] = pack_code<FMT>(__float_as_uint(v[c][q][2 * i]), sh[2 * i]) |
-                                  (pack_code<FMT>(__float_as_uint(v[c][q][2 * i + 1]), sh[2 * i + 1]) << 16);
+                        for (int c = 0; c < 2; ++c) r[c][i] = pack_pair<FMT>(v[c][q][2 * i], v[c][q][2 * i + 1], s0, s1);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            r[c][i] = pack_code<FMT>(__float_as_uint(v[c][q][2 * i]), (both[i] >> 7) & 0xFFu) |
+                                      (pack_code<FMT>(__float_as_uint(v[c][q][2 * i + 1]), both[i] >> 23) << 16);
+                }
                 if constexpr (FMT == TKD_BFP8) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) words[i] = r[0][i] | tkd_rotl(r[1][i], 8);
@@ -398,6 +459,12 @@ __global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const flo
         if constexpr (FMT != TKD_BF16) *reinterpret_cast<uint4*>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
     }
     if constexpr (FMT != TKD_BF16) {
+        __syncthreads();
+        uint32_t hi = 0, lo = 255;
+        for (int i = tid; i < nsa * KSA; i += kPackThreads) {
+            const uint32_t sh = *reinterpret_cast<const uint16_t*>(exps + 2 * i) >> 7;
+            hi = max(hi, sh), lo = min(lo, sh ? sh : 255u);
+        }
         hi = __reduce_max_sync(0xFFFFFFFFu, hi), lo = __reduce_min_sync(0xFFFFFFFFu, lo);
         if (lane == 0) shi[warp] = (int)hi, slo[warp] = (int)lo;
         __syncthreads();
@@ -412,11 +479,11 @@ __global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const flo
         constexpr int PT = 2 * XB, PW = 4 * PT;
         for (int i = tid; i < nsa * PW; i += kPackThreads) {
             const int sa = i / PW, wi = i % PW, wt = wi / PT, j = wi % PT;
-            const uint32_t e4 = *reinterpret_cast<const uint32_t*>(exps + sa * KSA + 32 * (j >> 1) + 8 * wt + 4 * (j & 1));
+            const uint2 e4 = *reinterpret_cast<const uint2*>(exps + 2 * (sa * KSA + 32 * (j >> 1) + 8 * wt + 4 * (j & 1)));
             uint32_t word = 0;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                const int sh = (int)((e4 >> (8 * r)) & 0xFFu);
+                const int sh = (int)(((r & 2 ? e4.y : e4.x) >> (16 * (r & 1) + 7)) & 0xFFu);
                 const int e = sh ? max(tkd_ezero(FMT), sh - top + tkd_ebias(FMT)) : tkd_ezero(FMT);
                 word |= tkd_exp_bits(FMT, (uint32_t)e, r);
             }
@@ -428,14 +495,14 @@ __global__ void __launch_bounds__(kPackThreads) tkd_pack_weight_kernel(const flo
 template <int FMT, int ORIENT>
 int launch_pack_weight(const float* src, int64_t ld, int64_t K, int64_t N, int64_t npad, const float* col_div, uint16_t* scale_out,
                        void* packed, uint8_t* emax, int* info, cudaStream_t st) {
-    const size_t smem = FMT == TKD_BF16 ? 0 : (size_t)(K + 63) / 64 * 64;
+    const size_t smem = FMT == TKD_BF16 ? 0 : (size_t)(K + 63) / 64 * 128;
     auto kern = scale_out ? tkd_pack_weight_kernel<FMT, ORIENT, 2>
                           : col_div ? tkd_pack_weight_kernel<FMT, ORIENT, 1> : tkd_pack_weight_kernel<FMT, ORIENT, 0>;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    kern<<<(unsigned)(npad / 16), kPackThreads, smem, st>>>(src, ld, (int)K, N, col_div, scale_out, static_cast<uint8_t*>(packed), emax, info);
+    kern<<<(unsigned)(npad / 16), pack_threads(scale_out ? 2 : 0), smem, st>>>(src, ld, (int)K, N, col_div, scale_out, static_cast<uint8_t*>(packed), emax, info);
     return (int)cudaGetLastError();
 }
 

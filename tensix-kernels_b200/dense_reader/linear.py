@@ -125,10 +125,12 @@ def native_weight(device, t, dtype, col_scale=False, sharded=True, max_banks=Non
     reports (width-sharded over the device's banks, or interleaved)."""
     assert dtype in NATIVE_TILES, f"dense_reader: weights are bfloat8_b, bfloat4_b or bfloat16, not {dtype}"
     n, k = t.shape
-    c = torch.empty(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch) if col_scale else \
-        torch.ones(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch)
     mc = sharded_memcfg(device, k, n, max_banks=max_banks) if sharded else ttnn.DRAM_MEMORY_CONFIG
-    w = ttnn.pack_weight(device, t, dtype, 0, memory_config=mc, col_scale=c if col_scale else None)
+    if col_scale:
+        w, c = ttnn.pack_weight_scaled(device, t, dtype, memory_config=mc)
+    else:
+        w = ttnn.pack_weight(device, t, dtype, 0, memory_config=mc)
+        c = torch.ones(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch)
     return w, ttnn.Tensor(c, ttnn.bfloat16, ttnn.TILE_LAYOUT, device, ttnn.DRAM_MEMORY_CONFIG)
 
 

@@ -549,8 +549,8 @@ def test_packing_in_one_pass_equals_the_passes(device, fmt, k, n):
         c = linear.bf16_ceil(w.abs().amax(dim=1).clamp(min=1e-8))
         div = c.to(device.torch) if scaled else None
         want, emax, f = ttnn._pack_in_passes(device, w.to(device.torch), _tkd.__dict__["FMT_" + fmt.upper()], 0, k, n, div)
-        cs = torch.zeros(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch) if scaled else None
-        got = [ttnn.pack_weight(device, w, DT[fmt], 0, col_scale=cs), ttnn.pack_weight(device, w, DT[fmt], 0, col_div=div),
+        own, cs = ttnn.pack_weight_scaled(device, w, DT[fmt]) if scaled else (ttnn.pack_weight(device, w, DT[fmt], 0), None)
+        got = [own, ttnn.pack_weight(device, w, DT[fmt], 0, col_div=div),
                ttnn.pack_weight(device, wide.to(device.torch)[:, :n], DT[fmt], 1, col_div=div)]
         for t in got:
             assert t.fmt == f and torch.equal(t.t, want)
