@@ -187,6 +187,15 @@ int tkd_matmul_workspace(const TkdMatmul* a, uint64_t* bytes);
  * weight and multiplies by it on the same stream without a synchronisation in between sets a->weights_fresh. */
 int tkd_matmul(const TkdMatmul* a, void* stream);
 
+/* tkd_matmul for more rows than 32 (m from 33 to TKD_ROWS_MAX; the reference's row slices, linear.py:179-184): one weight or
+ * pair, every output stage, no records, exchange, rotation or TKD_FMT_INT4 (TKD_ERR_UNSUPPORTED). A weight is read once for
+ * every 256 rows. The workspace is as tkd_matmul's and may be the same one; its size is tkd_matmul_rows_workspace's. A
+ * column's sum depends on K, the format, the row count and N (where a tile of columns is cut between CTAs), not on the rows'
+ * values. */
+#define TKD_ROWS_MAX 4096
+int tkd_matmul_rows_workspace(const TkdMatmul* a, uint64_t* bytes);
+int tkd_matmul_rows(const TkdMatmul* a, void* stream);
+
 /* tkd_matmul with the activations and the result in HOST memory (pinned, for the copies to be asynchronous): copies
  * x_host [m, k] bf16 into a->x, launches, copies a->out [m, ldo] to out_host, all on `stream`; a->x and a->out are the
  * caller's device staging buffers (ldx == k). The counterpart of a caller doing ttnn.from_torch(x) ... ttnn.to_torch(y)

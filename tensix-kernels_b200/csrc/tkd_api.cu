@@ -297,11 +297,8 @@ int tkd_matmul_workspace(const TkdMatmul* a, uint64_t* bytes) {
     return TKD_OK;
 }
 
-static int run_matmul(const TkdMatmul* a, void* workspace, uint64_t workspace_bytes, void* stream) {
-    Layout L;
-    const int rc = make_layout(a, &L, 0);
-    if (rc) return rc;
-    TkdParams& p = L.p;
+// A call's tensors and options against one another.
+static int check_pointers(const TkdMatmul* a) {
     if (!a->x || !a->out || a->ldx < a->k || a->ldx % 8 || (reinterpret_cast<uintptr_t>(a->x) & 15)) return TKD_ERR_BAD_ARG;
     for (int s = 0; s < a->nblocks; ++s) {
         const TkdBlock& b = a->block[s];
@@ -321,6 +318,102 @@ static int run_matmul(const TkdMatmul* a, void* workspace, uint64_t workspace_by
     if (a->epilogue == TKD_EPI_RESIDUAL && (!a->residual || a->residual_dtype != TKD_DT_BF16)) return TKD_ERR_BAD_ARG;
     if (a->epilogue == TKD_EPI_OUT32 && a->residual && a->residual_dtype != TKD_DT_F32) return TKD_ERR_BAD_ARG;
     if (a->epilogue != TKD_EPI_RESIDUAL && a->epilogue != TKD_EPI_OUT32 && a->residual) return TKD_ERR_BAD_ARG;
+    return TKD_OK;
+}
+
+// ---- more than 32 rows -----------------------------------------------------------------------------------------------
+
+// The launch of such a call, without the pointers into the workspace. sms 0: ask the device.
+static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_bytes, int sms) {
+    if (!a || !fmt_ok(a->fmt) || a->m < 33 || a->m > TKD_ROWS_MAX || a->k < 32 || a->k % 32 || a->k > (1 << 24)) return TKD_ERR_BAD_ARG;
+    if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_OUT32 || a->nblocks != 1 || a->topk_k) return TKD_ERR_BAD_ARG;
+    if ((a->epilogue == TKD_EPI_OUT32) != (a->out_dtype == TKD_DT_F32)) return TKD_ERR_BAD_ARG;
+    if (a->fmt == TKD_INT4 || a->hadamard || a->nranks > 1) return TKD_ERR_UNSUPPORTED;
+    const TkdBlock& b = a->block[0];
+    if (b.n < 1 || b.out_col0 < 0 || b.n > (1 << 28) || (a->epilogue == TKD_EPI_GLU_IL && b.n % 64)) return TKD_ERR_BAD_ARG;
+    memset(w, 0, sizeof(*w));
+    TkdWide& p = *w;
+    p.M = a->m, p.K = (int)a->k;
+    // rows of a tile: all of them up to 256, else as many in each tile as in the others
+    p.nrt = (p.M + 255) / 256;
+    p.nt = ((p.M + p.nrt - 1) / p.nrt + 15) / 16 * 16;
+    // (an MMA of up to 128 rows is shorter than its issue: two warps, an accumulator each)
+    p.nmma = p.nt <= 128 ? 2 : 1;
+    p.nset = p.nmma * p.nt * 2 <= 256 ? 2 : 1;
+    p.nx = p.nt <= 128 ? 8 : 4;
+    p.nkb = (p.K + 127) / 128 * 2;
+    const int64_t npad = tkd_padded_cols(b.n);
+    const int64_t panels = a->epilogue == TKD_EPI_GLU2 ? npad / 64 : npad / TKD_PANEL_COLS;
+    p.chunks = (p.K + tkd_chunk_k(a->fmt) - 1) / tkd_chunk_k(a->fmt);
+    const int64_t total = panels * p.nrt * p.chunks;
+    if (panels * p.nrt > kMaxPanels || total > (1 << 30)) return TKD_ERR_UNSUPPORTED;
+    p.total = (int)total;
+    if (sms <= 0) sms = sm_count();
+    if (sms <= 0) sms = 148;
+    if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
+    p.grid = (int)(total < sms ? total : sms);
+    p.panel_bytes = tkd_panel_bytes(a->fmt, a->k);
+    p.stage_bytes = 8 * tkd_subsa(a->fmt) * tkd_sab(a->fmt);
+    p.off_stage = TKD_SMEM_HEAD;
+    p.off_x = p.off_stage + 8 * 64 * 4;
+    p.off_ring = (int)align_up(p.off_x + 1023 + p.nx * p.nt * 128, 128);
+    p.nstages = (kMaxSmem - p.off_ring) / p.stage_bytes;
+    if (p.nstages > TKD_MAX_STAGES) p.nstages = TKD_MAX_STAGES;
+    if (p.nstages < 2) return TKD_ERR_UNSUPPORTED;
+    *smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
+    p.epi = a->epilogue, p.act = a->act, p.mul16 = 16, p.mul128 = 128;
+    // workspace: the counters every call shares, the cut tiles' partial sums, the x tiles
+    const int64_t scratch = (int64_t)p.grid * 2 * p.nt * 512;
+    *ws_bytes = (uint64_t)(kCounterBytes + scratch + (int64_t)p.nrt * p.nkb * p.nt * 128);
+    return TKD_OK;
+}
+
+int tkd_matmul_rows_workspace(const TkdMatmul* a, uint64_t* bytes) {
+    if (!bytes) return TKD_ERR_BAD_ARG;
+    int sms = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        sms = 148;
+    }
+    TkdWide w;
+    size_t smem;
+    return make_wide(a, &w, &smem, bytes, sms);
+}
+
+int tkd_matmul_rows(const TkdMatmul* a, void* stream) {
+    TkdWide p;
+    size_t smem;
+    uint64_t need;
+    const int rc = make_wide(a, &p, &smem, &need, 0);
+    if (rc) return rc;
+    const int ra = check_pointers(a);
+    if (ra) return ra;
+    if (!a->workspace || a->workspace_bytes < need) return TKD_ERR_WORKSPACE;
+    if (reinterpret_cast<uintptr_t>(a->workspace) & 255) return TKD_ERR_BAD_ARG;
+    const TkdBlock& b = a->block[0];
+    p.w = static_cast<const uint8_t*>(b.w), p.w2 = static_cast<const uint8_t*>(b.w_up), p.emax = b.emax, p.emax2 = b.emax_up;
+    p.n_valid = (int)b.n, p.out_col0 = (int)b.out_col0;
+    p.x = static_cast<const uint16_t*>(a->x), p.ldx = a->ldx;
+    p.scale = a->scale, p.scale2 = a->scale_up, p.scale_dt = a->scale_dtype;
+    p.res = a->residual, p.ldr = a->ldr, p.out = a->out, p.ldo = a->ldo;
+    uint8_t* ws = static_cast<uint8_t*>(a->workspace);
+    p.counters = reinterpret_cast<int*>(ws);
+    p.scratch = reinterpret_cast<float*>(ws + kCounterBytes);
+    p.xt = ws + kCounterBytes + (int64_t)p.grid * 2 * p.nt * 512;
+    p.status = a->status;
+    p.no_pdl = a->weights_fresh != 0;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return launch_err(a->fmt == TKD_BFP8 ? tkd_launch_wide_bfp8(p, smem, st)
+                                         : a->fmt == TKD_BFP4 ? tkd_launch_wide_bfp4(p, smem, st) : tkd_launch_wide_bf16(p, smem, st));
+}
+
+static int run_matmul(const TkdMatmul* a, void* workspace, uint64_t workspace_bytes, void* stream) {
+    Layout L;
+    const int rc = make_layout(a, &L, 0);
+    if (rc) return rc;
+    TkdParams& p = L.p;
+    const int ra = check_pointers(a);
+    if (ra) return ra;
     if (a->topk_k && !a->records) return TKD_ERR_BAD_ARG;
     if (!workspace || workspace_bytes < (uint64_t)L.ws_bytes) return TKD_ERR_WORKSPACE;
     if (workspace && (reinterpret_cast<uintptr_t>(workspace) & 255)) return TKD_ERR_BAD_ARG;

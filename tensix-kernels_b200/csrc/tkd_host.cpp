@@ -64,7 +64,7 @@ PyObject* host_matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (c10::cuda::current_device() != x.get_device()) guard.set_index(x.get_device());
         TkdMatmul a = *desc;
         at::Tensor made;
-        const bool f32 = a.out_dtype == TKD_DT_F32;
+        const bool f32 = a.out_dtype == TKD_DT_F32;  // (more than 32 rows: tkd_matmul_rows)
         if (!out) {
             const int64_t shape[4] = {1, 1, a.m, a.ldo};
             made = at::detail::empty_cuda(shape, f32 ? at::kFloat : at::kBFloat16, x.device(), std::nullopt);
@@ -77,7 +77,7 @@ PyObject* host_matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
         a.workspace_bytes = (uint64_t)ws.nbytes();
         void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
         int rc;
-        Py_BEGIN_ALLOW_THREADS rc = tkd_matmul(&a, stream);
+        Py_BEGIN_ALLOW_THREADS rc = a.m > 32 ? tkd_matmul_rows(&a, stream) : tkd_matmul(&a, stream);
         Py_END_ALLOW_THREADS if (rc) return tkd_error(rc, "tkd_matmul");
         if (made.defined()) return THPVariable_Wrap(std::move(made));
         Py_INCREF(args[2]);

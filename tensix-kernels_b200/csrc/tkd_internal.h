@@ -100,6 +100,41 @@ struct TkdParams {
     int stage_bytes;
 };
 
+// --- more than 32 rows (tkd_wide.cuh) ---
+#define TKD_WIDE_XT 8  // x tiles in shared memory, at most
+struct TkdWide {
+    const uint8_t *w, *w2;  // the packed stream (the gate's), the up weight's or null
+    const uint8_t *emax, *emax2;
+    int n_valid, out_col0;
+    int M, K;
+    int nt, nrt;        // rows of a tile (a multiple of 16, at most 256), row tiles
+    int chunks, total;  // chunks of K a tile; chunks of all tiles
+    int grid;
+    int64_t panel_bytes;
+    const uint16_t* x;
+    int64_t ldx;
+    uint8_t* xt;        // x in tiles of [nt][64 k], tile (row tile, k block)
+    int nkb;            // 64-k blocks of a row tile (K padded to 128)
+    int nmma, nset;     // MMA warps (and accumulators of a set), sets of accumulators
+    int nx, nstages, stage_bytes;
+    int off_stage, off_x, off_ring;  // shared-memory map
+    int epi, act;
+    const void *scale, *scale2;
+    int scale_dt;
+    const void* res;
+    int64_t ldr;
+    void* out;
+    int64_t ldo;
+    float* scratch;     // partial sums of cut tiles: two a CTA, [nt / 4][128 columns][4] floats
+    int* counters;      // per tile: parts delivered
+    int* status;
+    int no_pdl;
+    uint32_t mul16, mul128;
+};
+
+int tkd_launch_wide_bfp8(const TkdWide& p, size_t smem, cudaStream_t st);
+int tkd_launch_wide_bfp4(const TkdWide& p, size_t smem, cudaStream_t st);
+int tkd_launch_wide_bf16(const TkdWide& p, size_t smem, cudaStream_t st);
 int tkd_launch_stream(const TkdParams& p, int grid, size_t smem, cudaStream_t st);
 int tkd_launch_hadamard(const void* x, int64_t ldx, const uint32_t* signs, int rows, int K, void* out, int64_t ldo,
                         cudaStream_t st);

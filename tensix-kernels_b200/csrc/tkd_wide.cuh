@@ -1,0 +1,566 @@
+// tkd_wide.cuh: the matmul of more than 32 activation rows (a prompt's prefill, a large batch) against a packed weight, on
+// the fifth-generation tensor cores.
+//
+// The reference takes such calls as slices of rows, each reading all the weights again (dense_reader/linear.py:179-184). So
+// did this library: 512 rows through a [14336, 4096] bfloat8_b weight were 16 launches of the kernel for 32 rows, 387 us,
+// each bound by taking the weights apart, which is the same work for 32 rows as for 256. Here a weight is taken apart once
+// for up to 256 rows: a tile is 128 weight columns (the MMA's M: a panel of the stream) by NT rows (its N), all of K
+// accumulated in tensor memory.
+//
+//   tkd_wide_x_kernel  lays the activations out as the MMA's B operand first: tiles of NT rows x 64 k, K-major with the
+//                      128-byte swizzle, k in the order of the weight fragments, rows past M and k past K zero; each tile
+//                      contiguous, so that it comes into shared memory by one bulk copy.
+//   tkd_wide_kernel    warp 0 (and 2)  one lane issues the MMAs, A from tensor memory, B from shared memory. Up to 128 rows
+//                                      two warps share the units (of 128 k): an MMA of few rows is shorter than its issue.
+//                      warp 1          producer of the ring of weight chunks; warp 3: of the x tiles
+//                      warps 4-19      decode: tkd_stream_tc_kernel's, without the activations
+//                      warps 20-23     output: a thread is a column (a tensor-memory lane)
+//
+// Work split: tiles are numbered panel-major (the tiles of a panel run at the same time on different SMs and share its
+// chunks in L2), each of `chunks` chunks of K; all chunks are cut into equal contiguous runs, one per CTA. A tile that is
+// cut goes through scratch, a partial sum per CTA, and the CTA that delivers last adds them up in order of k: with 224 tiles
+// on 148 SMs (512 rows of the weight above) whole tiles would leave a quarter of the machine idle.
+#pragma once
+#include "tkd_stream_tc.cuh"
+
+namespace {
+
+constexpr int kWideWarps = 24, kWideRing = 1, kWideX = 3, kWideDecode0 = 4, kWideOut0 = 20;
+constexpr int kWideASlots = 4;                    // units of A in tensor memory, 64 columns each
+constexpr int kWideA0 = 256;                      // their first column: the accumulators have 0-255
+static_assert(kWideA0 + kWideASlots * 64 <= 512, "tensor memory");
+
+// One CTA lays out 64 rows of one tile: thread (row, piece of 8 k).
+__global__ void __launch_bounds__(512) tkd_wide_x_kernel(const uint16_t* __restrict__ x, int64_t ldx, int M, int K, int nt, int nkb,
+                                                         uint8_t* __restrict__ xt) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int kb = blockIdx.x, rt = blockIdx.z, r = blockIdx.y * 64 + (threadIdx.x >> 3), c = threadIdx.x & 7;
+    if (r >= nt) return;
+    const int row = rt * nt + r, k = kb * 64 + 8 * c;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (row < M && k < K) v = __ldg(reinterpret_cast<const uint4*>(x + (int64_t)row * ldx + k));
+    uint8_t* t = xt + ((int64_t)rt * nkb + kb) * nt * 128 + r * 128;
+    const int o0 = 64 * (c >> 2) + 8 * (c & 3), o1 = o0 + 32;  // (k 0-3 and k 4-7: see tkd_stream_tc.cuh)
+    *reinterpret_cast<uint2*>(t + ((((o0 >> 4) ^ (r & 7)) << 4) | (o0 & 15))) = make_uint2(v.x, v.y);
+    *reinterpret_cast<uint2*>(t + ((((o1 >> 4) ^ (r & 7)) << 4) | (o1 & 15))) = make_uint2(v.z, v.w);
+}
+
+// D (tensor memory) (+)= A (tensor memory) x B (shared memory), M 128, N from the instruction descriptor
+__device__ __forceinline__ void wide_mma(uint32_t d, uint32_t a, uint32_t blo, uint32_t bhi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+        ::"r"(d), "r"(a), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// A part of a CTA's run that lies in one tile.
+struct WideSeg {
+    int tile, c0, c1;  // chunks c0 .. c1 - 1 of the tile
+};
+__device__ __forceinline__ bool wide_next(const TkdWide& p, int& it, int i1, WideSeg& s) {
+    if (it >= i1) return false;
+    s.tile = it / p.chunks;
+    s.c0 = it - s.tile * p.chunks;
+    s.c1 = min(p.chunks, s.c0 + i1 - it);
+    it += s.c1 - s.c0;
+    return true;
+}
+__device__ __forceinline__ int wide_begin(const TkdWide& p, int cta) { return (int)((int64_t)p.total * cta / p.grid); }
+// the CTA whose run holds item i
+__device__ __forceinline__ int wide_owner(const TkdWide& p, int i) { return (int)((((int64_t)i + 1) * p.grid - 1) / p.total); }
+
+// The output warps: a thread is the column et of its tile's panel. Rows go in batches of 8 (of 16: 600 bytes of spills).
+template <int FMT>
+__device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, uint32_t tmem0, uint8_t* smem, uint32_t accfull0,
+                                            uint32_t accempty0, volatile int* sflag, uint32_t xs0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int CK = Fmt<FMT>::SUBSA * Fmt<FMT>::KSA;
+    const int lane = threadIdx.x & 31, ow = (threadIdx.x >> 5) & 3, et = ow * 32 + lane;
+    const int NT = p.nt, nm = p.nmma;
+    const bool glu2 = p.epi == TKD_EPI_GLU2, glu = glu2 || p.epi == TKD_EPI_GLU_IL;
+    const bool f32out = p.epi == TKD_EPI_OUT32, res32 = f32out && p.res, res16 = p.epi == TKD_EPI_RESIDUAL;
+    float* stage = reinterpret_cast<float*>(smem + p.off_stage);  // GLU: [8 rows][64 columns] of the up half
+    // GLU: the warps of a panel's gate columns (interleaved: 32 gate, their 32 up, ...; two weights: 64 and 64)
+    const bool gate = glu2 ? ow < 2 : (ow & 1) == 0;
+    const int gcol = glu2 ? (ow & 1) * 32 + lane : (ow >> 1) * 32 + lane;  // the column within the tile's 64 outputs
+    WideSeg sg;
+    uint32_t j = 0;
+    for (int it = i0; wide_next(p, it, i1, sg); ++j) {
+        const int panel = sg.tile / p.nrt, rt = sg.tile - panel * p.nrt;
+        const int n = glu2 ? (panel >> 1) * 128 + (panel & 1) * 64 + (et & 63) : panel * 128 + et;  // the column of its weight
+        const bool in_w = n < p.n_valid;
+        float colf = 1.f, colg = 1.f, cols = 1.f;
+        if constexpr (FMT != TKD_BF16) {
+            const int e = tkd_out_exp(FMT, (glu2 && et >= 64 ? p.emax2 : p.emax)[n >> 4]), e1 = e / 2, e2 = e - e1;
+            colf = __uint_as_float((uint32_t)(e1 + 127) << 23), colg = __uint_as_float((uint32_t)(e2 + 127) << 23);
+        }
+        if (p.scale_dt != TKD_DT_NONE && in_w) {
+            const void* sp = glu2 && et >= 64 ? p.scale2 : p.scale;
+            cols = p.scale_dt == TKD_DT_BF16 ? bf16_bits_to_f32(static_cast<const uint16_t*>(sp)[n]) : static_cast<const float*>(sp)[n];
+        }
+        // the output column this thread stores, or -1
+        int oc = -1;
+        if (!glu) {
+            if (in_w) oc = p.out_col0 + n;
+        } else if (gate) {
+            const int o = panel * 64 + gcol;
+            if (o < (glu2 ? p.n_valid : p.n_valid / 2)) oc = p.out_col0 + o;
+        }
+        const int row0 = rt * NT, rows = min(NT, p.M - row0);
+        const bool whole = sg.c0 == 0 && sg.c1 == p.chunks;
+        const int kv = min(p.K, sg.c1 * CK) - sg.c0 * CK;
+        const bool two = nm == 2 && kv > 128;
+        const uint32_t set = j % p.nset;
+        if (!mbar_wait_parked(accfull0 + 8 * set, (j / p.nset) & 1, p.status)) return;
+        tc_fence_after();
+        const uint32_t ta = tmem0 + ((uint32_t)(ow * 32) << 16) + set * nm * NT;
+        // eight rows of the segment's sums
+        auto load_acc = [&](int r, float (&v)[8]) {
+            uint32_t a[8], b[8];
+            auto ld = [&](uint32_t at, uint32_t (&q)[8]) {
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                             : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
+                             : "r"(at)
+                             : "memory");
+            };
+            ld(ta + r, a);
+            if (two) ld(ta + NT + r, b);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[m] = two ? __uint_as_float(a[m]) + __uint_as_float(b[m]) : __uint_as_float(a[m]);
+        };
+        auto release = [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(accempty0 + 8 * set);
+        };
+        // partial sums in scratch: [segment][row / 4][column][4]
+        const int64_t part = (int64_t)NT * 128;
+        int b0 = 0, nseg = 1;
+        bool staged = false;  // the partial sums are copied into the (then idle) x tiles first
+        int per = 0;          // ... so many rows at a time
+        if (!whole) {
+            float* dst = p.scratch + ((int64_t)blockIdx.x * 2 + (wide_begin(p, blockIdx.x) < sg.tile * p.chunks ? 1 : 0)) * part + et * 4;
+#pragma unroll 1
+            for (int r = 0; r < rows; r += 8) {
+                float v[8];
+                load_acc(r, v);
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    __stcg(reinterpret_cast<float4*>(dst + (r / 4 + q) * 512), make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+            }
+            release();
+            b0 = wide_owner(p, sg.tile * p.chunks);
+            nseg = wide_owner(p, sg.tile * p.chunks + p.chunks - 1) - b0 + 1;
+            bar_output_warps();  // (orders the 128 threads' stores before thread 0's release)
+            if (et == 0) {
+                const int last = atom_add_acq_rel(p.counters + sg.tile, 1) + 1 == nseg;
+                if (last) p.counters[sg.tile] = 0;
+                sflag[0] = last;
+            }
+            bar_output_warps();
+            const bool finish = sflag[0] != 0;
+            bar_output_warps();  // (sflag may be written again only after everyone has read it)
+            if (!finish) continue;
+            per = p.nx * NT * 128 / (nseg * 512) & ~7;
+            staged = it >= i1 && per >= 8;  // (this CTA's last tile: every x tile has been multiplied)
+        }
+        // where segment s of the tile left its sums
+        auto part_of = [&](int s) {
+            const int b = b0 + s;
+            return p.scratch + ((int64_t)b * 2 + (wide_begin(p, b) < sg.tile * p.chunks ? 1 : 0)) * part + et * 4;
+        };
+        // the residual of a batch, asked for a batch ahead: float32 a row, or bf16 a pair of columns of every other row
+        const bool odd = lane & 1;
+        const bool pairs = !f32out && !((reinterpret_cast<uintptr_t>(p.out) & 3) | (p.ldo & 1) | (p.out_col0 & 1)) &&
+                           !(res16 && ((reinterpret_cast<uintptr_t>(p.res) & 3) | (p.ldr & 1)));
+        const bool pair_ok = pairs && __shfl_xor_sync(0xFFFFFFFFu, oc, 1) >= 0 && oc >= 0;
+        uint32_t rq[8];
+        auto load_res = [&](int r) {
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                if (res32) {
+                    rq[m] = oc >= 0 && r + m < rows ? __float_as_uint(static_cast<const float*>(p.res)[(int64_t)(row0 + r + m) * p.ldr + oc]) : 0u;
+                } else if (pair_ok) {
+                    if (m < 4) {
+                        const int rr = r + 2 * m + odd;
+                        rq[m] = rr < rows ? *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.res) + (int64_t)(row0 + rr) * p.ldr + oc - odd) : 0u;
+                    }
+                } else {
+                    rq[m] = oc >= 0 && r + m < rows ? static_cast<const uint16_t*>(p.res)[(int64_t)(row0 + r + m) * p.ldr + oc] : 0u;
+                }
+            }
+        };
+        if (res32 || res16) load_res(0);
+        uint16_t* y16 = static_cast<uint16_t*>(p.out) + (int64_t)row0 * p.ldo + oc;
+        float* y32 = static_cast<float*>(p.out) + (int64_t)row0 * p.ldo + oc;
+#pragma unroll 1
+        for (int r = 0; r < rows; r += 8) {
+            float v[8];
+            if (whole) {
+                load_acc(r, v);
+            } else if (staged) {
+                if (r % per == 0) {
+                    const int n4 = min(per, NT - r) / 4;
+                    for (int s = 0; s < nseg; ++s) {
+                        const float* src = part_of(s) + r / 4 * 512;
+                        for (int q = 0; q < n4; ++q)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(xs0 + ((s * (per / 4) + q) * 128 + et) * 16), "l"(src + q * 512)
+                                         : "memory");
+                    }
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    for (int s = 0; s < nseg; ++s) {
+                        const uint4 w = lds128(xs0 + ((s * (per / 4) + (r % per) / 4 + q) * 128 + et) * 16);
+                        const float f[4] = {__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w)};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[4 * q + e] = s ? v[4 * q + e] + f[e] : f[e];
+                    }
+                }
+            } else {
+                for (int s = 0; s < nseg; ++s) {
+                    const float* src = part_of(s) + r / 4 * 512;
+                    float4 w[2];
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) w[q] = __ldcg(reinterpret_cast<const float4*>(src + q * 512));
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float f[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[4 * q + e] = s ? v[4 * q + e] + f[e] : f[e];
+                    }
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[m] = v[m] * colf * colg * cols;
+            if (glu) {
+                bar_output_warps();  // (the batch before has been read)
+                if (!gate)
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) stage[m * 64 + gcol] = v[m];
+                bar_output_warps();
+                if (!gate) continue;
+#pragma unroll
+                for (int m = 0; m < 8; ++m) v[m] = act_gate(v[m], p.act) * stage[m * 64 + gcol];
+            }
+            if (f32out) {
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    if (res32) v[m] += __uint_as_float(rq[m]);
+                    if (oc >= 0 && r + m < rows) y32[(int64_t)(r + m) * p.ldo] = v[m];
+                }
+                if (res32 && r + 8 < rows) load_res(r + 8);
+            } else {
+                // two columns a store: an even lane takes both columns' even rows, its neighbour the odd ones
+#pragma unroll
+                for (int m = 0; m < 8; m += 2) {
+                    const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[m] : v[m + 1], 1);
+                    if (pair_ok) {
+                        float lo = odd ? got : v[m], hi = odd ? v[m + 1] : got;
+                        if (res16) lo += __uint_as_float(rq[m >> 1] << 16), hi += __uint_as_float(rq[m >> 1] & 0xFFFF0000u);
+                        const int rr = r + m + odd;
+                        if (rr < rows)
+                            *reinterpret_cast<uint32_t*>(y16 + (int64_t)rr * p.ldo - odd) = f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
+                    } else if (oc >= 0) {
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            if (res16) v[m + e] += bf16_bits_to_f32((uint16_t)rq[m + e]);
+                            if (r + m + e < rows) y16[(int64_t)(r + m + e) * p.ldo] = f32_to_bf16_bits(v[m + e]);
+                        }
+                    }
+                }
+                if (res16 && r + 8 < rows) load_res(r + 8);
+            }
+        }
+        if (whole) release();
+    }
+}
+
+template <int FMT, bool KWHOLE>
+__global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __grid_constant__ TkdWide p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    using F = Fmt<FMT>;
+    constexpr int CK = F::SUBSA * F::KSA, SW = 16, G = kTcGroups;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * TKD_MAX_STAGES;
+    const uint32_t xfull0 = empty0 + 8 * TKD_MAX_STAGES, xempty0 = xfull0 + 8 * TKD_WIDE_XT;
+    const uint32_t afull0 = xempty0 + 8 * TKD_WIDE_XT, aempty0 = afull0 + 8 * kWideASlots;
+    const uint32_t accfull0 = aempty0 + 8 * kWideASlots, accempty0 = accfull0 + 16;
+    static_assert(8 * (2 * TKD_MAX_STAGES + 2 * TKD_WIDE_XT + 2 * kWideASlots + 4) <= TKD_SMEM_HEAD - 32, "barriers");
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + TKD_SMEM_HEAD - 32);
+    volatile int* sflag = reinterpret_cast<volatile int*>(smem + TKD_SMEM_HEAD - 16);
+    const uint32_t xs0 = (smem_u32(smem + p.off_x) + 1023u) & ~1023u;  // (the swizzle is a function of the address)
+    const uint32_t ring0 = smem_u32(smem + p.off_ring);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (tid == 0) {
+        for (int s = 0; s < p.nstages; ++s) mbar_init(full0 + 8 * s, 1), mbar_init(empty0 + 8 * s, SW);
+        for (int s = 0; s < p.nx; ++s) mbar_init(xfull0 + 8 * s, 1), mbar_init(xempty0 + 8 * s, 1);
+        for (int s = 0; s < kWideASlots; ++s) mbar_init(afull0 + 8 * s, SW / G), mbar_init(aempty0 + 8 * s, 1);
+        for (int s = 0; s < 2; ++s) mbar_init(accfull0 + 8 * s, p.nmma), mbar_init(accempty0 + 8 * s, 4);
+        sflag[0] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem0 = *tmem_slot;
+    const int i0 = wide_begin(p, blockIdx.x), i1 = wide_begin(p, blockIdx.x + 1);
+    const int K = p.K, nst = p.nstages, NT = p.nt, nx = p.nx;
+    const bool glu2 = p.epi == TKD_EPI_GLU2;
+    const int nsa_total = (K + F::KSA - 1) / F::KSA;
+    WideSeg sg;
+
+    if (warp == kWideRing) {
+        // ---------------------------------------------------------------- producer of the weight chunks
+        uint32_t st = 0;
+        bool ok = true;
+        for (int it = i0; ok && wide_next(p, it, i1, sg);) {
+            const int panel = sg.tile / p.nrt;
+            const uint8_t* src = p.w + (int64_t)(glu2 ? panel >> 1 : panel) * p.panel_bytes;
+            const uint8_t* src2 = glu2 ? p.w2 + (int64_t)(panel >> 1) * p.panel_bytes : nullptr;
+            for (int c = sg.c0; c < sg.c1; ++c, ++st) {
+                const uint32_t s = st % nst;
+                ok = mbar_wait_parked(empty0 + 8 * s, ((st / nst) & 1) ^ 1, p.status);
+                if (!ok) break;
+                const uint32_t gbytes = (uint32_t)min(F::SUBSA, nsa_total - c * F::SUBSA) * F::SAB;  // one group's share
+                const int64_t coff = (int64_t)c * (F::SUBSA * F::SAB * 8);
+                const uint32_t dst = ring0 + s * p.stage_bytes;
+                if (lane == 0) {
+                    mbar_expect_tx(full0 + 8 * s, 8 * gbytes);
+                    if (glu2) {
+                        const int64_t hoff = coff + (int64_t)(panel & 1) * 4 * gbytes;
+                        bulk_g2s(dst, src + hoff, 4 * gbytes, full0 + 8 * s);
+                        bulk_g2s(dst + 4 * gbytes, src2 + hoff, 4 * gbytes, full0 + 8 * s);
+                    } else {
+                        bulk_g2s(dst, src + coff, 8 * gbytes, full0 + 8 * s);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        if (!ok)  // (the copies in flight land before the CTA goes)
+            for (uint32_t back = 1; back <= (uint32_t)nst && back <= st; ++back)
+                for (uint32_t i = 0; i < 64; ++i)
+                    if (mbar_try_wait(full0 + 8 * ((st - back) % nst), ((st - back) / nst) & 1)) break;
+    } else if (warp == kWideX) {
+        // ---------------------------------------------------------------- producer of the x tiles, two a unit
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const uint32_t bytes = (uint32_t)NT * 128;
+        uint32_t st = 0;
+        bool ok = true;
+        for (int it = i0; ok && wide_next(p, it, i1, sg);) {
+            const uint8_t* src = p.xt + (int64_t)(sg.tile % p.nrt) * p.nkb * bytes;
+            const int kb1 = 2 * ((min(K, sg.c1 * CK) + 127) / 128);
+            for (int kb = sg.c0 * (CK / 64); kb < kb1; ++kb, ++st) {
+                const uint32_t s = st % nx;
+                ok = mbar_wait_parked(xempty0 + 8 * s, ((st / nx) & 1) ^ 1, p.status);
+                if (!ok) break;
+                if (lane == 0) {
+                    mbar_expect_tx(xfull0 + 8 * s, bytes);
+                    bulk_g2s(xs0 + s * bytes, src + (int64_t)kb * bytes, bytes, xfull0 + 8 * s);
+                }
+                __syncwarp();
+            }
+        }
+        if (!ok)
+            for (uint32_t back = 1; back <= (uint32_t)nx && back <= st; ++back)
+                for (uint32_t i = 0; i < 64; ++i)
+                    if (mbar_try_wait(xfull0 + 8 * ((st - back) % nx), ((st - back) / nx) & 1)) break;
+    } else if (warp == 0 || warp == 2) {
+        // ---------------------------------------------------------------- MMA issue. A unit belongs to the warp of its number's
+        // parity in the CTA's sequence (so a slot's barriers are one warp's and it sees every phase of them), an accumulator
+        // to the parity within the segment.
+        const int mw = warp >> 1, nm = p.nmma;
+        if (mw < nm) {
+            const uint64_t bd0 = tc_desc(xs0);
+            const uint32_t dhi = (uint32_t)(bd0 >> 32), blo0 = (uint32_t)bd0, xstep = (uint32_t)NT * 128 >> 4;
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)NT >> 3) << 17) | ((128u >> 4) << 24);
+            uint32_t us = 0, j = 0;
+            bool ok = true;
+            for (int it = i0; ok && wide_next(p, it, i1, sg); ++j) {
+                const int kv = min(K, sg.c1 * CK) - sg.c0 * CK, nu = (kv + 127) >> 7;
+                const uint32_t set = j % p.nset;
+                ok = mbar_wait(accempty0 + 8 * set, ((j / p.nset) & 1) ^ 1, p.status);
+                if (!ok) break;
+                tc_fence_after();
+                for (int ui = nm == 2 ? (int)((mw - us) & 1u) : 0; ui < nu; ui += nm) {
+                    const uint32_t g = us + ui, ps = g % kWideASlots;
+                    ok = mbar_wait(afull0 + 8 * ps, (g / kWideASlots) & 1, p.status);
+                    if (!ok) break;
+                    const int kleft = kv - 128 * ui, nb = kleft >= 128 ? 8 : kleft >> 4;
+                    const uint32_t d = tmem0 + (set * nm + (ui & (nm - 1))) * NT;
+                    uint32_t acc = ui >= nm;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t xq = 2 * g + h, s = xq % nx;
+                        ok = ok && mbar_wait(xfull0 + 8 * s, (xq / nx) & 1, p.status);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (tc_elect()) {
+                            const uint32_t al = tmem0 + kWideA0 + ps * 64 + h * 32, bl = blo0 + s * xstep;
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) {
+                                if (4 * h + b >= nb) break;
+                                wide_mma(d, al + 8 * b, bl + 2 * b, dhi, idesc, acc);
+                                acc = 1;
+                            }
+                            tc_commit(xempty0 + 8 * s);
+                            if (h == 1) tc_commit(aempty0 + 8 * ps);
+                        }
+                        acc = 1;
+                        __syncwarp();
+                    }
+                    if (!ok) break;
+                }
+                us += nu;
+                if (ok && tc_elect()) tc_commit(accfull0 + 8 * set);
+                __syncwarp();
+            }
+        }
+    } else if (warp >= kWideDecode0 && warp < kWideDecode0 + SW) {
+        // ---------------------------------------------------------------- decode warps, as tkd_stream_tc_kernel's: two groups of
+        // eight, a unit of two tiles of 64 k is one group's; a warp stores its 16 columns' share into tensor memory
+        const int cw = warp - kWideDecode0, qtr = warp & 3, sub4 = cw >> 2, grp = sub4 >> 1, rg = 2 * qtr + (sub4 & 1), t = lane & 3;
+        constexpr int EXPB = FMT == TKD_BFP4 ? 64 : (FMT == TKD_BFP8 ? 32 : 0), UPC = CK / 128, MU = (UPC + G - 1) / G;
+        const uint2 sh = make_uint2(p.mul16, p.mul128);
+        const uint32_t alane = tmem0 + ((uint32_t)(16 * rg) << 16) + kWideA0;
+        uint32_t slot = 0, phase = 0, useq = 0;
+        auto st_a = [&](uint32_t taddr, const uint32_t* r) {
+            asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+                         "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                         : "memory");
+        };
+        // 32 k (bfloat4_b: 64 k) of the warp's columns from shared memory at `sab` to tensor-memory columns tb on
+        auto decode_sa = [&](uint32_t sab, uint32_t tb) {
+            if constexpr (FMT == TKD_BF16) {
+                const uint4 a = lds128(sab + lane * 16), b = lds128(sab + 512 + lane * 16);
+                const uint32_t r[8] = {a.x, a.z, a.y, a.w, b.x, b.z, b.y, b.w};
+                st_a(tb, r);
+            } else {
+                uint32_t cw_[4], ew_[4];
+                const uint4 cv = lds128(sab + EXPB + lane * 16);
+                cw_[0] = cv.x, cw_[1] = cv.y, cw_[2] = cv.z, cw_[3] = cv.w;
+                if constexpr (FMT == TKD_BFP8) {
+                    const uint2 ev = lds64(sab + t * 8);
+                    ew_[0] = ev.x, ew_[1] = ev.y, ew_[2] = ew_[3] = 0;
+                } else {
+                    const uint4 ev = lds128(sab + t * 16);
+                    ew_[0] = ev.x, ew_[1] = ev.y, ew_[2] = ev.z, ew_[3] = ev.w;
+                }
+#pragma unroll
+                for (int q = 0; q < F::XB; ++q) {
+                    uint32_t r[8];
+#pragma unroll
+                    for (int jj = 0; jj < 2; ++jj) {
+                        uint32_t a0, a1, a2, a3, s0, s1;
+                        if constexpr (FMT == TKD_BFP4) {
+                            const uint32_t w = cw_[2 * q + jj], tt = __funnelshift_r(w, w, 8), ew = ew_[2 * q + jj];
+                            a0 = w & TKD_MASK_BFP4, a1 = shl_fma<4>(w, sh.x) & TKD_MASK_BFP4;
+                            a2 = tt & TKD_MASK_BFP4, a3 = shl_fma<4>(tt, sh.x) & TKD_MASK_BFP4;
+                            s0 = (ew & TKD_EMASK_BFP4) | TKD_EBASE_BFP4, s1 = (shl_fma<7>(ew, sh.y) & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
+                        } else {
+                            const uint32_t w0 = cw_[2 * jj], w1 = cw_[2 * jj + 1], ew = ew_[jj];
+                            a0 = w0 & TKD_MASK_BFP8, a1 = rot_and<8>(w0, TKD_MASK_BFP8);
+                            a2 = w1 & TKD_MASK_BFP8, a3 = rot_and<8>(w1, TKD_MASK_BFP8);
+                            s0 = ew & 0x7F807F80u, s1 = rot_and<8>(ew, 0x7F807F80u);
+                        }
+                        r[4 * jj] = mul_bf16x2(a0, s0), r[4 * jj + 1] = mul_bf16x2(a2, s1);
+                        r[4 * jj + 2] = mul_bf16x2(a1, s0), r[4 * jj + 3] = mul_bf16x2(a3, s1);
+                    }
+                    st_a(tb + 16 * q, r);
+                }
+            }
+        };
+        bool ok = true;
+        for (int it = i0; ok && wide_next(p, it, i1, sg);) {
+            for (int c = sg.c0; ok && c < sg.c1; ++c) {
+                ok = mbar_wait(full0 + 8 * slot, phase, p.status);
+                if (!ok) break;
+                const int nsa = KWHOLE ? F::SUBSA : min(F::SUBSA, nsa_total - c * F::SUBSA);
+                const int ntiles = (nsa * F::KSA + 63) / 64, nunits = (ntiles + 1) >> 1;
+                const int u0 = (int)((uint32_t)grp - useq) & (G - 1);
+                const uint32_t gb = ring0 + slot * p.stage_bytes + rg * nsa * F::SAB;
+#pragma unroll
+                for (int i = 0; i < MU; ++i) {
+                    const int u = u0 + G * i;
+                    if (u >= nunits) break;
+                    const uint32_t us = useq + u, ps = us % kWideASlots;
+                    ok = mbar_wait(aempty0 + 8 * ps, ((us / kWideASlots) & 1) ^ 1, p.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t ta = alane + ps * 64;
+#pragma unroll
+                    for (int sub = 0; sub < 2; ++sub) {
+                        const int ti = 2 * u + sub;
+                        if (ti >= ntiles) break;
+                        if constexpr (FMT == TKD_BFP4) {
+                            decode_sa(gb + ti * F::SAB, ta + sub * 32);
+                        } else {
+                            decode_sa(gb + 2 * ti * F::SAB, ta + sub * 32);
+                            if (2 * ti + 1 < nsa) decode_sa(gb + (2 * ti + 1) * F::SAB, ta + sub * 32 + 16);
+                        }
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(afull0 + 8 * ps);
+                }
+                useq += nunits;
+                __syncwarp();
+                if (ok && lane == 0) mbar_arrive(empty0 + 8 * slot);
+                if (++slot == (uint32_t)nst) slot = 0, phase ^= 1;
+            }
+        }
+    } else {
+        wide_output<FMT>(p, i0, i1, tmem0, smem, accfull0, accempty0, sflag, xs0);
+    }
+    // ---- the end: everyone comes here, also after a wait that gave up
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem0), "r"(512u) : "memory");
+    }
+}
+
+template <int FMT, bool KWHOLE>
+int launch_wide(const TkdWide& p, size_t smem, cudaStream_t st) {
+    auto kern = tkd_wide_kernel<FMT, KWHOLE>;
+    static bool allowed[64] = {false};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64 || !allowed[dev]) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < 64) allowed[dev] = true;
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = p.no_pdl ? 0 : 1;
+    cfg.gridDim = dim3((unsigned)p.nkb, (unsigned)((p.nt + 63) / 64), (unsigned)p.nrt), cfg.blockDim = dim3(512);
+    e = cudaLaunchKernelEx(&cfg, tkd_wide_x_kernel, p.x, p.ldx, p.M, p.K, p.nt, p.nkb, p.xt);
+    if (e != cudaSuccess) return (int)e;
+    cfg.gridDim = dim3((unsigned)p.grid), cfg.blockDim = dim3(kWideWarps * 32), cfg.dynamicSmemBytes = smem;
+    return (int)cudaLaunchKernelEx(&cfg, kern, p);
+}
+template <int FMT>
+int launch_wide_fmt(const TkdWide& p, size_t smem, cudaStream_t st) {
+    return p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0 ? launch_wide<FMT, true>(p, smem, st) : launch_wide<FMT, false>(p, smem, st);
+}
+
+}  // namespace

@@ -169,6 +169,19 @@ def row_slices(x, full_sync=False):
     return [(m0, min(32, m - m0)) for m0 in range(0, m, 32)]
 
 
+ROWS_MAX = 2048  # rows of one launch for more than 32 (its copy of x grows with them; the weights are read once per 256 rows)
+
+
+def _launch_rows(M, fmt, topk, exchange, hadamard):
+    """[(first row, rows)] of the launches a call of M rows makes: slices of up to 32, or more where tkd_matmul_rows serves."""
+    wide = M > 32 and fmt != _tkd.FMT_INT4 and topk is None and exchange is None and hadamard is None
+    parts = -(-M // (ROWS_MAX if wide else 32))
+    if not wide:
+        return [(m0, min(32, M - m0)) for m0 in range(0, M, 32)]
+    per = -(-M // parts)
+    return [(m0, min(per, M - m0)) for m0 in range(0, M, per)]
+
+
 def _raw(t):
     return t.t if isinstance(t, ttnn.Tensor) else t
 
@@ -395,7 +408,7 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
 
     A block list in place of w, [(w | (gate, up), col0_tiles), ...]: one launch over two to four weights of one K and
     dtype, each written at its col0_tiles (in 32-column tiles); bit for bit one call per block. More than 32 rows run
-    as slices of 32, each reading the weights once."""
+    as one launch (tkd_matmul_rows), or as slices of 32 with a top-k, an exchange or an int4 stream."""
     call_key = None
     if CACHE:
         # A call described before on this weight, whatever its tensors' addresses: everything was checked then.
@@ -507,8 +520,8 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     if segs:
         _block_kw_check(device, x, blocks_all, full_sync, opts, slices)
     launches, need = [], 0
-    for m0, _ in slices:
-        a, n = _describe_rows(x, blocks_all, scale, col_scales, y, min(32, M - m0), topk, act, residual, glu, out32,
+    for m0, m in _launch_rows(M, w.fmt, topk, exchange, hadamard):
+        a, n = _describe_rows(x, blocks_all, scale, col_scales, y, m, topk, act, residual, glu, out32,
                               opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, hadamard)
         launches.append((m0, a))
         need = max(need, n)
@@ -666,7 +679,9 @@ def _describe_rows(x, entries, scale, col_scales, y, m, topk, act, residual, glu
     a = _describe(_raw(x), m, blocks, epi, act, sc, sc_up, scale_dt, None if residual is None else _raw(residual), res_dt, _raw(y),
                   topk, ks, max_ctas)
     need = ctypes.c_uint64(0)
-    _tkd.check(_tkd.lib().tkd_matmul_workspace(ctypes.byref(a), ctypes.byref(need)), "tkd_matmul_workspace")
+    L = _tkd.lib()
+    _tkd.check((L.tkd_matmul_workspace if m <= 32 else L.tkd_matmul_rows_workspace)(ctypes.byref(a), ctypes.byref(need)),
+               "tkd_matmul_workspace")
     a.hadamard = _raw(hadamard).data_ptr() if hadamard is not None else None
     a.status = status_word(device).data_ptr()
     return a, need.value

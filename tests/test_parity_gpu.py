@@ -557,3 +557,38 @@ def test_packing_in_one_pass_equals_the_passes(device, fmt, k, n):
             assert emax is None or torch.equal(t.emax, emax)
         if scaled:
             assert torch.equal(cs.float().cpu().reshape(-1), c)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
+@pytest.mark.parametrize("m,k,n", [(33, 32, 16), (64, 1024 + 96, 144), (128, 2048, 1024 + 48), (129, 96, 320), (256, 4096, 208),
+                                   (257, 512, 64), (515, 1024 + 32, 640)])
+def test_prefill_rows_and_epilogues_against_oracle(device, fmt, m, k, n):
+    """tkd_matmul_rows: every output stage at the edges of its row tiles (one and two MMA warps, one and two sets of
+    accumulators, a last tile with rows to spare), K inside a tile of 64, a unit and a chunk, N inside a panel, and few CTAs
+    (whole tiles) against all (tiles cut between them). bf16 outputs within a rounding and the fp32 sums' error; the float32
+    ones within K products of relative error 2^-24 each, added at random: 1e-5 of the result's size."""
+    g = torch.Generator().manual_seed(m + k + n)
+    w, w2 = torch.randn(n, k, generator=g) * 0.02, torch.randn(n, k, generator=g) * 0.02
+    x = torch.randn(m, k, generator=g)
+    tx = dev_x(device, x)
+    (tw, ts), (tw2, _) = linear.native_weight(device, w, DT[fmt], col_scale=True), linear.native_weight(device, w2, DT[fmt])
+    wk, wk2 = (torch.from_numpy(orc.native_values(w, fmt, col_scale=True)[0]).double(), torch.from_numpy(orc.native_values(w2, fmt)[0]).double())
+    sc = ttnn.to_torch(ts).double().reshape(-1)
+    xd = x.to(torch.bfloat16).double()
+    plain, other = (xd @ wk), xd @ wk2
+    res = torch.randn(m, n, generator=g)
+    t32 = ttnn.from_torch(res.reshape(1, 1, m, n), dtype=ttnn.float32, layout=ttnn.TILE_LAYOUT, device=device)
+    tbf = ttnn.from_torch(res.to(torch.bfloat16).reshape(1, 1, m, n), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
+    for ctas in (None, 3):
+        close_bf16(host(linear.matmul(tx, tw, ts, max_ctas=ctas)), (plain * sc).numpy())
+        y32 = host(linear.matmul(tx, tw, None, residual=t32, out32=True, max_ctas=ctas)).double()
+        want = plain + res.double()
+        assert ((y32 - want).norm() / want.norm()).item() < 1e-5
+        close_bf16(host(linear.matmul(tx, tw2, None, residual=tbf, max_ctas=ctas)), (other + res.to(torch.bfloat16).double()).numpy())
+        glu = torch.nn.functional.silu(plain) * other
+        close_bf16(host(linear.matmul(tx, tw, None, w_up=tw2, glu=True, max_ctas=ctas)), glu.numpy())
+        if n % 64 == 0:
+            act = torch.nn.functional.gelu(plain, approximate="tanh")
+            half = act.reshape(m, -1, 2, 32)[:, :, 0].reshape(m, -1) * plain.reshape(m, -1, 2, 32)[:, :, 1].reshape(m, -1)
+            close_bf16(host(linear.matmul(tx, tw, None, glu=True, glu_act=1, max_ctas=ctas)), half.numpy())
+    linear.check_status(device)
