@@ -334,28 +334,48 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
     memset(w, 0, sizeof(*w));
     TkdWide& p = *w;
     p.M = a->m, p.K = (int)a->k;
-    // rows of a tile: all of them up to 256, else as many in each tile as in the others
-    p.nrt = (p.M + 255) / 256;
-    p.nt = ((p.M + p.nrt - 1) / p.nrt + 15) / 16 * 16;
+    p.nkb = (p.K + 127) / 128 * 2;
+    const int64_t npad = tkd_padded_cols(b.n);
+    const int64_t panels = a->epilogue == TKD_EPI_GLU2 ? npad / 64 : npad / TKD_PANEL_COLS;
+    const int chunk_k = tkd_chunk_k(a->fmt);
+    p.chunks = (p.K + chunk_k - 1) / chunk_k;
+    if (a->ks % chunk_k) return TKD_ERR_BAD_ARG;
+    if (sms <= 0) sms = sm_count();
+    if (sms <= 0) sms = 148;
+    if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
+    // The rows of a tile and the blocks it is cut into, by what the kernel measured (B200, us; K 4096, bfloat8_b): a unit of 128
+    // k takes 0.55 + nt / 600 (the decode, then the traffic of x from L2); a tile's output nt / 29; a cut tile's partial sums
+    // 2 + nt / 60 to store, and nt / 26 for each part that its last CTA adds up.
+    double best = 0;
+    for (int nrt = (p.M + 255) / 256, nrt1 = (p.M + 31) / 32; nrt <= nrt1; ++nrt) {
+        const int nt = ((p.M + nrt - 1) / nrt + 15) / 16 * 16;
+        if (panels * nrt > kMaxPanels) break;
+        for (int cut = 1; cut <= 8; ++cut) {
+            const int q = a->ks ? a->ks / chunk_k < p.chunks ? a->ks / chunk_k : p.chunks : (p.chunks + cut - 1) / cut;
+            const int blocks = (p.chunks + q - 1) / q;
+            const int64_t total = panels * nrt * blocks, grid = total < sms ? total : sms;
+            const int64_t run = (total + grid - 1) / grid;
+            const double units = (double)(run * q * chunk_k) / 128;
+            // parts of a tile: one whenever runs are whole tiles
+            const int parts = total % grid == 0 && run % blocks == 0 ? 1 : (int)((blocks + run - 2) / run) + 1;
+            const double us = units * (0.55 + nt / 600.) + (double)((run + blocks - 1) / blocks) * nt / 29. +
+                              (parts > 1 ? 2 + nt / 60. + (parts - 1) * nt / 26. : 0);
+            if (best == 0 || us < best) {
+                best = us;
+                p.nrt = nrt, p.nt = nt, p.q = q, p.blocks = blocks, p.total = (int)total, p.grid = (int)grid;
+            }
+            if (a->ks) break;
+        }
+    }
+    if (best == 0) return TKD_ERR_UNSUPPORTED;
     // (an MMA of up to 128 rows is shorter than its issue: two warps, an accumulator each)
     p.nmma = p.nt <= 128 ? 2 : 1;
     p.nset = p.nmma * p.nt * 2 <= 256 ? 2 : 1;
     p.nx = p.nt <= 128 ? 8 : 4;
-    p.nkb = (p.K + 127) / 128 * 2;
-    const int64_t npad = tkd_padded_cols(b.n);
-    const int64_t panels = a->epilogue == TKD_EPI_GLU2 ? npad / 64 : npad / TKD_PANEL_COLS;
-    p.chunks = (p.K + tkd_chunk_k(a->fmt) - 1) / tkd_chunk_k(a->fmt);
-    const int64_t total = panels * p.nrt * p.chunks;
-    if (panels * p.nrt > kMaxPanels || total > (1 << 30)) return TKD_ERR_UNSUPPORTED;
-    p.total = (int)total;
-    if (sms <= 0) sms = sm_count();
-    if (sms <= 0) sms = 148;
-    if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
-    p.grid = (int)(total < sms ? total : sms);
     p.panel_bytes = tkd_panel_bytes(a->fmt, a->k);
     p.stage_bytes = 8 * tkd_subsa(a->fmt) * tkd_sab(a->fmt);
     p.off_stage = TKD_SMEM_HEAD;
-    p.off_x = p.off_stage + 8 * 64 * 4;
+    p.off_x = p.off_stage + 16 * 64 * 4;
     p.off_ring = (int)align_up(p.off_x + 1023 + p.nx * p.nt * 128, 128);
     p.nstages = (kMaxSmem - p.off_ring) / p.stage_bytes;
     if (p.nstages > TKD_MAX_STAGES) p.nstages = TKD_MAX_STAGES;

@@ -108,7 +108,8 @@ struct TkdWide {
     int n_valid, out_col0;
     int M, K;
     int nt, nrt;        // rows of a tile (a multiple of 16, at most 256), row tiles
-    int chunks, total;  // chunks of K a tile; chunks of all tiles
+    int chunks;         // chunks of K a tile
+    int q, blocks, total;  // chunks a block; blocks a tile, of all tiles
     int grid;
     int64_t panel_bytes;
     const uint16_t* x;

@@ -13,19 +13,20 @@
 //   tkd_wide_kernel    warp 0 (and 2)  one lane issues the MMAs, A from tensor memory, B from shared memory. Up to 128 rows
 //                                      two warps share the units (of 128 k): an MMA of few rows is shorter than its issue.
 //                      warp 1          producer of the ring of weight chunks; warp 3: of the x tiles
-//                      warps 4-19      decode: tkd_stream_tc_kernel's, without the activations
-//                      warps 20-23     output: a thread is a column (a tensor-memory lane)
+//                      warps 4-7       output: a thread is a column (a tensor-memory lane). Before the decode warps: the
+//                                      schedulers favour older warps, and the next tile waits for these to free its accumulators
+//                      warps 8-23      decode: tkd_stream_tc_kernel's, without the activations
 //
 // Work split: tiles are numbered panel-major (the tiles of a panel run at the same time on different SMs and share its
-// chunks in L2), each of `chunks` chunks of K; all chunks are cut into equal contiguous runs, one per CTA. A tile that is
-// cut goes through scratch, a partial sum per CTA, and the CTA that delivers last adds them up in order of k: with 224 tiles
-// on 148 SMs (512 rows of the weight above) whole tiles would leave a quarter of the machine idle.
+// chunks in L2), each cut into `blocks` blocks of q chunks of K; all blocks are dealt out in equal contiguous runs, one per
+// CTA. A tile whose blocks fall to several CTAs goes through scratch, a partial sum per CTA, and the one that delivers last
+// adds them up in order of k. How many rows a tile has and how fine it is cut is the host's choice (make_wide).
 #pragma once
 #include "tkd_stream_tc.cuh"
 
 namespace {
 
-constexpr int kWideWarps = 24, kWideRing = 1, kWideX = 3, kWideDecode0 = 4, kWideOut0 = 20;
+constexpr int kWideWarps = 24, kWideRing = 1, kWideX = 3, kWideDecode0 = 8;
 constexpr int kWideASlots = 4;                    // units of A in tensor memory, 64 columns each
 constexpr int kWideA0 = 256;                      // their first column: the accumulators have 0-255
 static_assert(kWideA0 + kWideASlots * 64 <= 512, "tensor memory");
@@ -57,23 +58,54 @@ __device__ __forceinline__ void wide_mma(uint32_t d, uint32_t a, uint32_t blo, u
         : "memory");
 }
 
+// Stores under a predicate instead of a branch: the output stage is one warp a scheduler, and every branch costs it an
+// instruction fetch (about 80 cycles; eight of them a batch of rows were most of the stage).
+__device__ __forceinline__ void st_if(bool ok, void* at, uint32_t v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b32 [%0], %1;\n\t}" ::"l"(at), "r"(v), "r"((uint32_t)ok) : "memory");
+}
+__device__ __forceinline__ void st16_if(bool ok, void* at, uint16_t v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(at), "h"(v), "r"((uint32_t)ok) : "memory");
+}
+// two floats as a bf16 pair, the first in the lower half
+__device__ __forceinline__ uint32_t f32x2_to_bf16x2(float lo, float hi) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
+
 // A part of a CTA's run that lies in one tile.
 struct WideSeg {
     int tile, c0, c1;  // chunks c0 .. c1 - 1 of the tile
 };
 __device__ __forceinline__ bool wide_next(const TkdWide& p, int& it, int i1, WideSeg& s) {
     if (it >= i1) return false;
-    s.tile = it / p.chunks;
-    s.c0 = it - s.tile * p.chunks;
-    s.c1 = min(p.chunks, s.c0 + i1 - it);
-    it += s.c1 - s.c0;
+    s.tile = it / p.blocks;
+    const int b0 = it - s.tile * p.blocks, b1 = min(p.blocks, b0 + i1 - it);
+    s.c0 = b0 * p.q, s.c1 = min(p.chunks, b1 * p.q);
+    it += b1 - b0;
     return true;
 }
 __device__ __forceinline__ int wide_begin(const TkdWide& p, int cta) { return (int)((int64_t)p.total * cta / p.grid); }
 // the CTA whose run holds item i
 __device__ __forceinline__ int wide_owner(const TkdWide& p, int i) { return (int)((((int64_t)i + 1) * p.grid - 1) / p.total); }
 
-// The output warps: a thread is the column et of its tile's panel. Rows go in batches of 8 (of 16: 600 bytes of spills).
+__device__ __forceinline__ void tmem_ld16(uint32_t at, uint32_t (&q)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]), "=r"(q[9]),
+                   "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+                 : "r"(at)
+                 : "memory");
+}
+// (the registers named, so that nothing reads them before the wait)
+__device__ __forceinline__ void tmem_wait16(uint32_t (&q)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]), "+r"(q[7]), "+r"(q[8]), "+r"(q[9]),
+                   "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15])
+                 :
+                 : "memory");
+}
+
+// The output warps: a thread is the column et of its tile's panel. Rows go in batches of 16.
 template <int FMT>
 __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, uint32_t tmem0, uint8_t* smem, uint32_t accfull0,
                                             uint32_t accempty0, volatile int* sflag, uint32_t xs0) {
@@ -83,7 +115,7 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
     const int NT = p.nt, nm = p.nmma;
     const bool glu2 = p.epi == TKD_EPI_GLU2, glu = glu2 || p.epi == TKD_EPI_GLU_IL;
     const bool f32out = p.epi == TKD_EPI_OUT32, res32 = f32out && p.res, res16 = p.epi == TKD_EPI_RESIDUAL;
-    float* stage = reinterpret_cast<float*>(smem + p.off_stage);  // GLU: [8 rows][64 columns] of the up half
+    float* stage = reinterpret_cast<float*>(smem + p.off_stage);  // GLU: [16 rows][64 columns] of the up half
     // GLU: the warps of a panel's gate columns (interleaved: 32 gate, their 32 up, ...; two weights: 64 and 64)
     const bool gate = glu2 ? ow < 2 : (ow & 1) == 0;
     const int gcol = glu2 ? (ow & 1) * 32 + lane : (ow >> 1) * 32 + lane;  // the column within the tile's 64 outputs
@@ -93,14 +125,14 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
         const int panel = sg.tile / p.nrt, rt = sg.tile - panel * p.nrt;
         const int n = glu2 ? (panel >> 1) * 128 + (panel & 1) * 64 + (et & 63) : panel * 128 + et;  // the column of its weight
         const bool in_w = n < p.n_valid;
-        float colf = 1.f, colg = 1.f, cols = 1.f;
+        float colf = 1.f, colg = 1.f;  // the column's factor: 2^e of its group in two normal floats, times its scale
         if constexpr (FMT != TKD_BF16) {
             const int e = tkd_out_exp(FMT, (glu2 && et >= 64 ? p.emax2 : p.emax)[n >> 4]), e1 = e / 2, e2 = e - e1;
             colf = __uint_as_float((uint32_t)(e1 + 127) << 23), colg = __uint_as_float((uint32_t)(e2 + 127) << 23);
         }
         if (p.scale_dt != TKD_DT_NONE && in_w) {
             const void* sp = glu2 && et >= 64 ? p.scale2 : p.scale;
-            cols = p.scale_dt == TKD_DT_BF16 ? bf16_bits_to_f32(static_cast<const uint16_t*>(sp)[n]) : static_cast<const float*>(sp)[n];
+            colg *= p.scale_dt == TKD_DT_BF16 ? bf16_bits_to_f32(static_cast<const uint16_t*>(sp)[n]) : static_cast<const float*>(sp)[n];
         }
         // the output column this thread stores, or -1
         int oc = -1;
@@ -118,167 +150,196 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
         if (!mbar_wait_parked(accfull0 + 8 * set, (j / p.nset) & 1, p.status)) return;
         tc_fence_after();
         const uint32_t ta = tmem0 + ((uint32_t)(ow * 32) << 16) + set * nm * NT;
-        // eight rows of the segment's sums
-        auto load_acc = [&](int r, float (&v)[8]) {
-            uint32_t a[8], b[8];
-            auto ld = [&](uint32_t at, uint32_t (&q)[8]) {
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                             : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
-                             : "r"(at)
-                             : "memory");
-            };
-            ld(ta + r, a);
-            if (two) ld(ta + NT + r, b);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        // sixteen rows of the segment's sums
+        auto sums = [&](int r, float (&v)[16]) {
+            uint32_t a[16], b[16];
+            tmem_ld16(ta + r, a);
+            if (two) tmem_ld16(ta + NT + r, b);
+            tmem_wait16(a);
+            if (two) {
+                tmem_wait16(b);
 #pragma unroll
-            for (int m = 0; m < 8; ++m) v[m] = two ? __uint_as_float(a[m]) + __uint_as_float(b[m]) : __uint_as_float(a[m]);
+                for (int m = 0; m < 16; ++m) v[m] = __uint_as_float(a[m]) + __uint_as_float(b[m]);
+            } else {
+#pragma unroll
+                for (int m = 0; m < 16; ++m) v[m] = __uint_as_float(a[m]);
+            }
         };
         auto release = [&]() {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(accempty0 + 8 * set);
         };
-        // partial sums in scratch: [segment][row / 4][column][4]
+        // ---- a cut tile: partial sums in scratch, [segment][row / 4][column][4]. The later of two CTAs adds the other's to its
+        // own, still in tensor memory, without storing that; of more than two each stores its own, and the last adds them all.
         const int64_t part = (int64_t)NT * 128;
-        int b0 = 0, nseg = 1;
-        bool staged = false;  // the partial sums are copied into the (then idle) x tiles first
-        int per = 0;          // ... so many rows at a time
-        if (!whole) {
-            float* dst = p.scratch + ((int64_t)blockIdx.x * 2 + (wide_begin(p, blockIdx.x) < sg.tile * p.chunks ? 1 : 0)) * part + et * 4;
-#pragma unroll 1
-            for (int r = 0; r < rows; r += 8) {
-                float v[8];
-                load_acc(r, v);
-#pragma unroll
-                for (int q = 0; q < 2; ++q)
-                    __stcg(reinterpret_cast<float4*>(dst + (r / 4 + q) * 512), make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
-            }
-            release();
-            b0 = wide_owner(p, sg.tile * p.chunks);
-            nseg = wide_owner(p, sg.tile * p.chunks + p.chunks - 1) - b0 + 1;
-            bar_output_warps();  // (orders the 128 threads' stores before thread 0's release)
-            if (et == 0) {
-                const int last = atom_add_acq_rel(p.counters + sg.tile, 1) + 1 == nseg;
-                if (last) p.counters[sg.tile] = 0;
-                sflag[0] = last;
-            }
-            bar_output_warps();
-            const bool finish = sflag[0] != 0;
-            bar_output_warps();  // (sflag may be written again only after everyone has read it)
-            if (!finish) continue;
-            per = p.nx * NT * 128 / (nseg * 512) & ~7;
-            staged = it >= i1 && per >= 8;  // (this CTA's last tile: every x tile has been multiplied)
-        }
-        // where segment s of the tile left its sums
+        const int b0 = whole ? 0 : wide_owner(p, sg.tile * p.blocks);
+        const int nseg = whole ? 1 : wide_owner(p, sg.tile * p.blocks + p.blocks - 1) - b0 + 1, own = (int)blockIdx.x - b0;
+        // where segment s of the tile leaves its sums
         auto part_of = [&](int s) {
-            const int b = b0 + s;
-            return p.scratch + ((int64_t)b * 2 + (wide_begin(p, b) < sg.tile * p.chunks ? 1 : 0)) * part + et * 4;
+            return p.scratch + ((int64_t)(b0 + s) * 2 + (wide_begin(p, b0 + s) < sg.tile * p.blocks ? 1 : 0)) * part + et * 4;
         };
-        // the residual of a batch, asked for a batch ahead: float32 a row, or bf16 a pair of columns of every other row
+        bool staged = false;  // the other parts are copied into the (then idle) x tiles first, `per` rows at a time
+        int per = 0;
+        if (!whole) {
+            bool last = false;
+            if (nseg == 2) {
+                if (et == 0) sflag[0] = atom_add_acq_rel(p.counters + sg.tile, 0) == 1;
+                bar_output_warps();
+                last = sflag[0] != 0;
+                bar_output_warps();  // (sflag may be written again only after everyone has read it)
+            }
+            if (!last) {
+                float* dst = part_of(own);
+#pragma unroll 1
+                for (int r = 0; r < rows; r += 16) {
+                    float v[16];
+                    sums(r, v);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        __stcg(reinterpret_cast<float4*>(dst + r * 128 + q * 512), make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+                }
+                bar_output_warps();  // (orders the 128 threads' stores before thread 0's release)
+                if (et == 0) sflag[0] = atom_add_acq_rel(p.counters + sg.tile, 1) == nseg - 1;
+                bar_output_warps();
+                last = sflag[0] != 0;
+                bar_output_warps();
+            }
+            if (!last) {
+                release();
+                continue;
+            }
+            if (et == 0) p.counters[sg.tile] = 0;
+            per = p.nx * NT * 128 / ((nseg == 2 ? 1 : nseg) * 512) & ~15;
+            staged = it >= i1 && per >= 16;  // (this CTA's last tile: every x tile has been multiplied)
+        }
+        // ---- the output stage, sixteen rows at a time (a warp has its scheduler nearly to itself here: the loop is bound by the
+        // latency of its chains, so the rows go side by side; eight at a time a tile of 256 rows took twice as long)
         const bool odd = lane & 1;
         const bool pairs = !f32out && !((reinterpret_cast<uintptr_t>(p.out) & 3) | (p.ldo & 1) | (p.out_col0 & 1)) &&
                            !(res16 && ((reinterpret_cast<uintptr_t>(p.res) & 3) | (p.ldr & 1)));
-        const bool pair_ok = pairs && __shfl_xor_sync(0xFFFFFFFFu, oc, 1) >= 0 && oc >= 0;
+        const bool fast = __all_sync(0xFFFFFFFFu, pairs && oc >= 0);  // (two columns a store)
+        const uint32_t pick = odd ? 0x3276u : 0x5410u;  // (own word first: an even lane both lower halves, an odd one both upper)
+        // fast, with a residual: the pairs of columns of every other row of a batch, asked for a batch ahead
         uint32_t rq[8];
         auto load_res = [&](int r) {
+            const uint16_t* rp = static_cast<const uint16_t*>(p.res) + (int64_t)(row0 + r + odd) * p.ldr + oc - odd;
 #pragma unroll
             for (int m = 0; m < 8; ++m) {
-                if (res32) {
-                    rq[m] = oc >= 0 && r + m < rows ? __float_as_uint(static_cast<const float*>(p.res)[(int64_t)(row0 + r + m) * p.ldr + oc]) : 0u;
-                } else if (pair_ok) {
-                    if (m < 4) {
-                        const int rr = r + 2 * m + odd;
-                        rq[m] = rr < rows ? *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.res) + (int64_t)(row0 + rr) * p.ldr + oc - odd) : 0u;
-                    }
-                } else {
-                    rq[m] = oc >= 0 && r + m < rows ? static_cast<const uint16_t*>(p.res)[(int64_t)(row0 + r + m) * p.ldr + oc] : 0u;
-                }
+                // (a row past the last reads the last of its kind again)
+                rq[m] = *reinterpret_cast<const uint32_t*>(rp);
+                if (r + 2 * m + 2 + odd < rows) rp += 2 * p.ldr;
             }
         };
-        if (res32 || res16) load_res(0);
+        if (fast && res16 && odd < rows) load_res(0);
         uint16_t* y16 = static_cast<uint16_t*>(p.out) + (int64_t)row0 * p.ldo + oc;
-        float* y32 = static_cast<float*>(p.out) + (int64_t)row0 * p.ldo + oc;
+        int staged_from = 0, staged_to = 0;  // the rows whose other parts lie in the x tiles
 #pragma unroll 1
-        for (int r = 0; r < rows; r += 8) {
-            float v[8];
-            if (whole) {
-                load_acc(r, v);
-            } else if (staged) {
-                if (r % per == 0) {
-                    const int n4 = min(per, NT - r) / 4;
-                    for (int s = 0; s < nseg; ++s) {
-                        const float* src = part_of(s) + r / 4 * 512;
-                        for (int q = 0; q < n4; ++q)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(xs0 + ((s * (per / 4) + q) * 128 + et) * 16), "l"(src + q * 512)
-                                         : "memory");
+        for (int r = 0; r < rows; r += 16) {
+            float v[16];
+            if (staged && r >= staged_to) {
+                staged_from = r, staged_to = r + per;
+                const int n4 = min(per, NT - r) / 4;
+                for (int s = nseg == 2 ? 1 - own : 0, i = 0; s < nseg && (nseg > 2 || i == 0); ++s, ++i) {
+                    const float* src = part_of(s) + r * 128;
+                    const uint32_t dst = xs0 + (i * (per / 4) * 128 + et) * 16;
+#pragma unroll 8
+                    for (int q = 0; q < n4; ++q)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + q * 2048), "l"(src + q * 512) : "memory");
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+            }
+            // + sixteen rows of the i-th part that is added here, segment s's
+            auto add = [&](int s, int i) {
+                float4 f[4];
+                if (staged) {
+                    const uint32_t at = xs0 + ((i * (per / 4) + (r - staged_from) / 4) * 128 + et) * 16;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint4 w = lds128(at + 2048 * q);
+                        f[q] = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
                     }
-                    asm volatile("cp.async.wait_all;" ::: "memory");
+                } else {
+                    const float4* src = reinterpret_cast<const float4*>(part_of(s) + r * 128);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) f[q] = __ldcg(src + 128 * q);
                 }
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    for (int s = 0; s < nseg; ++s) {
-                        const uint4 w = lds128(xs0 + ((s * (per / 4) + (r % per) / 4 + q) * 128 + et) * 16);
-                        const float f[4] = {__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w)};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) v[4 * q + e] = s ? v[4 * q + e] + f[e] : f[e];
-                    }
-                }
+                for (int q = 0; q < 4; ++q) v[4 * q] += f[q].x, v[4 * q + 1] += f[q].y, v[4 * q + 2] += f[q].z, v[4 * q + 3] += f[q].w;
+            };
+            if (nseg <= 2) {
+                sums(r, v);
+                if (nseg == 2) add(1 - own, 0);  // (which of two terms comes first does not matter)
             } else {
-                for (int s = 0; s < nseg; ++s) {
-                    const float* src = part_of(s) + r / 4 * 512;
-                    float4 w[2];
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) w[q] = __ldcg(reinterpret_cast<const float4*>(src + q * 512));
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const float f[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) v[4 * q + e] = s ? v[4 * q + e] + f[e] : f[e];
-                    }
-                }
+                for (int m = 0; m < 16; ++m) v[m] = 0.f;
+#pragma unroll 1
+                for (int s = 0; s < nseg; ++s) add(s, s);  // in order of k
             }
 #pragma unroll
-            for (int m = 0; m < 8; ++m) v[m] = v[m] * colf * colg * cols;
+            for (int m = 0; m < 16; ++m) v[m] = v[m] * colf * colg;
             if (glu) {
                 bar_output_warps();  // (the batch before has been read)
                 if (!gate)
 #pragma unroll
-                    for (int m = 0; m < 8; ++m) stage[m * 64 + gcol] = v[m];
+                    for (int m = 0; m < 16; ++m) stage[m * 64 + gcol] = v[m];
                 bar_output_warps();
                 if (!gate) continue;
 #pragma unroll
-                for (int m = 0; m < 8; ++m) v[m] = act_gate(v[m], p.act) * stage[m * 64 + gcol];
+                for (int m = 0; m < 16; ++m) v[m] = act_gate(v[m], p.act) * stage[m * 64 + gcol];
             }
-            if (f32out) {
+            if (fast) {
+                // an even lane stores both columns of the even rows, its neighbour those of the odd ones
+                uint16_t* yp = y16 + (int64_t)(r + odd) * p.ldo - odd;
+                const int left = rows - r - odd;  // (rows from this lane's first on)
+                uint32_t w[8];
+                if (!res16) {
 #pragma unroll
-                for (int m = 0; m < 8; ++m) {
-                    if (res32) v[m] += __uint_as_float(rq[m]);
-                    if (oc >= 0 && r + m < rows) y32[(int64_t)(r + m) * p.ldo] = v[m];
-                }
-                if (res32 && r + 8 < rows) load_res(r + 8);
-            } else {
-                // two columns a store: an even lane takes both columns' even rows, its neighbour the odd ones
-#pragma unroll
-                for (int m = 0; m < 8; m += 2) {
-                    const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[m] : v[m + 1], 1);
-                    if (pair_ok) {
-                        float lo = odd ? got : v[m], hi = odd ? v[m + 1] : got;
-                        if (res16) lo += __uint_as_float(rq[m >> 1] << 16), hi += __uint_as_float(rq[m >> 1] & 0xFFFF0000u);
-                        const int rr = r + m + odd;
-                        if (rr < rows)
-                            *reinterpret_cast<uint32_t*>(y16 + (int64_t)rr * p.ldo - odd) = f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
-                    } else if (oc >= 0) {
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            if (res16) v[m + e] += bf16_bits_to_f32((uint16_t)rq[m + e]);
-                            if (r + m + e < rows) y16[(int64_t)(r + m + e) * p.ldo] = f32_to_bf16_bits(v[m + e]);
-                        }
+                    for (int m = 0; m < 8; ++m) {
+                        const uint32_t mine = f32x2_to_bf16x2(v[2 * m], v[2 * m + 1]);
+                        w[m] = __byte_perm(mine, __shfl_xor_sync(0xFFFFFFFFu, mine, 1), pick);
                     }
+                } else {
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) {
+                        const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[2 * m] : v[2 * m + 1], 1);
+                        const float lo = odd ? got : v[2 * m], hi = odd ? v[2 * m + 1] : got;
+                        w[m] = f32x2_to_bf16x2(lo + __uint_as_float(rq[m] << 16), hi + __uint_as_float(rq[m] & 0xFFFF0000u));
+                    }
+                    if (r + 16 + odd < rows) load_res(r + 16);
                 }
-                if (res16 && r + 8 < rows) load_res(r + 8);
+#pragma unroll
+                for (int m = 0; m < 8; ++m, yp += 2 * p.ldo) st_if(2 * m < left, yp, w[m]);
+            } else if (f32out && !res32) {
+                float* yp = static_cast<float*>(p.out) + (int64_t)(row0 + r) * p.ldo + oc;
+                const int left = oc >= 0 ? rows - r : 0;
+#pragma unroll
+                for (int m = 0; m < 16; ++m, yp += p.ldo) st_if(m < left, yp, __float_as_uint(v[m]));
+            } else if (oc >= 0) {
+                int64_t at = (int64_t)(row0 + r) * p.ldo + oc, ra = (int64_t)(row0 + r) * p.ldr + oc;
+                const int esz = f32out ? 4 : 2, rsz = res32 ? 4 : 2;
+                char *yp = static_cast<char*>(p.out) + at * esz;
+                const char* rp = static_cast<const char*>(p.res) + ra * rsz;
+                uint32_t q[16];
+                if (res32 || res16) {
+#pragma unroll
+                    for (int m = 0; m < 16; ++m) {
+                        q[m] = res32 ? *reinterpret_cast<const uint32_t*>(rp) : (uint32_t)*reinterpret_cast<const uint16_t*>(rp) << 16;
+                        if (r + m + 1 < rows) rp += p.ldr * rsz;
+                    }
+#pragma unroll
+                    for (int m = 0; m < 16; ++m) v[m] += __uint_as_float(q[m]);
+                }
+#pragma unroll
+                for (int m = 0; m < 16; ++m, yp += p.ldo * esz) {
+                    if (f32out)
+                        st_if(r + m < rows, yp, __float_as_uint(v[m]));
+                    else
+                        st16_if(r + m < rows, yp, f32_to_bf16_bits(v[m]));
+                }
             }
         }
-        if (whole) release();
+        release();
     }
 }
 
