@@ -365,9 +365,10 @@ __global__ void __launch_bounds__(pack_threads(SCALE)) tkd_pack_weight_kernel(co
             load8(v[1][q], n1, in1, sa * KSA + 32 * q + 8 * t);
         }
         if constexpr (SCALE != 0) {
-            // (own scales) v / d correctly rounded from the correctly rounded reciprocal r: q = v r, then q + (v - q d) r
-            // (P. Markstein, IBM J. Res. Dev. 34, 1990; a bf16 divisor is not the exceptional one whose significand bits are
-            // all set). It needs v - q d exact: a block whose largest quotients lie near the denormals is divided again below.
+            // (own scales) v / d correctly rounded: q = v r, r the rounded reciprocal, then q + (v - q d) r (P. Markstein, IBM J. Res.
+            // Dev. 34, 1990). q is within 1.5 units of its last place, d has 8 significant bits: v - q d is exact, the last sum
+            // is v / d within 2^-23 units, and a quotient by such a d lies at least 2^-9 units from where rounding changes.
+            // It needs v - q d in the normal numbers: a block whose largest quotients lie near the denormals is divided below.
             if (SCALE == 2 && FMT != TKD_BF16 && !slow) {
 #pragma unroll
                 for (int q = 0; q < XB; ++q)

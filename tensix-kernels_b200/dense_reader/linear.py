@@ -82,6 +82,7 @@ _CALLS_MAX = 256
 _WEIGHT_CALLS = 64  # described calls kept with a weight, at most
 _CHOICE = {}     # the plan cache
 _WORKSPACE = {}  # device id -> zeroed uint8 tensor
+_OUTGROWN = []   # workspaces replaced by larger ones
 _STATUS = {}     # device id -> int32 status word
 
 
@@ -197,7 +198,11 @@ def _ws_key(device):
 def _workspace(device, nbytes):
     ws = _WORKSPACE.get(_ws_key(device))
     if ws is None or ws.numel() < nbytes:
-        # (zeroed once: the kernel leaves its counters at zero)
+        # (zeroed once: the kernel leaves its counters at zero. The one outgrown stays alive for the CUDA graphs that hold its
+        # address; sizes at least double, so all of them together are smaller than twice the last)
+        if ws is not None:
+            _OUTGROWN.append(ws)
+            nbytes = max(nbytes, 2 * ws.numel())
         ws = _WORKSPACE[_ws_key(device)] = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device.torch)
     return ws
 
@@ -418,7 +423,7 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
             y = call.run(x, out, opts.get("residual"))
             return out if out is not None else ttnn.Tensor(y, call.out_dtype, ttnn.TILE_LAYOUT, call.device, memory_config)
     y, call = _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0, w_up, max_banks, opts)
-    if call_key is not None and call.exchange is None:
+    if call_key is not None:
         if len(first.calls) >= _WEIGHT_CALLS:
             first.calls.clear()
         first.calls[call_key] = call

@@ -592,3 +592,28 @@ def test_prefill_rows_and_epilogues_against_oracle(device, fmt, m, k, n):
             half = act.reshape(m, -1, 2, 32)[:, :, 0].reshape(m, -1) * plain.reshape(m, -1, 2, 32)[:, :, 1].reshape(m, -1)
             close_bf16(host(linear.matmul(tx, tw, None, glu=True, glu_act=1, max_ctas=ctas)), half.numpy())
     linear.check_status(device)
+
+
+def test_graph_keeps_its_workspace(device):
+    """A captured call replays rightly after larger calls have outgrown its workspace, whose memory others may have by then."""
+    g = torch.Generator().manual_seed(96)
+    k, n = 4096, 1024 + 128
+    tw, _ = linear.native_weight(device, torch.randn(n, k, generator=g) * 0.02, ttnn.bfloat8_b)
+    slot, linear.WORKSPACE_SLOT = linear.WORKSPACE_SLOT, "graph"
+    try:
+        x = dev_x(device, torch.randn(2, k, generator=g))
+        want = host(linear.matmul(x, tw, None)).clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = linear.matmul(x, tw, None)
+        before = linear._WORKSPACE[(device.id, "graph")].numel()
+        linear.matmul(dev_x(device, torch.randn(300, k, generator=g)), tw, None)
+        assert linear._WORKSPACE[(device.id, "graph")].numel() >= 2 * before
+        junk = [torch.full((1 << 20,), 7, dtype=torch.int32, device=device.torch) for _ in range(8)]
+        y.t.zero_()
+        graph.replay()
+        assert torch.equal(host(y), want)
+        del junk, graph
+    finally:
+        linear.WORKSPACE_SLOT = slot
+    linear.check_status(device)
