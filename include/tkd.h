@@ -272,16 +272,21 @@ typedef struct {
                                 b) * (x U + b); down: the n columns of y = sum over the slots of h_q @ D_q */
     int64_t ldo;
     void* workspace;         /* down: tkd_moe_workspace bytes, zeroed once by the caller before the first use (the kernel
-                                returns its counters to zero); calls that share one must be ordered on one stream */
+                                returns its counters to zero); calls that share one must be ordered on one stream. by_union:
+                                tkd_moe_rows_workspace bytes, for gate_up too (one of its own; with none, or too little, its
+                                work is spread over the SMs less evenly; down then runs fewer CTAs) */
     uint64_t workspace_bytes;
     int32_t fmt;             /* TKD_FMT_BFP4, or TKD_FMT_BF16: experts whose values no bfloat4_b stream holds (the K-block
                                 layout, moe8.py:507-527 kblock: shared exponents along K), kept exactly at 2 bytes a weight;
                                 emax is then unused */
+    int32_t out_rows;        /* by_union: rows of out; those from `rows` on are written with zeros (0: none) */
+    int32_t* status;         /* by_union: one int32 (or NULL): TKD_ERR_TIMEOUT is written here if a wait gives up */
 } TkdMoe;
 
 int tkd_moe_workspace(const TkdMoe* a, uint64_t* bytes);
-/* Rows whose activations do not fit in shared memory together are taken in passes (the experts' weights are read again
- * for each, from L2). TKD_ERR_UNSUPPORTED: not even one row of k_in inputs fits. */
+/* The workspace of a by_union call of gate_up (down 0) or down, whatever its slots: for a->experts, n and rows. */
+int tkd_moe_rows_workspace(const TkdMoe* a, int down, uint64_t* bytes);
+/* TKD_ERR_UNSUPPORTED: one row of k_in inputs does not fit in shared memory (by_union: never). */
 int tkd_moe_gate_up(const TkdMoe* a, void* stream);
 int tkd_moe_down(const TkdMoe* a, void* stream);
 /* The router's top k and their weights, into the ids and weights the ops above read: stands in for moe8.route

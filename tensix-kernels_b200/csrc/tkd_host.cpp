@@ -88,8 +88,8 @@ PyObject* host_matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
 }
 
-// moe(descriptor's address, x, ids, routing weights (gate_up) or None (down), workspace (down) or None) -> the output:
-// bf16 [1, 1, 1, ldo], or with by_union [1, 1, 32, ldo] with zeros in the rows past the descriptor's.
+// moe(descriptor's address, x, ids, routing weights (gate_up) or None (down), workspace or None) -> the output: bf16
+// [1, 1, 1, ldo], or with by_union [1, 1, 32, ldo] (the kernel writes zeros into the rows past the descriptor's).
 PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 5 || !all_tensors(args, {1, 2}, {3, 4})) return type_error("tkd_host.moe: descriptor, x, ids, w, workspace");
     const auto* desc = static_cast<const TkdMoe*>(PyLong_AsVoidPtr(args[0]));
@@ -108,10 +108,6 @@ PyObject* host_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (w) a.route_w = w->data_ptr(), a.ld_w = w->stride(-2);
         if (ws) a.workspace = ws->data_ptr(), a.workspace_bytes = (uint64_t)ws->nbytes();
         a.out = out.data_ptr();
-        if (a.by_union && a.rows < 32) {
-            const cudaError_t e = cudaMemsetAsync(static_cast<char*>(a.out) + (size_t)a.rows * a.ldo * 2, 0, (size_t)(32 - a.rows) * a.ldo * 2, stream);
-            if (e != cudaSuccess) return tkd_error(TKD_ERR_CUDA + (int)e, "cudaMemsetAsync");
-        }
         int rc;
         Py_BEGIN_ALLOW_THREADS rc = w ? tkd_moe_gate_up(&a, stream) : tkd_moe_down(&a, stream);
         Py_END_ALLOW_THREADS if (rc) return tkd_error(rc, w ? "tkd_moe_gate_up" : "tkd_moe_down");

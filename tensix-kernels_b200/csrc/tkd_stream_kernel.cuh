@@ -160,6 +160,15 @@ __device__ __forceinline__ void bar_output_warps() { asm volatile("bar.sync 1, 1
 __device__ __forceinline__ float bf16_bits_to_f32(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 __device__ __forceinline__ uint16_t f32_to_bf16_bits(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
 
+// Stores under a predicate instead of a branch: an output stage is one warp a scheduler, and every branch costs it an
+// instruction fetch (about 80 cycles; eight of them a batch of rows were most of the prefill kernel's).
+__device__ __forceinline__ void st_if(bool ok, void* at, uint32_t v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b32 [%0], %1;\n\t}" ::"l"(at), "r"(v), "r"((uint32_t)ok) : "memory");
+}
+__device__ __forceinline__ void st16_if(bool ok, void* at, uint16_t v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(at), "h"(v), "r"((uint32_t)ok) : "memory");
+}
+
 // dense_ops.h:44-59 of the reference: silu, and gelu_tanh as x * sigmoid(2 u), u = sqrt(2 / pi) (x + 0.044715 x^3)
 __device__ __forceinline__ float act_gate(float g, int act) {
     const float u = act ? g * (1.5957691216f + 0.0713548162f * (g * g)) : g;

@@ -58,14 +58,6 @@ __device__ __forceinline__ void wide_mma(uint32_t d, uint32_t a, uint32_t blo, u
         : "memory");
 }
 
-// Stores under a predicate instead of a branch: the output stage is one warp a scheduler, and every branch costs it an
-// instruction fetch (about 80 cycles; eight of them a batch of rows were most of the stage).
-__device__ __forceinline__ void st_if(bool ok, void* at, uint32_t v) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b32 [%0], %1;\n\t}" ::"l"(at), "r"(v), "r"((uint32_t)ok) : "memory");
-}
-__device__ __forceinline__ void st16_if(bool ok, void* at, uint16_t v) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(at), "h"(v), "r"((uint32_t)ok) : "memory");
-}
 // two floats as a bf16 pair, the first in the lower half
 __device__ __forceinline__ uint32_t f32x2_to_bf16x2(float lo, float hi) {
     uint32_t d;

@@ -45,6 +45,7 @@ class TkdMoe(ctypes.Structure):
         ("rows", c_i32), ("x", c_vp), ("ldx", c_i64), ("ids", c_vp), ("ids32", c_i32), ("k", c_i32), ("ld_ids", c_i64),
         ("route_w", c_vp), ("ld_w", c_i64), ("by_union", c_i32), ("slots", c_i32), ("act", c_i32), ("bias", c_vp),
         ("out", c_vp), ("ldo", c_i64), ("workspace", c_vp), ("workspace_bytes", c_u64), ("fmt", c_i32),
+        ("out_rows", c_i32), ("status", c_vp),
     ]
 
 
@@ -78,6 +79,7 @@ SYMBOLS = {
     "tkd_noalloc_scratch_address": (c_i32, [ctypes.POINTER(c_vp)]),
     "tkd_hadamard": (c_i32, [c_vp, c_i64, c_vp, c_i32, c_i32, c_vp, c_i64, c_vp]),
     "tkd_moe_workspace": (c_i32, [ctypes.POINTER(TkdMoe), ctypes.POINTER(c_u64)]),
+    "tkd_moe_rows_workspace": (c_i32, [ctypes.POINTER(TkdMoe), c_i32, ctypes.POINTER(c_u64)]),
     "tkd_moe_gate_up": (c_i32, [ctypes.POINTER(TkdMoe), c_vp]),
     "tkd_moe_down": (c_i32, [ctypes.POINTER(TkdMoe), c_vp]),
     "tkd_moe_route": (c_i32, [c_vp, c_i64, c_i32, c_i32, c_i32, c_i32, c_vp, ctypes.c_double, c_i32, c_i32, c_i32, c_i32, c_u32,

@@ -45,6 +45,7 @@ from common import ttnn_like as ttnn
 from common.device import dram_banks
 from dense_reader import _tkd
 from dense_reader import cache as _cache
+from dense_reader import linear
 
 TILE = 32
 TB = 576  # a bfloat4_b tile: 64 exponent bytes, then 1024 codes of a sign and 3 magnitude bits
@@ -438,7 +439,10 @@ class _Op:
         if gu:
             a.act, a.bias = ACTS[act], P["gu_bias_t"].data_ptr() if P["gu_bias"] else None
         need = ctypes.c_uint64(0)
-        if not gu:
+        if by_union:
+            a.out_rows, a.status = TILE, linear.status_word(P["_device"]).data_ptr()
+            _tkd.check(_tkd.lib().tkd_moe_rows_workspace(ctypes.byref(a), int(not gu), ctypes.byref(need)), "tkd_moe_rows_workspace")
+        elif not gu:
             _tkd.check(_tkd.lib().tkd_moe_workspace(ctypes.byref(a), ctypes.byref(need)), "tkd_moe_workspace")
         self.need, self.address, self.weights = need.value, ctypes.addressof(a), weights.data_ptr()
         self.ids_dtype, self.launch = (ttnn.uint32 if ids32 else ttnn.uint16), _tkd.host().moe
@@ -467,19 +471,24 @@ def _op(P, what, x, ids, w, rows, k, ids32, by_union, act=None):
     return op
 
 
+def _workspace(P, what, op):
+    """The op's workspace, kept with the layer, one a kind of op: zeroed once (the kernels return their counters to zero; calls
+    on one layer run in stream order). One outgrown stays alive for the CUDA graphs that hold its address."""
+    held = P["_ws"].setdefault(what, [])
+    if not held or held[-1].numel() < op.need:
+        held.append(torch.zeros(op.need, dtype=torch.uint8, device=P["_device"].torch))
+    return held[-1]
+
+
 def _gate_up(x, P, ids, w, k, rows, ids32, by_union, act, memory_config):
     op = _op(P, "gu", x, ids, w, rows, k, ids32, by_union, act)
-    out = op.launch(op.address, x.t, ids.t, w.t, None)
+    out = op.launch(op.address, x.t, ids.t, w.t, _workspace(P, "gu rows", op) if by_union else None)
     return ttnn.Tensor(out, ttnn.bfloat16, ttnn.TILE_LAYOUT, x._device, memory_config)
 
 
 def _down(h, P, ids, k, rows, ids32, by_union, memory_config):
     op = _op(P, "dn", h, ids, None, rows, k, ids32, by_union)
-    ws = P["_ws"].get("dn")
-    if ws is None or ws.numel() < op.need:
-        # (zeroed once: the kernel returns its counters to zero; calls on one layer run in stream order)
-        ws = P["_ws"]["dn"] = torch.zeros(op.need, dtype=torch.uint8, device=h._device.torch)
-    out = op.launch(op.address, h.t, ids.t, None, ws)
+    out = op.launch(op.address, h.t, ids.t, None, _workspace(P, "dn rows" if by_union else "dn", op))
     return ttnn.Tensor(out, ttnn.bfloat16, ttnn.TILE_LAYOUT, h._device, memory_config)
 
 

@@ -20,6 +20,7 @@ pytestmark = pytest.mark.gpu
 
 from common import ttnn_like as ttnn  # noqa: E402
 from common.testing import check, raises, same  # noqa: E402
+from dense_reader import linear  # noqa: E402
 from moe import moe8  # noqa: E402
 from oracle import oracle as orc  # noqa: E402
 
@@ -428,3 +429,58 @@ def test_kblock_pack_holds_the_host_quantisers_values(device):
         raises("a K-block cache taken as an ordinary one", moe8.PackCacheMismatch, lambda: moe8.pack_cached(device, tmp / "l"))
     finally:
         shutil.rmtree(tmp, ignore_errors=True)
+
+
+@pytest.mark.parametrize("e,h,i,k,rows,bad", [
+    (4, 32, 32, 2, 8, False),       # fewer blocks of work than CTAs
+    (16, 544, 96, 4, 9, True),      # K past a chunk and inside a super-atom, two tiles of rows, ids past the experts
+    (64, 96, 640, 16, 17, False),   # four tiles a CTA and more: gate_up deals out whole ones
+    (8, 1056, 288, 8, 25, False),   # four tiles of rows; every expert chosen by every row
+    (3, 64, 64, 3, 24, "all"),      # no id names an expert
+])
+@pytest.mark.parametrize("kblock", [False, True])
+def test_rows_at_the_edges_of_their_tiles(device, e, h, i, k, rows, bad, kblock):
+    """gate_up_rows and down_rows against the oracle where a tile is cut between CTAs or not, with and without a workspace for
+    gate_up, and a second call on the same workspaces bit for bit. Bars: the reference's."""
+    gu, dn = experts(e + h, 0.05, e, h, i, kblock=kblock)
+    P = moe8.pack(device, gu, dn, kblock=kblock)
+    g = torch.Generator().manual_seed(h + rows)
+    ids = torch.stack([torch.randperm(e, generator=g)[:k] for _ in range(rows)])
+    if bad == "all":
+        ids += e
+    elif bad:
+        ids[1, 0] = e + 5
+        ids[:, k - 1] = e
+    wts = torch.softmax(torch.randn(rows, k, generator=g), -1).to(BF)
+    x = make_x(rows, 19, h)
+    tid = dev(device, ids.to(torch.int16).reshape(1, 1, rows, k), ttnn.uint16)
+    twt = dev(device, wts.reshape(1, 1, rows, k), ttnn.bfloat16)
+    tx = dev(device, x.reshape(1, 1, rows, h), ttnn.bfloat16)
+    u = moe8.union(ids, e)
+    want_h, want_y = torch.zeros(rows, len(u) * i, dtype=torch.float64), torch.zeros(rows, h, dtype=torch.float64)
+    for r in range(rows):
+        valid = [(s, v) for s, v in enumerate(ids[r].tolist()) if v < e]
+        if not valid:
+            continue
+        oy, oh = orc.moe_reference(x[r : r + 1].float().numpy(), gu.float().numpy(), dn.float().numpy(), [v for _, v in valid],
+                                   [float(wts[r, s]) for s, _ in valid], "silu")
+        want_y[r] = torch.from_numpy(oy)[0]
+        for j, (_, v) in enumerate(valid):
+            q = u.index(v)
+            want_h[r, q * i : (q + 1) * i] = torch.from_numpy(oh[0, j * i : (j + 1) * i])
+    th = moe8.gate_up_rows(tx, P, tid, twt, k, rows)
+    ty = moe8.down_rows(th, P, tid, k, rows)
+    hd, yd = host(th, th.shape[-1]), host(ty, h)
+    if u:
+        check(f"rows {rows} of {e} experts: h", hd[:rows, : len(u) * i], want_h, rel=REL)
+        check(f"rows {rows} of {e} experts: y", yd[:rows], want_y, rel=REL)
+    assert not hd[:rows, len(u) * i :].any() and not hd[rows:].any() and not yd[rows:].any()
+    assert u or not yd.any()
+    th2 = moe8.gate_up_rows(tx, P, tid, twt, k, rows)
+    same("h again", host(th2, th.shape[-1]), hd)
+    same("y again", host(moe8.down_rows(th2, P, tid, k, rows), h), yd)
+    op = moe8._op(P, "gu", tx, tid, twt, rows, k, False, True, "silu")
+    bare = ttnn.Tensor(op.launch(op.address, tx.t, tid.t, twt.t, None), ttnn.bfloat16, ttnn.TILE_LAYOUT, device, None)
+    if u:
+        check("h without a workspace", host(bare, th.shape[-1])[:rows, : len(u) * i], want_h, rel=REL)
+    linear.check_status(device)
