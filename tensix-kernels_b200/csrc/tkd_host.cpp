@@ -147,6 +147,33 @@ PyObject* host_route(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
 }
 
+// pick(records, x, head rows, out, ids_out or None, (records, rows, k, top, vocabulary, whether rounded)): tkd_head_pick.
+PyObject* host_pick(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 6 || !all_tensors(args, {0, 1, 2, 3}, {4})) return type_error("tkd_host.pick: records, x, head, out, ids_out, settings");
+    int nrec, rows, k, top, round;
+    unsigned vocab;
+    if (!PyArg_ParseTuple(args[5], "iiiiIi", &nrec, &rows, &k, &top, &vocab, &round)) return nullptr;
+    try {
+        const at::Tensor &rec = THPVariable_Unpack(args[0]), &x = THPVariable_Unpack(args[1]), &head = THPVariable_Unpack(args[2]);
+        const at::Tensor &out = THPVariable_Unpack(args[3]), *ids = tensor_or_null(args[4]);
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != x.get_device()) guard.set_index(x.get_device());
+        void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
+        const int64_t dim = x.size(-1), ld_head = head.size(-1);
+        const auto* rp = static_cast<const uint32_t*>(rec.data_ptr());
+        const void *xp = x.data_ptr(), *hp = head.data_ptr();
+        auto* op = static_cast<uint32_t*>(out.data_ptr());
+        auto* ip = ids ? static_cast<uint32_t*>(ids->data_ptr()) : nullptr;
+        int rc;
+        Py_BEGIN_ALLOW_THREADS rc = tkd_head_pick(rp, nrec, rows, k, top, vocab, xp, dim, (int)dim, hp, ld_head, round, op, ip, stream);
+        Py_END_ALLOW_THREADS if (rc) return tkd_error(rc, "tkd_head_pick");
+        Py_RETURN_NONE;
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
 // This thread's int in pinned host memory, which a packing kernel sets when its weight is wide: read after the stream has been
 // waited for, with nothing copied back.
 struct WideWord {
@@ -210,6 +237,7 @@ PyMethodDef methods[] = {
     fast<host_moe>("moe"),
     fast<host_route>("route"),
     fast<host_pack>("pack"),
+    fast<host_pick>("pick"),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "tkd_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

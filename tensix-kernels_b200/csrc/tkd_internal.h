@@ -46,7 +46,7 @@ struct TkdSegDev {
 };
 
 struct TkdParams {
-    TkdSegDev seg[4];
+    TkdSegDev seg[TKD_MAX_BLOCKS];
     int nseg;
     int fmt, M, K;
     const uint16_t* x;  // bf16 bits, row-major, ldx elements a row

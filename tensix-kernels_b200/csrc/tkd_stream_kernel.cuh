@@ -189,9 +189,7 @@ __device__ __forceinline__ void cursor_init(Cursor& c, const TkdParams& p, int64
     c.panel = (int)idiv(p, it, p.nslices);
     c.slice = (int)(it - (int64_t)c.panel * p.nslices);
     c.seg = 0;
-#pragma unroll
-    for (int s = 1; s < 4; ++s)
-        if (s < p.nseg && c.panel >= p.seg[s].panel0) c.seg = s;
+    while (c.seg + 1 < p.nseg && c.panel >= p.seg[c.seg + 1].panel0) ++c.seg;
     c.pl = c.panel - p.seg[c.seg].panel0;
 }
 __device__ __forceinline__ void cursor_next(Cursor& c, const TkdParams& p) {
@@ -385,74 +383,106 @@ __device__ __forceinline__ uint32_t topk_key(uint16_t b) {
     return (uint32_t)(b ^ (0x8000u | (0x7FFFu & (0u - (uint32_t)(b >> 15))))) & 0xFFFFu;
 }
 
+// The largest of a lane's candidates below `bound` (all of them: bound ~0).
+template <int N>
+__device__ __forceinline__ uint32_t topk_best(const uint32_t (&cand)[N], uint32_t bound) {
+    uint32_t best = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+        if (cand[j] < bound) best = max(best, cand[j]);
+    return best;
+}
+
 // The top-k records of the unit of columns that panel c.pl belongs to, made by the CTA whose output warps complete the
-// unit's last panel, from the bf16 outputs themselves (all four output warps call this after a panel's output stage).
+// unit's last panel, from the bf16 outputs themselves (all four output warps call this after a panel's output stage). A
+// candidate is key << 16 | 0xFFFF - its column in the unit: key descending, column ascending. Each warp finds the best k of its
+// quarter of the unit (16 columns a lane; a round is one warp-wide maximum in hardware, and only the lane that gave it looks
+// through its candidates again), a row after the other, then a warp merges a row's four lists. (Every round's maximum over
+// the four warps through shared memory, with two barriers a round, took 8 rows of 8 some 5 us a unit.)
 __device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c, const TkdSegDev& sg, int et, int ow, int lane,
                                              float* tbuf, volatile int* sflag, uint16_t* y16, int topk_k, int npeers) {
-                // ------------------------------------------------------------ top-k records: one per unit of columns,
-                // made by the CTA that completes the unit's last panel, from the bf16 outputs themselves
-                const int upanels = p.topk_unit / TKD_PANEL_COLS;
-                const int unit = c.pl / upanels;
-                const int in_unit = min(upanels, p.total_panels - unit * upanels);
-                __threadfence();
-                bar_output_warps();
-                if (et == 0) {
-                    const int old = atomicAdd(p.unit_counters + unit, 1);
-                    const int last = old + 1 == in_unit;
-                    if (last) p.unit_counters[unit] = 0;
-                    sflag[0] = last;
-                }
-                bar_output_warps();
-                const bool scan = sflag[0] != 0;
-                bar_output_warps();
-                if (!scan) return;
-                __threadfence();
-                const uint16_t* ysrc = p.write_y ? y16 + sg.out_col0 : p.ytmp;
-                const int64_t ldy = p.write_y ? p.ldo : p.ld_ytmp;
-                const int col0 = unit * p.topk_unit;  // the unit's first column (call-relative)
-                uint32_t* red = reinterpret_cast<uint32_t*>(tbuf);
-                const size_t rec_at = (size_t)(p.topk_slot0 + unit) * 2 * p.topk_rows * topk_k;
-                uint32_t* rec = p.records + rec_at;
-                for (int r = 0; r < p.topk_rows; ++r) {
-                    // candidates: (key << 16 | 0xFFFF - position in unit) orders by key descending, then column ascending;
-                    // this thread's 16 (a unit holds at most 2048 columns) are loaded once
-                    uint32_t cand[16];
-    #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int cc = et + j * TKD_PANEL_COLS, col = col0 + cc;
-                        uint32_t key = 0;
-                        if (cc < p.topk_unit && col < p.topk_n && col < sg.n_valid)
-                            key = topk_key(__ldcg(ysrc + (size_t)r * ldy + col));
-                        cand[j] = key ? (key << 16) | (0xFFFFu - (uint32_t)cc) : 0u;
+    const int upanels = p.topk_unit / TKD_PANEL_COLS, seg_panels = p.total_panels / p.nseg;
+    const int unit = c.pl / upanels, slot = c.seg * ((seg_panels + upanels - 1) / upanels) + unit;
+    const int in_unit = min(upanels, seg_panels - unit * upanels);
+    __threadfence();
+    bar_output_warps();
+    if (et == 0) {
+        const int old = atomicAdd(p.unit_counters + slot, 1);
+        const int last = old + 1 == in_unit;
+        if (last) p.unit_counters[slot] = 0;
+        sflag[0] = last;
+    }
+    bar_output_warps();
+    const bool scan = sflag[0] != 0;
+    bar_output_warps();
+    if (!scan) return;
+    __threadfence();
+    const uint16_t* ysrc = p.write_y ? y16 + sg.out_col0 : p.ytmp + (int64_t)sg.panel0 * TKD_PANEL_COLS;
+    const int64_t ldy = p.write_y ? p.ldo : p.ld_ytmp;
+    const int col0 = unit * p.topk_unit, c0 = ow * 512 + lane * 16;  // the unit's first column, this lane's first in the unit
+    // this lane's columns that count
+    const int64_t limit = min(min((int64_t)p.topk_n, (int64_t)sg.n_valid) - col0, (int64_t)p.topk_unit);
+    const int have = (int)max((int64_t)0, min((int64_t)16, limit - c0));
+    uint32_t* red = reinterpret_cast<uint32_t*>(tbuf);  // [row][warp][k]
+    auto load = [&](int r, uint32_t (&w)[8]) {
+        const uint16_t* s = ysrc + (size_t)r * ldy + col0 + c0;
+        if (!p.write_y) {
+            if (have) {
+                const uint4 a = __ldcg(reinterpret_cast<const uint4*>(s)), b = __ldcg(reinterpret_cast<const uint4*>(s) + 1);
+                w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const uint32_t v = j < have ? __ldcg(s + j) : 0u;
+                w[j >> 1] = j & 1 ? w[j >> 1] | v << 16 : v;
+            }
+        }
+    };
+    uint32_t next[8] = {};
+    load(0, next);
+    for (int r = 0; r < p.topk_rows; ++r) {
+        uint32_t cand[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const uint32_t key = topk_key((uint16_t)(next[j >> 1] >> (16 * (j & 1))));
+            cand[j] = j < have && key ? (key << 16) | (0xFFFFu - (uint32_t)(c0 + j)) : 0u;
+        }
+        if (r + 1 < p.topk_rows) load(r + 1, next);
+        uint32_t best = topk_best(cand, 0xFFFFFFFFu);
+        for (int q = 0; q < topk_k; ++q) {
+            const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, best);
+            if (lane == 0) red[(r * 4 + ow) * topk_k + q] = m;  // (0: nothing left)
+            if (best == m) best = topk_best(cand, m);
+        }
+    }
+    bar_output_warps();
+    const size_t rec_at = (size_t)(p.topk_slot0 + slot) * 2 * p.topk_rows * topk_k;
+    uint32_t* rec = p.records + rec_at;
+    const uint32_t base = p.topk_base + (uint32_t)c.seg * (uint32_t)sg.n_valid + (uint32_t)col0;
+    for (int r = ow; r < p.topk_rows; r += 4) {
+        uint32_t cand[8];  // (4 k candidates, k at most 64)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cand[j] = lane + 32 * j < 4 * topk_k ? red[r * 4 * topk_k + lane + 32 * j] : 0u;
+        uint32_t best = topk_best(cand, 0xFFFFFFFFu);
+        for (int q = 0; q < topk_k; ++q) {
+            const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, best);
+            if (best == m) best = topk_best(cand, m);
+            if (lane == 0) {
+                const uint32_t key = m >> 16, idx = m ? base + (0xFFFFu - (m & 0xFFFFu)) : 0xFFFFFFFFu;
+                const int at_k = r * topk_k + q, at_i = (p.topk_rows + r) * topk_k + q;
+                rec[at_k] = key;
+                rec[at_i] = idx;
+#pragma unroll 1
+                for (int pq = 0; pq < npeers; ++pq)
+                    if (p.peer_records[pq]) {
+                        p.peer_records[pq][rec_at + at_k] = key;
+                        p.peer_records[pq][rec_at + at_i] = idx;
                     }
-                    uint32_t bound = 0xFFFFFFFFu;
-                    for (int q = 0; q < topk_k; ++q) {
-                        uint32_t best = 0;
-    #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (cand[j] < bound && cand[j] > best) best = cand[j];
-    #pragma unroll
-                        for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
-                        if (lane == 0) red[ow] = best;
-                        bar_output_warps();
-                        best = max(max(red[0], red[1]), max(red[2], red[3]));
-                        bar_output_warps();
-                        bound = best;  // (0: nothing left, the remaining slots stay empty)
-                        if (et == 0) {
-                            const uint32_t key = best >> 16;
-                            const uint32_t idx = best ? p.topk_base + (uint32_t)col0 + (0xFFFFu - (best & 0xFFFFu)) : 0xFFFFFFFFu;
-                            const int at_k = r * topk_k + q, at_i = (p.topk_rows + r) * topk_k + q;
-                            rec[at_k] = key;
-                            rec[at_i] = idx;
-    #pragma unroll 1
-                            for (int pq = 0; pq < npeers; ++pq)
-                                if (p.peer_records[pq]) {
-                                    p.peer_records[pq][rec_at + at_k] = key;
-                                    p.peer_records[pq][rec_at + at_i] = idx;
-                                }
-                        }
-                    }
-                }
+            }
+        }
+    }
+    bar_output_warps();  // (the lists have been read)
 }
 
 // The end of an exchanged call, run by every output warp after its last panel.
@@ -1017,7 +1047,7 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
                                     for (int q = 0; q < npeers; ++q)
                                         if (p.peer_out[q]) static_cast<uint16_t*>(p.peer_out[q])[(size_t)m * p.ldo + ocol] = b;
                                 }
-                                if (topk_k && !p.write_y && m < p.topk_rows) p.ytmp[(size_t)m * p.ld_ytmp + n] = b;
+                                if (topk_k && !p.write_y && m < p.topk_rows) p.ytmp[(size_t)m * p.ld_ytmp + c.panel * TKD_PANEL_COLS + et] = b;
                             }
                     }
                 }

@@ -846,7 +846,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                                     for (int q = 0; q < npeers; ++q)
                                         if (p.peer_out[q]) static_cast<uint16_t*>(p.peer_out[q])[at] = b;
                                 }
-                                if (topk_k && !p.write_y && r0 + m < p.topk_rows) p.ytmp[(size_t)(r0 + m) * p.ld_ytmp + n] = b;
+                                if (topk_k && !p.write_y && r0 + m < p.topk_rows) p.ytmp[(size_t)(r0 + m) * p.ld_ytmp + c.panel * TKD_PANEL_COLS + et] = b;
                             }
                         }
                     }

@@ -138,81 +138,103 @@ __device__ __forceinline__ uint32_t rank16(uint32_t kk) {
     return kk == 0x7FFFu ? 0x8000u : kk;
 }
 
+constexpr int kPickWarps = 16, kPickOwn = 8;
+
+// The best `top` (at most 32) of a warp's candidates, lane t the t-th: (rank, id), rank 0 where there are none. A candidate's
+// word is rank << 12 | 4095 - its place, so that an equal rank keeps the earlier place; a round is one warp-wide maximum in
+// hardware, and the lane that gave it moves on to its next.
+template <int N>
+__device__ __forceinline__ void pick_rounds(const uint32_t (&word)[N], const uint32_t (&id)[N], int top, int lane, uint32_t& rank_out,
+                                            uint32_t& id_out) {
+    uint32_t best = 0, bid = 0;
+    auto next = [&](uint32_t bound) {
+        best = 0;
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (word[j] < bound && word[j] > best) best = word[j], bid = id[j];
+    };
+    next(0xFFFFFFFFu);
+    rank_out = 0, id_out = 0;
+    for (int t = 0; t < top; ++t) {
+        const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, best);
+        if (m >> 12 == 0) break;
+        const uint32_t src = __ballot_sync(0xFFFFFFFFu, best == m);
+        const uint32_t won = __shfl_sync(0xFFFFFFFFu, bid, __ffs(src) - 1);
+        if (lane == t) rank_out = m >> 12, id_out = won;
+        if (best == m) next(m);
+    }
+}
+
 // One CTA per row r of the step.
 //   1. The best `top` slots of row r over the records in order (record by record, slot by slot), by key (RECORDS: by
-//      rank16, and top is 1); an equal key keeps the earlier slot; a slot with key 0 or an id at or past `vocab` is empty.
+//      rank16, and top is 1); an equal key keeps the earlier slot; a slot with key 0 or an id at or past `vocab` is empty. A
+//      warp takes a run of slots, 256 at a time beside its best so far; one warp merges the warps' lists.
 //   2. (not RECORDS) Their exact logits: bf16 x row times the candidates' bf16 head rows, float32 sums (a warp per
 //      candidate: every lane sums its 8-element pieces in order, then a shuffle tree), rounded to bf16 with `round`.
 //   3. The pick: the largest logit (order32), the lowest id among equals. Row r of out (32 words):
 //      [token, the first candidate by the device's own logit, count, 0 ...]; count is the candidates held (RECORDS: all
 //      valid slots). No valid slot: [0, 0xFFFFFFFF, 0].
+// Bound by latency: as `top` rounds over all slots read anew, with two barriers each, and one candidate after the other, it
+// took a fifth of a vocabulary's call.
 template <bool RECORDS>
-__global__ void __launch_bounds__(kThreads) tkd_head_pick_kernel(const uint32_t* __restrict__ records, int nrec, int rows,
-                                                                 int k, int top, uint32_t vocab,
-                                                                 const uint16_t* __restrict__ x, int64_t ldx, int dim,
-                                                                 const uint16_t* __restrict__ head, int64_t ld_head,
-                                                                 int round, const uint32_t* __restrict__ tmap,
-                                                                 uint32_t* __restrict__ out, uint32_t* __restrict__ ids_out) {
-    __shared__ unsigned long long red[kThreads / 32];
-    __shared__ uint32_t cid[32], clogit[32];
-    __shared__ int held, nvalid[kThreads / 32];
+__global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const uint32_t* __restrict__ records, int nrec, int rows,
+                                                                        int k, int top, uint32_t vocab,
+                                                                        const uint16_t* __restrict__ x, int64_t ldx, int dim,
+                                                                        const uint16_t* __restrict__ head, int64_t ld_head,
+                                                                        int round, const uint32_t* __restrict__ tmap,
+                                                                        uint32_t* __restrict__ out, uint32_t* __restrict__ ids_out) {
+    __shared__ uint32_t srank[kPickWarps][32], sid[kPickWarps][32], cid[32], clogit[32];
+    __shared__ int held, nvalid[kPickWarps];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = nrec * k;
-    auto slot = [&](int c, uint32_t& id) -> uint32_t {
-        const int rec = c / k, q = c - rec * k;
-        const uint32_t* page = records + (size_t)rec * 2 * rows * k;
-        const uint32_t key = __ldg(page + r * k + q) & 0xFFFFu;
-        id = __ldg(page + (rows + r) * k + q);
-        return key && id < vocab ? key : 0u;
-    };
-    // packed (rank, ~position): the 64-bit order is "larger rank first, earlier slot first"
-    auto packed = [&](int c) -> unsigned long long {
-        uint32_t id;
-        const uint32_t key = slot(c, id);
-        return key ? ((unsigned long long)(RECORDS ? rank16(key) : key) << 32) | (uint32_t)~(uint32_t)c : 0ull;
-    };
+    const int n = nrec * k, per = (n + kPickWarps - 1) / kPickWarps, c1 = min(n, (warp + 1) * per);
+    uint32_t rank = 0, id = 0;  // lane t: the t-th so far
     int mine = 0;
-    for (int c = tid; c < n; c += kThreads) mine += packed(c) != 0;
+    for (int c0 = warp * per; c0 < c1; c0 += 32 * kPickOwn) {
+        uint32_t word[kPickOwn + 1], ids[kPickOwn + 1];
 #pragma unroll
-    for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xFFFFFFFFu, mine, o);
+        for (int j = 0; j < kPickOwn; ++j) {
+            const int c = c0 + 32 * j + lane;
+            word[j] = ids[j] = 0;
+            if (c < c1) {
+                const int rec = c / k, q = c - rec * k;
+                const uint32_t* page = records + (size_t)rec * 2 * rows * k;
+                const uint32_t key = __ldg(page + r * k + q) & 0xFFFFu;
+                ids[j] = __ldg(page + (rows + r) * k + q);
+                if (key && ids[j] < vocab) {
+                    word[j] = (RECORDS ? rank16(key) : key) << 12 | (uint32_t)(4095 - 32 - 32 * j - lane);
+                    ++mine;
+                }
+            }
+        }
+        word[kPickOwn] = rank ? rank << 12 | (uint32_t)(4095 - lane) : 0u, ids[kPickOwn] = id;
+        pick_rounds(word, ids, top, lane, rank, id);
+    }
+    srank[warp][lane] = rank, sid[warp][lane] = id;
+    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
     if (lane == 0) nvalid[warp] = mine;
-    if (tid == 0) held = 0;
-    unsigned long long bound = ~0ull;
-    for (int t = 0; t < top; ++t) {
-        unsigned long long best = 0;
-        for (int c = tid; c < n; c += kThreads) {
-            const unsigned long long v = packed(c);
-            if (v < bound && v > best) best = v;
-        }
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t word[kPickWarps], ids[kPickWarps];
 #pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            best = other > best ? other : best;
+        for (int w = 0; w < kPickWarps; ++w) {
+            const uint32_t rk = srank[w][lane];
+            word[w] = rk ? rk << 12 | (uint32_t)(4095 - 32 * w - lane) : 0u, ids[w] = sid[w][lane];
         }
-        if (lane == 0) red[warp] = best;
-        __syncthreads();
-        best = red[0];
-#pragma unroll
-        for (int w = 1; w < kThreads / 32; ++w) best = red[w] > best ? red[w] : best;
-        if (tid == 0 && best) {
-            uint32_t id;
-            (void)slot((int)~(uint32_t)best, id);
-            cid[t] = id;
-            held = t + 1;
-        }
-        __syncthreads();
-        bound = best;
-        if (!best) break;
+        pick_rounds(word, ids, top, lane, rank, id);
+        cid[lane] = id;
+        const uint32_t any = __ballot_sync(0xFFFFFFFFu, rank != 0);
+        if (lane == 0) held = __popc(any);
     }
     __syncthreads();
     const int nc = held;
     if constexpr (!RECORDS) {
         const uint16_t* xr = x + (size_t)r * ldx;
-        for (int c = warp; c < nc; c += kThreads / 32) {
+        for (int c = warp; c < nc; c += kPickWarps) {
             const uint16_t* wr = head + (size_t)cid[c] * ld_head;
             float acc = 0.f;
+#pragma unroll 8
             for (int d = lane * 8; d < dim; d += 256) {
                 const uint4 wv = __ldg(reinterpret_cast<const uint4*>(wr + d));
                 const uint4 xv = __ldg(reinterpret_cast<const uint4*>(xr + d));
@@ -233,27 +255,20 @@ __global__ void __launch_bounds__(kThreads) tkd_head_pick_kernel(const uint32_t*
         }
         __syncthreads();
     }
-    if (tid == 0) {
-        uint32_t best = 0xFFFFFFFFu, best_key = 0, count = (uint32_t)nc;
-        bool any = false;
+    if (warp == 0) {
+        const bool have = lane < nc;
+        uint32_t best = 0xFFFFFFFFu, count = (uint32_t)nc;
         if constexpr (RECORDS) {
-            count = 0;
-            for (int w = 0; w < kThreads / 32; ++w) count += (uint32_t)nvalid[w];
-            if (nc) best = cid[0], any = true;
-        } else {
-            for (int c = 0; c < nc; ++c) {
-                const uint32_t kk = clogit[c], id = cid[c];
-                if (!any || kk > best_key || (kk == best_key && id < best)) best_key = kk, best = id, any = true;
-            }
+            count = (uint32_t)__reduce_add_sync(0xFFFFFFFFu, lane < kPickWarps ? nvalid[lane] : 0);
+            if (nc) best = cid[0];
+        } else if (nc) {
+            const uint32_t logit = have ? clogit[lane] : 0u, most = __reduce_max_sync(0xFFFFFFFFu, logit);
+            best = __reduce_min_sync(0xFFFFFFFFu, have && logit == most ? cid[lane] : 0xFFFFFFFFu);
         }
-        uint32_t tok = any ? best : 0u;
-        if (RECORDS && any && tmap) tok = __ldg(tmap + best);
-        uint32_t* o = out + (size_t)r * 32;
-        o[0] = tok;
-        o[1] = nc ? cid[0] : 0xFFFFFFFFu;
-        o[2] = count;
-        for (int w = 3; w < 32; ++w) o[w] = 0;
-        if (ids_out && r == 0) ids_out[0] = tok;
+        uint32_t tok = nc ? best : 0u;
+        if (RECORDS && nc && tmap) tok = __ldg(tmap + best);
+        out[(size_t)r * 32 + lane] = lane == 0 ? tok : lane == 1 ? (nc ? cid[0] : 0xFFFFFFFFu) : lane == 2 ? count : 0u;
+        if (ids_out && r == 0 && lane == 0) ids_out[0] = tok;
     }
 }
 
@@ -263,7 +278,7 @@ int launch_pick(const uint32_t* records, int nrec, int rows, int k, int top, uin
                 uint32_t* ids_out, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)rows);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kPickWarps * 32);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

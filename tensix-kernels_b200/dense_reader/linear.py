@@ -232,8 +232,10 @@ def _describe(x, m, entries, epi, act, scale, scale_up, scale_dt, residual, res_
     a.fmt, a.m, a.k = w0.fmt, m, w0.k
     a.ldx = x.shape[-1]
     a.nblocks, a.epilogue, a.act = len(entries), epi, act
+    if len(entries) > 4:
+        a.blocks = ctypes.cast((_tkd.TkdBlock * len(entries))(), ctypes.POINTER(_tkd.TkdBlock))  # (the pointer keeps the array)
     for i, (g, u, c0) in enumerate(entries):
-        b = a.block[i]
+        b = a.blocks[i] if len(entries) > 4 else a.block[i]
         b.w, b.emax = g.t.data_ptr(), (g.emax.data_ptr() if g.emax is not None else None)
         if u is not None:
             b.w_up, b.emax_up = u.t.data_ptr(), (u.emax.data_ptr() if u.emax is not None else None)
@@ -535,6 +537,39 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     call = _Call(device, launches, need, (scale, col_scales, *scales, hadamard, topk and topk["r"], *others), y.dtype, exchange)
     call.run(x, y, residual)
     return y, call
+
+
+def records_together(x, weights, topk, out):
+    """The top-k records of several weights of one K, dtype and width N, each as matmul(x, w, None, topk={**topk, "slot0":
+    slot0 + b * units, "base": base + b * N}, out=out) for weight b leaves them (units: topk_units(N)), by one launch for every
+    _tkd.MAX_BLOCKS of them. weights: a tuple; topk: matmul's with write_y False; out: a tensor of matmul's output shape, not
+    written."""
+    first = weights[0]
+    key = ("records", x.t.shape, out.t.shape, id(weights), id(topk["r"]), topk["k"], topk["rows"], topk["slot0"],
+           topk["base"], topk["n"], TOPK_UNIT, KS, MAX_CTAS)
+    call = first.calls.get(key) if CACHE else None
+    if call is not None and call.fits(x, out):
+        for a in call.launches:
+            call.launch(a[2], x.t, out.t, None, _workspace(call.device, call.need), 0)
+        return
+    N, units = first.n, topk_units(first.n)
+    assert not topk.get("write_y", False) and x.dtype == ttnn.bfloat16 and x.shape[-1] == first.k and x.shape[-2] <= 32
+    assert all(type(w) is ttnn.Weight and (w.k, w.n, w.fmt) == (first.k, N, first.fmt) for w in weights)
+    assert 1 <= topk["rows"] <= 16 and topk["rows"] * topk["k"] <= 64 and topk["rows"] <= x.shape[-2] and out.shape[-1] >= N, topk
+    launches, need = [], 0
+    for b0 in range(0, len(weights), _tkd.MAX_BLOCKS):
+        part = weights[b0 : b0 + _tkd.MAX_BLOCKS]
+        spec = {**topk, "slot0": topk["slot0"] + b0 * units, "base": topk["base"] + b0 * N}
+        a, n = _describe_rows(x, [(w, None, 0) for w in part], None, None, out, x.shape[-2], spec, 0, None, False, False, KS or 0, MAX_CTAS or 0)
+        launches.append((0, a, ctypes.addressof(a)))
+        need = max(need, n)
+    call = _Call(x.device(), launches, need, (topk["r"], *weights[1:], weights), out.dtype, None)
+    for a in launches:
+        call.launch(a[2], x.t, out.t, None, _workspace(call.device, need), 0)
+    if CACHE:
+        if len(first.calls) >= _WEIGHT_CALLS:
+            first.calls.clear()
+        first.calls[key] = call
 
 
 _PLAIN = {int, bool, str, type(None)}

@@ -85,9 +85,29 @@ def pick(records, x, rows_t, nrows, k, top=16, logits="bf16", out=None, valid=No
     valid count, 0 ...]. valid: a padded head's real vocabulary (ids at or past it are empty slots; default the table's
     rows). A row with no valid candidate gets token 0 and count 0. ids_out: also row 0's token into this one-element
     uint32 tensor. (head_pick.py:101-220)"""
+    key = (records.t.shape, records.dtype, x.t.shape, x.dtype, rows_t.t.shape, rows_t.dtype, rows_t.layout, id(rows_t._mc), nrows, k,
+           top, logits, valid)
+    settings = _PICKS.get(key)
+    if settings is None:
+        settings = _pick_settings(records, x, rows_t, nrows, k, top, logits, valid)
+        if len(_PICKS) >= 256:
+            _PICKS.clear()
+        _PICKS[key] = settings
+    if out is None:
+        out = _out_page(x.device())
+    if ids_out is not None:
+        check_ids_out(ids_out)
+    _tkd.host().pick(records.t, x.t, rows_t.t, out.t, None if ids_out is None else ids_out.t, settings[0])
+    return out
+
+
+_PICKS = {}  # the settings of picks checked before, by shapes and options (a memory config is named by its identity and kept)
+
+
+def _pick_settings(records, x, rows_t, nrows, k, top, logits, valid):
+    """pick's arguments checked, as the native call takes them."""
     assert logits in ("bf16", "float32"), logits
     assert 1 <= top <= 32 and 1 <= nrows <= TILE, (top, nrows)
-    device = x.device()
     dim = x.shape[-1]
     assert dim % TILE == 0, dim
     assert x.dtype == ttnn.bfloat16 and nrows <= x.shape[-2], (x.dtype, x.shape, nrows)
@@ -95,16 +115,7 @@ def pick(records, x, rows_t, nrows, k, top=16, logits="bf16", out=None, valid=No
     nrec = _record_count(records, nrows, k)
     vocab = rows_t.shape[-2] if valid is None else int(valid)
     assert 1 <= vocab <= rows_t.shape[-2], (valid, rows_t.shape)
-    if out is None:
-        out = _out_page(device)
-    if ids_out is not None:
-        check_ids_out(ids_out)
-    with torch.cuda.device(device.torch):
-        _tkd.check(_tkd.lib().tkd_head_pick(
-            records.t.data_ptr(), nrec, nrows, k, top, vocab, x.t.data_ptr(), x.t.shape[-1], dim, rows_t.t.data_ptr(),
-            rows_t.t.shape[-1], int(logits == "bf16"), out.t.data_ptr(), ids_out.t.data_ptr() if ids_out is not None else None,
-            _stream()), "tkd_head_pick")
-    return out
+    return (nrec, nrows, k, top, vocab, int(logits == "bf16")), rows_t._mc
 
 
 def token_map(device, ids):

@@ -14,6 +14,7 @@ lm_head_topk/tests/test_lm_head.py: a random bf16 head [8192, 1024] as four bflo
 - both picks with k 4 at 1 and 3 rows.
 """
 
+import numpy as np
 import pytest
 import torch
 
@@ -23,6 +24,7 @@ from common import ttnn_like as ttnn  # noqa: E402
 from common.testing import same  # noqa: E402
 from dense_reader import linear  # noqa: E402
 from lm_head_topk import head_pick, lmhead  # noqa: E402
+from oracle import oracle as orc  # noqa: E402
 
 VOCAB, DIM, CHUNKS = 8192, 1024, 4
 
@@ -168,3 +170,68 @@ def test_records_pick(device):
     assert int(ttnn.to_torch(ids_out).reshape(-1)[0]) == int(tmap[best][0])
     for h in (plain, picked, mapped):
         h.deallocate()
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("blocks,step,rows,k,unit", [(2, 96, 1, 8, 2048), (5, 2048 + 160, 16, 4, 2048), (17, 288, 5, 8, 128), (4, 2048, 1, 64, 512)])
+def test_blocks_together_equal_a_call_each(device, fmt, blocks, step, rows, k, unit):
+    """The head's blocks in one launch (two for 17) leave the records that a call for each leaves, bit for bit, and those are
+    the canonical top-k of the outputs: blocks that end inside a panel and a unit, one row and more than the four warps that
+    merge, lists of one lane and of many, equal logits by the dozen, ids that count from a block's base."""
+    g = torch.Generator().manual_seed(blocks + step)
+    dim = 256
+    w = (torch.randn(blocks * step, dim, generator=g) * 4).round() / 64
+    x = (torch.randn(rows, dim, generator=g) * 2).round().to(torch.bfloat16)
+    tx = ttnn.from_torch(x.reshape(1, 1, rows, dim), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
+    ws = tuple(linear.native_weight(device, w[i * step : (i + 1) * step], lmhead.FORMATS[fmt])[0] for i in range(blocks))
+    was, linear.TOPK_UNIT = linear.TOPK_UNIT, unit
+    try:
+        units = linear.topk_units(step)
+        one, each = (linear.topk_result(device, 1 + blocks * units, rows, k) for _ in range(2))
+        y = ttnn.allocate_tensor_on_device([1, 1, rows, step], ttnn.bfloat16, ttnn.TILE_LAYOUT, device)
+        spec = {"k": k, "rows": rows, "n": step - 7, "write_y": False}
+        for _ in range(2):  # (described, then as kept)
+            linear.records_together(tx, ws, {**spec, "r": one, "slot0": 1, "base": 50}, y)
+        for b, tw in enumerate(ws):
+            linear.matmul(tx, tw, None, out=y, topk={**spec, "r": each, "slot0": 1 + b * units, "base": 50 + b * step})
+            out = ttnn.to_torch(linear.matmul(tx, tw, None)).reshape(rows, step)
+            rec = ttnn.to_torch(each).reshape(-1, 2, rows, k).numpy().view(np.uint32)
+            for u in range(units):
+                c0, c1 = u * unit, min((u + 1) * unit, step - 7)
+                for r in range(rows):
+                    keys, idx = orc.topk_canonical(orc.bf16_bits(out[r, c0:c1].float()), max(0, c1 - c0), k, 50 + b * step + c0)
+                    assert np.array_equal(rec[1 + b * units + u, 0, r], keys) and np.array_equal(rec[1 + b * units + u, 1, r], idx), (b, u, r)
+    finally:
+        linear.TOPK_UNIT = was
+    assert torch.equal(ttnn.to_torch(one), ttnn.to_torch(each))
+    linear.check_status(device)
+
+
+@pytest.mark.parametrize("nrec,rows,k,top", [(1, 1, 4, 1), (75, 3, 8, 16), (600, 2, 8, 32), (40, 32, 16, 5)])
+def test_pick_takes_the_earliest_of_equal_keys(device, nrec, rows, k, top):
+    """The pick's candidates against the host's stable order over records full of equal keys, empty slots and ids past the
+    vocabulary, with fewer and more slots than the warps take at a time: the first candidate, the count and the token."""
+    gen = np.random.default_rng(nrec + top)
+    dim, vocab = 64, nrec * rows * k // 2 + 8
+    words = np.zeros((nrec, 2, rows, k), np.uint32)
+    words[:, 0] = gen.integers(0x8000, 0x8010, size=(nrec, rows, k))
+    words[:, 0][gen.random((nrec, rows, k)) < 0.2] = 0
+    words[:, 1] = gen.permutation(nrec * rows * k).reshape(nrec, rows, k)
+    r = linear.topk_result(device, nrec, rows, k)
+    r.t.copy_(torch.from_numpy(words.view(np.int32)).reshape(r.t.shape))
+    g = torch.Generator().manual_seed(nrec)
+    table = (torch.randn(vocab, dim, generator=g) * 4).round().to(torch.bfloat16)
+    x = (torch.randn(rows, dim, generator=g) * 2).round().to(torch.bfloat16)  # (whole numbers: exact sums, whatever their order)
+    tx = ttnn.from_torch(x.reshape(1, 1, rows, dim), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
+    tok, best, count = head_pick.tokens(head_pick.pick(r, tx, head_pick.head_rows(device, table), rows, k, top=top, logits="float32"), rows)
+    rtok, _, rcount = head_pick.tokens(head_pick.pick_records(r, rows, k, vocab), rows)
+    for t in range(rows):
+        keys, ids = words[:, 0, t].reshape(-1).astype(np.int64), words[:, 1, t].reshape(-1).astype(np.int64)
+        keys[ids >= vocab] = 0
+        order = np.argsort(-keys, kind="stable")
+        order = order[keys[order] > 0]
+        cand = ids[order][:top]
+        z = (x[t].float() @ table[torch.from_numpy(cand)].float().T).numpy()
+        want = cand[z == z.max()].min()
+        assert (int(tok[t]), int(best[t]), int(count[t])) == (want, cand[0], len(cand)), t
+        assert (int(rtok[t]), int(rcount[t])) == (ids[order][0], len(order)), t
