@@ -113,7 +113,7 @@ typedef struct {
     int64_t k;
     const void* x;          /* bf16 [m, k], ldx elements a row (at most 2^26 for m > 8), 16-byte aligned rows */
     int64_t ldx;
-    int32_t nblocks;        /* 1, or 2..4 for a block list (linear.py:615-624); up to TKD_MAX_BLOCKS through `blocks` */
+    int32_t nblocks;        /* 1, or 2..4 for a block list (linear.py:615-624) */
     int32_t epilogue;       /* TKD_EPI_* */
     TkdBlock block[4];
     int32_t act;            /* GLU: 0 silu, 1 gelu_tanh (common/kernels/dense_ops.h:44-59) */
@@ -128,8 +128,8 @@ typedef struct {
     int64_t ldo;
     /* top-k records (dense_reader/kernels/dense_writer.cpp:185-258; record layout linear.py:771-785): one record per
      * topk_unit columns, record slot0 + unit; a record is keys[rows][k] then indices[rows][k], uint32 each. Within a
-     * record: key descending, index ascending among equal keys. topk_k 0: none. Several blocks: all of one n, without
-     * scales; block b's records begin at topk_slot0 + b * (units of a block), its indices at topk_base + b * n. */
+     * record: key descending, index ascending among equal keys. topk_k 0: none. Several blocks, or a
+     * block of several weights (repeats): all of one n, without scales; the b-th's records begin at topk_slot0 + b * (its units), its indices at topk_base + b * n. */
     void* records;
     int32_t topk_k, topk_rows, topk_unit, topk_slot0, topk_write_y;
     uint32_t topk_base;
@@ -169,9 +169,10 @@ typedef struct {
                                (s * x) per block of 1024 inputs, unnormalised, exactly as tkd_hadamard does it (its sign
                                words), inside the kernel's own copy of x: k a multiple of 1024, and x must fit in shared
                                memory beside the ring (TKD_ERR_UNSUPPORTED otherwise: call tkd_hadamard first) */
-    const TkdBlock* blocks; /* or NULL. HOST memory: nblocks entries in place of block[] (read during the call) */
+    int32_t repeats;        /* 0 or 1, or: block[0] is so many weights of n columns each, their streams back to back (every one
+                               padded to whole panels) and their emax arrays too. For records without y: each weight's as
+                               a block's of its own (LM head: a vocabulary's blocks in one launch) */
 } TkdMatmul;
-#define TKD_MAX_BLOCKS 16
 #define TKD_MAX_RANKS 8
 #define TKD_FLAG_SEQ 8      /* flags[0..7]: calls completed by rank r, as told by r; flags[8]: calls completed here */
 #define TKD_FLAG_WORDS 16

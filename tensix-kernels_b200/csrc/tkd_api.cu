@@ -39,8 +39,6 @@ int sm_count() {
     return cached[dev];
 }
 
-inline const TkdBlock& block_of(const TkdMatmul* a, int s) { return a->blocks ? a->blocks[s] : a->block[s]; }
-
 struct Layout {
     TkdParams p;
     int grid;
@@ -57,7 +55,7 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms) {
     // (the int4 weight with group scales is the reference's one-token op; more rows go through its dequantised
     // bfloat8_b form, as there: int4/w4a16.py dequantize)
     if (a->fmt == TKD_INT4 && a->m > 8) return TKD_ERR_UNSUPPORTED;
-    if (a->nblocks < 1 || a->nblocks > (a->blocks ? TKD_MAX_BLOCKS : 4)) return TKD_ERR_BAD_ARG;
+    if (a->nblocks < 1 || a->nblocks > 4) return TKD_ERR_BAD_ARG;
     if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_OUT32) return TKD_ERR_BAD_ARG;
     const bool glu = a->epilogue == TKD_EPI_GLU_IL || a->epilogue == TKD_EPI_GLU2;
     if (a->nblocks > 1 && !(a->epilogue == TKD_EPI_PLAIN || a->epilogue == TKD_EPI_GLU2)) return TKD_ERR_BAD_ARG;
@@ -66,6 +64,11 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms) {
     if ((a->epilogue == TKD_EPI_OUT32) != (a->out_dtype == TKD_DT_F32)) return TKD_ERR_BAD_ARG;
     if (a->out_dtype != TKD_DT_F32 && a->out_dtype != TKD_DT_BF16) return TKD_ERR_BAD_ARG;
     if (a->nranks < 0 || a->nranks > TKD_MAX_RANKS || (a->nranks > 1 && (a->rank < 0 || a->rank >= a->nranks)))
+        return TKD_ERR_BAD_ARG;
+
+    const int repeats = a->repeats > 1 ? a->repeats : 1;
+    if (a->repeats < 0 || (repeats > 1 && (!a->topk_k || a->topk_write_y || a->nblocks > 1 || a->epilogue != TKD_EPI_PLAIN ||
+                                           a->scale_dtype != TKD_DT_NONE || repeats > (1 << 16))))
         return TKD_ERR_BAD_ARG;
 
     TkdParams& p = L->p;
@@ -98,10 +101,12 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms) {
     int panels = 0;
     L->weight_bytes = 0;
     for (int s = 0; s < a->nblocks; ++s) {
-        const TkdBlock& b = block_of(a, s);
+        const TkdBlock& b = a->block[s];
         if (b.n < 1 || b.out_col0 < 0 || b.n > (1 << 28)) return TKD_ERR_BAD_ARG;
         if (glu && a->epilogue == TKD_EPI_GLU_IL && b.n % 64) return TKD_ERR_BAD_ARG;
-        const int64_t npad = tkd_padded_cols(b.n);
+        const int64_t npad = tkd_padded_cols(b.n) * repeats;
+        if (npad > (1 << 28)) return TKD_ERR_BAD_ARG;
+        if (repeats > 1) p.rep_panels = (int)(npad / repeats / TKD_PANEL_COLS);
         TkdSegDev& d = p.seg[s];
         d.w = static_cast<const uint8_t*>(b.w);
         d.w2 = static_cast<const uint8_t*>(b.w_up);
@@ -170,8 +175,8 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms) {
         p.topk_base = a->topk_base;
         p.topk_n = a->topk_n;
         for (int s = 1; s < a->nblocks; ++s)
-            if (block_of(a, s).n != block_of(a, 0).n) return TKD_ERR_BAD_ARG;
-        units = a->nblocks * ((panels / a->nblocks * TKD_PANEL_COLS + a->topk_unit - 1) / a->topk_unit);
+            if (a->block[s].n != a->block[0].n) return TKD_ERR_BAD_ARG;
+        units = a->nblocks * repeats * ((panels / (a->nblocks * repeats) * TKD_PANEL_COLS + a->topk_unit - 1) / a->topk_unit);
     }
     // workspace map. The counters live in a fixed region at the start, the same for every call: they must stay zero
     // between calls, so no call's slice sums or outputs may ever be laid over another call's counters.
@@ -305,7 +310,7 @@ int tkd_matmul_workspace(const TkdMatmul* a, uint64_t* bytes) {
 static int check_pointers(const TkdMatmul* a) {
     if (!a->x || !a->out || a->ldx < a->k || a->ldx % 8 || (reinterpret_cast<uintptr_t>(a->x) & 15)) return TKD_ERR_BAD_ARG;
     for (int s = 0; s < a->nblocks; ++s) {
-        const TkdBlock& b = block_of(a, s);
+        const TkdBlock& b = a->block[s];
         if (!b.w || (reinterpret_cast<uintptr_t>(b.w) & 15)) return TKD_ERR_BAD_ARG;
         if (has_emax(a->fmt) && !b.emax) return TKD_ERR_BAD_ARG;
         if (a->epilogue == TKD_EPI_GLU2) {
@@ -333,7 +338,7 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
     if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_OUT32 || a->nblocks != 1 || a->topk_k) return TKD_ERR_BAD_ARG;
     if ((a->epilogue == TKD_EPI_OUT32) != (a->out_dtype == TKD_DT_F32)) return TKD_ERR_BAD_ARG;
     if (a->fmt == TKD_INT4 || a->hadamard || a->nranks > 1) return TKD_ERR_UNSUPPORTED;
-    const TkdBlock& b = block_of(a, 0);
+    const TkdBlock& b = a->block[0];
     if (b.n < 1 || b.out_col0 < 0 || b.n > (1 << 28) || (a->epilogue == TKD_EPI_GLU_IL && b.n % 64)) return TKD_ERR_BAD_ARG;
     memset(w, 0, sizeof(*w));
     TkdWide& p = *w;
@@ -414,7 +419,7 @@ int tkd_matmul_rows(const TkdMatmul* a, void* stream) {
     if (ra) return ra;
     if (!a->workspace || a->workspace_bytes < need) return TKD_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(a->workspace) & 255) return TKD_ERR_BAD_ARG;
-    const TkdBlock& b = block_of(a, 0);
+    const TkdBlock& b = a->block[0];
     p.w = static_cast<const uint8_t*>(b.w), p.w2 = static_cast<const uint8_t*>(b.w_up), p.emax = b.emax, p.emax2 = b.emax_up;
     p.n_valid = (int)b.n, p.out_col0 = (int)b.out_col0;
     p.x = static_cast<const uint16_t*>(a->x), p.ldx = a->ldx;

@@ -46,7 +46,7 @@ struct TkdSegDev {
 };
 
 struct TkdParams {
-    TkdSegDev seg[TKD_MAX_BLOCKS];
+    TkdSegDev seg[4];
     int nseg;
     int fmt, M, K;
     const uint16_t* x;  // bf16 bits, row-major, ldx elements a row
@@ -73,6 +73,7 @@ struct TkdParams {
     uint32_t* records;
     int topk_k, topk_rows, topk_unit, topk_slot0, write_y;
     uint32_t topk_base;
+    int rep_panels;      // the call's weight is several of this many panels each, back to back (0: one)
     int64_t topk_n;
     uint16_t* ytmp;      // bf16 outputs of a call that does not write y: [rows][ld_ytmp]
     int64_t ld_ytmp;

@@ -189,7 +189,9 @@ __device__ __forceinline__ void cursor_init(Cursor& c, const TkdParams& p, int64
     c.panel = (int)idiv(p, it, p.nslices);
     c.slice = (int)(it - (int64_t)c.panel * p.nslices);
     c.seg = 0;
-    while (c.seg + 1 < p.nseg && c.panel >= p.seg[c.seg + 1].panel0) ++c.seg;
+#pragma unroll
+    for (int s = 1; s < 4; ++s)
+        if (s < p.nseg && c.panel >= p.seg[s].panel0) c.seg = s;
     c.pl = c.panel - p.seg[c.seg].panel0;
 }
 __device__ __forceinline__ void cursor_next(Cursor& c, const TkdParams& p) {
@@ -401,9 +403,11 @@ __device__ __forceinline__ uint32_t topk_best(const uint32_t (&cand)[N], uint32_
 // the four warps through shared memory, with two barriers a round, took 8 rows of 8 some 5 us a unit.)
 __device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c, const TkdSegDev& sg, int et, int ow, int lane,
                                              float* tbuf, volatile int* sflag, uint16_t* y16, int topk_k, int npeers) {
-    const int upanels = p.topk_unit / TKD_PANEL_COLS, seg_panels = p.total_panels / p.nseg;
-    const int unit = c.pl / upanels, slot = c.seg * ((seg_panels + upanels - 1) / upanels) + unit;
-    const int in_unit = min(upanels, seg_panels - unit * upanels);
+    // (the weight's number in the call, by block or by repeat, its panels, and the panel's number in it)
+    const int upanels = p.topk_unit / TKD_PANEL_COLS, wpanels = p.rep_panels ? p.rep_panels : p.total_panels / p.nseg;
+    const int wi = p.rep_panels ? c.pl / wpanels : c.seg, pl = p.rep_panels ? c.pl - wi * wpanels : c.pl;
+    const int unit = pl / upanels, slot = wi * ((wpanels + upanels - 1) / upanels) + unit;
+    const int in_unit = min(upanels, wpanels - unit * upanels);
     __threadfence();
     bar_output_warps();
     if (et == 0) {
@@ -417,7 +421,7 @@ __device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c
     bar_output_warps();
     if (!scan) return;
     __threadfence();
-    const uint16_t* ysrc = p.write_y ? y16 + sg.out_col0 : p.ytmp + (int64_t)sg.panel0 * TKD_PANEL_COLS;
+    const uint16_t* ysrc = p.write_y ? y16 + sg.out_col0 : p.ytmp + (int64_t)(c.panel - pl) * TKD_PANEL_COLS;
     const int64_t ldy = p.write_y ? p.ldo : p.ld_ytmp;
     const int col0 = unit * p.topk_unit, c0 = ow * 512 + lane * 16;  // the unit's first column, this lane's first in the unit
     // this lane's columns that count
@@ -459,7 +463,7 @@ __device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c
     bar_output_warps();
     const size_t rec_at = (size_t)(p.topk_slot0 + slot) * 2 * p.topk_rows * topk_k;
     uint32_t* rec = p.records + rec_at;
-    const uint32_t base = p.topk_base + (uint32_t)c.seg * (uint32_t)sg.n_valid + (uint32_t)col0;
+    const uint32_t base = p.topk_base + (uint32_t)wi * (uint32_t)sg.n_valid + (uint32_t)col0;
     for (int r = ow; r < p.topk_rows; r += 4) {
         uint32_t cand[8];  // (4 k candidates, k at most 64)
 #pragma unroll
@@ -874,11 +878,13 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
             const uint32_t pb = NPB == 2 ? pi & 1 : 0;
             // this thread's column within its weight; its group's exponent byte and its scale are asked for now, so
             // that their latency passes while the streaming warps are still at work
-            const int n = glu2 ? c.pl * 64 + (et & 63) : c.pl * TKD_PANEL_COLS + et;
+            const int plw = !PLAIN && p.rep_panels ? c.pl % p.rep_panels : c.pl;  // (the panel's number in its weight)
+            const int n = glu2 ? c.pl * 64 + (et & 63) : plw * TKD_PANEL_COLS + et;
             const bool in_w = n < sg.n_valid;
             int ebyte = 0;
             float sc = 1.f;
-            if constexpr (FMT == TKD_BFP8 || FMT == TKD_BFP4) ebyte = (glu2 && et >= 64 ? sg.emax2 : sg.emax)[n >> 4];
+            if constexpr (FMT == TKD_BFP8 || FMT == TKD_BFP4)
+                ebyte = (glu2 && et >= 64 ? sg.emax2 : sg.emax)[(PLAIN || glu2 ? n : c.pl * TKD_PANEL_COLS + et) >> 4];
             if (p.scale_dt != TKD_DT_NONE && in_w) {
                 const void* sp = glu2 && et >= 64 ? p.scale2 : p.scale;
                 sc = p.scale_dt == TKD_DT_BF16 ? bf16_bits_to_f32(static_cast<const uint16_t*>(sp)[n])

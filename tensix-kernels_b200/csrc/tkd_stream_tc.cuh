@@ -476,12 +476,13 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 cursor_next(c, p);
             const Flow f = flow_of(c, p, it, i0, i1);
             const TkdSegDev& sg = p.seg[c.seg];
-            const int n = glu2 ? c.pl * 64 + (et & 63) : c.pl * TKD_PANEL_COLS + et;
+            const int plw = p.rep_panels ? c.pl % p.rep_panels : c.pl;  // (the panel's number in its weight)
+            const int n = glu2 ? c.pl * 64 + (et & 63) : plw * TKD_PANEL_COLS + et;
             const bool in_w = n < sg.n_valid;
             int ebyte = 0;
             float sc = 1.f;
             if (f.deliver) {
-                if constexpr (FMT != TKD_BF16) ebyte = (glu2 && et >= 64 ? sg.emax2 : sg.emax)[n >> 4];
+                if constexpr (FMT != TKD_BF16) ebyte = (glu2 && et >= 64 ? sg.emax2 : sg.emax)[(glu2 ? n : c.pl * TKD_PANEL_COLS + et) >> 4];
                 if (p.scale_dt != TKD_DT_NONE && in_w) {
                     const void* sp = glu2 && et >= 64 ? p.scale2 : p.scale;
                     sc = p.scale_dt == TKD_DT_BF16 ? bf16_bits_to_f32(static_cast<const uint16_t*>(sp)[n])

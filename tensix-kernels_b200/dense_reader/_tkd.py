@@ -33,11 +33,8 @@ class TkdMatmul(ctypes.Structure):
         ("status", c_vp), ("ks", c_i32), ("max_ctas", c_i32),
         ("nranks", c_i32), ("rank", c_i32), ("peer_out", c_vp * 7), ("peer_records", c_vp * 7), ("peer_flags", c_vp * 7),
         ("flags", c_vp), ("exchange_wait", c_i32), ("weights_fresh", c_i32), ("hadamard", c_vp),
-        ("blocks", ctypes.POINTER(TkdBlock)),
+        ("repeats", c_i32),
     ]
-
-
-MAX_BLOCKS = 16
 
 
 MAX_RANKS, FLAG_SEQ, FLAG_WORDS = 8, 8, 16

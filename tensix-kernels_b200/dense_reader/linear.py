@@ -232,10 +232,8 @@ def _describe(x, m, entries, epi, act, scale, scale_up, scale_dt, residual, res_
     a.fmt, a.m, a.k = w0.fmt, m, w0.k
     a.ldx = x.shape[-1]
     a.nblocks, a.epilogue, a.act = len(entries), epi, act
-    if len(entries) > 4:
-        a.blocks = ctypes.cast((_tkd.TkdBlock * len(entries))(), ctypes.POINTER(_tkd.TkdBlock))  # (the pointer keeps the array)
     for i, (g, u, c0) in enumerate(entries):
-        b = a.blocks[i] if len(entries) > 4 else a.block[i]
+        b = a.block[i]
         b.w, b.emax = g.t.data_ptr(), (g.emax.data_ptr() if g.emax is not None else None)
         if u is not None:
             b.w_up, b.emax_up = u.t.data_ptr(), (u.emax.data_ptr() if u.emax is not None else None)
@@ -541,8 +539,8 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
 
 def records_together(x, weights, topk, out):
     """The top-k records of several weights of one K, dtype and width N, each as matmul(x, w, None, topk={**topk, "slot0":
-    slot0 + b * units, "base": base + b * N}, out=out) for weight b leaves them (units: topk_units(N)), by one launch for every
-    _tkd.MAX_BLOCKS of them. weights: a tuple; topk: matmul's with write_y False; out: a tensor of matmul's output shape, not
+    slot0 + b * units, "base": base + b * N}, out=out) for weight b leaves them (units: topk_units(N)): by one launch for weights
+    that lie back to back in device memory, as lm_head_topk's do, else one for every four. weights: a tuple; topk: matmul's with write_y False; out: a tensor of matmul's output shape, not
     written."""
     first = weights[0]
     key = ("records", x.t.shape, out.t.shape, id(weights), id(topk["r"]), topk["k"], topk["rows"], topk["slot0"],
@@ -557,10 +555,14 @@ def records_together(x, weights, topk, out):
     assert all(type(w) is ttnn.Weight and (w.k, w.n, w.fmt) == (first.k, N, first.fmt) for w in weights)
     assert 1 <= topk["rows"] <= 16 and topk["rows"] * topk["k"] <= 64 and topk["rows"] <= x.shape[-2] and out.shape[-1] >= N, topk
     launches, need = [], 0
-    for b0 in range(0, len(weights), _tkd.MAX_BLOCKS):
-        part = weights[b0 : b0 + _tkd.MAX_BLOCKS]
+    after = lambda t, i: None if t is None else t.data_ptr() + i * t.numel()  # noqa: E731  (byte tensors)
+    adjacent = all(w.t.data_ptr() == after(first.t, i) and (w.emax is None or w.emax.data_ptr() == after(first.emax, i))
+                   for i, w in enumerate(weights))
+    for b0 in range(0, len(weights), len(weights) if adjacent else 4):
+        part = weights[:1] if adjacent else weights[b0 : b0 + 4]
         spec = {**topk, "slot0": topk["slot0"] + b0 * units, "base": topk["base"] + b0 * N}
-        a, n = _describe_rows(x, [(w, None, 0) for w in part], None, None, out, x.shape[-2], spec, 0, None, False, False, KS or 0, MAX_CTAS or 0)
+        a, n = _describe_rows(x, [(w, None, 0) for w in part], None, None, out, x.shape[-2], spec, 0, None, False, False, KS or 0,
+                              MAX_CTAS or 0, repeats=len(weights) if adjacent else 0)
         launches.append((0, a, ctypes.addressof(a)))
         need = max(need, n)
     call = _Call(x.device(), launches, need, (topk["r"], *weights[1:], weights), out.dtype, None)
@@ -692,7 +694,8 @@ def matmul_host(x_host, out_host, x, w, scale, *, topk=None, out=None, col0=0, w
     return out
 
 
-def _describe_rows(x, entries, scale, col_scales, y, m, topk, act, residual, glu, out32, ks=0, max_ctas=0, hadamard=None):
+def _describe_rows(x, entries, scale, col_scales, y, m, topk, act, residual, glu, out32, ks=0, max_ctas=0, hadamard=None,
+                   repeats=0):
     """(the descriptor of one launch over m rows of x, without its tensors' addresses; the workspace it needs).
     (linear.py:828-1070)"""
     device = x.device()
@@ -718,6 +721,7 @@ def _describe_rows(x, entries, scale, col_scales, y, m, topk, act, residual, glu
     blocks = [(g, u, c0 * TILE) for g, u, c0 in entries]
     a = _describe(_raw(x), m, blocks, epi, act, sc, sc_up, scale_dt, None if residual is None else _raw(residual), res_dt, _raw(y),
                   topk, ks, max_ctas)
+    a.repeats = repeats
     need = ctypes.c_uint64(0)
     L = _tkd.lib()
     _tkd.check((L.tkd_matmul_workspace if m <= 32 else L.tkd_matmul_rows_workspace)(ctypes.byref(a), ctypes.byref(need)),

@@ -172,10 +172,11 @@ def test_records_pick(device):
         h.deallocate()
 
 
+@pytest.mark.parametrize("adjacent", [False, True])
 @pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
 @pytest.mark.parametrize("blocks,step,rows,k,unit", [(2, 96, 1, 8, 2048), (5, 2048 + 160, 16, 4, 2048), (17, 288, 5, 8, 128), (4, 2048, 1, 64, 512)])
-def test_blocks_together_equal_a_call_each(device, fmt, blocks, step, rows, k, unit):
-    """The head's blocks in one launch (two for 17) leave the records that a call for each leaves, bit for bit, and those are
+def test_blocks_together_equal_a_call_each(device, fmt, blocks, step, rows, k, unit, adjacent):
+    """The head's blocks in one launch (back to back in memory; else one for four) leave the records that a call for each leaves, bit for bit, and those are
     the canonical top-k of the outputs: blocks that end inside a panel and a unit, one row and more than the four warps that
     merge, lists of one lane and of many, equal logits by the dozen, ids that count from a block's base."""
     g = torch.Generator().manual_seed(blocks + step)
@@ -184,6 +185,11 @@ def test_blocks_together_equal_a_call_each(device, fmt, blocks, step, rows, k, u
     x = (torch.randn(rows, dim, generator=g) * 2).round().to(torch.bfloat16)
     tx = ttnn.from_torch(x.reshape(1, 1, rows, dim), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
     ws = tuple(linear.native_weight(device, w[i * step : (i + 1) * step], lmhead.FORMATS[fmt])[0] for i in range(blocks))
+    if adjacent:
+        streams, emaxes = torch.stack([t.t for t in ws]), torch.stack([t.emax for t in ws])
+        for i, t in enumerate(ws):
+            t.t, t.emax = streams[i], emaxes[i]
+        torch.cuda.synchronize()
     was, linear.TOPK_UNIT = linear.TOPK_UNIT, unit
     try:
         units = linear.topk_units(step)
