@@ -185,7 +185,8 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms) {
     L->off_units = (int64_t)kMaxPanels * 4;
     L->off_misc = (int64_t)(kMaxPanels + kMaxUnits) * 4;
     L->off_scratch = kCounterBytes;
-    const int64_t scratch = p.nslices > 1 ? (int64_t)panels * p.nslices * 2 * p.M * TKD_PANEL_COLS * 4 : 0;
+    // (the kernel for up to eight rows reads eight rows of every slice)
+    const int64_t scratch = p.nslices > 1 ? ((int64_t)panels * p.nslices * 2 * p.M + (p.M > 1 && p.M < 8 ? 8 : 0)) * TKD_PANEL_COLS * 4 : 0;
     L->off_ytmp = align_up(L->off_scratch + scratch, 256);
     p.ld_ytmp = (int64_t)panels * TKD_PANEL_COLS;
     const int64_t ytmp = a->topk_k && !a->topk_write_y ? (int64_t)a->topk_rows * p.ld_ytmp * 2 : 0;

@@ -26,7 +26,7 @@ namespace {
 __device__ __forceinline__ float moe_glu(float gt, float u, int act) {
     if (act == 2) {
         const float gc = fminf(gt, 7.f);
-        return gc / (1.f + __expf(-1.702f * gc)) * (fminf(fmaxf(u, -7.f), 7.f) + 1.f);
+        return over_one_plus_exp(gc, -1.702f * gc) * (fminf(fmaxf(u, -7.f), 7.f) + 1.f);
     }
     return act_gate(gt, act) * u;
 }

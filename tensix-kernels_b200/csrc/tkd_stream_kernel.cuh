@@ -168,11 +168,30 @@ __device__ __forceinline__ void st_if(bool ok, void* at, uint32_t v) {
 __device__ __forceinline__ void st16_if(bool ok, void* at, uint16_t v) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(at), "h"(v), "r"((uint32_t)ok) : "memory");
 }
+// two floats as a bf16 pair, the first in the lower half
+__device__ __forceinline__ uint32_t f32x2_to_bf16x2(float lo, float hi) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
 
+
+// a / (1 + e^t), |error| about two units in the last place, without a branch: the division's slow path (a call for extreme
+// operands) kept an output stage's rows from running side by side, 250 ns a row. The reciprocal of the hardware, corrected by
+// one step of Newton's iteration; a divisor past 2^64 is taken down by 2^64 first, so that its reciprocal stays a normal number.
+__device__ __forceinline__ float over_one_plus_exp(float a, float t) {
+    const float d = 1.f + __expf(fminf(t, 88.7f));
+    const float k = d > 0x1p64f ? 0x1p-64f : 1.f, dk = d * k;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(dk));
+    r = fmaf(r, fmaf(-dk, r, 1.f), r);
+    const float q = a * r * k;
+    return t > 88.72f ? a * 0.f : q;  // (where e^t is no number any more the quotient is none; a NaN stays one)
+}
 // dense_ops.h:44-59 of the reference: silu, and gelu_tanh as x * sigmoid(2 u), u = sqrt(2 / pi) (x + 0.044715 x^3)
 __device__ __forceinline__ float act_gate(float g, int act) {
     const float u = act ? g * (1.5957691216f + 0.0713548162f * (g * g)) : g;
-    return g / (1.f + __expf(-u));
+    return over_one_plus_exp(g, -u);
 }
 
 // Quotients of item counts: 32-bit arithmetic when the launch's numbers allow it (p.small): a 64-bit division is a long
@@ -949,27 +968,33 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
                         }
                         tot[0] = t0 + t1;
                     } else {
+                        // Two slices' loads in flight together, 32 (64: spills, slower), at fixed distances from two addresses: one warp a scheduler
+                        // runs an instruction in four cycles or more, and 64 addresses took 2.2 us of a 9.8 us launch of
+                        // 8 rows. (A row past M is another's, or the workspace's last bytes: it is not used.)
+                        float t0[MR], t1[MR];
+                        const size_t step = (size_t)2 * M * TKD_PANEL_COLS;
+                        const float *h0 = s0 + (pe - 1) * step, *h1 = h0 + step / 2;
+#pragma unroll
+                        for (int m = 0; m < MR; ++m) t0[m] = __ldcg(h0 + m * TKD_PANEL_COLS), t1[m] = __ldcg(h1 + m * TKD_PANEL_COLS);
 #pragma unroll 1
-                        for (int hh = 0; hh < 2; ++hh) {
-                            {
-                                float th[MR];
+                        for (int s = pe; s < p.nslices; s += 2) {
+                            float a0[MR], a1[MR], b0[MR], b1[MR];
+                            const bool more = s + 1 < p.nslices;
+                            const float *f0 = h0 + step, *f1 = h1 + step;
+                            h0 = more ? f0 + step : f0, h1 = more ? f1 + step : f1;
 #pragma unroll
-                                for (int m = 0; m < MR; ++m)
-                                    if (m < M) th[m] = term(pe - 1, hh, m);
-#pragma unroll 1
-                                for (int s = pe; s < p.nslices; ++s) {
-                                    float v[MR];
+                            for (int m = 0; m < MR; ++m) {
+                                a0[m] = __ldcg(f0 + m * TKD_PANEL_COLS), a1[m] = __ldcg(f1 + m * TKD_PANEL_COLS);
+                                b0[m] = __ldcg(h0 + m * TKD_PANEL_COLS), b1[m] = __ldcg(h1 + m * TKD_PANEL_COLS);
+                            }
 #pragma unroll
-                                    for (int m = 0; m < MR; ++m)
-                                        if (m < M) v[m] = term(s, hh, m);
-#pragma unroll
-                                    for (int m = 0; m < MR; ++m)
-                                        if (m < M) th[m] += v[m];
-                                }
-#pragma unroll
-                                for (int m = 0; m < MR; ++m) tot[m] = hh == 0 ? th[m] : tot[m] + th[m];
+                            for (int m = 0; m < MR; ++m) {
+                                t0[m] += a0[m], t1[m] += a1[m];
+                                if (more) t0[m] += b0[m], t1[m] += b1[m];
                             }
                         }
+#pragma unroll
+                        for (int m = 0; m < MR; ++m) tot[m] = t0[m] + t1[m];
                     }
                 }
                 bar_output_warps();  // sflag may be written again only after everyone has read it
@@ -1020,38 +1045,41 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
                 if (ocol >= 0) {
                     // (the residual is read for every row before anything is stored: the output may be the residual's own
                     // memory, and loads placed after stores to what may be the same address would wait for each other row
-                    // by row)
-                    if (p.epi == TKD_EPI_OUT32) {
-                        if (p.res_dt == TKD_DT_F32) {
-    #pragma unroll
-                            for (int m = 0; m < R; ++m)
-                                if (m < M) tot[m] += static_cast<const float*>(p.res)[(size_t)m * p.ldr + ocol];
+                    // by row; a row past M reads the last again)
+                    const bool f32out = p.epi == TKD_EPI_OUT32;
+                    if (p.res_dt != TKD_DT_NONE) {
+                        const int rsz = p.res_dt == TKD_DT_F32 ? 4 : 2;
+                        const char* rp = static_cast<const char*>(p.res) + (int64_t)ocol * rsz;
+                        uint32_t q[R];
+#pragma unroll
+                        for (int m = 0; m < R; ++m) {
+                            q[m] = rsz == 4 ? *reinterpret_cast<const uint32_t*>(rp) : (uint32_t)*reinterpret_cast<const uint16_t*>(rp) << 16;
+                            if (m + 1 < M) rp += p.ldr * rsz;
                         }
-                        float* y32 = static_cast<float*>(p.out);
-    #pragma unroll
+#pragma unroll
+                        for (int m = 0; m < R; ++m) tot[m] += __uint_as_float(q[m]);
+                    }
+                    char* yp = static_cast<char*>(p.out) + (int64_t)ocol * (f32out ? 4 : 2);
+#pragma unroll
+                    for (int m = 0; m < R; ++m, yp += p.ldo * (f32out ? 4 : 2)) {
+                        if (f32out)
+                            st_if(m < M, yp, __float_as_uint(tot[m]));
+                        else
+                            st16_if(store && m < M, yp, f32_to_bf16_bits(tot[m]));
+                    }
+                    if constexpr (!PLAIN) {
+#pragma unroll
                         for (int m = 0; m < R; ++m)
                             if (m < M) {
-                                y32[(size_t)m * p.ldo + ocol] = tot[m];
-    #pragma unroll 1
-                                for (int q = 0; q < npeers; ++q)
-                                    if (p.peer_out[q]) static_cast<float*>(p.peer_out[q])[(size_t)m * p.ldo + ocol] = tot[m];
-                            }
-                    } else {
-                        if (p.epi == TKD_EPI_RESIDUAL) {
-    #pragma unroll
-                            for (int m = 0; m < R; ++m)
-                                if (m < M)
-                                    tot[m] += bf16_bits_to_f32(static_cast<const uint16_t*>(p.res)[(size_t)m * p.ldr + ocol]);
-                        }
-    #pragma unroll
-                        for (int m = 0; m < R; ++m)
-                            if (m < M) {
+                                const size_t at = (size_t)m * p.ldo + ocol;
                                 const uint16_t b = f32_to_bf16_bits(tot[m]);
-                                if (store) {
-                                    y16[(size_t)m * p.ldo + ocol] = b;
-    #pragma unroll 1
-                                    for (int q = 0; q < npeers; ++q)
-                                        if (p.peer_out[q]) static_cast<uint16_t*>(p.peer_out[q])[(size_t)m * p.ldo + ocol] = b;
+#pragma unroll 1
+                                for (int q = 0; q < npeers; ++q) {
+                                    if (!p.peer_out[q] || !(f32out || store)) continue;
+                                    if (f32out)
+                                        static_cast<float*>(p.peer_out[q])[at] = tot[m];
+                                    else
+                                        static_cast<uint16_t*>(p.peer_out[q])[at] = b;
                                 }
                                 if (topk_k && !p.write_y && m < p.topk_rows) p.ytmp[(size_t)m * p.ld_ytmp + c.panel * TKD_PANEL_COLS + et] = b;
                             }
@@ -1108,6 +1136,7 @@ int launch_rows(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     if (p.M == 1 && p.x_smem && !p.topk_k && !p.npeers) return launch_one<FMT, true, true, KWHOLE, true>(p, grid, smem, st);
     if (p.M == 1 && p.x_smem) return launch_one<FMT, true, false, KWHOLE, true>(p, grid, smem, st);
     // (9 to 32 rows run tkd_stream_tc_kernel: the caller never gets here with them)
+    if (p.x_smem && !p.topk_k && !p.npeers) return launch_one<FMT, false, true, KWHOLE, true>(p, grid, smem, st);
     if (p.x_smem) return launch_one<FMT, false, false, KWHOLE, true>(p, grid, smem, st);
     return launch_one<FMT, false, false, KWHOLE, false>(p, grid, smem, st);
 }

@@ -95,7 +95,9 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-template <int FMT, bool KWHOLE>
+// PLAIN: no top-k records and no exchange with other GPUs: that code falls away (it is the code's length that costs: the output
+// stage runs once or twice a CTA, from the instruction cache's misses).
+template <int FMT, bool KWHOLE, bool PLAIN>
 __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const __grid_constant__ TkdParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     const int64_t i0 = idiv(p, T * blockIdx.x, gridDim.x), i1 = idiv(p, T * (blockIdx.x + 1), gridDim.x);
     const int nst = p.nstages;
     const int M = p.M, K = p.K;
-    const int topk_k = p.topk_k, npeers = p.npeers;
+    const int topk_k = PLAIN ? 0 : p.topk_k, npeers = PLAIN ? 0 : p.npeers;
     const bool glu2 = p.epi == TKD_EPI_GLU2;
     const int nsa_total = (K + F::KSA - 1) / F::KSA;
     if (i0 >= i1) return;  // (before any tensor memory is held; the grid is never larger than the item count)
@@ -150,16 +152,19 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     auto item_at = [&](int64_t j) { return j < lead ? tail0 + j : i0 + (j - lead); };
 
     // tensor memory: all 512 columns (two sets of two accumulators of 32, then the A slots of 64), allocated and freed by
-    // the MMA warp
+    // the MMA warp. The allocation takes a microsecond: the producer, which has no use for it, goes ahead.
     if (warp == kTcMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem0 = *tmem_slot;
+    uint32_t tmem0 = 0;
+    if (warp != kTcProducerWarp) {
+        tc_fence_before();
+        asm volatile("bar.sync 2, %0;" ::"n"((kTcWarps - 1) * 32) : "memory");
+        tc_fence_after();
+        tmem0 = *tmem_slot;
+    }
 
     if (warp == kTcProducerWarp) {
         // ---------------------------------------------------------------- producer (as in tkd_stream_kernel; the whole
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 cursor_next(c, p);
             const Flow f = flow_of(c, p, it, i0, i1);
             const TkdSegDev& sg = p.seg[c.seg];
-            const int plw = p.rep_panels ? c.pl % p.rep_panels : c.pl;  // (the panel's number in its weight)
+            const int plw = !PLAIN && p.rep_panels ? c.pl % p.rep_panels : c.pl;  // (the panel's number in its weight)
             const int n = glu2 ? c.pl * 64 + (et & 63) : plw * TKD_PANEL_COLS + et;
             const bool in_w = n < sg.n_valid;
             int ebyte = 0;
@@ -550,11 +555,12 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 if (lane == 0) mbar_arrive(accempty0 + 8 * buf);
             }
             if (f.store) {
-                // the running sums into the scratch slot of (panel, slice): [row][128 columns] (the first half of a slot
-                // as tkd_stream_kernel lays it out; there is no second half here)
-                float* scr = p.scratch + (size_t)(c.panel * p.nslices + c.slice) * 2 * M * TKD_PANEL_COLS + et;
-#pragma unroll 1
-                for (int m = 0; m < M; ++m) __stcg(scr + (size_t)m * TKD_PANEL_COLS, trow[m]);
+                // the running sums into the scratch slot of (panel, slice): [row / 4][128 columns][4] (within a slot's first half
+                // as tkd_stream_kernel lays it out, rounded up to four rows; there is no second half here)
+                float* scr = p.scratch + (size_t)(c.panel * p.nslices + c.slice) * 2 * M * TKD_PANEL_COLS + et * 4;
+#pragma unroll
+                for (int m = 0; m < 32; m += 4)
+                    if (m < M) __stcg(reinterpret_cast<float4*>(scr + m * TKD_PANEL_COLS), *reinterpret_cast<const float4*>(trow + m));
             }
             if (!f.deliver) continue;
             bool finish = !f.split;
@@ -575,62 +581,58 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                     const int64_t owner = idiv(p, (pfirst + 1) * gridDim.x - 1, T);
                     const int64_t oend = idiv(p, T * (owner + 1), gridDim.x);
                     const int pe = (int)min((int64_t)p.nslices, oend - pfirst);
-                    const float* s0 = p.scratch + pfirst * 2 * M * TKD_PANEL_COLS + et;
-                    auto term = [&](int s, int m) { return __ldcg(s0 + ((size_t)(s * 2) * M + m) * TKD_PANEL_COLS); };
                     const int ns = p.nslices - pe + 1;  // sums to add: the owner's, then one per later slice
-                    if (j == nitems - 1 && (size_t)ns * M * 512 <= (size_t)nst * p.stage_bytes) {
-                        // The CTA's last item: the ring is idle, and the sums (M x 512 bytes a slice, contiguous) are copied
-                        // into it 16 bytes at a time, all copies in flight together (one trip to L2 instead of one per 32
-                        // loads a thread), then added up in slice order from shared memory.
-                        const uint32_t ring_a = smem_u32(ring);
-                        const int per = M * 32;  // 16-byte pieces of a slice's sums
-                        for (int si = 0; si < ns; ++si) {
-                            const float* src = p.scratch + ((pfirst + pe - 1 + si) * 2 * M) * TKD_PANEL_COLS;
-                            const uint32_t dst = ring_a + si * per * 16;
-                            for (int q = et; q < per; q += 128)
-                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + q * 16), "l"(src + q * 4)
-                                             : "memory");
+                    auto part = [&](int si) { return p.scratch + (size_t)(pfirst + pe - 1 + si) * 2 * M * TKD_PANEL_COLS + et * 4; };
+                    const int m4 = (M + 3) >> 2;
+                    // The CTA's last item: the ring is idle, and this column's sums of every slice come into it with all
+                    // copies in flight together (one trip to L2 instead of one for every four rows), then are added up in
+                    // slice order from shared memory.
+                    const bool staged = j == nitems - 1 && (size_t)ns * m4 * 2048 <= (size_t)nst * p.stage_bytes;
+                    const uint32_t ring_c = smem_u32(ring) + et * 16;
+                    if (staged) {
+                        uint32_t dst = ring_c;
+                        for (int si = 0; si < ns; ++si, dst += m4 * 2048) {
+                            const float* src = part(si);
+#pragma unroll
+                            for (int q = 0; q < 8; ++q)
+                                if (q < m4)
+                                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + q * 2048), "l"(src + q * 512) : "memory");
                         }
                         asm volatile("cp.async.wait_all;" ::: "memory");
-                        bar_output_warps();
-                        const float* rs = reinterpret_cast<const float*>(ring) + et;
+                    }
+                    // eight rows of four slices at a time, their loads side by side (a row past M: what lies there)
+                    const float* src0 = part(0);
+                    const size_t step = (size_t)2 * M * TKD_PANEL_COLS;
 #pragma unroll 1
-                        for (int rb = 0; rb < M; rb += 8) {  // (eight rows' loads at a time; a row past M re-reads the last)
-                            float th[8];
-#pragma unroll
-                            for (int m = 0; m < 8; ++m) th[m] = rs[(size_t)min(rb + m, M - 1) * TKD_PANEL_COLS];
+                    for (int r = 0; r < m4; r += 2) {
+                        float4 th[2] = {};
 #pragma unroll 1
-                            for (int si = 1; si < ns; ++si) {
-                                float v[8];
+                        for (int s4 = 0; s4 < ns; s4 += 4) {
+                            float4 v[4][2];
 #pragma unroll
-                                for (int m = 0; m < 8; ++m) v[m] = rs[((size_t)si * M + min(rb + m, M - 1)) * TKD_PANEL_COLS];
+                            for (int u = 0; u < 4; ++u) {
+                                const int si = min(s4 + u, ns - 1);
+                                const float4* src_g = reinterpret_cast<const float4*>(src0 + si * step + r * 512);
+                                const uint32_t src_s = ring_c + (si * m4 + r) * 2048;
 #pragma unroll
-                                for (int m = 0; m < 8; ++m) th[m] += v[m];
-                            }
-                            *reinterpret_cast<float4*>(trow + rb) = make_float4(th[0], th[1], th[2], th[3]);
-                            *reinterpret_cast<float4*>(trow + rb + 4) = make_float4(th[4], th[5], th[6], th[7]);
-                        }
-                    } else
-#pragma unroll 1
-                    for (int rb = 0; rb < M; rb += 8) {
-                        float th[8];
-#pragma unroll 1
-                        for (int s = pe - 1; s < p.nslices; s += 4) {
-                            float v[4][8];
-#pragma unroll
-                            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                                for (int m = 0; m < 8; ++m) v[q][m] = term(min(s + q, p.nslices - 1), min(rb + m, M - 1));
-#pragma unroll
-                            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                                for (int m = 0; m < 8; ++m) {
-                                    if (s + q >= p.nslices) continue;
-                                    th[m] = s + q == pe - 1 ? v[q][m] : th[m] + v[q][m];
+                                for (int q = 0; q < 2; ++q) {
+                                    if (staged) {
+                                        const uint4 w = lds128(src_s + q * 2048);
+                                        v[u][q] = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+                                    } else {
+                                        v[u][q] = __ldcg(src_g + q * 128);
+                                    }
                                 }
+                            }
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+                                if (s4 + u < ns)
+#pragma unroll
+                                    for (int q = 0; q < 2; ++q)
+                                        th[q] = make_float4(th[q].x + v[u][q].x, th[q].y + v[u][q].y, th[q].z + v[u][q].z, th[q].w + v[u][q].w);
                         }
-                        *reinterpret_cast<float4*>(trow + rb) = make_float4(th[0], th[1], th[2], th[3]);
-                        *reinterpret_cast<float4*>(trow + rb + 4) = make_float4(th[4], th[5], th[6], th[7]);
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) *reinterpret_cast<float4*>(trow + 4 * (r + q)) = th[q];
                     }
                 }
                 bar_output_warps();  // sflag may be written again only after everyone has read it
@@ -648,6 +650,91 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 }
                 const float cols = p.scale_dt != TKD_DT_NONE && in_w ? sc : 1.f;
                 const bool glu = p.epi == TKD_EPI_GLU_IL || glu2;
+                if constexpr (PLAIN) {
+                    // A thread keeps its column, sixteen rows at a time. GLU: the up columns' sums go back scaled first, then
+                    // the gate columns' threads make the outputs.
+                    const bool gate = glu2 ? ow < 2 : !(ow & 1);
+                    int oc = -1;  // the output column this thread stores
+                    if (!glu) {
+                        if (in_w) oc = sg.out_col0 + n;
+                    } else if (gate) {
+                        const int o = c.pl * 64 + (glu2 ? et : (ow >> 1) * 32 + lane);
+                        if (o < (glu2 ? sg.n_valid : sg.n_valid / 2)) oc = sg.out_col0 + o;
+                    }
+                    const float* up = trow + (glu2 ? 64 : 32) * MP;
+                    if (glu) {
+                        if (!gate)
+#pragma unroll 1
+                            for (int r = 0; r < M; r += 4) {
+                                const float4 u = *reinterpret_cast<const float4*>(trow + r);
+                                *reinterpret_cast<float4*>(trow + r) = make_float4(u.x * colf * colg * cols, u.y * colf * colg * cols,
+                                                                                   u.z * colf * colg * cols, u.w * colf * colg * cols);
+                            }
+                        bar_output_warps();
+                    }
+                    const bool f32out = p.epi == TKD_EPI_OUT32, odd = lane & 1;
+                    const int esz = f32out ? 4 : 2, rsz = p.res_dt == TKD_DT_F32 ? 4 : 2;
+                    // (two bf16 columns a store: an even lane takes both columns' even rows, its neighbour the odd ones)
+                    const bool fast = !f32out && !((reinterpret_cast<uintptr_t>(p.out) & 3) | (p.ldo & 1) | (sg.out_col0 & 1)) &&
+                                      __all_sync(0xFFFFFFFFu, oc >= 0);
+                    const uint32_t pick = odd ? 0x3276u : 0x5410u;
+                    if (!glu || gate)
+#pragma unroll 1
+                        for (int r = 0; r < M; r += 16) {
+                            float v[16];
+                            uint32_t q[16];
+                            const bool res = p.res && oc >= 0;
+                            if (res) {
+                                // (a row past M reads the last again)
+                                const char* rp = static_cast<const char*>(p.res) + ((int64_t)r * p.ldr + oc) * rsz;
+#pragma unroll
+                                for (int m = 0; m < 16; ++m) {
+                                    q[m] = rsz == 4 ? *reinterpret_cast<const uint32_t*>(rp) : (uint32_t)*reinterpret_cast<const uint16_t*>(rp) << 16;
+                                    if (r + m + 1 < M) rp += p.ldr * rsz;
+                                }
+                            }
+#pragma unroll
+                            for (int m = 0; m < 16; m += 4) {
+                                const float4 g = *reinterpret_cast<const float4*>(trow + r + m);
+                                v[m] = g.x, v[m + 1] = g.y, v[m + 2] = g.z, v[m + 3] = g.w;
+                            }
+#pragma unroll
+                            for (int m = 0; m < 16; ++m) v[m] = v[m] * colf * colg * cols;
+                            if (glu) {
+#pragma unroll
+                                for (int m = 0; m < 16; m += 4) {
+                                    const float4 u = *reinterpret_cast<const float4*>(up + r + m);
+                                    v[m] = act_gate(v[m], p.act) * u.x, v[m + 1] = act_gate(v[m + 1], p.act) * u.y;
+                                    v[m + 2] = act_gate(v[m + 2], p.act) * u.z, v[m + 3] = act_gate(v[m + 3], p.act) * u.w;
+                                }
+                            }
+                            if (res) {
+#pragma unroll
+                                for (int m = 0; m < 16; ++m) v[m] += __uint_as_float(q[m]);
+                            }
+                            if (fast) {
+                                uint16_t* yp = y16 + (int64_t)(r + odd) * p.ldo + oc - odd;
+                                const int left = M - r - odd;
+#pragma unroll
+                                for (int m = 0; m < 8; ++m, yp += 2 * p.ldo) {
+                                    const uint32_t mine = f32x2_to_bf16x2(v[2 * m], v[2 * m + 1]);
+                                    st_if(2 * m < left, yp, __byte_perm(mine, __shfl_xor_sync(0xFFFFFFFFu, mine, 1), pick));
+                                }
+                            } else {
+                                char* yp = static_cast<char*>(p.out) + ((int64_t)r * p.ldo + oc) * esz;
+                                const int left = oc >= 0 ? M - r : 0;
+#pragma unroll
+                                for (int m = 0; m < 16; ++m, yp += p.ldo * esz) {
+                                    if (f32out)
+                                        st_if(m < left, yp, __float_as_uint(v[m]));
+                                    else
+                                        st16_if(m < left, yp, f32_to_bf16_bits(v[m]));
+                                }
+                            }
+                        }
+                    if (glu) bar_output_warps();  // (the up columns have been read)
+                    continue;
+                }
                 if (topk_k == 0) {
                     // No records: the panel leaves through a transposition in shared memory. Every thread scales its own
                     // column in place; then a lane is a ROW and a warp takes every fourth group of 8 output columns:
@@ -869,9 +956,9 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     }
 }
 
-template <int FMT, bool KWHOLE>
+template <int FMT, bool KWHOLE, bool PLAIN>
 int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
-    auto kern = tkd_stream_tc_kernel<FMT, KWHOLE>;
+    auto kern = tkd_stream_tc_kernel<FMT, KWHOLE, PLAIN>;
     static bool allowed[64] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -897,8 +984,9 @@ int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
 template <int FMT>
 int launch_fmt_all(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     if (p.tc) {
-        return p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0 ? launch_tc<FMT, true>(p, grid, smem, st)
-                                                           : launch_tc<FMT, false>(p, grid, smem, st);
+        const bool whole = p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0;
+        if (!p.topk_k && !p.npeers) return whole ? launch_tc<FMT, true, true>(p, grid, smem, st) : launch_tc<FMT, false, true>(p, grid, smem, st);
+        return whole ? launch_tc<FMT, true, false>(p, grid, smem, st) : launch_tc<FMT, false, false>(p, grid, smem, st);
     }
     return launch_fmt<FMT>(p, grid, smem, st);
 }

@@ -58,13 +58,6 @@ __device__ __forceinline__ void wide_mma(uint32_t d, uint32_t a, uint32_t blo, u
         : "memory");
 }
 
-// two floats as a bf16 pair, the first in the lower half
-__device__ __forceinline__ uint32_t f32x2_to_bf16x2(float lo, float hi) {
-    uint32_t d;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
-    return d;
-}
-
 // A part of a CTA's run that lies in one tile.
 struct WideSeg {
     int tile, c0, c1;  // chunks c0 .. c1 - 1 of the tile
@@ -361,14 +354,19 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
         sflag[0] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncthreads();
+    // (the allocation takes a microsecond: the producers, which have no use for it, go ahead)
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem0 = *tmem_slot;
+    uint32_t tmem0 = 0;
+    if (warp != kWideRing && warp != kWideX) {
+        tc_fence_before();
+        asm volatile("bar.sync 2, %0;" ::"n"((kWideWarps - 2) * 32) : "memory");
+        tc_fence_after();
+        tmem0 = *tmem_slot;
+    }
     const int i0 = wide_begin(p, blockIdx.x), i1 = wide_begin(p, blockIdx.x + 1);
     const int K = p.K, nst = p.nstages, NT = p.nt, nx = p.nx;
     const bool glu2 = p.epi == TKD_EPI_GLU2;
