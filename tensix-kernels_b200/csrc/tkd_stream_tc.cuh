@@ -158,13 +158,10 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    uint32_t tmem0 = 0;
-    if (warp != kTcProducerWarp) {
-        tc_fence_before();
-        asm volatile("bar.sync 2, %0;" ::"n"((kTcWarps - 1) * 32) : "memory");
-        tc_fence_after();
-        tmem0 = *tmem_slot;
-    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem0 = *tmem_slot;
 
     if (warp == kTcProducerWarp) {
         // ---------------------------------------------------------------- producer (as in tkd_stream_kernel; the whole

@@ -354,19 +354,14 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
         sflag[0] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
-    // (the allocation takes a microsecond: the producers, which have no use for it, go ahead)
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    uint32_t tmem0 = 0;
-    if (warp != kWideRing && warp != kWideX) {
-        tc_fence_before();
-        asm volatile("bar.sync 2, %0;" ::"n"((kWideWarps - 2) * 32) : "memory");
-        tc_fence_after();
-        tmem0 = *tmem_slot;
-    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem0 = *tmem_slot;
     const int i0 = wide_begin(p, blockIdx.x), i1 = wide_begin(p, blockIdx.x + 1);
     const int K = p.K, nst = p.nstages, NT = p.nt, nx = p.nx;
     const bool glu2 = p.epi == TKD_EPI_GLU2;
