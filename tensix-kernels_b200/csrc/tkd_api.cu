@@ -49,7 +49,8 @@ struct Layout {
 };
 
 // Everything a launch needs except the device pointers into the workspace. sms 0: ask the device.
-int make_layout(const TkdMatmul* a, Layout* L, int sms) {
+// counted: the kernel with the counters and slice sums of the workspace, even where tkd_narrow_kernel could run.
+int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     if (!a || !fmt_ok(a->fmt)) return TKD_ERR_BAD_ARG;
     if (a->m < 1 || a->m > 32 || a->k < 32 || a->k % 32 || a->k > (1 << 24)) return TKD_ERR_BAD_ARG;
     // (the int4 weight with group scales is the reference's one-token op; more rows go through its dequantised
@@ -145,6 +146,18 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms) {
         const int64_t x_row = (a->k + chunk_k - 1) / chunk_k * chunk_k * 2 + (a->m > 1 ? 64 : 0);
         if (p.off_xt + a->m * x_row + 4 * (int64_t)p.stage_bytes + 256 <= kMaxSmem) {
             p.x_smem = 1;
+            p.x_stride = (int)x_row;
+            xt_bytes = a->m * x_row;
+        }
+        // Items of 32 columns over all of K (tkd_narrow.cuh) where the call is a plain one and K makes four slices of nearly
+        // the same length: a streaming warp stays with one slice, and where the last is short, its warps wait for the others'.
+        // (Three stages are enough there: 100 KB of loads in flight on an SM, of the 60 that its share of the memory's rate
+        // needs, and eight rows of K 5632 in bf16 would not fit beside four.)
+        const int64_t narrow_xt = p.off_pbuf + 2 * 8 * 32 * (a->m > 1 ? 8 : 1) * 4;
+        if (!counted && p.nslices == 4 && 4 * p.ks - p.K < p.ks / 2 && !a->topk_k && a->nranks <= 1 &&
+            narrow_xt + a->m * x_row + 3 * (int64_t)p.stage_bytes + 128 <= kMaxSmem) {
+            p.narrow = p.x_smem = 1;
+            p.off_xt = (int)narrow_xt;
             p.x_stride = (int)x_row;
             xt_bytes = a->m * x_row;
         }
@@ -437,9 +450,9 @@ int tkd_matmul_rows(const TkdMatmul* a, void* stream) {
                                          : a->fmt == TKD_BFP4 ? tkd_launch_wide_bfp4(p, smem, st) : tkd_launch_wide_bf16(p, smem, st));
 }
 
-static int run_matmul(const TkdMatmul* a, void* workspace, uint64_t workspace_bytes, void* stream) {
+static int run_matmul(const TkdMatmul* a, void* workspace, uint64_t workspace_bytes, void* stream, bool counted = false) {
     Layout L;
-    const int rc = make_layout(a, &L, 0);
+    const int rc = make_layout(a, &L, 0, counted);
     if (rc) return rc;
     TkdParams& p = L.p;
     const int ra = check_pointers(a);
@@ -540,7 +553,7 @@ static int noalloc_address(void** out, bool* first) {
 
 int tkd_matmul_noalloc(const TkdMatmul* a, void* stream) {
     Layout L;
-    const int rc = make_layout(a, &L, 0);
+    const int rc = make_layout(a, &L, 0, true);
     if (rc) return rc;
     if ((uint64_t)L.ws_bytes > (uint64_t)TKD_NOALLOC_SCRATCH_BYTES) return TKD_ERR_FIXED_SCRATCH;
     void* ptr = nullptr;
@@ -552,7 +565,8 @@ int tkd_matmul_noalloc(const TkdMatmul* a, void* stream) {
         const cudaError_t e = cudaMemsetAsync(ptr, 0, (size_t)kCounterBytes, static_cast<cudaStream_t>(stream));
         if (e != cudaSuccess) return cuda_err(e);
     }
-    return run_matmul(a, ptr, TKD_NOALLOC_SCRATCH_BYTES, stream);
+    // (its counters and their reset are part of this entry point: it stays with the kernel that uses them)
+    return run_matmul(a, ptr, TKD_NOALLOC_SCRATCH_BYTES, stream, true);
 }
 
 int tkd_matmul_noalloc_reset(void* stream) {

@@ -93,6 +93,7 @@ struct TkdParams {
     int exchange_wait;
     int tc;              // 9 to 32 rows: the tensor-memory kernel (tkd_stream_tc.cuh); off_xt is where its operand tiles go
     int x_smem;          // 1 to 8 rows, and all of x (K rounded up to a chunk) fits in shared memory at off_xt
+    int narrow;          // ... and the call runs tkd_narrow_kernel (tkd_narrow.cuh)
     int x_stride;        // ... bytes from one row of it to the next
     int no_pdl;          // launch without programmatic dependent launch (the weights may still be being written)
     const uint32_t* had;  // TKD_INT4: sign words of the block Hadamard applied to x in shared memory first (or null)
