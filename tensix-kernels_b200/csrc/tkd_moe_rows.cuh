@@ -233,8 +233,8 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
 #pragma unroll
                                 for (int jj = 0; jj < 2; ++jj) {
                                     const uint32_t w = cwd[jj], w8 = __funnelshift_r(w, w, 8);
-                                    const uint32_t s0 = (ewd[jj] & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
-                                    const uint32_t s1 = (shl_fma<7>(ewd[jj], sh.y) & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
+                                    const uint32_t s0 = and_or(ewd[jj], TKD_EMASK_BFP4, ebase(sh));
+                                    const uint32_t s1 = and_or(shl_fma<7>(ewd[jj], sh.y), TKD_EMASK_BFP4, ebase(sh));
                                     const uint32_t a0 = mul_bf16x2(w & TKD_MASK_BFP4, s0), a1 = mul_bf16x2(shl_fma<4>(w, sh.x) & TKD_MASK_BFP4, s0);
                                     const uint32_t a2 = mul_bf16x2(w8 & TKD_MASK_BFP4, s1), a3 = mul_bf16x2(shl_fma<4>(w8, sh.x) & TKD_MASK_BFP4, s1);
 #pragma unroll

@@ -21,6 +21,11 @@ namespace {
 
 constexpr int kNarrowWarps = 19;
 
+__device__ __forceinline__ void sts32(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts64(uint32_t a, float v, float w) {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v), "f"(w) : "memory");
+}
+
 // Where item `pl` of a segment lies: the panel and the two groups in it.
 struct NarrowItem {
     int panel, ga, gb;
@@ -43,7 +48,6 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + TKD_MAX_STAGES);
     const uint32_t pfull0 = smem_u32(bars + 2 * TKD_MAX_STAGES), pempty0 = pfull0 + 16, xbar = pfull0 + 32;
-    uint2* hdr = reinterpret_cast<uint2*>(smem + 512);          // a stage's flags and its chunk's number in the slices
     float* pbuf = reinterpret_cast<float*>(smem + p.off_pbuf);  // [2 items][4 slices][2 halves][32 columns][MR]
     const uint32_t ring_a = smem_u32(smem + p.off_ring), xt0 = smem_u32(smem + p.off_xt);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -60,7 +64,6 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
     const int nst = p.nstages, M = ONE ? 1 : p.M, K = p.K, cps = p.ks / CK, nch = (K + CK - 1) / CK;
     const int nsa_total = (K + F::KSA - 1) / F::KSA;
     const bool glu = p.epi == TKD_EPI_GLU2 || p.epi == TKD_EPI_GLU_IL;
-    const int depth = cps;
     auto seg_of = [&](int it) {
         int s = 0;
 #pragma unroll
@@ -79,7 +82,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
             const TkdSegDev& sg = p.seg[seg_of(it)];
             const NarrowItem n = narrow_item(p, it - 4 * sg.panel0);
             const uint8_t* src = (g && p.epi == TKD_EPI_GLU2 ? sg.w2 : sg.w) + (int64_t)n.panel * p.panel_bytes;
-            for (int i = 0; i < depth; ++i, ++st) {
+            for (int i = 0; i < cps; ++i, ++st) {
                 const uint32_t q = st % nst;
                 ok = __all_sync(0xFFFFFFFFu, mbar_wait_parked(empty0 + 8 * q, ((st / nst) & 1) ^ 1, p.status));
                 if (!ok) break;
@@ -87,10 +90,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
                 const bool mine = lane < 8 && c < nch && (glu || !g);
                 const uint32_t gb = mine ? (uint32_t)min(F::SUBSA, nsa_total - c * F::SUBSA) * F::SAB : 0u, bytes = glu ? gb : 2 * gb;
                 const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, bytes);
-                if (lane == 0) {
-                    hdr[q] = make_uint2((i == 0 ? ST_FIRST : 0u) | (i == depth - 1 ? ST_LAST | (it == i1 - 1 ? ST_END : 0u) : 0u), (uint32_t)i);
-                    mbar_expect_tx(full0 + 8 * q, all);
-                }
+                if (lane == 0) mbar_expect_tx(full0 + 8 * q, all);
                 __syncwarp();
                 if (mine)
                     bulk_g2s(ring_a + q * p.stage_bytes + s * 2 * GB + g * gb, src + (int64_t)c * (GB * 8) + (int64_t)(g ? n.gb : n.ga) * gb, bytes,
@@ -119,58 +119,60 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
             for (int r = 0; r < M; ++r) bulk_g2s(xt0 + (ONE ? 0 : r * p.x_stride), p.x + (int64_t)r * p.ldx, (uint32_t)(K * 2), xbar);
         }
         const int g = lane >> 2, t = lane & 3;
-        const uint32_t hdr_a = smem_u32(hdr), exp_lane = FMT == TKD_INT4 ? g * 8 : t * (EXPB / 4);
-        const uint32_t lane_off = sl * 2 * GB + h * F::SAB;
+        const uint32_t exp_lane = FMT == TKD_INT4 ? g * 8 : t * (EXPB / 4);
+        const uint32_t lane_off = sl * 2 * GB + gsel * GB + h * F::SAB;
         // (a lane whose row lies beyond M reads row M - 1: a column of B only feeds its own column of D)
         const uint32_t xs_lane = xt0 + (ONE ? 0 : min(g, M - 1) * p.x_stride) + (8 * t + h * F::KSA) * 2;
         const uint2 sh = make_uint2(p.mul16, p.mul128);
         const uint16_t* const no_x[1] = {nullptr};
         const uint4 no_pre[F::SUBSA / 2 * F::XB][1] = {};
         float acc[2][1][4];
-        uint32_t slot = 0, phase = 0, j = 0;
-        const bool x_here = mbar_wait(xbar, 0, p.status);
+        bool ok = mbar_wait(xbar, 0, p.status);
         if constexpr (FMT == TKD_INT4)
-            if (p.had && x_here) hadamard_rows<ONE>(p, xt0, cw, lane, M);
-        while (x_here) {
-            if (!mbar_wait(full0 + 8 * slot, phase, p.status)) break;
-            const uint2 hd = lds64(hdr_a + 8 * slot);
-            const uint32_t fl = hd.x;
-            if (fl & ST_FIRST) {
+            if (p.had && ok) hadamard_rows<ONE>(p, xt0, cw, lane, M);
+        const int c0 = sl * cps, mine = min(cps, nch - c0);  // (the last slice may have fewer chunks)
+        const uint32_t xs0 = xs_lane + c0 * CK * 2;
+        const uint32_t ring_end = ring_a + nst * p.stage_bytes;
+        uint32_t at = ring_a, bar = full0, phase = 0;  // the stage, its barrier, its parity
+        // (where this lane's sums go, of two buffers)
+        uint32_t pc = smem_u32(pbuf) + (((sl * 2 + h) * 32 + gsel * 16 + g) * MR + (ONE ? 0 : 2 * t)) * 4, pbar = pfull0, pphase = 1;
+        int other = 8 * 32 * MR * 4;
+        for (int j = 0; ok && j < i1 - i0; ++j) {
 #pragma unroll
-                for (int a = 0; a < 2; ++a) acc[a][0][0] = acc[a][0][1] = acc[a][0][2] = acc[a][0][3] = 0.f;
-            }
-            const int c = sl * cps + (int)hd.y, kc = c * CK;
-            const uint32_t sb = ring_a + slot * p.stage_bytes + lane_off;
-            if (c < nch) {  // (not past K; a slice has cps chunks)
-                if (KWHOLE || kc + CK <= K) {
-                    const uint32_t a = sb + gsel * GB;
-                    chunk_mma<FMT, 1, 2, true, false, true>(acc, a + EXPB + lane * 16, a + exp_lane, no_pre, no_x, kc, K, h, F::SUBSA, sh,
-                                                            xs_lane + kc * 2);
-                } else {
-                    const int nsa = nsa_total - c * F::SUBSA;
-                    const uint32_t a = sb + gsel * nsa * F::SAB;
-                    chunk_mma<FMT, 1, 2, false, false, true>(acc, a + EXPB + lane * 16, a + exp_lane, no_pre, no_x, kc, K, h, nsa, sh,
-                                                             xs_lane + kc * 2);
+            for (int a = 0; a < 2; ++a) acc[a][0][0] = acc[a][0][1] = acc[a][0][2] = acc[a][0][3] = 0.f;
+            uint32_t xs = xs0;
+#pragma unroll 1
+            for (int i = 0; i < cps; ++i, xs += CK * 2) {
+                ok = mbar_wait(bar, phase, p.status);
+                if (!ok) break;
+                const uint32_t a = at + lane_off;
+                if (i < mine) {
+                    if (KWHOLE || (c0 + i + 1) * CK <= K) {
+                        chunk_mma<FMT, 1, 2, true, false, true>(acc, a + EXPB + lane * 16, a + exp_lane, no_pre, no_x, 0, K, h, F::SUBSA, sh, xs);
+                    } else {
+                        const int nsa = nsa_total - (c0 + i) * F::SUBSA;  // (the groups lie closer together)
+                        const uint32_t b = a - gsel * (GB - nsa * F::SAB);
+                        chunk_mma<FMT, 1, 2, false, false, true>(acc, b + EXPB + lane * 16, b + exp_lane, no_pre, no_x, (c0 + i) * CK, K, h, nsa, sh, xs);
+                    }
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar + 8 * TKD_MAX_STAGES);
+                at += p.stage_bytes, bar += 8;
+                if (at == ring_end) at = ring_a, bar = full0, phase ^= 1;
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty0 + 8 * slot);
-            if (++slot == (uint32_t)nst) slot = 0, phase ^= 1;
-            if (!(fl & ST_LAST)) continue;
+            if (!ok) break;
             // ---- the item's sums of this slice, half and group
-            const uint32_t b = j & 1;
-            if (!mbar_wait(pempty0 + 8 * b, ((j >> 1) & 1) ^ 1, p.status)) break;
-            float* pc = pbuf + (((size_t)b * 8 + sl * 2 + h) * 32 + gsel * 16 + g) * MR;
+            if (!mbar_wait(pbar + 16, pphase, p.status)) break;
             if constexpr (ONE) {
-                if (t == 0) pc[0] = acc[0][0][0] + acc[1][0][0], pc[8] = acc[0][0][2] + acc[1][0][2];
+                if (t == 0) sts32(pc, acc[0][0][0] + acc[1][0][0]), sts32(pc + 32, acc[0][0][2] + acc[1][0][2]);
             } else {
-                *reinterpret_cast<float2*>(pc + 2 * t) = make_float2(acc[0][0][0] + acc[1][0][0], acc[0][0][1] + acc[1][0][1]);
-                *reinterpret_cast<float2*>(pc + 8 * MR + 2 * t) = make_float2(acc[0][0][2] + acc[1][0][2], acc[0][0][3] + acc[1][0][3]);
+                sts64(pc, acc[0][0][0] + acc[1][0][0], acc[0][0][1] + acc[1][0][1]);
+                sts64(pc + 8 * MR * 4, acc[0][0][2] + acc[1][0][2], acc[0][0][3] + acc[1][0][3]);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(pfull0 + 8 * b);
-            ++j;
-            if (fl & ST_END) break;
+            if (lane == 0) mbar_arrive(pbar);
+            pc += other, other = -other, pbar ^= 8;
+            if (pbar == pfull0) pphase ^= 1;
         }
     } else {
         // ---------------------------------------------------------------- output warps

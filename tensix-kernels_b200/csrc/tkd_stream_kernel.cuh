@@ -36,6 +36,7 @@
 #include <stdint.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "tkd_internal.h"
 #include "tkd_layout.h"
@@ -118,6 +119,13 @@ __device__ __forceinline__ uint32_t shl_fma(uint32_t w, uint32_t pow2) {
     return d;
 #endif
 }
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+// TKD_EBASE_BFP4, as a value the compiler cannot see through (sh: the multipliers of shl_fma)
+__device__ __forceinline__ uint32_t ebase(const uint2 sh) { return sh.y * (TKD_EBASE_BFP4 / 128); }
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -125,7 +133,7 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -271,12 +279,14 @@ __device__ __forceinline__ void block_mma(float (&acc)[NA][MT][4], const uint32_
         uint32_t a0, a1, a2, a3;
         uint32_t s0, s1;
         if constexpr (FMT == TKD_BFP4) {
-            // (five integer-pipe operations and three multiplies for the 8 codes and 4 exponents of a word each)
+            // (seven integer-pipe operations and three multiplies for the 8 codes and 4 exponents of a word each. and_or wants its
+            // third operand in a register: with two constants it was two operations, and the loop 11 % longer.)
+            const uint32_t base = ebase(sh);
             const uint32_t w = cw[jj], t = __funnelshift_r(w, w, 8);
             a0 = w & TKD_MASK_BFP4, a1 = shl_fma<4>(w, sh.x) & TKD_MASK_BFP4;
             a2 = t & TKD_MASK_BFP4, a3 = shl_fma<4>(t, sh.x) & TKD_MASK_BFP4;
-            s0 = (ew[jj] & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
-            s1 = (shl_fma<7>(ew[jj], sh.y) & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
+            s0 = and_or(ew[jj], TKD_EMASK_BFP4, base);
+            s1 = and_or(shl_fma<7>(ew[jj], sh.y), TKD_EMASK_BFP4, base);
         } else {
             const uint32_t w0 = cw[2 * jj], w1 = cw[2 * jj + 1];
             a0 = w0 & TKD_MASK_BFP8, a1 = rot_and<8>(w0, TKD_MASK_BFP8);
@@ -301,6 +311,24 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
     return v;
+}
+
+// ... at a constant distance from an address: the load's own offset, no instruction for it
+template <int OFF>
+__device__ __forceinline__ uint4 lds128_at(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+%5];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a), "n"(OFF));
+    return v;
+}
+template <int OFF>
+__device__ __forceinline__ uint2 lds64_at(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2+%3];" : "=r"(v.x), "=r"(v.y) : "r"(a), "n"(OFF));
+    return v;
+}
+template <class F, int... I>
+__device__ __forceinline__ void unrolled(std::integer_sequence<int, I...>, F f) {
+    (f(std::integral_constant<int, I>{}), ...);
 }
 
 // What a stage of the ring holds for the streaming warps besides the weights: a 16-byte header the producer writes.
@@ -328,50 +356,50 @@ __device__ __forceinline__ void chunk_mma(float (&acc)[NA][MT][4], uint32_t code
                                           uint32_t xt_a = 0) {
     using F = Fmt<FMT>;
     constexpr int NPW = F::SUBSA / 2;  // super-atoms a warp takes of a chunk
-#pragma unroll
-    for (int i = 0; i < NPW; ++i) {
-        if (!FULL && h + 2 * i >= nsa) break;
+    unrolled(std::make_integer_sequence<int, NPW>{}, [&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        if (!FULL && h + 2 * i >= nsa) return;
         uint32_t cw[F::XB][4], ew[F::XB][2];
         if constexpr (FMT == TKD_BFP4) {
-            const uint4 ev = lds128(exp_a + 2 * i * F::SAB), cv = lds128(code_a + 2 * i * F::SAB);
+            const uint4 ev = lds128_at<2 * i * F::SAB>(exp_a), cv = lds128_at<2 * i * F::SAB>(code_a);
             cw[0][0] = cv.x, cw[0][1] = cv.y, cw[1][0] = cv.z, cw[1][1] = cv.w;
             cw[0][2] = cw[0][3] = cw[1][2] = cw[1][3] = 0;
             ew[0][0] = ev.x, ew[0][1] = ev.y, ew[1][0] = ev.z, ew[1][1] = ev.w;
         } else if constexpr (FMT == TKD_INT4) {
             // (exp_a: this lane's two scale words of the super-atom, one per k32 block: columns g and g + 8)
-            const uint2 sv = lds64(exp_a + 2 * i * F::SAB);
-            const uint4 cv = lds128(code_a + 2 * i * F::SAB);
+            const uint2 sv = lds64_at<2 * i * F::SAB>(exp_a);
+            const uint4 cv = lds128_at<2 * i * F::SAB>(code_a);
             cw[0][0] = cv.x, cw[0][1] = cv.y, cw[1][0] = cv.z, cw[1][1] = cv.w;
             cw[0][2] = cw[0][3] = cw[1][2] = cw[1][3] = 0;
             ew[0][0] = sv.x, ew[1][0] = sv.y, ew[0][1] = ew[1][1] = 0;
         } else if constexpr (FMT == TKD_BFP8) {
-            const uint2 ev = lds64(exp_a + 2 * i * F::SAB);
-            const uint4 cv = lds128(code_a + 2 * i * F::SAB);
+            const uint2 ev = lds64_at<2 * i * F::SAB>(exp_a);
+            const uint4 cv = lds128_at<2 * i * F::SAB>(code_a);
             cw[0][0] = cv.x, cw[0][1] = cv.y, cw[0][2] = cv.z, cw[0][3] = cv.w;
             ew[0][0] = ev.x, ew[0][1] = ev.y;
         }
-#pragma unroll
-        for (int q = 0; q < F::XB; ++q) {
+        unrolled(std::make_integer_sequence<int, F::XB>{}, [&](auto qc) {
+            constexpr int q = decltype(qc)::value;
             const int k = kc + 2 * i * F::KSA + 32 * q;  // (+ h * KSA, which xb carries)
-            if (!FULL && k + h * F::KSA >= K) break;     // a K that ends inside a super-atom
+            if (!FULL && k + h * F::KSA >= K) return;    // a K that ends inside a super-atom
             uint4 xv[MT];
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 if constexpr (XSM)  // (the one row of x, whole, in shared memory: xt_a is this lane's address at k = kc)
-                    xv[m] = lds128(xt_a + (2 * i * F::KSA + 32 * q) * 2);
+                    xv[m] = lds128_at<(2 * i * F::KSA + 32 * q) * 2>(xt_a);
                 else if constexpr (FULL && PRE)
                     xv[m] = xpre[i * F::XB + q][m];
                 else
                     xv[m] = ldg_x(xb[m] + k);
             }
             if constexpr (FMT == TKD_BF16) {
-#pragma unroll
-                for (int jj = 0; jj < 2; ++jj) {
-                    const uint4 a = lds128(code_a + 2 * i * F::SAB + jj * 512);
+                unrolled(std::make_integer_sequence<int, 2>{}, [&](auto jc) {
+                    constexpr int jj = decltype(jc)::value;
+                    const uint4 a = lds128_at<2 * i * F::SAB + jj * 512>(code_a);
 #pragma unroll
                     for (int m = 0; m < MT; ++m)
                         mma_bf16(acc[jj % NA][m], a.x, a.y, a.z, a.w, jj ? xv[m].z : xv[m].x, jj ? xv[m].w : xv[m].y);
-                }
+                });
             } else if constexpr (FMT == TKD_INT4) {
                 // The k32 block's codes (bf16 subnormals q * 2^-129) times the activations times 2^64, summed from zero;
                 // then the block's scale (s * 2^65, a pair of bf16 in ew[q][0]: column g low, g + 8 high) takes the sum
@@ -395,8 +423,8 @@ __device__ __forceinline__ void chunk_mma(float (&acc)[NA][MT][4], uint32_t code
             } else {
                 block_mma<FMT, MT, NA>(acc, cw[q], ew[q], xv, sh);
             }
-        }
-    }
+        });
+    });
 }
 
 // bf16 output as the top-k records order it: a monotone 16-bit key, 0 below every value (dense_writer.cpp:215).

@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                             const uint32_t w = cwd[2 * q + jj], tt = __funnelshift_r(w, w, 8), ew = ewd[2 * q + jj];
                             a0 = w & TKD_MASK_BFP4, a1 = shl_fma<4>(w, sh.x) & TKD_MASK_BFP4;
                             a2 = tt & TKD_MASK_BFP4, a3 = shl_fma<4>(tt, sh.x) & TKD_MASK_BFP4;
-                            s0 = (ew & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
-                            s1 = (shl_fma<7>(ew, sh.y) & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
+                            s0 = and_or(ew, TKD_EMASK_BFP4, ebase(sh));
+                            s1 = and_or(shl_fma<7>(ew, sh.y), TKD_EMASK_BFP4, ebase(sh));
                         } else {
                             const uint32_t w0 = cwd[2 * jj], w1 = cwd[2 * jj + 1], ew = ewd[jj];
                             a0 = w0 & TKD_MASK_BFP8, a1 = rot_and<8>(w0, TKD_MASK_BFP8);

@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
                             const uint32_t w = cw_[2 * q + jj], tt = __funnelshift_r(w, w, 8), ew = ew_[2 * q + jj];
                             a0 = w & TKD_MASK_BFP4, a1 = shl_fma<4>(w, sh.x) & TKD_MASK_BFP4;
                             a2 = tt & TKD_MASK_BFP4, a3 = shl_fma<4>(tt, sh.x) & TKD_MASK_BFP4;
-                            s0 = (ew & TKD_EMASK_BFP4) | TKD_EBASE_BFP4, s1 = (shl_fma<7>(ew, sh.y) & TKD_EMASK_BFP4) | TKD_EBASE_BFP4;
+                            s0 = and_or(ew, TKD_EMASK_BFP4, ebase(sh)), s1 = and_or(shl_fma<7>(ew, sh.y), TKD_EMASK_BFP4, ebase(sh));
                         } else {
                             const uint32_t w0 = cw_[2 * jj], w1 = cw_[2 * jj + 1], ew = ew_[jj];
                             a0 = w0 & TKD_MASK_BFP8, a1 = rot_and<8>(w0, TKD_MASK_BFP8);
