@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
         float acc[2][1][4];
         bool ok = mbar_wait(xbar, 0, p.status);
         if constexpr (FMT == TKD_INT4)
-            if (p.had && ok) hadamard_rows<ONE>(p, xt0, cw, lane, M);
+            rows_for_int4<ONE>(p, xt0, cw, lane, M);
         const int c0 = sl * cps, mine = min(cps, nch - c0);  // (the last slice may have fewer chunks)
         const uint32_t xs0 = xs_lane + c0 * CK * 2;
         const uint32_t ring_end = ring_a + nst * p.stage_bytes;

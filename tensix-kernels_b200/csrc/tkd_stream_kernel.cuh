@@ -349,6 +349,7 @@ enum : uint32_t {
 // loaded before the stage was waited for, when PRE).
 // XSM: a one-row call keeps all of x in shared memory (zero-filled up to a whole chunk): xt_a is the address of this
 // lane's 16 bytes of the chunk's first block.
+constexpr uint32_t kInt4Scale = 0x5F805F80u;  // 2^64, twice
 template <int FMT, int MT, int NA, bool FULL, bool PRE, bool XSM = false>
 __device__ __forceinline__ void chunk_mma(float (&acc)[NA][MT][4], uint32_t code_a, uint32_t exp_a,
                                           const uint4 (&xpre)[Fmt<FMT>::SUBSA / 2 * Fmt<FMT>::XB][MT],
@@ -414,7 +415,10 @@ __device__ __forceinline__ void chunk_mma(float (&acc)[NA][MT][4], uint32_t code
                         const uint32_t a0 = w & TKD_MASK_BFP4, a1 = shl_fma<4>(w, sh.x) & TKD_MASK_BFP4;
                         const uint32_t a2 = t8 & TKD_MASK_BFP4, a3 = shl_fma<4>(t8, sh.x) & TKD_MASK_BFP4;
                         const uint32_t x0 = jj ? xv[m].z : xv[m].x, x1 = jj ? xv[m].w : xv[m].y;
-                        mma_bf16(tmp, a0, a1, a2, a3, mul_bf16x2(x0, 0x5F805F80u), mul_bf16x2(x1, 0x5F805F80u));
+                        if constexpr (XSM)  // (x lies there times 2^64 already: rows_for_int4)
+                            mma_bf16(tmp, a0, a1, a2, a3, x0, x1);
+                        else
+                            mma_bf16(tmp, a0, a1, a2, a3, mul_bf16x2(x0, kInt4Scale), mul_bf16x2(x1, kInt4Scale));
                     }
                     float(&a)[4] = acc[q % NA][m];
                     a[0] = fmaf(tmp[0], s_lo, a[0]), a[1] = fmaf(tmp[1], s_lo, a[1]);
@@ -572,7 +576,7 @@ constexpr int kStreamWarps = 16;
 // x: x' = H_1024 (s * x), unnormalised. A warp takes a (row, block of 1024) at a time, a lane 32
 // consecutive inputs in registers: five butterfly stages inside the lane, five across lanes by shuffles,
 // in the order and with the operands of tkd_hadamard_kernel (stage h pairs i and i + h: a + c, a - c),
-// so both give the same bits; then bf16 again, in place.
+// so both give the same bits; then bf16 again, in place, times 2^64 (chunk_mma).
 template <bool ONE>
 __device__ __forceinline__ void hadamard_rows(const TkdParams& p, uint32_t xt0, int cw, int lane, int M) {
     const int nblk = p.K >> 10;
@@ -614,13 +618,28 @@ __device__ __forceinline__ void hadamard_rows(const TkdParams& p, uint32_t xt0, 
             uint32_t o[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                o[j] = (uint32_t)f32_to_bf16_bits(v[8 * q + 2 * j]) |
-                       ((uint32_t)f32_to_bf16_bits(v[8 * q + 2 * j + 1]) << 16);
+                o[j] = (uint32_t)f32_to_bf16_bits(v[8 * q + 2 * j] * 0x1p64f) |
+                       ((uint32_t)f32_to_bf16_bits(v[8 * q + 2 * j + 1] * 0x1p64f) << 16);
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(xa + 16 * q), "r"(o[0]), "r"(o[1]), "r"(o[2]),
                          "r"(o[3])
                          : "memory");
         }
     }
+    asm volatile("bar.sync 2, %0;" ::"n"(kStreamWarps * 32) : "memory");
+}
+// A TKD_INT4 call's rows of x in shared memory: rotated if the call says so, and times 2^64, which every product with a code needs
+// (once here; in the loop it was two of some nineteen operations for 256 weights).
+template <bool ONE>
+__device__ __forceinline__ void rows_for_int4(const TkdParams& p, uint32_t xt0, int cw, int lane, int M) {
+    if (p.had) return hadamard_rows<ONE>(p, xt0, cw, lane, M);
+    for (int r = 0; r < M; ++r)
+        for (int e = cw * 32 + lane; e < p.K / 8; e += kStreamWarps * 32) {
+            const uint32_t a = xt0 + (ONE ? 0 : r * p.x_stride) + e * 16;
+            const uint4 v = lds128(a);
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(mul_bf16x2(v.x, kInt4Scale)), "r"(mul_bf16x2(v.y, kInt4Scale)),
+                         "r"(mul_bf16x2(v.z, kInt4Scale)), "r"(mul_bf16x2(v.w, kInt4Scale))
+                         : "memory");
+        }
     asm volatile("bar.sync 2, %0;" ::"n"(kStreamWarps * 32) : "memory");
 }
 
@@ -812,7 +831,7 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
             // 13 us launch, all of it before the first chunk.)
             x_here = mbar_wait(xbar, 0, p.status);  // (the copies were issued right after the wait for the kernel before)
             if constexpr (FMT == TKD_INT4) {
-                if (p.had && x_here) hadamard_rows<ONE>(p, xt0, cw, lane, M);
+                rows_for_int4<ONE>(p, xt0, cw, lane, M);  // (every warp: it has a barrier)
             }
         }
         while (x_here) {
