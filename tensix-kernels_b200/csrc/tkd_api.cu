@@ -39,6 +39,19 @@ int sm_count() {
     return cached[dev];
 }
 
+// Clusters of four CTAs that the tensor-memory kernel of a format can run at a time on the current device: asked once.
+int tc_cluster_count(int fmt, size_t smem) {
+    static std::atomic<int> cached[64][4];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = cached[dev][fmt].load(std::memory_order_relaxed);
+    if (!n) {
+        n = 1 + (fmt == TKD_BFP8 ? tkd_tc_clusters_bfp8(smem) : fmt == TKD_BFP4 ? tkd_tc_clusters_bfp4(smem) : tkd_tc_clusters_bf16(smem));
+        cached[dev][fmt].store(n, std::memory_order_relaxed);
+    }
+    return n - 1;
+}
+
 struct Layout {
     TkdParams p;
     int grid;
@@ -168,10 +181,31 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     if (p.nstages < 2) return TKD_ERR_UNSUPPORTED;
     L->smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
 
+    const bool on_device = sms <= 0;
     if (sms <= 0) sms = sm_count();
     if (sms <= 0) sms = 148;
     if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
     L->grid = (int)(p.total_items < sms ? p.total_items : sms);
+    // 9 to 32 rows: clusters of four CTAs, one to a slice (tkd_stream_tc.cuh), for a plain call of four slices. They take whole
+    // panels and leave some SMs idle (a GPC's number of SMs is not a multiple of four: 132 of 148 CTAs on a B200), so they are
+    // taken where no CTA gets more items for it; from four items on the other form's SMs that have one less leave theirs to the rest.
+    if (p.tc && !counted && on_device && p.nslices == 4 && !a->topk_k && a->nranks <= 1) {
+        const int off_xt = p.off_tbuf + 2 * 4 * 8 * 32 * 16, off_ring = (int)align_up(off_xt + 1024 + TKD_TC_SLOTS * 2 * 4096, 128);
+        const int stages = (int)((kMaxSmem - off_ring) / p.stage_bytes < TKD_MAX_STAGES ? (kMaxSmem - off_ring) / p.stage_bytes : TKD_MAX_STAGES);
+        const size_t smem = (size_t)off_ring + (size_t)stages * p.stage_bytes;
+        int clusters = tc_cluster_count(a->fmt, smem);
+        if (clusters > sms / 4) clusters = sms / 4;
+        if (clusters > panels) clusters = panels;
+        if (clusters > 0) {
+            const int items = (panels + clusters - 1) / clusters;  // of a CTA, at most
+            if (items <= 3 && items <= (4 * panels + sms - 1) / sms) {
+                p.tc_cluster = 1;
+                p.off_xt = off_xt, p.off_ring = off_ring, p.nstages = stages;
+                L->smem = smem;
+                L->grid = 4 * clusters;
+            }
+        }
+    }
     p.small = (p.total_items + 1) * (int64_t)(L->grid + 1) < (1ll << 32);
 
     // top-k

@@ -92,6 +92,7 @@ struct TkdParams {
     int* grid_counter;   // CTAs of this call that have finished their output (returns to zero)
     int exchange_wait;
     int tc;              // 9 to 32 rows: the tensor-memory kernel (tkd_stream_tc.cuh); off_xt is where its operand tiles go
+    int tc_cluster;      // ... in clusters of four CTAs, a slice each
     int x_smem;          // 1 to 8 rows, and all of x (K rounded up to a chunk) fits in shared memory at off_xt
     int narrow;          // ... and the call runs tkd_narrow_kernel (tkd_narrow.cuh)
     int x_stride;        // ... bytes from one row of it to the next
@@ -139,6 +140,9 @@ int tkd_launch_wide_bfp8(const TkdWide& p, size_t smem, cudaStream_t st);
 int tkd_launch_wide_bfp4(const TkdWide& p, size_t smem, cudaStream_t st);
 int tkd_launch_wide_bf16(const TkdWide& p, size_t smem, cudaStream_t st);
 int tkd_launch_stream(const TkdParams& p, int grid, size_t smem, cudaStream_t st);
+int tkd_tc_clusters_bfp8(size_t smem);  // clusters of four CTAs of the tensor-memory kernel that run at a time (0: cannot tell)
+int tkd_tc_clusters_bfp4(size_t smem);
+int tkd_tc_clusters_bf16(size_t smem);
 int tkd_launch_hadamard(const void* x, int64_t ldx, const uint32_t* signs, int rows, int K, void* out, int64_t ldo,
                         cudaStream_t st);
 int tkd_launch_topk_merge(const uint32_t* records, int nrec, int rows, int k, int top, uint32_t* out, cudaStream_t st);

@@ -7,3 +7,4 @@ int tkd_launch_stream_bf16(const TkdParams& p, int grid, size_t smem, cudaStream
     if (p.narrow) return launch_narrow<TKD_BF16>(p, grid, smem, st);
     return launch_fmt_all<TKD_BF16>(p, grid, smem, st);
 }
+int tkd_tc_clusters_bf16(size_t smem) { return tc_clusters<TKD_BF16>(smem); }

@@ -7,3 +7,4 @@ int tkd_launch_stream_bfp4(const TkdParams& p, int grid, size_t smem, cudaStream
     if (p.narrow) return launch_narrow<TKD_BFP4>(p, grid, smem, st);
     return launch_fmt_all<TKD_BFP4>(p, grid, smem, st);
 }
+int tkd_tc_clusters_bfp4(size_t smem) { return tc_clusters<TKD_BFP4>(smem); }

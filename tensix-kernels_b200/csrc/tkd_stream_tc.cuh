@@ -95,9 +95,46 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// The other CTAs of a cluster: an address of this CTA's shared memory in CTA `cta`'s, a store there, an arrival there, and the
+// wait for what others stored and announced here.
+__device__ __forceinline__ uint32_t cl_map(uint32_t a, uint32_t cta) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(cta));
+    return r;
+}
+__device__ __forceinline__ void cl_st128(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+__device__ __forceinline__ void cl_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool cl_wait(uint32_t bar, uint32_t parity, int* status) {
+    for (uint32_t i = 0; i < kWaitRounds; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity), "r"(kWaitHintNs)
+            : "memory");
+        if (ok) return true;
+    }
+    if (status) atomicExch(status, kStatusTimeout);
+    return false;
+}
+__device__ __forceinline__ void cl_barrier_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cl_barrier_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+constexpr int kTcExchange = 4 * 8 * 32 * 16;  // bytes: [slice][4 rows][32 columns][4] sums of 32 rows, one of two buffers
+
 // PLAIN: no top-k records and no exchange with other GPUs: that code falls away (it is the code's length that costs: the output
 // stage runs once or twice a CTA, from the instruction cache's misses).
-template <int FMT, bool KWHOLE, bool PLAIN>
+// CL (plain calls of four slices): the CTAs come in clusters of four, a cluster takes whole panels and a CTA of it always the
+// same slice. The four sums of a panel meet in shared memory: every CTA finishes 32 of the panel's columns (GLU: 16 gate
+// columns and their 16 up columns), and an output warp sends each column's sums of its slice to the CTA that finishes it. The
+// sums and their order are those of the other form, whose panels end in a chain of trips through L2 by one CTA alone: sums
+// stored 0.6 us, counted in 0.9, added up 2.4, put out 1.0 (32 rows, [4096, 4096] of bfloat8_b, 11.5 us from start to end).
+template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false>
 __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const __grid_constant__ TkdParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
@@ -109,6 +146,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + TKD_MAX_STAGES);
     const uint32_t afull0 = smem_u32(bars + 2 * TKD_MAX_STAGES), aempty0 = afull0 + 8 * kTcSlots;
     const uint32_t accfull0 = aempty0 + 8 * kTcSlots, accempty0 = accfull0 + 16;
+    const uint32_t xfull0 = accempty0 + 16, xempty0 = xfull0 + 16;  // CL: of the exchange buffers
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + TKD_SMEM_HEAD - 32);
     volatile int* sflag = reinterpret_cast<volatile int*>(smem + TKD_SMEM_HEAD - 16);
     uint4* hdr = reinterpret_cast<uint4*>(smem + 512);
@@ -131,6 +169,10 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
         for (int s = 0; s < 2; ++s) {
             mbar_init(accfull0 + 8 * s, kTcMmaWarps);
             mbar_init(accempty0 + 8 * s, 4);
+            if constexpr (CL) {
+                mbar_init(xfull0 + 8 * s, p.epi == TKD_EPI_GLU2 || p.epi == TKD_EPI_GLU_IL ? 8 : 4);
+                mbar_init(xempty0 + 8 * s, 16);
+            }
         }
         sflag[0] = sflag[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -138,18 +180,23 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     __syncthreads();
 
     const int64_t T = p.total_items;
-    const int64_t i0 = idiv(p, T * blockIdx.x, gridDim.x), i1 = idiv(p, T * (blockIdx.x + 1), gridDim.x);
+    // CL: the cluster's panels, this CTA's slice of each; as items they are p.nslices apart
+    const int rank = CL ? (int)(blockIdx.x & 3) : 0;
+    const int64_t pan0 = CL ? (int64_t)p.total_panels * (blockIdx.x >> 2) / (gridDim.x >> 2) : 0;
+    const int64_t pan1 = CL ? (int64_t)p.total_panels * ((blockIdx.x >> 2) + 1) / (gridDim.x >> 2) : 0;
+    const int64_t i0 = CL ? pan0 * p.nslices + rank : idiv(p, T * blockIdx.x, gridDim.x);
+    const int64_t i1 = CL ? pan1 * p.nslices + rank : idiv(p, T * (blockIdx.x + 1), gridDim.x);
     const int nst = p.nstages;
     const int M = p.M, K = p.K;
     const int topk_k = PLAIN ? 0 : p.topk_k, npeers = PLAIN ? 0 : p.npeers;
     const bool glu2 = p.epi == TKD_EPI_GLU2;
     const int nsa_total = (K + F::KSA - 1) / F::KSA;
     if (i0 >= i1) return;  // (before any tensor memory is held; the grid is never larger than the item count)
-    const int64_t lastp0 = idiv(p, i1 - 1, p.nslices) * p.nslices;
+    const int64_t lastp0 = CL ? i0 : idiv(p, i1 - 1, p.nslices) * p.nslices;
     const int64_t tail0 = lastp0 > i0 && lastp0 + p.nslices > i1 ? lastp0 : i1;
     const int64_t lead = i1 - tail0;
-    const int64_t nitems = i1 - i0;
-    auto item_at = [&](int64_t j) { return j < lead ? tail0 + j : i0 + (j - lead); };
+    const int64_t nitems = CL ? pan1 - pan0 : i1 - i0;
+    auto item_at = [&](int64_t j) { return CL ? i0 + j * p.nslices : j < lead ? tail0 + j : i0 + (j - lead); };
 
     // tensor memory: all 512 columns (two sets of two accumulators of 32, then the A slots of 64), allocated and freed by
     // the MMA warp. The allocation takes a microsecond: the producer, which has no use for it, goes ahead.
@@ -158,6 +205,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if constexpr (CL) cl_barrier_arrive();  // (this CTA's barriers are ready; waited for before the first use of another's)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -175,7 +223,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
             for (int64_t j = 0; j < nitems && ok; ++j) {
                 c = cn;
                 if (j + 1 < nitems) {
-                    if (j + 1 == lead)
+                    if (CL || j + 1 == lead)
                         cursor_init(cn, p, item_at(j + 1));
                     else
                         cursor_next(cn, p);
@@ -420,7 +468,9 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
             const uint64_t bd0 = tc_desc(ops0);
             const uint32_t dhi = (uint32_t)(bd0 >> 32), blo0 = (uint32_t)bd0, alo0 = tmem0 + kTcA0;
             for (int64_t j = 0; j < nitems && ok; ++j) {
-                if (j == 0 || j == lead) {
+                if (CL) {
+                    slice = rank;
+                } else if (j == 0 || j == lead) {
                     const int64_t it = item_at(j);
                     slice = (int)(it - idiv(p, it, p.nslices) * p.nslices);
                 } else if (++slice == p.nslices) {
@@ -468,9 +518,126 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
         const int et = ow * 32 + lane;    // the panel column (= A row = tensor-memory lane) this thread owns
         Cursor c;
         bool ok = true;
+        if constexpr (CL) {
+            cl_barrier_wait();
+            const bool glu = glu2 || p.epi == TKD_EPI_GLU_IL, up = glu && lane >= 16, f32out = p.epi == TKD_EPI_OUT32;
+            const int m4 = (M + 3) >> 2, rsz = p.res_dt == TKD_DT_F32 ? 4 : 2, osz = f32out ? 4 : 2;
+            // the CTA that finishes this thread's column of the panel, and the column's number there
+            const uint32_t to = glu ? (glu2 ? 2 * (ow & 1) : 2 * (ow >> 1)) + (lane >> 4) : ow;
+            const int pos = glu ? (glu2 ? ow >> 1 : ow & 1) * 16 + (lane & 15) : lane;
+            const uint32_t xb0 = smem_u32(tbuf), send0 = cl_map(xb0 + (rank * 256 + pos) * 16, to), sent0 = cl_map(xfull0, to);
+            const uint32_t freed0 = cl_map(xempty0, lane & 3);
+            const bool two = min(p.ks, K - rank * p.ks) > 128;
+            for (int64_t j = 0; j < nitems; ++j) {
+                const uint32_t buf = (uint32_t)j & 1, par = ((uint32_t)j >> 1) & 1;
+                cursor_init(c, p, item_at(j));
+                const TkdSegDev& sg = p.seg[c.seg];
+                // the column this thread finishes (rows 8 ow ..), its factors and its residuals
+                int n, oc;
+                if (glu2) {
+                    n = c.pl * 64 + 16 * rank + (lane & 15);
+                    oc = !up && n < sg.n_valid ? sg.out_col0 + n : -1;
+                } else if (glu) {
+                    const int o = c.pl * 64 + 16 * rank + (lane & 15);
+                    n = c.pl * TKD_PANEL_COLS + 64 * (rank >> 1) + 16 * (rank & 1) + (up ? 32 : 0) + (lane & 15);
+                    oc = !up && o < sg.n_valid / 2 ? sg.out_col0 + o : -1;
+                } else {
+                    n = c.pl * TKD_PANEL_COLS + 32 * rank + lane;
+                    oc = n < sg.n_valid ? sg.out_col0 + n : -1;
+                }
+                const bool other = up && glu2;
+                float f1 = 1.f, f2 = 1.f, sc = 1.f;
+                if constexpr (FMT != TKD_BF16) {
+                    const int e = tkd_out_exp(FMT, (other ? sg.emax2 : sg.emax)[n >> 4]), e1 = e / 2;
+                    f1 = __uint_as_float((uint32_t)(e1 + 127) << 23), f2 = __uint_as_float((uint32_t)(e - e1 + 127) << 23);
+                }
+                if (p.scale_dt != TKD_DT_NONE && n < sg.n_valid) {
+                    const void* sp = other ? p.scale2 : p.scale;
+                    sc = p.scale_dt == TKD_DT_BF16 ? bf16_bits_to_f32(static_cast<const uint16_t*>(sp)[n]) : static_cast<const float*>(sp)[n];
+                }
+                const int left = M - 8 * ow;  // rows from this warp's first on
+                uint32_t q[8] = {};
+                if (p.res_dt != TKD_DT_NONE && oc >= 0 && left > 0) {
+                    // (a row past M reads the last again)
+                    const char* rp = static_cast<const char*>(p.res) + ((int64_t)(8 * ow) * p.ldr + oc) * rsz;
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) {
+                        q[m] = rsz == 4 ? *reinterpret_cast<const uint32_t*>(rp) : (uint32_t)*reinterpret_cast<const uint16_t*>(rp) << 16;
+                        if (m + 1 < left) rp += p.ldr * rsz;
+                    }
+                }
+                // this slice's sums d0 + d1, to the CTAs that finish them
+                ok = mbar_wait(accfull0 + 8 * buf, par, p.status) && cl_wait(xempty0 + 8 * buf, par ^ 1, p.status);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t ta = tmem0 + ((uint32_t)(ow * 32) << 16) + kTcAcc0 + buf * 64, send = send0 + buf * kTcExchange;
+#pragma unroll 1
+                for (int h = 0; h < m4; h += 2) {
+                    uint32_t r0[8], r1[8] = {};
+                    auto ld8 = [&](uint32_t addr, uint32_t (&r)[8]) {
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                                     : "r"(addr)
+                                     : "memory");
+                    };
+                    ld8(ta + 4 * h, r0);
+                    if (two) ld8(ta + 32 + 4 * h, r1);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float v[8];
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) v[m] = two ? __uint_as_float(r0[m]) + __uint_as_float(r1[m]) : __uint_as_float(r0[m]);
+                    cl_st128(send + h * 512, v[0], v[1], v[2], v[3]);
+                    cl_st128(send + h * 512 + 512, v[4], v[5], v[6], v[7]);
+                }
+                tc_fence_before();
+                asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accempty0 + 8 * buf);
+                if (lane == 0 || (glu && lane == 16)) cl_arrive(sent0 + 8 * buf);
+                // the four slices' sums of this CTA's columns
+                ok = cl_wait(xfull0 + 8 * buf, par, p.status);
+                if (!ok) break;
+                float v[8];
+                if (left > 0) {
+                    const uint32_t at = xb0 + buf * kTcExchange + (2 * ow * 32 + lane) * 16;
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        const uint4 lo = lds128(at + s * 4096), hi = lds128(at + s * 4096 + 512);
+                        const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                        for (int m = 0; m < 8; ++m) v[m] = s ? v[m] + __uint_as_float(w[m]) : __uint_as_float(w[m]);
+                    }
+                }
+                __syncwarp();
+                if (lane < 4) cl_arrive(freed0 + 8 * buf);
+                if (left <= 0) continue;
+#pragma unroll
+                for (int m = 0; m < 8; ++m) v[m] = v[m] * f1 * f2 * sc;
+                if (glu) {
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) {
+                        const float u = __shfl_xor_sync(0xFFFFFFFFu, v[m], 16);
+                        v[m] = act_gate(v[m], p.act) * u;
+                    }
+                }
+                if (p.res_dt != TKD_DT_NONE) {
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) v[m] += __uint_as_float(q[m]);
+                }
+                char* yp = static_cast<char*>(p.out) + ((int64_t)(8 * ow) * p.ldo + oc) * osz;
+                const int rows = oc >= 0 ? left : 0;
+#pragma unroll
+                for (int m = 0; m < 8; ++m, yp += p.ldo * osz) {
+                    if (f32out)
+                        st_if(m < rows, yp, __float_as_uint(v[m]));
+                    else
+                        st16_if(m < rows, yp, f32_to_bf16_bits(v[m]));
+                }
+            }
+        }
         float* const trow = tbuf + (size_t)et * MP;
         uint16_t* y16 = static_cast<uint16_t*>(p.out);
-        for (int64_t j = 0; j < nitems && ok; ++j) {
+        for (int64_t j = 0; !CL && j < nitems && ok; ++j) {
             const int64_t it = item_at(j);
             if (j == 0 || j == lead)
                 cursor_init(c, p, it);
@@ -946,6 +1113,13 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     // ---- the end: everyone is here (a role whose wait gave up falls through to this point too), and the tensor memory
     // goes back
     tc_fence_before();
+    if constexpr (CL) {
+        // (no CTA goes while another may still store or arrive in its shared memory)
+        if (warp < kTcOutputWarp0) cl_barrier_wait();
+        __syncwarp();
+        cl_barrier_arrive();
+        cl_barrier_wait();
+    }
     __syncthreads();
     if (warp == kTcMmaWarp) {
         tc_fence_after();
@@ -953,9 +1127,23 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     }
 }
 
-template <int FMT, bool KWHOLE, bool PLAIN>
+template <int FMT, bool KWHOLE, bool PLAIN, bool CL>
+cudaLaunchConfig_t tc_config(int grid, size_t smem, cudaStream_t st, bool pdl, cudaLaunchAttribute (&attr)[2]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kTcWarps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    int n = 0;
+    if (CL) attr[n].id = cudaLaunchAttributeClusterDimension, attr[n].val.clusterDim = {4, 1, 1}, ++n;
+    if (pdl) attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization, attr[n].val.programmaticStreamSerializationAllowed = 1, ++n;
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cfg;
+}
+template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false>
 int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
-    auto kern = tkd_stream_tc_kernel<FMT, KWHOLE, PLAIN>;
+    auto kern = tkd_stream_tc_kernel<FMT, KWHOLE, PLAIN, CL>;
     static bool allowed[64] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -965,23 +1153,30 @@ int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
         if (e != cudaSuccess) return (int)e;
         if (dev >= 0 && dev < 64) allowed[dev] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kTcWarps * 32);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = p.no_pdl ? 0 : 1;
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = tc_config<FMT, KWHOLE, PLAIN, CL>(grid, smem, st, !p.no_pdl, attr);
     return (int)cudaLaunchKernelEx(&cfg, kern, p);
+}
+// Clusters of four that the device runs at a time (a CTA takes an SM; a cluster's SMs lie in one GPC), 0 if it cannot tell.
+template <int FMT>
+int tc_clusters(size_t smem) {
+    auto kern = tkd_stream_tc_kernel<FMT, true, true, true>;
+    int n = 0;
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = tc_config<FMT, true, true, true>(4, smem, nullptr, false, attr);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return n;
 }
 
 template <int FMT>
 int launch_fmt_all(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     if (p.tc) {
         const bool whole = p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0;
+        if (p.tc_cluster) return whole ? launch_tc<FMT, true, true, true>(p, grid, smem, st) : launch_tc<FMT, false, true, true>(p, grid, smem, st);
         if (!p.topk_k && !p.npeers) return whole ? launch_tc<FMT, true, true>(p, grid, smem, st) : launch_tc<FMT, false, true>(p, grid, smem, st);
         return whole ? launch_tc<FMT, true, false>(p, grid, smem, st) : launch_tc<FMT, false, false>(p, grid, smem, st);
     }
