@@ -432,7 +432,7 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
     p.panel_bytes = tkd_panel_bytes(a->fmt, a->k);
     p.stage_bytes = 8 * tkd_subsa(a->fmt) * tkd_sab(a->fmt);
     p.off_stage = TKD_SMEM_HEAD;
-    p.off_x = p.off_stage + 16 * 64 * 4;
+    p.off_x = p.off_stage + (p.nset == 1 ? 5 : 1) * 16 * 64 * 4;  // (GLU: a staging buffer for each worker of the output)
     p.off_ring = (int)align_up(p.off_x + 1023 + p.nx * p.nt * 128, 128);
     p.nstages = (kMaxSmem - p.off_ring) / p.stage_bytes;
     if (p.nstages > TKD_MAX_STAGES) p.nstages = TKD_MAX_STAGES;

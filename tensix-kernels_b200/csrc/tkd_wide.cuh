@@ -13,7 +13,7 @@
 //   tkd_wide_kernel    warp 0 (and 2)  one lane issues the MMAs, A from tensor memory, B from shared memory. Up to 128 rows
 //                                      two warps share the units (of 128 k): an MMA of few rows is shorter than its issue.
 //                      warp 1          producer of the ring of weight chunks; warp 3: of the x tiles
-//                      warps 4-7       output: a thread is a column (a tensor-memory lane). Before the decode warps: the
+//                      warps 4-7       output: a thread is a column (a tensor-memory lane); the decode warps help where they cannot go on. Before the decode warps: the
 //                                      schedulers favour older warps, and the next tile waits for these to free its accumulators
 //                      warps 8-23      decode: tkd_stream_tc_kernel's, without the activations
 //
@@ -27,6 +27,7 @@
 namespace {
 
 constexpr int kWideWarps = 24, kWideRing = 1, kWideX = 3, kWideDecode0 = 8;
+constexpr int kWideWorkers = 5;  // of a tile's output: the output warps and four times four decode warps
 constexpr int kWideASlots = 4;                    // units of A in tensor memory, 64 columns each
 constexpr int kWideA0 = 256;                      // their first column: the accumulators have 0-255
 static_assert(kWideA0 + kWideASlots * 64 <= 512, "tensor memory");
@@ -90,23 +91,32 @@ __device__ __forceinline__ void tmem_wait16(uint32_t (&q)[16]) {
                  : "memory");
 }
 
-// The output warps: a thread is the column et of its tile's panel. Rows go in batches of 16.
-template <int FMT>
-__device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, uint32_t tmem0, uint8_t* smem, uint32_t accfull0,
-                                            uint32_t accempty0, volatile int* sflag, uint32_t xs0) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+// The output of segment j of the CTA's run: a thread is the column et of its tile's panel, rows go in batches of 16. Four warps
+// (one to a quarter of the tensor memory's lanes) are a worker, and worker wk of nwk takes every nwk-th batch: the output
+// warps alone where a second set of accumulators lets the next tile's MMAs run beside them; with the decode warps as workers
+// 1-4 where there is one set, since nothing can run before it is free (256 rows: 9 us with four warps, of 77 for 512 rows of
+// [4096, 14336] in which a CTA has two tiles).
+template <int FMT, int EK, int nwk>
+__device__ __forceinline__ void wide_segment(const TkdWide& p, const WideSeg& sg, uint32_t j, bool more, int wk, uint32_t tmem0,
+                                             uint8_t* smem, uint32_t accfull0, uint32_t accempty0, volatile int* sflag, uint32_t xs0) {
     constexpr int CK = Fmt<FMT>::SUBSA * Fmt<FMT>::KSA;
     const int lane = threadIdx.x & 31, ow = (threadIdx.x >> 5) & 3, et = ow * 32 + lane;
-    const int NT = p.nt, nm = p.nmma;
-    const bool glu2 = p.epi == TKD_EPI_GLU2, glu = glu2 || p.epi == TKD_EPI_GLU_IL;
-    const bool f32out = p.epi == TKD_EPI_OUT32, res32 = f32out && p.res, res16 = p.epi == TKD_EPI_RESIDUAL;
-    float* stage = reinterpret_cast<float*>(smem + p.off_stage);  // GLU: [16 rows][64 columns] of the up half
+    const bool leader = wk == 0 && et == 0;
+    const int NT = p.nt, nm = p.nmma, r0 = 16 * wk, rstep = 16 * nwk;
+    constexpr bool glu = EK == TKD_EPI_GLU2, f32out = EK == TKD_EPI_OUT32, res16 = EK == TKD_EPI_RESIDUAL;
+    const bool glu2 = glu && p.epi == TKD_EPI_GLU2, res32 = f32out && p.res;
+    float* stage = reinterpret_cast<float*>(smem + p.off_stage) + wk * 1024;  // GLU: [16 rows][64 columns] of the up half
     // GLU: the warps of a panel's gate columns (interleaved: 32 gate, their 32 up, ...; two weights: 64 and 64)
     const bool gate = glu2 ? ow < 2 : (ow & 1) == 0;
     const int gcol = glu2 ? (ow & 1) * 32 + lane : (ow >> 1) * 32 + lane;  // the column within the tile's 64 outputs
-    WideSeg sg;
-    uint32_t j = 0;
-    for (int it = i0; wide_next(p, it, i1, sg); ++j) {
+    auto bar_workers = [&]() {
+        if (nwk > 1)
+            asm volatile("bar.sync 3, %0;" ::"n"(kWideWorkers * 128) : "memory");
+        else
+            bar_output_warps();
+    };
+    auto bar_worker = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(4 + wk) : "memory"); };
+    {
         const int panel = sg.tile / p.nrt, rt = sg.tile - panel * p.nrt;
         const int n = glu2 ? (panel >> 1) * 128 + (panel & 1) * 64 + (et & 63) : panel * 128 + et;  // the column of its weight
         const bool in_w = n < p.n_valid;
@@ -152,8 +162,11 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
         };
         auto release = [&]() {
             tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(accempty0 + 8 * set);
+            if (nwk > 1)
+                bar_workers();
+            else
+                __syncwarp();
+            if (wk == 0 && lane == 0) mbar_arrive(accempty0 + 8 * set);
         };
         // ---- a cut tile: partial sums in scratch, [segment][row / 4][column][4]. The later of two CTAs adds the other's to its
         // own, still in tensor memory, without storing that; of more than two each stores its own, and the last adds them all.
@@ -169,34 +182,34 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
         if (!whole) {
             bool last = false;
             if (nseg == 2) {
-                if (et == 0) sflag[0] = atom_add_acq_rel(p.counters + sg.tile, 0) == 1;
-                bar_output_warps();
+                if (leader) sflag[0] = atom_add_acq_rel(p.counters + sg.tile, 0) == 1;
+                bar_workers();
                 last = sflag[0] != 0;
-                bar_output_warps();  // (sflag may be written again only after everyone has read it)
+                bar_workers();  // (sflag may be written again only after everyone has read it)
             }
             if (!last) {
                 float* dst = part_of(own);
 #pragma unroll 1
-                for (int r = 0; r < rows; r += 16) {
+                for (int r = r0; r < rows; r += rstep) {
                     float v[16];
                     sums(r, v);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                         __stcg(reinterpret_cast<float4*>(dst + r * 128 + q * 512), make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
                 }
-                bar_output_warps();  // (orders the 128 threads' stores before thread 0's release)
-                if (et == 0) sflag[0] = atom_add_acq_rel(p.counters + sg.tile, 1) == nseg - 1;
-                bar_output_warps();
+                bar_workers();  // (orders all threads' stores before thread 0's release)
+                if (leader) sflag[0] = atom_add_acq_rel(p.counters + sg.tile, 1) == nseg - 1;
+                bar_workers();
                 last = sflag[0] != 0;
-                bar_output_warps();
+                bar_workers();
             }
             if (!last) {
                 release();
-                continue;
+                return;
             }
-            if (et == 0) p.counters[sg.tile] = 0;
+            if (leader) p.counters[sg.tile] = 0;
             per = p.nx * NT * 128 / ((nseg == 2 ? 1 : nseg) * 512) & ~15;
-            staged = it >= i1 && per >= 16;  // (this CTA's last tile: every x tile has been multiplied)
+            staged = !more && (nwk > 1 ? nseg == 2 && per >= NT : per >= 16);  // (this CTA's last tile: every x tile has been multiplied)
         }
         // ---- the output stage, sixteen rows at a time (a warp has its scheduler nearly to itself here: the loop is bound by the
         // latency of its chains, so the rows go side by side; eight at a time a tile of 256 rows took twice as long)
@@ -216,11 +229,22 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
                 if (r + 2 * m + 2 + odd < rows) rp += 2 * p.ldr;
             }
         };
-        if (fast && res16 && odd < rows) load_res(0);
+        if (fast && res16 && r0 + odd < rows) load_res(r0);
         uint16_t* y16 = static_cast<uint16_t*>(p.out) + (int64_t)row0 * p.ldo + oc;
         int staged_from = 0, staged_to = 0;  // the rows whose other parts lie in the x tiles
+        if (staged && nwk > 1) {
+            // (one other part, and room for all of it: each thread copies its own batches')
+            const float* src = part_of(1 - own);
+            for (int r = r0; r < rows; r += rstep)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(xs0 + ((r / 4 + q) * 128 + et) * 16), "l"(src + r * 128 + q * 512)
+                                 : "memory");
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            staged_to = NT;
+        }
 #pragma unroll 1
-        for (int r = 0; r < rows; r += 16) {
+        for (int r = r0; r < rows; r += rstep) {
             float v[16];
             if (staged && r >= staged_to) {
                 staged_from = r, staged_to = r + per;
@@ -264,11 +288,11 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
 #pragma unroll
             for (int m = 0; m < 16; ++m) v[m] = v[m] * colf * colg;
             if (glu) {
-                bar_output_warps();  // (the batch before has been read)
+                bar_worker();  // (the batch before has been read)
                 if (!gate)
 #pragma unroll
                     for (int m = 0; m < 16; ++m) stage[m * 64 + gcol] = v[m];
-                bar_output_warps();
+                bar_worker();
                 if (!gate) continue;
 #pragma unroll
                 for (int m = 0; m < 16; ++m) v[m] = act_gate(v[m], p.act) * stage[m * 64 + gcol];
@@ -291,7 +315,7 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
                         const float lo = odd ? got : v[2 * m], hi = odd ? v[2 * m + 1] : got;
                         w[m] = f32x2_to_bf16x2(lo + __uint_as_float(rq[m] << 16), hi + __uint_as_float(rq[m] & 0xFFFF0000u));
                     }
-                    if (r + 16 + odd < rows) load_res(r + 16);
+                    if (r + rstep + odd < rows) load_res(r + rstep);
                 }
 #pragma unroll
                 for (int m = 0; m < 8; ++m, yp += 2 * p.ldo) st_if(2 * m < left, yp, w[m]);
@@ -328,7 +352,9 @@ __device__ __forceinline__ void wide_output(const TkdWide& p, int i0, int i1, ui
     }
 }
 
-template <int FMT, bool KWHOLE>
+// EK: the kind of output (TKD_EPI_GLU2 for both GLU forms). One kernel for all of them was 3 us slower at any size: every launch
+// fetches its code anew, and most of it was outputs that the call does not have. SHARED: the decode warps share the output.
+template <int FMT, bool KWHOLE, int EK, bool SHARED>
 __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __grid_constant__ TkdWide p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
@@ -475,9 +501,10 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
                 __syncwarp();
             }
         }
-    } else if (warp >= kWideDecode0 && warp < kWideDecode0 + SW) {
-        // ---------------------------------------------------------------- decode warps, as tkd_stream_tc_kernel's: two groups of
+    } else {
+        // ---------------------------------------------------------------- output warps (4-7), and decode warps, as tkd_stream_tc_kernel's: two groups of
         // eight, a unit of two tiles of 64 k is one group's; a warp stores its 16 columns' share into tensor memory
+        const bool decode = warp >= kWideDecode0;
         const int cw = warp - kWideDecode0, qtr = warp & 3, sub4 = cw >> 2, grp = sub4 >> 1, rg = 2 * qtr + (sub4 & 1), t = lane & 3;
         constexpr int EXPB = FMT == TKD_BFP4 ? 64 : (FMT == TKD_BFP8 ? 32 : 0), UPC = CK / 128, MU = (UPC + G - 1) / G;
         const uint2 sh = make_uint2(p.mul16, p.mul128);
@@ -530,8 +557,9 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
             }
         };
         bool ok = true;
+        uint32_t j = 0;
         for (int it = i0; ok && wide_next(p, it, i1, sg);) {
-            for (int c = sg.c0; ok && c < sg.c1; ++c) {
+            for (int c = decode ? sg.c0 : sg.c1; ok && c < sg.c1; ++c) {
                 ok = mbar_wait(full0 + 8 * slot, phase, p.status);
                 if (!ok) break;
                 const int nsa = KWHOLE ? F::SUBSA : min(F::SUBSA, nsa_total - c * F::SUBSA);
@@ -568,9 +596,12 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
                 if (ok && lane == 0) mbar_arrive(empty0 + 8 * slot);
                 if (++slot == (uint32_t)nst) slot = 0, phase ^= 1;
             }
+            // (the output and the residual may be the kernel before's: waited for once)
+            if (j == 0 && (SHARED || !decode)) asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (ok && (SHARED || !decode))
+                wide_segment<FMT, EK, SHARED ? kWideWorkers : 1>(p, sg, j, it < i1, SHARED ? 1 + sub4 : 0, tmem0, smem, accfull0, accempty0, sflag, xs0);
+            ++j;
         }
-    } else {
-        wide_output<FMT>(p, i0, i1, tmem0, smem, accfull0, accempty0, sflag, xs0);
     }
     // ---- the end: everyone comes here, also after a wait that gave up
     tc_fence_before();
@@ -581,9 +612,9 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
     }
 }
 
-template <int FMT, bool KWHOLE>
+template <int FMT, bool KWHOLE, int EK, bool SHARED>
 int launch_wide(const TkdWide& p, size_t smem, cudaStream_t st) {
-    auto kern = tkd_wide_kernel<FMT, KWHOLE>;
+    auto kern = tkd_wide_kernel<FMT, KWHOLE, EK, SHARED>;
     static bool allowed[64] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -604,9 +635,21 @@ int launch_wide(const TkdWide& p, size_t smem, cudaStream_t st) {
     cfg.gridDim = dim3((unsigned)p.grid), cfg.blockDim = dim3(kWideWarps * 32), cfg.dynamicSmemBytes = smem;
     return (int)cudaLaunchKernelEx(&cfg, kern, p);
 }
+template <int FMT, int EK>
+int launch_wide_k(const TkdWide& p, size_t smem, cudaStream_t st) {
+    const bool whole = p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0;
+    if (p.nset == 1) return whole ? launch_wide<FMT, true, EK, true>(p, smem, st) : launch_wide<FMT, false, EK, true>(p, smem, st);
+    return whole ? launch_wide<FMT, true, EK, false>(p, smem, st) : launch_wide<FMT, false, EK, false>(p, smem, st);
+}
 template <int FMT>
 int launch_wide_fmt(const TkdWide& p, size_t smem, cudaStream_t st) {
-    return p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0 ? launch_wide<FMT, true>(p, smem, st) : launch_wide<FMT, false>(p, smem, st);
+    switch (p.epi) {
+        case TKD_EPI_GLU2:
+        case TKD_EPI_GLU_IL: return launch_wide_k<FMT, TKD_EPI_GLU2>(p, smem, st);
+        case TKD_EPI_RESIDUAL: return launch_wide_k<FMT, TKD_EPI_RESIDUAL>(p, smem, st);
+        case TKD_EPI_OUT32: return launch_wide_k<FMT, TKD_EPI_OUT32>(p, smem, st);
+        default: return launch_wide_k<FMT, TKD_EPI_PLAIN>(p, smem, st);
+    }
 }
 
 }  // namespace
