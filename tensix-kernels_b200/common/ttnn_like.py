@@ -192,10 +192,11 @@ def _stream_ptr():
     return torch.cuda.current_stream().cuda_stream
 
 
-def pack_weight(device, wt, dtype, orient, col_div=None, memory_config=None):
+def pack_weight(device, wt, dtype, orient, col_div=None, memory_config=None, into=(None, None)):
     """A float matrix (orient 0: [N, K] as torch's [out, in]; 1: [K, N]) -> Weight, on the GPU in one launch
-    (tkd_pack_weight). col_div: divisors of the columns."""
-    return _packed(device, wt, dtype, orient, col_div, memory_config, False)[0]
+    (tkd_pack_weight). col_div: divisors of the columns. into: byte tensors for the stream and its exponents (a weight too
+    wide for its format's stream has its own all the same)."""
+    return _packed(device, wt, dtype, orient, col_div, memory_config, False, into)[0]
 
 
 def pack_weight_scaled(device, wt, dtype, memory_config=None):
@@ -204,7 +205,7 @@ def pack_weight_scaled(device, wt, dtype, memory_config=None):
     return _packed(device, wt, dtype, 0, None, memory_config, True)
 
 
-def _packed(device, wt, dtype, orient, col_div, memory_config, own):
+def _packed(device, wt, dtype, orient, col_div, memory_config, own, into=(None, None)):
     fmt = FMT[dtype]
     src = wt.to(device.torch, torch.float32)
     ld, width = src.stride(0), src.shape[1]
@@ -213,7 +214,7 @@ def _packed(device, wt, dtype, orient, col_div, memory_config, own):
     n, k = (src.shape[0], width) if orient == 0 else (width, src.shape[0])
     assert k % TILE == 0, f"K {k} is not a multiple of 32"
     div = None if col_div is None else col_div.to(device.torch, torch.float32).contiguous()
-    stream, emax, scale, state = _tkd.host().pack(fmt, src, orient, div, own)
+    stream, emax, scale, state = _tkd.host().pack(fmt, src, orient, div, own, *into)
     if state:
         # (a wide weight, or a K past what one pass takes)
         with torch.cuda.device(device.torch):

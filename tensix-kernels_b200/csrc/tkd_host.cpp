@@ -187,11 +187,11 @@ struct WideWord {
     }
 };
 
-// pack(format, float32 matrix, orientation, divisors or None, own scales) -> (stream, emax or None, scales or None, state):
-// tkd_pack_weight into new tensors, waited for (launches read weights ahead of stream order). state 0: done; 1: the weight
+// pack(format, float32 matrix, orientation, divisors or None, own scales, stream or None, emax or None) -> (stream, emax or None,
+// scales or None, state): tkd_pack_weight into the tensors given or into new ones, waited for (launches read weights ahead of stream order). state 0: done; 1: the weight
 // is wide; 2: this K is not taken (then nothing was packed).
 PyObject* host_pack(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 5 || !all_tensors(args, {1}, {3})) return type_error("tkd_host.pack: format, matrix, orientation, divisors, own scales");
+    if (n != 7 || !all_tensors(args, {1}, {3, 5, 6})) return type_error("tkd_host.pack: format, matrix, orientation, divisors, own scales, stream, emax");
     const int fmt = (int)PyLong_AsLong(args[0]), orient = (int)PyLong_AsLong(args[2]), own = PyObject_IsTrue(args[4]);
     if (PyErr_Occurred()) return nullptr;
     static thread_local WideWord word;
@@ -205,8 +205,14 @@ PyObject* host_pack(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (!wide) return tkd_error(TKD_ERR_CUDA + (int)cudaGetLastError(), "cudaHostAlloc");
         *wide = 0;
         auto bytes = [&](int64_t b) { return at::detail::empty_cuda({b}, at::kByte, src.device(), std::nullopt); };
-        at::Tensor stream = bytes(tkd_packed_bytes(fmt, k, cols)), emax, scales;
-        if (fmt != TKD_FMT_BF16) emax = bytes(tkd_padded_cols(cols) / 16);
+        auto given = [&](int i, int64_t b) -> at::Tensor {
+            const at::Tensor* t = tensor_or_null(args[i]);
+            if (t && (!t->is_cuda() || t->get_device() != src.get_device() || !t->is_contiguous() || (int64_t)t->nbytes() != b))
+                throw std::runtime_error("tkd_host.pack: a tensor given for the result has another size, device or layout");
+            return t ? *t : at::Tensor(bytes(b));
+        };
+        at::Tensor stream = given(5, tkd_packed_bytes(fmt, k, cols)), emax, scales;
+        if (fmt != TKD_FMT_BF16) emax = given(6, tkd_padded_cols(cols) / 16);
         if (own) scales = at::detail::empty_cuda({1, 1, 1, cols}, at::kBFloat16, src.device(), std::nullopt);
         cudaStream_t st = c10::cuda::getCurrentCUDAStream(src.get_device()).stream();
         int rc;
