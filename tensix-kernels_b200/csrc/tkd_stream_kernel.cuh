@@ -202,6 +202,35 @@ __device__ __forceinline__ float act_gate(float g, int act) {
     return over_one_plus_exp(g, -u);
 }
 
+// The kind of output an instance of a kernel serves: an epilogue (TKD_EPI_GLU2: both GLU forms), or whichever the call has. Every
+// launch fetches its code anew, so the code of other outputs costs time without running: 0.35 us of a launch of 32 rows, 0.9 of
+// one with several items a CTA. (Not so the kernel for up to eight rows: its outputs are short, and the launches of a layer share
+// one instance's code: a layer of eight rows took 27.1 us with an instance for each kind, 26.8 with one.)
+constexpr int EK_ANY = -1;
+template <int EK>
+__device__ __forceinline__ int epi_of(int epi) {
+    return EK == EK_ANY || EK == TKD_EPI_GLU2 ? epi : EK;
+}
+template <int EK>
+__device__ __forceinline__ bool glu_of(int epi) {
+    return EK == EK_ANY ? epi == TKD_EPI_GLU2 || epi == TKD_EPI_GLU_IL : EK == TKD_EPI_GLU2;
+}
+template <int EK>  // (the type of the residual: TKD_EPI_RESIDUAL has a bf16 one, TKD_EPI_OUT32 a float32 one or none)
+__device__ __forceinline__ int res_of(int res_dt) {
+    return EK == EK_ANY || EK == TKD_EPI_OUT32 ? res_dt : EK == TKD_EPI_RESIDUAL ? TKD_DT_BF16 : TKD_DT_NONE;
+}
+// f(an instance's EK) for a call's epilogue
+template <class F>
+int for_epilogue(int epi, F f) {
+    switch (epi) {
+        case TKD_EPI_GLU2:
+        case TKD_EPI_GLU_IL: return f(std::integral_constant<int, TKD_EPI_GLU2>{});
+        case TKD_EPI_RESIDUAL: return f(std::integral_constant<int, TKD_EPI_RESIDUAL>{});
+        case TKD_EPI_OUT32: return f(std::integral_constant<int, TKD_EPI_OUT32>{});
+        default: return f(std::integral_constant<int, TKD_EPI_PLAIN>{});
+    }
+}
+
 // Quotients of item counts: 32-bit arithmetic when the launch's numbers allow it (p.small): a 64-bit division is a long
 // subroutine on the GPU, and these sit on every CTA's way to its first copy and on the way to a panel's completion.
 __device__ __forceinline__ int64_t idiv(const TkdParams& p, int64_t num, int64_t den) {

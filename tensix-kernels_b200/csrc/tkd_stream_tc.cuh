@@ -134,7 +134,7 @@ constexpr int kTcExchange = 4 * 8 * 32 * 16;  // bytes: [slice][4 rows][32 colum
 // columns and their 16 up columns), and an output warp sends each column's sums of its slice to the CTA that finishes it. The
 // sums and their order are those of the other form, whose panels end in a chain of trips through L2 by one CTA alone: sums
 // stored 0.6 us, counted in 0.9, added up 2.4, put out 1.0 (32 rows, [4096, 4096] of bfloat8_b, 11.5 us from start to end).
-template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false>
+template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false, int EK = EK_ANY>
 __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const __grid_constant__ TkdParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
             mbar_init(accfull0 + 8 * s, kTcMmaWarps);
             mbar_init(accempty0 + 8 * s, 4);
             if constexpr (CL) {
-                mbar_init(xfull0 + 8 * s, p.epi == TKD_EPI_GLU2 || p.epi == TKD_EPI_GLU_IL ? 8 : 4);
+                mbar_init(xfull0 + 8 * s, glu_of<EK>(p.epi) ? 8 : 4);
                 mbar_init(xempty0 + 8 * s, 16);
             }
         }
@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     const int nst = p.nstages;
     const int M = p.M, K = p.K;
     const int topk_k = PLAIN ? 0 : p.topk_k, npeers = PLAIN ? 0 : p.npeers;
-    const bool glu2 = p.epi == TKD_EPI_GLU2;
+    const int epi = epi_of<EK>(p.epi), res_dt = res_of<EK>(p.res_dt);
+    const bool glu2 = glu_of<EK>(p.epi) && epi == TKD_EPI_GLU2;
     const int nsa_total = (K + F::KSA - 1) / F::KSA;
     if (i0 >= i1) return;  // (before any tensor memory is held; the grid is never larger than the item count)
     const int64_t lastp0 = CL ? i0 : idiv(p, i1 - 1, p.nslices) * p.nslices;
@@ -520,8 +521,8 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
         bool ok = true;
         if constexpr (CL) {
             cl_barrier_wait();
-            const bool glu = glu2 || p.epi == TKD_EPI_GLU_IL, up = glu && lane >= 16, f32out = p.epi == TKD_EPI_OUT32;
-            const int m4 = (M + 3) >> 2, rsz = p.res_dt == TKD_DT_F32 ? 4 : 2, osz = f32out ? 4 : 2;
+            const bool glu = glu_of<EK>(p.epi), up = glu && lane >= 16, f32out = epi == TKD_EPI_OUT32;
+            const int m4 = (M + 3) >> 2, rsz = res_dt == TKD_DT_F32 ? 4 : 2, osz = f32out ? 4 : 2;
             // the CTA that finishes this thread's column of the panel, and the column's number there
             const uint32_t to = glu ? (glu2 ? 2 * (ow & 1) : 2 * (ow >> 1)) + (lane >> 4) : ow;
             const int pos = glu ? (glu2 ? ow >> 1 : ow & 1) * 16 + (lane & 15) : lane;
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 }
                 const int left = M - 8 * ow;  // rows from this warp's first on
                 uint32_t q[8] = {};
-                if (p.res_dt != TKD_DT_NONE && oc >= 0 && left > 0) {
+                if (res_dt != TKD_DT_NONE && oc >= 0 && left > 0) {
                     // (a row past M reads the last again)
                     const char* rp = static_cast<const char*>(p.res) + ((int64_t)(8 * ow) * p.ldr + oc) * rsz;
 #pragma unroll
@@ -620,7 +621,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                         v[m] = act_gate(v[m], p.act) * u;
                     }
                 }
-                if (p.res_dt != TKD_DT_NONE) {
+                if (res_dt != TKD_DT_NONE) {
 #pragma unroll
                     for (int m = 0; m < 8; ++m) v[m] += __uint_as_float(q[m]);
                 }
@@ -658,12 +659,12 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                                                    : static_cast<const float*>(sp)[n];
                 }
             }
-            if (f.deliver && p.res && topk_k == 0) {
+            if (f.deliver && res_dt != TKD_DT_NONE && topk_k == 0) {
                 // the panel's residual on its way to L2 while the slice is still being multiplied: row et & 31, line et >> 5
                 // of the row's 128 (GLU: 64) columns
-                const int rr = et & 31, ln = et >> 5, rsz_ = p.res_dt == TKD_DT_F32 ? 4 : 2;
-                const int ncol = (p.epi == TKD_EPI_GLU_IL || glu2) ? 64 : TKD_PANEL_COLS;
-                const int nout_valid = p.epi == TKD_EPI_GLU_IL ? sg.n_valid / 2 : sg.n_valid;  // (only elements that exist)
+                const int rr = et & 31, ln = et >> 5, rsz_ = res_dt == TKD_DT_F32 ? 4 : 2;
+                const int ncol = glu_of<EK>(p.epi) ? 64 : TKD_PANEL_COLS;
+                const int nout_valid = epi == TKD_EPI_GLU_IL ? sg.n_valid / 2 : sg.n_valid;  // (only elements that exist)
                 if (rr < M && ln * 128 < ncol * rsz_ && c.pl * ncol + ln * (128 / rsz_) < nout_valid) {
                     const char* rp = static_cast<const char*>(p.res) +
                                      ((size_t)rr * p.ldr + sg.out_col0 + (size_t)c.pl * ncol) * rsz_ + ln * 128;
@@ -813,7 +814,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                     colf = __uint_as_float((uint32_t)(e1 + 127) << 23), colg = __uint_as_float((uint32_t)(e2 + 127) << 23);
                 }
                 const float cols = p.scale_dt != TKD_DT_NONE && in_w ? sc : 1.f;
-                const bool glu = p.epi == TKD_EPI_GLU_IL || glu2;
+                const bool glu = glu_of<EK>(p.epi);
                 if constexpr (PLAIN) {
                     // A thread keeps its column, sixteen rows at a time. GLU: the up columns' sums go back scaled first, then
                     // the gate columns' threads make the outputs.
@@ -836,8 +837,8 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                             }
                         bar_output_warps();
                     }
-                    const bool f32out = p.epi == TKD_EPI_OUT32, odd = lane & 1;
-                    const int esz = f32out ? 4 : 2, rsz = p.res_dt == TKD_DT_F32 ? 4 : 2;
+                    const bool f32out = epi == TKD_EPI_OUT32, odd = lane & 1;
+                    const int esz = f32out ? 4 : 2, rsz = res_dt == TKD_DT_F32 ? 4 : 2;
                     // (two bf16 columns a store: an even lane takes both columns' even rows, its neighbour the odd ones)
                     const bool fast = !f32out && !((reinterpret_cast<uintptr_t>(p.out) & 3) | (p.ldo & 1) | (sg.out_col0 & 1)) &&
                                       __all_sync(0xFFFFFFFFu, oc >= 0);
@@ -847,7 +848,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                         for (int r = 0; r < M; r += 16) {
                             float v[16];
                             uint32_t q[16];
-                            const bool res = p.res && oc >= 0;
+                            const bool res = res_dt != TKD_DT_NONE && oc >= 0;
                             if (res) {
                                 // (a row past M reads the last again)
                                 const char* rp = static_cast<const char*>(p.res) + ((int64_t)r * p.ldr + oc) * rsz;
@@ -924,13 +925,13 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                         const int left = sg.n_valid - c.pl * TKD_PANEL_COLS;  // columns of this panel that exist (a multiple of 64)
                         nv = left >= 128 ? 64 : (left >= 64 ? 32 : 0);
                     }
-                    const bool f32out = p.epi == TKD_EPI_OUT32;
+                    const bool f32out = epi == TKD_EPI_OUT32;
                     const int esz = f32out ? 4 : 2;
                     const bool vec = ((reinterpret_cast<uintptr_t>(p.out) | (uintptr_t)(p.ldo * esz) | (uintptr_t)(oc0 * esz)) & 15) == 0;
                     const int r = lane;
                     // the residual of this lane's groups, asked for with 16-byte loads two groups ahead (four round trips to
                     // L2 one after the other were most of this stage)
-                    const bool res32 = f32out && p.res_dt == TKD_DT_F32, res16 = p.epi == TKD_EPI_RESIDUAL;
+                    const bool res32 = f32out && res_dt == TKD_DT_F32, res16 = epi == TKD_EPI_RESIDUAL;
                     const int rsz = res32 ? 4 : 2;
                     const bool rvec = vec && (res32 || res16) &&
                                       ((reinterpret_cast<uintptr_t>(p.res) | (uintptr_t)(p.ldr * rsz) | (uintptr_t)(oc0 * rsz)) & 15) == 0;
@@ -1073,11 +1074,11 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
 #pragma unroll
                         for (int m = 0; m < 8; ++m)
                             v[m] = glu ? act_gate(gp[r0 + m], p.act) * up[r0 + m] : trow[r0 + m] * colf * colg * cols;
-                        if (p.epi == TKD_EPI_OUT32 && p.res_dt == TKD_DT_F32) {
+                        if (epi == TKD_EPI_OUT32 && res_dt == TKD_DT_F32) {
 #pragma unroll
                             for (int m = 0; m < 8; ++m)
                                 if (r0 + m < M) v[m] += static_cast<const float*>(p.res)[(size_t)(r0 + m) * p.ldr + ocol];
-                        } else if (p.epi == TKD_EPI_RESIDUAL) {
+                        } else if (epi == TKD_EPI_RESIDUAL) {
 #pragma unroll
                             for (int m = 0; m < 8; ++m)
                                 if (r0 + m < M)
@@ -1087,7 +1088,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                         for (int m = 0; m < 8; ++m) {
                             if (r0 + m >= M) break;
                             const size_t at = (size_t)(r0 + m) * p.ldo + ocol;
-                            if (p.epi == TKD_EPI_OUT32) {
+                            if (epi == TKD_EPI_OUT32) {
                                 static_cast<float*>(p.out)[at] = v[m];
                                 for (int q = 0; q < npeers; ++q)
                                     if (p.peer_out[q]) static_cast<float*>(p.peer_out[q])[at] = v[m];
@@ -1127,7 +1128,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     }
 }
 
-template <int FMT, bool KWHOLE, bool PLAIN, bool CL>
+template <bool CL>
 cudaLaunchConfig_t tc_config(int grid, size_t smem, cudaStream_t st, bool pdl, cudaLaunchAttribute (&attr)[2]) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -1141,9 +1142,9 @@ cudaLaunchConfig_t tc_config(int grid, size_t smem, cudaStream_t st, bool pdl, c
     cfg.numAttrs = n;
     return cfg;
 }
-template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false>
+template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false, int EK = EK_ANY>
 int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
-    auto kern = tkd_stream_tc_kernel<FMT, KWHOLE, PLAIN, CL>;
+    auto kern = tkd_stream_tc_kernel<FMT, KWHOLE, PLAIN, CL, EK>;
     static bool allowed[64] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1154,16 +1155,16 @@ int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
         if (dev >= 0 && dev < 64) allowed[dev] = true;
     }
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = tc_config<FMT, KWHOLE, PLAIN, CL>(grid, smem, st, !p.no_pdl, attr);
+    const cudaLaunchConfig_t cfg = tc_config<CL>(grid, smem, st, !p.no_pdl, attr);
     return (int)cudaLaunchKernelEx(&cfg, kern, p);
 }
 // Clusters of four that the device runs at a time (a CTA takes an SM; a cluster's SMs lie in one GPC), 0 if it cannot tell.
 template <int FMT>
 int tc_clusters(size_t smem) {
-    auto kern = tkd_stream_tc_kernel<FMT, true, true, true>;
+    auto kern = tkd_stream_tc_kernel<FMT, true, true, true, TKD_EPI_PLAIN>;
     int n = 0;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = tc_config<FMT, true, true, true>(4, smem, nullptr, false, attr);
+    const cudaLaunchConfig_t cfg = tc_config<true>(4, smem, nullptr, false, attr);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -1176,8 +1177,14 @@ template <int FMT>
 int launch_fmt_all(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     if (p.tc) {
         const bool whole = p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0;
-        if (p.tc_cluster) return whole ? launch_tc<FMT, true, true, true>(p, grid, smem, st) : launch_tc<FMT, false, true, true>(p, grid, smem, st);
-        if (!p.topk_k && !p.npeers) return whole ? launch_tc<FMT, true, true>(p, grid, smem, st) : launch_tc<FMT, false, true>(p, grid, smem, st);
+        if (!p.topk_k && !p.npeers) {
+            // (a K that ends inside a chunk, the rare case: one instance for all outputs)
+            if (!whole) return p.tc_cluster ? launch_tc<FMT, false, true, true>(p, grid, smem, st) : launch_tc<FMT, false, true>(p, grid, smem, st);
+            return for_epilogue(p.epi, [&](auto ek) {
+                constexpr int EK = decltype(ek)::value;
+                return p.tc_cluster ? launch_tc<FMT, true, true, true, EK>(p, grid, smem, st) : launch_tc<FMT, true, true, false, EK>(p, grid, smem, st);
+            });
+        }
         return whole ? launch_tc<FMT, true, false>(p, grid, smem, st) : launch_tc<FMT, false, false>(p, grid, smem, st);
     }
     return launch_fmt<FMT>(p, grid, smem, st);

@@ -643,13 +643,7 @@ int launch_wide_k(const TkdWide& p, size_t smem, cudaStream_t st) {
 }
 template <int FMT>
 int launch_wide_fmt(const TkdWide& p, size_t smem, cudaStream_t st) {
-    switch (p.epi) {
-        case TKD_EPI_GLU2:
-        case TKD_EPI_GLU_IL: return launch_wide_k<FMT, TKD_EPI_GLU2>(p, smem, st);
-        case TKD_EPI_RESIDUAL: return launch_wide_k<FMT, TKD_EPI_RESIDUAL>(p, smem, st);
-        case TKD_EPI_OUT32: return launch_wide_k<FMT, TKD_EPI_OUT32>(p, smem, st);
-        default: return launch_wide_k<FMT, TKD_EPI_PLAIN>(p, smem, st);
-    }
+    return for_epilogue(p.epi, [&](auto ek) { return launch_wide_k<FMT, decltype(ek)::value>(p, smem, st); });
 }
 
 }  // namespace
