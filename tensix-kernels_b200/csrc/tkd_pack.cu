@@ -251,6 +251,15 @@ __global__ void tkd_unpack_kernel(int fmt, int64_t K, int64_t npad, const uint8_
 // in the 126 MB L2), else as many as fit
 __host__ __device__ constexpr int pack_threads(int scale) { return scale == 2 ? 512 : 256; }
 
+// The largest of three magnitudes, a NaN if there is one: one operation for two values, where an AND and a maximum each were four
+// on the half-rate integer pipe, which the kernel keeps busy (a [14336, 4096] call with its own scales: bfloat8_b 126 to 113 us,
+// bfloat4_b 107 to 105).
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+    float d;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 // |v|'s bits rounded up to bf16, as a float (linear.bf16_ceil), of at least 1e-8
 __device__ __forceinline__ float pack_col_scale(uint32_t bits) {
     const float a = __uint_as_float(bits), s = a < 1e-8f ? 1e-8f : a;  // (a NaN stays)
@@ -326,16 +335,16 @@ __global__ void __launch_bounds__(pack_threads(SCALE)) tkd_pack_weight_kernel(co
         if (in0) d0 = col_div[n0];
         if (in1) d1 = col_div[n1];
     } else if constexpr (SCALE == 2) {
-        uint32_t m0 = 0, m1 = 0;
-#pragma unroll 4
+        float f0 = 0.f, f1 = 0.f;
+#pragma unroll 2  // (four need 75 registers: one CTA an SM)
         for (int b = warp; b < K / 32; b += kPackWarps) {
             float v0[8], v1[8];
             load8(v0, n0, in0, 32 * b + 8 * t);
             load8(v1, n1, in1, 32 * b + 8 * t);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)  // (magnitudes order as their bits do, a NaN above all)
-                m0 = max(m0, __float_as_uint(v0[i]) & 0x7FFFFFFFu), m1 = max(m1, __float_as_uint(v1[i]) & 0x7FFFFFFFu);
+            for (int i = 0; i < 8; i += 2) f0 = max3_abs(f0, v0[i], v0[i + 1]), f1 = max3_abs(f1, v1[i], v1[i + 1]);
         }
+        uint32_t m0 = __float_as_uint(f0), m1 = __float_as_uint(f1);  // (magnitudes order as their bits do, a NaN above all)
 #pragma unroll
         for (int o = 1; o < 4; o <<= 1) {
             m0 = max(m0, __shfl_xor_sync(0xFFFFFFFFu, m0, o));
