@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     auto item_at = [&](int64_t j) { return CL ? i0 + j * p.nslices : j < lead ? tail0 + j : i0 + (j - lead); };
 
     // tensor memory: all 512 columns (two sets of two accumulators of 32, then the A slots of 64), allocated and freed by
-    // the MMA warp. The allocation takes a microsecond: the producer, which has no use for it, goes ahead.
+    // the MMA warp.
     if (warp == kTcMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u)
                      : "memory");
