@@ -229,6 +229,8 @@ def _describe(x, m, entries, epi, act, scale, scale_up, scale_dt, residual, res_
     """The TkdMatmul of one row slice, without the activation, output and residual addresses."""
     a = _tkd.TkdMatmul()
     w0 = entries[0][0]
+    # (the library is told one format and no stream's size)
+    assert all(t is None or t.fmt == w0.fmt for g, u, _ in entries for t in (g, u)), "dense_reader: streams of several formats"
     a.fmt, a.m, a.k = w0.fmt, m, w0.k
     a.ldx = x.shape[-1]
     a.nblocks, a.epilogue, a.act = len(entries), epi, act
@@ -485,6 +487,8 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
         assert glu, "dense_reader: w_up is the GLU's up weight (glu=True)"
         assert (w_up.dtype, tuple(w_up.padded_shape)) == (w.dtype, tuple(w.padded_shape)), "dense_reader: gate and up differ"
         assert str(w_up.memory_config()) == str(w.memory_config()), "dense_reader: gate and up differ"
+        if w_up.fmt != w.fmt:
+            ((w, w_up, _),) = _one_stream_format([(w, w_up, 0)])
         extra["glu2"] = True
     opts = {**opts, **extra}
     M = x.shape[-2]
@@ -519,8 +523,6 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     if topk is not None:
         assert M <= 32, "dense_reader: top-k needs one row slice"
         assert 1 <= topk["rows"] <= 16 and topk["rows"] * topk["k"] <= 64 and topk["rows"] <= M, topk
-    if w_up is not None and w_up.fmt != w.fmt:
-        ((w, w_up, _),) = _one_stream_format([(w, w_up, 0)])
     slices = choose(device, x, w, full_sync, **opts)
     if segs:
         _block_kw_check(device, x, blocks_all, full_sync, opts, slices)

@@ -1,0 +1,70 @@
+"""What linear.matmul describes and keeps, without a GPU: the descriptors' formats and addresses, and which calls a kept one
+serves. Tensors are host ones and no launch is made."""
+
+import pytest
+import torch
+
+from common import ttnn_like as ttnn
+from dense_reader import _tkd, linear
+
+
+class Device:
+    """Stands in for a GPU: tensors made on it are the host's."""
+
+    id, sms, torch = 0, 148, torch.device("cpu")
+
+    def dram_grid_size(self):
+        return ttnn.Grid(8, 1)
+
+
+DEVICE = Device()
+
+
+def weight(k, n, dtype=ttnn.bfloat8_b, wide=False):
+    fmt = _tkd.FMT_BF16 if wide else ttnn.FMT[dtype]
+    stream = torch.zeros(_tkd.lib().tkd_packed_bytes(fmt, k, n), dtype=torch.uint8)
+    emax = None if fmt == _tkd.FMT_BF16 else torch.zeros(_tkd.lib().tkd_padded_cols(n) // 16, dtype=torch.uint8)
+    return ttnn.Weight(stream, emax, k, n, dtype, DEVICE, linear.sharded_memcfg(DEVICE, k, n), fmt=fmt)
+
+
+def tensor(*shape, dtype=ttnn.bfloat16):
+    return ttnn.Tensor(torch.zeros(*shape, dtype=ttnn._TORCH[dtype]), dtype, ttnn.TILE_LAYOUT, DEVICE, None)
+
+
+@pytest.fixture
+def ran(monkeypatch):
+    """The calls that linear.matmul would have launched, in order."""
+    calls = []
+
+    def run(call, x, out, residual):
+        calls.append(call)
+        return out.t if out is not None else torch.zeros(1, 1, x.t.shape[-2], call.launches[0][1].ldo)
+
+    def twin(w):
+        if w.fmt == _tkd.FMT_BF16:
+            return w
+        if getattr(w, "_bf16_twin", None) is None:
+            w._bf16_twin = weight(w.k, w.n, w.dtype, wide=True)
+        return w._bf16_twin
+
+    monkeypatch.setattr(linear._Call, "run", run)
+    monkeypatch.setattr(ttnn, "as_bf16_stream", twin)
+    return calls
+
+
+@pytest.mark.parametrize("m", [1, 16, 64])
+@pytest.mark.parametrize("dtype", [ttnn.bfloat8_b, ttnn.bfloat4_b])
+@pytest.mark.parametrize("which", ["gate", "up"])
+def test_a_gate_and_an_up_weight_of_two_stream_formats(ran, m, dtype, which):
+    """A wide weight is held as a bf16 stream: its partner is streamed as bf16 too, since a launch is told one format."""
+    gate, up = weight(256, 128, dtype, wide=which == "gate"), weight(256, 128, dtype, wide=which == "up")
+    x = tensor(1, 1, m, 256)
+    for _ in range(2):
+        linear.matmul(x, gate, None, w_up=up, glu=True)
+    linear.linear(x, (gate, up), None, activation="swiglu")
+    for call in ran:
+        ((_, a),) = call.launches
+        assert a.fmt == _tkd.FMT_BF16 and a.epilogue == _tkd.EPI_GLU2
+        assert a.block[0].w == ttnn.as_bf16_stream(gate).t.data_ptr() and a.block[0].w_up == ttnn.as_bf16_stream(up).t.data_ptr()
+        assert not a.block[0].emax and not a.block[0].emax_up
+    assert len(ran) == 3

@@ -103,6 +103,26 @@ def test_wide_weight_runs(device, fmt):
     linear.check_status(device)
 
 
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("m", [1, 16, 64])
+@pytest.mark.parametrize("which", ["gate", "up"])
+def test_wide_gate_or_up_weight(device, fmt, m, which):
+    """Two weights of which one is wide (a bf16 stream) and one is not: one launch streams both as bf16."""
+    g = torch.Generator().manual_seed(67 + m)
+    n, k = 192, 512
+    w = [torch.randn(n, k, generator=g) * 0.02 for _ in range(2)]
+    w[which == "up"][:, 7] = torch.randn(n, generator=g) * 1e-17
+    gate, up = (linear.native_weight(device, v, DT[fmt])[0] for v in w)
+    assert (gate.wide, up.wide) == (which == "gate", which == "up")
+    x = torch.randn(m, k, generator=g)
+    G, U = (torch.from_numpy(orc.matmul_f64(x, orc.native_values(v, fmt)[0])) for v in w)
+    want = (torch.nn.functional.silu(G) * U).numpy()
+    for _ in range(2):  # (described, then kept)
+        close_bf16(host(linear.matmul(dev_x(device, x), gate, None, w_up=up, glu=True)), want)
+    close_bf16(host(linear.linear(dev_x(device, x), (gate, up), None, activation="swiglu")), want)
+    linear.check_status(device)
+
+
 @pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
 @pytest.mark.parametrize("m", [1, 4, 8, 13, 32])
 def test_matmul_against_oracle(device, fmt, m):
