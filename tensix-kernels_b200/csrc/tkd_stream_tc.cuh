@@ -751,8 +751,8 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                     const int m4 = (M + 3) >> 2;
                     // The CTA's last item: the ring is idle, and this column's sums of every slice come into it with all
                     // copies in flight together (one trip to L2 instead of one for every four rows), then are added up in
-                    // slice order from shared memory.
-                    const bool staged = j == nitems - 1 && (size_t)ns * m4 * 2048 <= (size_t)nst * p.stage_bytes;
+                    // slice order from shared memory. (An odd m4's last read takes four rows past the last slice's.)
+                    const bool staged = j == nitems - 1 && (size_t)(ns * m4 + (m4 & 1)) * 2048 <= (size_t)nst * p.stage_bytes;
                     const uint32_t ring_c = smem_u32(ring) + et * 16;
                     if (staged) {
                         uint32_t dst = ring_c;

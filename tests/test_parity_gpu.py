@@ -172,6 +172,20 @@ def test_many_rows_epilogues_against_oracle(device, fmt, m, n):
     linear.check_status(device)
 
 
+@pytest.mark.parametrize("m", [9, 12, 13])
+def test_a_panels_sums_as_large_as_the_ring(device, m):
+    """9 to 12 rows of a panel of 24 slices, a CTA each: their sums, three lots of four rows a slice, take the whole of the ring
+    that they are added up in (72 times 2 KB), and the lots are read in pairs."""
+    g = torch.Generator().manual_seed(68 + m)
+    n, k = 128, 24 * 512
+    w, x = torch.randn(n, k, generator=g) * 0.02, torch.randn(m, k, generator=g)
+    tw, _ = linear.native_weight(device, w, ttnn.bfloat4_b)
+    plan = linear.plan(device, dev_x(device, x), tw, noscale=True, ks=512)
+    assert (plan["SLICES"], plan["PANELS"], plan["GRID"]) == (24, 1, 24)
+    close_bf16(host(linear.matmul(dev_x(device, x), tw, None, ks=512)), orc.matmul_f64(x, orc.native_values(w, "bfp4")[0]))
+    linear.check_status(device)
+
+
 def test_config_shapes_full_size(device):
     """The benchmark configurations at their own sizes against the oracle over every column: the README example
     (one token through a [4096, 2048] bfloat8_b weight), the MLP gate/up pair (two [14336, 4096] bfloat4_b weights,
