@@ -76,19 +76,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait: false (and the status word set) when the phase never completes.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status) {
-    for (uint32_t i = 0; i < kWaitRounds; ++i)
+// Warps that meet at named barriers do not leave when one's wait gives up: another's may have been met just in time, and its
+// barriers would wait for the first without a bound. They go on with whatever lies there (the status word says so), no longer
+// patient: a later wait is one look.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, bool patient = true) {
+    for (uint32_t i = 0, n = patient ? kWaitRounds : 1u; i < n; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     if (status) atomicExch(status, kStatusTimeout);
     return false;
 }
 // The same for the roles that spend most of the kernel waiting (the producer lane, the output warps): between tries the
 // warp sleeps, so that its polling does not take issue slots and integer-pipe cycles from the streaming warps.
-__device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, int* status) {
+__device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, int* status, bool patient = true) {
 #ifdef TKD_NO_PARKED_SLEEP
-    return mbar_wait(bar, parity, status);
+    return mbar_wait(bar, parity, status, patient);
 #else
-    for (uint32_t i = 0; i < (kWaitRounds << 2); ++i) {  // (a failing try_wait has itself waited microseconds)
+    for (uint32_t i = 0, n = patient ? kWaitRounds << 2 : 1u; i < n; ++i) {  // (a failing try_wait has itself waited microseconds)
         if (mbar_try_wait(bar, parity)) return true;
         __nanosleep(TKD_PARK_NS);
     }

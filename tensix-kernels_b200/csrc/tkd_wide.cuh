@@ -95,10 +95,11 @@ __device__ __forceinline__ void tmem_wait16(uint32_t (&q)[16]) {
 // (one to a quarter of the tensor memory's lanes) are a worker, and worker wk of nwk takes every nwk-th batch: the output
 // warps alone where a second set of accumulators lets the next tile's MMAs run beside them; with the decode warps as workers
 // 1-4 where there is one set, since nothing can run before it is free (256 rows: 9 us with four warps, of 77 for 512 rows of
-// [4096, 14336] in which a CTA has two tiles).
+// [4096, 14336] in which a CTA has two tiles). met: whether the warp's waits so far were (it goes on either way: see mbar_wait).
 template <int FMT, int EK, int nwk>
 __device__ __forceinline__ void wide_segment(const TkdWide& p, const WideSeg& sg, uint32_t j, bool more, int wk, uint32_t tmem0,
-                                             uint8_t* smem, uint32_t accfull0, uint32_t accempty0, volatile int* sflag, uint32_t xs0) {
+                                             uint8_t* smem, uint32_t accfull0, uint32_t accempty0, volatile int* sflag, uint32_t xs0,
+                                             bool& met) {
     constexpr int CK = Fmt<FMT>::SUBSA * Fmt<FMT>::KSA;
     const int lane = threadIdx.x & 31, ow = (threadIdx.x >> 5) & 3, et = ow * 32 + lane;
     const bool leader = wk == 0 && et == 0;
@@ -142,7 +143,7 @@ __device__ __forceinline__ void wide_segment(const TkdWide& p, const WideSeg& sg
         const int kv = min(p.K, sg.c1 * CK) - sg.c0 * CK;
         const bool two = nm == 2 && kv > 128;
         const uint32_t set = j % p.nset;
-        if (!mbar_wait_parked(accfull0 + 8 * set, (j / p.nset) & 1, p.status)) return;
+        if (!mbar_wait_parked(accfull0 + 8 * set, (j / p.nset) & 1, p.status, met)) met = false;
         tc_fence_after();
         const uint32_t ta = tmem0 + ((uint32_t)(ow * 32) << 16) + set * nm * NT;
         // sixteen rows of the segment's sums
@@ -556,10 +557,11 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
                 }
             }
         };
-        bool ok = true;
+        bool met = true;
         uint32_t j = 0;
-        for (int it = i0; ok && wide_next(p, it, i1, sg);) {
-            for (int c = decode ? sg.c0 : sg.c1; ok && c < sg.c1; ++c) {
+        for (int it = i0; wide_next(p, it, i1, sg);) {
+            bool ok = true;
+            for (int c = decode && met ? sg.c0 : sg.c1; ok && c < sg.c1; ++c) {
                 ok = mbar_wait(full0 + 8 * slot, phase, p.status);
                 if (!ok) break;
                 const int nsa = KWHOLE ? F::SUBSA : min(F::SUBSA, nsa_total - c * F::SUBSA);
@@ -596,10 +598,12 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
                 if (ok && lane == 0) mbar_arrive(empty0 + 8 * slot);
                 if (++slot == (uint32_t)nst) slot = 0, phase ^= 1;
             }
+            met = met && ok;
             // (the output and the residual may be the kernel before's: waited for once)
             if (j == 0 && (SHARED || !decode)) asm volatile("griddepcontrol.wait;" ::: "memory");
-            if (ok && (SHARED || !decode))
-                wide_segment<FMT, EK, SHARED ? kWideWorkers : 1>(p, sg, j, it < i1, SHARED ? 1 + sub4 : 0, tmem0, smem, accfull0, accempty0, sflag, xs0);
+            if (SHARED || !decode)
+                wide_segment<FMT, EK, SHARED ? kWideWorkers : 1>(p, sg, j, it < i1, SHARED ? 1 + sub4 : 0, tmem0, smem, accfull0, accempty0, sflag,
+                                                                 xs0, met);
             ++j;
         }
     }
