@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
             }
         }
         uint32_t np = 0;
+        bool met = true;
         int qw = -1;  // the slot whose routing weights are in wrow
         float* const col = pbuf + (size_t)et * MP;
         for (int it = i0; it < i1; ++np) {
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
                     bg = bf16_bits_to_f32(b[0]), bu = bf16_bits_to_f32(b[32]);
                 }
             }
-            if (!mbar_wait_parked(pfull, np & 1, p.status)) break;
+            if (!mbar_wait_parked(pfull, np & 1, p.status, met)) met = false;  // (and on: see mbar_wait)
             float v[RW];  // the column's sums
 #pragma unroll
             for (int m = 0; m < RW; m += 4) {
