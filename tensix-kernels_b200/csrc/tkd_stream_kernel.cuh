@@ -967,8 +967,8 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
         Cursor c;
         uint32_t pi = 0;
         float tot[MR];
-        bool ok = true;
-        for (int64_t j = 0; j < i1 - i0 && ok; ++j) {
+        bool met = true;
+        for (int64_t j = 0; j < i1 - i0; ++j) {
             const int64_t it = j < lead ? tail0 + j : i0 + (j - lead);
             if (j == 0 || j == lead)
                 cursor_init(c, p, it);
@@ -992,8 +992,7 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
                 sc = p.scale_dt == TKD_DT_BF16 ? bf16_bits_to_f32(static_cast<const uint16_t*>(sp)[n])
                                                : static_cast<const float*>(sp)[n];
             }
-            ok = mbar_wait_parked(pfull0 + 8 * pb, (NPB == 2 ? pi >> 1 : pi) & 1, p.status);
-            if (!ok) break;
+            if (!mbar_wait_parked(pfull0 + 8 * pb, (NPB == 2 ? pi >> 1 : pi) & 1, p.status, met)) met = false;
             bool finish = !f.split;
             if (!f.split) {
                 // the two halves' sums cover the whole panel

@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
         }
         float* const trow = tbuf + (size_t)et * MP;
         uint16_t* y16 = static_cast<uint16_t*>(p.out);
-        for (int64_t j = 0; !CL && j < nitems && ok; ++j) {
+        for (int64_t j = 0; !CL && j < nitems; ++j) {
             const int64_t it = item_at(j);
             if (j == 0 || j == lead)
                 cursor_init(c, p, it);
@@ -672,8 +672,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 }
             }
             const uint32_t buf = (uint32_t)j & 1;
-            ok = mbar_wait(accfull0 + 8 * buf, ((uint32_t)j >> 1) & 1, p.status);
-            if (!ok) break;
+            if (!mbar_wait(accfull0 + 8 * buf, ((uint32_t)j >> 1) & 1, p.status, ok)) ok = false;  // (and on: see mbar_wait)
             tc_fence_after();
             {
                 // the slice's sum d0 + d1 (d1 only if the slice has a second unit), sixteen rows at a time: both
