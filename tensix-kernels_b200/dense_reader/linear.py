@@ -447,6 +447,10 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
                 check_banks(u, max_banks)
     check_banks(w_up, max_banks)
     assert fidelity in FIDELITY, fidelity
+    # the caller's weights (what is launched may be a twin of one: see _one_stream_format)
+    own = [w, w_up]
+    if is_block_list(w):
+        own = [u for wt, _ in w for u in (wt if isinstance(wt, (list, tuple)) else (wt,))]
     segs = ()
     if isinstance(w, (list, tuple)):
         assert is_block_list(w), "dense_reader: w is one weight or a block list [(w | (gate, up), col0_tiles), ...]"
@@ -534,7 +538,8 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
         need = max(need, n)
     scales = col_scales if isinstance(col_scales, (tuple, list)) else (col_scales,)
     others = [t for g, u, _ in blocks_all for t in (g, u)][1:]
-    call = _Call(device, launches, need, (scale, col_scales, *scales, hadamard, topk and topk["r"], *others), y.dtype, exchange)
+    keep = [t for t in (scale, col_scales, *scales, hadamard, topk and topk["r"], *others, *own) if t is not own[0]]
+    call = _Call(device, launches, need, keep, y.dtype, exchange)
     call.run(x, y, residual)
     return y, call
 
@@ -580,19 +585,19 @@ _PLAIN = {int, bool, str, type(None)}
 
 
 def _call_key(x, w, scale, topk, out, col0, w_up, max_banks, fidelity, opts):
-    """(the weight a call is kept with, what else shapes it). Objects are named by their identities: the kept call keeps
-    them alive, so the identities stay theirs."""
+    """(the weight a call is kept with, what else shapes it). Weights are named by their serial numbers, which never come back;
+    other objects by their identities: the kept call keeps those alive."""
     if type(w) is list or type(w) is tuple:
         try:
-            wk = tuple([(id(e[0]) if type(e[0]) is not tuple and type(e[0]) is not list else tuple(map(id, e[0])), e[1]) for e in w])
+            wk = tuple([(e[0].serial if type(e[0]) is ttnn.Weight else tuple([u.serial for u in e[0]]), e[1]) for e in w])
             first = w[0][0]
             if type(first) is tuple or type(first) is list:
                 first = first[0]
-        except (TypeError, IndexError):
+        except (TypeError, IndexError, AttributeError):
             return None, None  # (not a block list: the full path says so)
     else:
         first, wk = w, None
-    if type(first) is not ttnn.Weight:
+    if type(first) is not ttnn.Weight or not (w_up is None or type(w_up) is ttnn.Weight):
         return None, None
     ok = ()
     if opts:
@@ -601,8 +606,8 @@ def _call_key(x, w, scale, topk, out, col0, w_up, max_banks, fidelity, opts):
     tk = None
     if topk is not None:
         tk = (id(topk["r"]), topk["k"], topk["rows"], topk["slot0"], topk["base"], topk["n"], topk.get("write_y", False), TOPK_UNIT)
-    return first, (x.t.shape, None if out is None else out.t.shape, wk, id(scale), id(w_up), col0, max_banks, fidelity, ok, tk,
-                   KS, MAX_CTAS, dev.MAX_BANKS)
+    return first, (x.t.shape, None if out is None else out.t.shape, wk, id(scale), None if w_up is None else w_up.serial, col0, max_banks,
+                   fidelity, ok, tk, KS, MAX_CTAS, dev.MAX_BANKS)
 
 
 class _Call:

@@ -68,3 +68,32 @@ def test_a_gate_and_an_up_weight_of_two_stream_formats(ran, m, dtype, which):
         assert a.block[0].w == ttnn.as_bf16_stream(gate).t.data_ptr() and a.block[0].w_up == ttnn.as_bf16_stream(up).t.data_ptr()
         assert not a.block[0].emax and not a.block[0].emax_up
     assert len(ran) == 3
+
+
+@pytest.mark.parametrize("form", ["list", "pairs", "w_up"])
+def test_a_kept_call_is_its_weights_own(ran, form):
+    """The first weight wide, another not, so that the other is launched as its bf16 twin: a later weight in its place (at its
+    object's address too, once it is gone) is another call, and a freed one's call is not run again."""
+    k, n, x = 256, 128, tensor(1, 1, 4, 256)
+    first, g2 = weight(k, n, wide=True), weight(k, n, wide=True)
+
+    def call(w):
+        if form == "w_up":
+            linear.matmul(x, first, None, w_up=w, glu=True)
+        else:
+            linear.matmul(x, [((first, g2), 0), ((w, w), n // 32)] if form == "pairs" else [(first, 0), (w, n // 32)], None)
+        ((_, a),) = ran[-1].launches
+        at = {"list": a.block[1].w, "pairs": a.block[1].w_up, "w_up": a.block[0].w_up}[form]
+        assert at == ttnn.as_bf16_stream(w).t.data_ptr()
+
+    for _ in range(20):
+        w = weight(k, n)
+        call(w)
+        call(w)
+        assert ran[-1] is ran[-2]
+        del w
+    w = weight(k, n)
+    call(w)
+    kept = ran[-1]
+    ttnn.deallocate(w)
+    assert not kept.fits(x, None)
