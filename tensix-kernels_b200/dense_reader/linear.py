@@ -584,6 +584,22 @@ def records_together(x, weights, topk, out):
 _PLAIN = {int, bool, str, type(None)}
 
 
+class _Unnamed(Exception):
+    """An option that nothing a kept call holds can name: the call is described anew each time."""
+
+
+def _option_key(k, v):
+    """What names an option that is no plain value: all that is checked of a residual, and the identities of objects that the
+    kept call holds (a list's elements: the list may be changed)."""
+    if k == "residual" and type(v) is ttnn.Tensor:
+        return v.t.shape, id(v.dtype), id(v.layout), id(v._mc.memory_layout)
+    if k == "col_scales":
+        return tuple(map(id, v)) if type(v) is tuple or type(v) is list else id(v)
+    if k == "hadamard" or k == "exchange":
+        return id(v)
+    raise _Unnamed
+
+
 def _call_key(x, w, scale, topk, out, col0, w_up, max_banks, fidelity, opts):
     """(the weight a call is kept with, what else shapes it). Weights are named by their serial numbers, which never come back;
     other objects by their identities: the kept call keeps those alive."""
@@ -601,11 +617,14 @@ def _call_key(x, w, scale, topk, out, col0, w_up, max_banks, fidelity, opts):
         return None, None
     ok = ()
     if opts:
-        ok = tuple([(k, v if type(v) in _PLAIN else tuple(map(id, v)) if type(v) is tuple else
-                     (v.t.shape, id(v.dtype)) if k == "residual" and type(v) is ttnn.Tensor else id(v)) for k, v in opts.items()])
+        try:
+            ok = tuple([(k, v if type(v) in _PLAIN else _option_key(k, v)) for k, v in opts.items()])
+        except _Unnamed:
+            return None, None
     tk = None
     if topk is not None:
-        tk = (id(topk["r"]), topk["k"], topk["rows"], topk["slot0"], topk["base"], topk["n"], topk.get("write_y", False), TOPK_UNIT)
+        tk = (id(topk["r"]), int(topk["k"]), int(topk["rows"]), int(topk["slot0"]), int(topk["base"]), int(topk["n"]),
+              bool(topk.get("write_y", False)), TOPK_UNIT)
     return first, (x.t.shape, None if out is None else out.t.shape, wk, id(scale), None if w_up is None else w_up.serial, col0, max_banks,
                    fidelity, ok, tk, KS, MAX_CTAS, dev.MAX_BANKS)
 

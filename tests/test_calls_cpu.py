@@ -1,6 +1,7 @@
 """What linear.matmul describes and keeps, without a GPU: the descriptors' formats and addresses, and which calls a kept one
 serves. Tensors are host ones and no launch is made."""
 
+import numpy as np
 import pytest
 import torch
 
@@ -18,6 +19,12 @@ class Device:
 
 
 DEVICE = Device()
+
+
+class DeviceScale(torch.Tensor):
+    """A host tensor where the device's is asked for."""
+
+    is_cuda = True
 
 
 def weight(k, n, dtype=ttnn.bfloat8_b, wide=False):
@@ -97,3 +104,27 @@ def test_a_kept_call_is_its_weights_own(ran, form):
     kept = ran[-1]
     ttnn.deallocate(w)
     assert not kept.fits(x, None)
+
+
+def test_options_that_a_kept_call_does_not_hold(ran):
+    """Options that are no plain values (a number of another type, whose object is gone after the call) and lists that change
+    name no kept call; a residual that is refused is refused beside a kept call too."""
+    k, n, x = 256, 128, tensor(1, 1, 4, 256)
+    gate, up = weight(k, n), weight(k, n)
+    for i in range(40):
+        linear.matmul(x, gate, None, w_up=up, glu=True, glu_act=np.int64(i & 1))
+        assert ran[-1].launches[0][1].act == i & 1
+    scales = [torch.ones(n), torch.ones(n)]
+    for t in scales:
+        t.__class__ = DeviceScale
+    linear.matmul(x, gate, None, w_up=up, glu=True, col_scales=scales)
+    other = torch.ones(n)
+    other.__class__ = DeviceScale
+    scales[1] = other
+    linear.matmul(x, gate, None, w_up=up, glu=True, col_scales=scales)
+    assert ran[-1].launches[0][1].scale_up == other.data_ptr()
+    linear.matmul(x, gate, None, residual=tensor(1, 1, 4, n))
+    sharded = tensor(1, 1, 4, n)
+    sharded._mc = gate.memory_config()
+    with pytest.raises(AssertionError):
+        linear.matmul(x, gate, None, residual=sharded)
