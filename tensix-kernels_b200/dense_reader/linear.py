@@ -23,6 +23,7 @@ What differs from the reference, by necessity or on purpose:
 import ctypes
 import itertools
 import sys
+import weakref
 from pathlib import Path
 
 import torch
@@ -83,6 +84,7 @@ _WEIGHT_CALLS = 64  # described calls kept with a weight, at most
 _CHOICE = {}     # the plan cache
 _WORKSPACE = {}  # device id -> zeroed uint8 tensor
 _OUTGROWN = []   # workspaces replaced by larger ones
+_COUNTED = []    # (device id, a weak reference) of every workspace, the mixture-of-experts layers' too
 _STATUS = {}     # device id -> int32 status word
 
 
@@ -203,7 +205,14 @@ def _workspace(device, nbytes):
         if ws is not None:
             _OUTGROWN.append(ws)
             nbytes = max(nbytes, 2 * ws.numel())
-        ws = _WORKSPACE[_ws_key(device)] = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device.torch)
+        ws = _WORKSPACE[_ws_key(device)] = new_workspace(device, max(nbytes, 1 << 20))
+    return ws
+
+
+def new_workspace(device, nbytes):
+    """A zeroed workspace for the kernels' counters and sums, which check_status knows of while it lives."""
+    ws = torch.zeros(nbytes, dtype=torch.uint8, device=device.torch)
+    _COUNTED[:] = [r for r in _COUNTED if r[1]() is not None] + [(device.id, weakref.ref(ws))]
     return ws
 
 
@@ -219,9 +228,13 @@ def check_status(device):
     """Synchronise and raise if a kernel of this device reported an error (a bounded wait that gave up)."""
     code = int(status_word(device).item())
     if code:
+        # Every workspace's counters may be mid-count. They are zeroed where they are: captured graphs hold their addresses.
+        torch.cuda.synchronize(device.torch)
         status_word(device).zero_()
-        for key in [k for k in _WORKSPACE if k[0] == device.id]:
-            _WORKSPACE.pop(key)  # their counters may be mid-count
+        for ws in [r() for at, r in _COUNTED if at == device.id]:
+            if ws is not None:
+                ws.zero_()
+        torch.cuda.synchronize(device.torch)
         raise _tkd.TkdError(code, "a kernel reported")
 
 

@@ -476,7 +476,7 @@ def _workspace(P, what, op):
     on one layer run in stream order). One outgrown stays alive for the CUDA graphs that hold its address."""
     held = P["_ws"].setdefault(what, [])
     if not held or held[-1].numel() < op.need:
-        held.append(torch.zeros(op.need, dtype=torch.uint8, device=P["_device"].torch))
+        held.append(linear.new_workspace(P["_device"], op.need))
     return held[-1]
 
 

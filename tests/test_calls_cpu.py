@@ -128,3 +128,32 @@ def test_options_that_a_kept_call_does_not_hold(ran):
     sharded._mc = gate.memory_config()
     with pytest.raises(AssertionError):
         linear.matmul(x, gate, None, residual=sharded)
+
+
+def test_an_error_zeroes_every_workspace(monkeypatch):
+    """A kernel that gave up a wait may leave counters mid-count, in linear's workspaces (one outgrown, which a graph may hold,
+    among them) and in a mixture-of-experts layer's: check_status zeroes them all in place."""
+    from moe import moe8
+
+    for name in ("_WORKSPACE", "_STATUS"):
+        monkeypatch.setattr(linear, name, {})
+    for name in ("_OUTGROWN", "_COUNTED"):
+        monkeypatch.setattr(linear, name, [])
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    layer, op = {"_ws": {}, "_device": DEVICE}, type("Op", (), {"need": 4096})
+    small = linear._workspace(DEVICE, 1 << 20)
+    large = linear._workspace(DEVICE, 3 << 20)
+    own = moe8._workspace(layer, "gu rows", op)
+    assert small is not large
+    gone = linear.new_workspace(DEVICE, 64)
+    del gone
+    for ws in (small, large, own):
+        ws.fill_(3)
+    linear.check_status(DEVICE)  # (no error: nothing is touched)
+    assert all((ws == 3).all() for ws in (small, large, own))
+    linear.status_word(DEVICE).fill_(3)
+    with pytest.raises(_tkd.TkdError):
+        linear.check_status(DEVICE)
+    assert not any(ws.any() for ws in (small, large, own)) and not linear.status_word(DEVICE).any()
+    assert linear._workspace(DEVICE, 64) is large and moe8._workspace(layer, "gu rows", op) is own
+    linear.check_status(DEVICE)
