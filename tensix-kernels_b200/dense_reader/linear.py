@@ -175,10 +175,16 @@ def row_slices(x, full_sync=False):
 ROWS_MAX = 2048  # rows of one launch for more than 32 (its copy of x grows with them; the weights are read once per 256 rows)
 
 
-def _launch_rows(M, fmt, topk, exchange, hadamard):
-    """[(first row, rows)] of the launches a call of M rows makes: slices of up to 32, or more where tkd_matmul_rows serves."""
-    wide = M > 32 and fmt != _tkd.FMT_INT4 and topk is None and exchange is None and hadamard is None
-    parts = -(-M // (ROWS_MAX if wide else 32))
+# What a launch has counters for (the head of a workspace): tiles of 128 columns (and, past 32 rows, of up to 256 rows), top-k units
+MAX_TILES, MAX_UNITS = 48 * 1024, 16 * 1024
+
+
+def _launch_rows(M, panels, fmt, topk, exchange, hadamard):
+    """[(first row, rows)] of the launches a call of M rows over so many panels of columns makes: slices of up to 32, or more where
+    tkd_matmul_rows serves."""
+    most = min(ROWS_MAX, 256 * (MAX_TILES // panels))
+    wide = M > 32 and most and fmt != _tkd.FMT_INT4 and topk is None and exchange is None and hadamard is None
+    parts = -(-M // (most if wide else 32))
     if not wide:
         return [(m0, min(32, M - m0)) for m0 in range(0, M, 32)]
     per = -(-M // parts)
@@ -544,7 +550,8 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     if segs:
         _block_kw_check(device, x, blocks_all, full_sync, opts, slices)
     launches, need = [], 0
-    for m0, m in _launch_rows(M, w.fmt, topk, exchange, hadamard):
+    panels = -(-w.shape[-1] // 128) * (1 if w_up is None else 2)
+    for m0, m in _launch_rows(M, panels, w.fmt, topk, exchange, hadamard):
         a, n = _describe_rows(x, blocks_all, scale, col_scales, y, m, topk, act, residual, glu, out32,
                               opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, hadamard)
         launches.append((m0, a))
@@ -578,11 +585,13 @@ def records_together(x, weights, topk, out):
     after = lambda t, i: None if t is None else t.data_ptr() + i * t.numel()  # noqa: E731  (byte tensors)
     adjacent = all(w.t.data_ptr() == after(first.t, i) and (w.emax is None or w.emax.data_ptr() == after(first.emax, i))
                    for i, w in enumerate(weights))
-    for b0 in range(0, len(weights), len(weights) if adjacent else 4):
-        part = weights[:1] if adjacent else weights[b0 : b0 + 4]
+    most = max(1, min(len(weights) if adjacent else 4, MAX_TILES // (-(-N // 128)), MAX_UNITS // units))
+    for b0 in range(0, len(weights), most):
+        part = weights[b0 : b0 + most]
+        repeats = len(part) if adjacent else 0
         spec = {**topk, "slot0": topk["slot0"] + b0 * units, "base": topk["base"] + b0 * N}
-        a, n = _describe_rows(x, [(w, None, 0) for w in part], None, None, out, x.shape[-2], spec, 0, None, False, False, KS or 0,
-                              MAX_CTAS or 0, repeats=len(weights) if adjacent else 0)
+        a, n = _describe_rows(x, [(w, None, 0) for w in (part[:1] if adjacent else part)], None, None, out, x.shape[-2], spec, 0, None, False,
+                              False, KS or 0, MAX_CTAS or 0, repeats=repeats)
         launches.append((0, a, ctypes.addressof(a)))
         need = max(need, n)
     call = _Call(x.device(), launches, need, (topk["r"], *weights[1:], weights), out.dtype, None)

@@ -1,6 +1,8 @@
 """What linear.matmul describes and keeps, without a GPU: the descriptors' formats and addresses, and which calls a kept one
 serves. Tensors are host ones and no launch is made."""
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -157,3 +159,52 @@ def test_an_error_zeroes_every_workspace(monkeypatch):
     assert not any(ws.any() for ws in (small, large, own)) and not linear.status_word(DEVICE).any()
     assert linear._workspace(DEVICE, 64) is large and moe8._workspace(layer, "gu rows", op) is own
     linear.check_status(DEVICE)
+
+
+@pytest.mark.parametrize("rows,n,two", [(33, 128, False), (2048, 151936, False), (2048, 1 << 20, False), (512, 1 << 20, True),
+                                        (700, 6291456, False), (2049, 4096, True)])
+def test_rows_of_wide_outputs_are_launched_as_they_can_be(rows, n, two):
+    """More than 32 rows over so many columns that a launch has no counter for every tile of them: fewer rows a launch."""
+    panels = -(-n // 128) * (2 if two else 1)
+    at = 0
+    for row0, m in linear._launch_rows(rows, panels, _tkd.FMT_BFP4, None, None, None):
+        assert row0 == at and m >= 1
+        at += m
+        a, need = _tkd.TkdMatmul(), ctypes.c_uint64()
+        a.fmt, a.m, a.k, a.nblocks, a.out_dtype = _tkd.FMT_BFP4, m, 64, 1, _tkd.DT_BF16
+        a.epilogue = _tkd.EPI_GLU2 if two else _tkd.EPI_PLAIN
+        a.block[0].n = n
+        L = _tkd.lib()
+        _tkd.check((L.tkd_matmul_workspace if m <= 32 else L.tkd_matmul_rows_workspace)(ctypes.byref(a), ctypes.byref(need)), "workspace")
+    assert at == rows
+
+
+@pytest.mark.parametrize("adjacent", [True, False])
+@pytest.mark.parametrize("unit,launches", [(2048, 1), (128, 2)])
+def test_records_of_many_columns_are_launched_as_they_can_be(monkeypatch, adjacent, unit, launches):
+    """A head's blocks in one launch only as far as it has counters for their units; every block's slots and indices once."""
+    made = []
+    host = type("Host", (), {"matmul": staticmethod(lambda a, *rest: made.append(_tkd.TkdMatmul.from_buffer_copy(
+        (ctypes.c_char * ctypes.sizeof(_tkd.TkdMatmul)).from_address(a))))})
+    monkeypatch.setattr(_tkd, "host", lambda: host)
+    monkeypatch.setattr(linear, "TOPK_UNIT", unit)
+    monkeypatch.setattr(linear, "_workspace", lambda device, need: torch.zeros(1))
+    k, n, count = 32, 1 << 20, 3
+    L = _tkd.lib()
+    streams = torch.zeros(count, L.tkd_packed_bytes(_tkd.FMT_BFP4, k, n), dtype=torch.uint8)
+    emaxes = torch.zeros(count, n // 16, dtype=torch.uint8)
+    order = range(count) if adjacent else (2, 0, 1)
+    mc = linear.sharded_memcfg(DEVICE, k, n)
+    weights = tuple(ttnn.Weight(streams[i], emaxes[i], k, n, ttnn.bfloat4_b, DEVICE, mc) for i in order)
+    units = linear.topk_units(n)
+    r = tensor(1, 1, count * units, 2, dtype=ttnn.uint32)
+    topk = {"r": r, "k": 1, "rows": 1, "slot0": 5, "base": 7, "n": n}
+    for _ in range(2):
+        linear.records_together(tensor(1, 1, 1, k), weights, topk, tensor(1, 1, 1, n))
+    assert len(made) == 2 * launches
+    got = []
+    for a in made[: len(made) // 2]:
+        for b in range(max(a.nblocks, a.repeats)):
+            at = a.block[0].w + b * streams.shape[1] if a.repeats else a.block[b].w
+            got.append((at, a.topk_slot0 + b * units, a.topk_base + b * n))
+    assert got == [(w.t.data_ptr(), 5 + b * units, 7 + b * n) for b, w in enumerate(weights)]
