@@ -571,12 +571,15 @@ def records_together(x, weights, topk, out):
     written."""
     first = weights[0]
     key = ("records", x.t.shape, out.t.shape, id(weights), id(topk["r"]), topk["k"], topk["rows"], topk["slot0"],
-           topk["base"], topk["n"], TOPK_UNIT, KS, MAX_CTAS)
+           topk["base"], topk["n"], TOPK_UNIT, KS, MAX_CTAS, dev.MAX_BANKS)
     call = first.calls.get(key) if CACHE else None
     if call is not None and call.fits(x, out):
         for a in call.launches:
             call.launch(a[2], x.t, out.t, None, _workspace(call.device, call.need), 0)
         return
+    for w in weights:
+        check_banks(w)
+    assert x.memory_config().memory_layout == ttnn.TensorMemoryLayout.INTERLEAVED, x.memory_config()
     N, units = first.n, topk_units(first.n)
     assert not topk.get("write_y", False) and x.dtype == ttnn.bfloat16 and x.shape[-1] == first.k and x.shape[-2] <= 32
     assert all(type(w) is ttnn.Weight and (w.k, w.n, w.fmt) == (first.k, N, first.fmt) for w in weights)

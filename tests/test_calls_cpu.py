@@ -208,3 +208,16 @@ def test_records_of_many_columns_are_launched_as_they_can_be(monkeypatch, adjace
             at = a.block[0].w + b * streams.shape[1] if a.repeats else a.block[b].w
             got.append((at, a.topk_slot0 + b * units, a.topk_base + b * n))
     assert got == [(w.t.data_ptr(), 5 + b * units, 7 + b * n) for b, w in enumerate(weights)]
+
+
+def test_records_together_refuses_what_matmul_refuses(monkeypatch):
+    monkeypatch.setattr(_tkd, "host", lambda: type("Host", (), {"matmul": staticmethod(lambda *a: None)}))
+    weights = (weight(64, 128), weight(64, 128))
+    topk = {"r": tensor(1, 1, 2, 2, dtype=ttnn.uint32), "k": 1, "rows": 1, "slot0": 0, "base": 0, "n": 128}
+    x, out = tensor(1, 1, 1, 64), tensor(1, 1, 1, 128)
+    x._mc = weights[0].memory_config()
+    with pytest.raises(AssertionError):
+        linear.records_together(x, weights, topk, out)
+    monkeypatch.setattr(linear.dev, "MAX_BANKS", 4)
+    with pytest.raises(ValueError):
+        linear.records_together(tensor(1, 1, 1, 64), weights, topk, out)
