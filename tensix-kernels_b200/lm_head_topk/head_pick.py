@@ -86,7 +86,7 @@ def pick(records, x, rows_t, nrows, k, top=16, logits="bf16", out=None, valid=No
     rows). A row with no valid candidate gets token 0 and count 0. ids_out: also row 0's token into this one-element
     uint32 tensor. (head_pick.py:101-220)"""
     key = (records.t.shape, records.dtype, x.t.shape, x.dtype, rows_t.t.shape, rows_t.dtype, rows_t.layout, id(rows_t._mc), nrows, k,
-           top, logits, valid)
+           top, logits, None if valid is None else int(valid))
     settings = _PICKS.get(key)
     if settings is None:
         settings = _pick_settings(records, x, rows_t, nrows, k, top, logits, valid)

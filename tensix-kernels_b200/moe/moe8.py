@@ -545,7 +545,8 @@ def route(logits, ids, w, k, *, kind="softmax", bias=None, ids32=False, experts=
     4). groups=(n_group, topk_group): the sigmoid kind with a bias; a group's score the sum of its two largest keys, the
     topk_group best groups kept. slot: that id as slot k of every row at weight 1.0 (ids and w hold k + 1). Returns w."""
     key = (logits.t.shape, ids.t.shape, w.t.shape, k, kind, None if bias is None else bias.t.shape, ids32, experts,
-           None if shared is None else shared.t.shape, scale, norm, groups and tuple(groups), slot)
+           None if shared is None else shared.t.shape, float(scale), bool(norm),
+           None if groups is None else (int(groups[0]), int(groups[1])), None if slot is None else int(slot))
     settings = _ROUTES.get(key)
     if (settings is None or logits.dtype is not ttnn.float32 or ids.dtype is not (ttnn.uint32 if ids32 else ttnn.uint16)
             or w.dtype is not ttnn.bfloat16 or (bias is not None and bias.dtype is not ttnn.float32)

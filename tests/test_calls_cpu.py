@@ -210,6 +210,30 @@ def test_records_of_many_columns_are_launched_as_they_can_be(monkeypatch, adjace
     assert got == [(w.t.data_ptr(), 5 + b * units, 7 + b * n) for b, w in enumerate(weights)]
 
 
+def test_settings_given_as_arrays(monkeypatch):
+    """head_pick.pick and moe8.route keep their checked settings by value: numbers given as arrays and tensors serve as before, and
+    an array changed in place is read anew."""
+    from lm_head_topk import head_pick
+    from moe import moe8
+
+    made = []
+    host = type("Host", (), {"pick": staticmethod(lambda *a: made.append(a[5])), "route": staticmethod(lambda *a: made.append(a[5]))})
+    monkeypatch.setattr(_tkd, "host", lambda: host)
+    records, x = tensor(1, 1, 4, 16, dtype=ttnn.uint32), tensor(1, 1, 1, 64)
+    rows_t = ttnn.Tensor(torch.zeros(1, 1, 128, 64, dtype=torch.bfloat16), ttnn.bfloat16, ttnn.ROW_MAJOR_LAYOUT, DEVICE, None)
+    valid = np.array(100)
+    for v in (100, 90):
+        valid[...] = v
+        head_pick.pick(records, x, rows_t, 1, 8, valid=valid)
+        assert made[-1][4] == v
+    logits, ids, w = tensor(1, 1, 1, 64, dtype=ttnn.float32), tensor(1, 1, 1, 8, dtype=ttnn.uint16), tensor(1, 1, 1, 8)
+    bias, scale = tensor(1, 1, 1, 64, dtype=ttnn.float32), torch.tensor(1.0)
+    for v in (1.0, 2.5):
+        scale.fill_(v)
+        moe8.route(logits, ids, w, 8, kind="sigmoid", bias=bias, scale=scale, groups=np.array([4, 2]))
+        assert made[-1][4] == v and made[-1][6:8] == (4, 2)
+
+
 def test_records_together_refuses_what_matmul_refuses(monkeypatch):
     monkeypatch.setattr(_tkd, "host", lambda: type("Host", (), {"matmul": staticmethod(lambda *a: None)}))
     weights = (weight(64, 128), weight(64, 128))
