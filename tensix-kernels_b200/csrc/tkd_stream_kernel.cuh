@@ -188,17 +188,20 @@ __device__ __forceinline__ uint32_t f32x2_to_bf16x2(float lo, float hi) {
 }
 
 
-// a / (1 + e^t), |error| about two units in the last place, without a branch: the division's slow path (a call for extreme
-// operands) kept an output stage's rows from running side by side, 250 ns a row. The reciprocal of the hardware, corrected by
-// one step of Newton's iteration; a divisor past 2^64 is taken down by 2^64 first, so that its reciprocal stays a normal number.
+// a / (1 + e^t) as the division gives it, without a branch: the division's slow path (a call for extreme operands) kept an output
+// stage's rows from running side by side, 250 ns a row. The hardware's reciprocal, corrected by one step of Newton's iteration,
+// then the quotient by its exact remainder (P. Markstein, IBM J. Res. Dev. 34, 1990). A divisor past 2^64 is taken down by 2^64
+// first, so that its reciprocal stays a normal number. A divisor past the largest number, and an infinite a, whose remainder is no
+// number (t is minus infinity then: a minus infinity has a divisor without end), are the division's too.
 __device__ __forceinline__ float over_one_plus_exp(float a, float t) {
-    const float d = 1.f + __expf(fminf(t, 88.7f));
+    const float d = 1.f + __expf(t);
     const float k = d > 0x1p64f ? 0x1p-64f : 1.f, dk = d * k;
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(dk));
     r = fmaf(r, fmaf(-dk, r, 1.f), r);
-    const float q = a * r * k;
-    return t > 88.72f ? a * 0.f : q;  // (where e^t is no number any more the quotient is none; a NaN stays one)
+    float q = a * r;
+    q = fmaf(fminf(fmaf(-dk, q, a), 0x1.fffffep127f), r, q) * k;
+    return d > 0x1.fffffep127f ? a * 0.f : q;
 }
 // dense_ops.h:44-59 of the reference: silu, and gelu_tanh as x * sigmoid(2 u), u = sqrt(2 / pi) (x + 0.044715 x^3)
 __device__ __forceinline__ float act_gate(float g, int act) {

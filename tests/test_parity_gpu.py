@@ -703,3 +703,35 @@ def test_plain_calls_equal_the_counted_kernels(device, dtype, k, m):
         torch.cuda.synchronize()
         assert status.item() == 0 and torch.isfinite(outs[0]).all() and not (outs[0] == 7.0).all()
         assert torch.equal(outs[0], outs[1]), (epi, cols)
+
+
+@pytest.mark.parametrize("m", [1, 3, 20, 40])
+@pytest.mark.parametrize("act", [0, 1])
+def test_activations_over_their_range(device, m, act):
+    """act(gate) * up, the gates any float32 (a weight of 1 times its column's scale), up 1: within a rounding to bf16 of the
+    float64 value over the whole range, and at the edges: where e^-u passes 2^64 and the largest float32, at infinities and NaN.
+    2^-8 for the rounding (8 significant bits), and for e^t in float32 2^-23 |t| (t's rounding and its product's with log2 e) and 2^-21 (the
+    exponential's own two units, the sum and the quotient)."""
+    g = torch.Generator().manual_seed(99)
+    edges = torch.tensor([0.0, -0.0, 44.36, -44.36, -44.37, -88.69, -88.7, -88.71, -88.72, -88.7228, -88.7229, -88.73, -104.0, 88.7, 1e30, -1e30,
+                          7.9, -7.9, -7.91, -10.0, -10.1, -10.2, float("inf"), float("-inf"), float("nan")])
+    gates = torch.cat([edges, torch.rand(2000, generator=g) * 200 - 100, torch.randn(2000, generator=g) * 4,
+                       torch.randn(71, generator=g) * torch.exp2(torch.rand(71, generator=g) * 60 - 40)])
+    n, k = gates.numel(), 32
+    one = torch.zeros(n, k)
+    one[:, 0] = 1.0
+    gate, up = (linear.native_weight(device, one, ttnn.bfloat16)[0] for _ in range(2))
+    x = torch.zeros(m, k)
+    x[:, 0] = 1.0
+    scales = (gates.to(device.torch), torch.ones(n, device=device.torch))
+    got = host(linear.matmul(dev_x(device, x), gate, None, w_up=up, glu=True, glu_act=act, col_scales=scales)).double()
+    v = gates.double()
+    t = -v if act == 0 else -(v * (1.5957691216 + 0.0713548162 * v * v))
+    want = v / (1 + torch.exp(t))  # (-inf / inf: no number)
+    for row in got:
+        assert torch.equal(row.isnan(), want.isnan()) and torch.equal(row.isinf(), want.isinf())
+        ok = want.isfinite()
+        # (past e^88.72 the float32 sum has no end and the quotient is zero: below 2^-119 anything counts as zero)
+        bound = want[ok].abs() * (2.0**-8 + 2.0**-23 * t[ok].abs().clamp(max=90) + 2.0**-21) + 2.0**-119
+        assert ((row[ok] - want[ok]).abs() <= bound).all()
+    linear.check_status(device)
