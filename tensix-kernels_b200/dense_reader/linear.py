@@ -248,13 +248,14 @@ def _describe(x, m, entries, epi, act, scale, scale_up, scale_dt, residual, res_
     """The TkdMatmul of one row slice, without the activation, output and residual addresses."""
     a = _tkd.TkdMatmul()
     w0 = entries[0][0]
-    # (the library is told one format and no stream's size)
-    assert all(t is None or t.fmt == w0.fmt for g, u, _ in entries for t in (g, u)), "dense_reader: streams of several formats"
-    a.fmt, a.m, a.k = w0.fmt, m, w0.k
+    fmt = a.fmt = w0.fmt
+    a.m, a.k = m, w0.k
     a.ldx = x.shape[-1]
     a.nblocks, a.epilogue, a.act = len(entries), epi, act
     for i, (g, u, c0) in enumerate(entries):
         b = a.block[i]
+        # (the library is told one format and no stream's size)
+        assert g.fmt == fmt and (u is None or u.fmt == fmt), "dense_reader: streams of several formats in one launch"
         b.w, b.emax = g.t.data_ptr(), (g.emax.data_ptr() if g.emax is not None else None)
         if u is not None:
             b.w_up, b.emax_up = u.t.data_ptr(), (u.emax.data_ptr() if u.emax is not None else None)
@@ -468,7 +469,7 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     assert fidelity in FIDELITY, fidelity
     # the caller's weights (what is launched may be a twin of one: see _one_stream_format)
     own = [w, w_up]
-    if is_block_list(w):
+    if not isinstance(w, ttnn.Weight) and is_block_list(w):
         own = [u for wt, _ in w for u in (wt if isinstance(wt, (list, tuple)) else (wt,))]
     segs = ()
     if isinstance(w, (list, tuple)):
@@ -558,7 +559,8 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
         need = max(need, n)
     scales = col_scales if isinstance(col_scales, (tuple, list)) else (col_scales,)
     others = [t for g, u, _ in blocks_all for t in (g, u)][1:]
-    keep = [t for t in (scale, col_scales, *scales, hadamard, topk and topk["r"], *others, *own) if t is not own[0]]
+    held = {id(t): t for t in (scale, col_scales, *scales, hadamard, topk and topk["r"], *others, *own[1:])}
+    keep = [t for t in held.values() if t is not None and t is not own[0]]
     call = _Call(device, launches, need, keep, y.dtype, exchange)
     call.run(x, y, residual)
     return y, call
