@@ -76,7 +76,7 @@ MAX_CTAS = None
 
 _TENSIX_OPTS = {"cores_per_bank", "split", "rows", "xs", "kb", "kw", "sbw", "noscale", "glu2", "budget", "mt"}
 _OPTS = _TENSIX_OPTS | {"glu", "glu_act", "residual", "residual_mode", "out32", "blocks", "max_banks", "col_scales", "ks",
-                        "max_ctas", "exchange", "hadamard"}
+                        "max_ctas", "exchange", "hadamard", "fixed_sums"}
 
 _CALLS = {}      # matmul_host's calls by the identity of their arguments (a hit goes straight to the library)
 _CALLS_MAX = 256
@@ -179,11 +179,11 @@ ROWS_MAX = 2048  # rows of one launch for more than 32 (its copy of x grows with
 MAX_TILES, MAX_UNITS = 48 * 1024, 16 * 1024
 
 
-def _launch_rows(M, panels, fmt, topk, exchange, hadamard):
+def _launch_rows(M, panels, fmt, topk, exchange, hadamard, fixed_sums=False):
     """[(first row, rows)] of the launches a call of M rows over so many panels of columns makes: slices of up to 32, or more where
     tkd_matmul_rows serves."""
     most = min(ROWS_MAX, 256 * (MAX_TILES // panels))
-    wide = M > 32 and most and fmt != _tkd.FMT_INT4 and topk is None and exchange is None and hadamard is None
+    wide = M > 32 and most and fmt != _tkd.FMT_INT4 and topk is None and exchange is None and hadamard is None and not fixed_sums
     parts = -(-M // (most if wide else 32))
     if not wide:
         return [(m0, min(32, M - m0)) for m0 in range(0, M, 32)]
@@ -430,12 +430,15 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
     buffer, are also written to every other rank's buffer, and the call completes when all ranks' have arrived.
     col_scales=(gate scales, up scales) float32 [N] each with w_up (or one float32 vector in the
     interleaved weight's column order with glu); a float32 residual with out32 (y = x @ w + residual in float32);
+    fixed_sums=True: more than 32 rows run as slices of 32 as well, whose sums depend on K, the format and ks alone; those of one
+    launch depend on where its tiles are cut, which goes by N, the rows and the number of CTAs (a weight's columns, or a part of
+    them on each GPU, may then differ in a rounding).
     hadamard= (the sign words of ternary_matmul.t2.hadamard_signs; int4-stream weights only): x is rotated by the block
     Hadamard inside the kernel first.
 
     A block list in place of w, [(w | (gate, up), col0_tiles), ...]: one launch over two to four weights of one K and
     dtype, each written at its col0_tiles (in 32-column tiles); bit for bit one call per block. More than 32 rows run
-    as one launch (tkd_matmul_rows), or as slices of 32 with a top-k, an exchange or an int4 stream."""
+    as one launch (tkd_matmul_rows), or as slices of 32 with fixed_sums, a top-k, an exchange or an int4 stream."""
     call_key = None
     if CACHE:
         # A call described before on this weight, whatever its tensors' addresses: everything was checked then.
@@ -552,7 +555,7 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
         _block_kw_check(device, x, blocks_all, full_sync, opts, slices)
     launches, need = [], 0
     panels = -(-w.shape[-1] // 128) * (1 if w_up is None else 2)
-    for m0, m in _launch_rows(M, panels, w.fmt, topk, exchange, hadamard):
+    for m0, m in _launch_rows(M, panels, w.fmt, topk, exchange, hadamard, bool(opts.get("fixed_sums"))):
         a, n = _describe_rows(x, blocks_all, scale, col_scales, y, m, topk, act, residual, glu, out32,
                               opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, hadamard)
         launches.append((m0, a))

@@ -4,7 +4,8 @@ The reference runs on one device; on a box of GPUs large weights (the LM head, t
 split by output columns, each rank packs and streams only its own columns (linear.native_weight on its rows of the
 [out, in] matrix, linear.matmul on the replicated activations), and the small results are joined by one all-gather:
 the [M, N_local] outputs, or the top-k records followed by a merge every rank does for itself. There is no sharding of
-K, so no reduction and no dependence of any value on the number of GPUs.
+K, so no reduction, and no dependence of any value on the number of GPUs: with up to 32 rows, through an Exchange, or with
+linear.matmul's fixed_sums (more rows in one launch are summed where its tiles are cut, which goes by the columns it has).
 
 Two ways to join: torch.distributed's collectives (gather_outputs, gather_records: NCCL on GPUs, gloo in the CPU
 tests of the host logic), or Exchange: the stream kernel itself stores every output element and record into the other

@@ -245,3 +245,14 @@ def test_records_together_refuses_what_matmul_refuses(monkeypatch):
     monkeypatch.setattr(linear.dev, "MAX_BANKS", 4)
     with pytest.raises(ValueError):
         linear.records_together(tensor(1, 1, 1, 64), weights, topk, out)
+
+
+@pytest.mark.parametrize("m", [33, 64, 300])
+def test_fixed_sums_are_slices_of_32_rows(ran, m):
+    w, x = weight(256, 128), tensor(1, 1, m, 256)
+    linear.matmul(x, w, None)
+    assert [a.m for _, a in ran[-1].launches] == [m]
+    linear.matmul(x, w, None, fixed_sums=True)
+    assert [(at, a.m) for at, a in ran[-1].launches] == [(at, min(32, m - at)) for at in range(0, m, 32)]
+    linear.matmul(x, w, None, fixed_sums=False)
+    assert [a.m for _, a in ran[-1].launches] == [m]

@@ -735,3 +735,21 @@ def test_activations_over_their_range(device, m, act):
         bound = want[ok].abs() * (2.0**-8 + 2.0**-23 * t[ok].abs().clamp(max=90) + 2.0**-21) + 2.0**-119
         assert ((row[ok] - want[ok]).abs() <= bound).all()
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
+@pytest.mark.parametrize("m", [7, 32, 40, 100])
+def test_column_shards_give_the_whole_weights_bits(device, fmt, m):
+    """A weight's columns in parts, as the GPUs of a box hold them, give what the whole weight gives bit for bit: up to 32 rows, and
+    with fixed_sums for more."""
+    g = torch.Generator().manual_seed(97 + m)
+    k, n = 4096, 2560
+    w = torch.randn(n, k, generator=g) * 0.02
+    x = dev_x(device, torch.randn(m, k, generator=g))
+    opts = {"fixed_sums": True} if m > 32 else {}
+    whole = host(linear.matmul(x, linear.native_weight(device, w, DT[fmt])[0], None, **opts))
+    for parts in (2, 5):
+        cols = n // parts
+        got = [host(linear.matmul(x, linear.native_weight(device, w[i * cols : (i + 1) * cols], DT[fmt])[0], None, **opts)) for i in range(parts)]
+        assert torch.equal(torch.cat(got, dim=1), whole), parts
+    linear.check_status(device)
