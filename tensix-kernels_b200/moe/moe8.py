@@ -473,8 +473,9 @@ def _op(P, what, x, ids, w, rows, k, ids32, by_union, act=None):
 
 def _workspace(P, what, op):
     """The op's workspace, kept with the layer, one a kind of op: zeroed once (the kernels return their counters to zero; calls
-    on one layer run in stream order). One outgrown stays alive for the CUDA graphs that hold its address."""
-    held = P["_ws"].setdefault(what, [])
+    on one layer that may overlap, on several streams, each have linear.WORKSPACE_SLOT of their own). One outgrown stays alive for
+    the CUDA graphs that hold its address."""
+    held = P["_ws"].setdefault((what, linear.WORKSPACE_SLOT), [])
     if not held or held[-1].numel() < op.need:
         held.append(linear.new_workspace(P["_device"], op.need))
     return held[-1]

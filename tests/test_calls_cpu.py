@@ -256,3 +256,18 @@ def test_fixed_sums_are_slices_of_32_rows(ran, m):
     assert [(at, a.m) for at, a in ran[-1].launches] == [(at, min(32, m - at)) for at in range(0, m, 32)]
     linear.matmul(x, w, None, fixed_sums=False)
     assert [a.m for _, a in ran[-1].launches] == [m]
+
+
+def test_a_moe_layers_workspaces_go_by_slot(monkeypatch):
+    """Calls on one layer that may overlap pick their workspaces as linear's do: gate_up_rows counts in one too."""
+    from moe import moe8
+
+    monkeypatch.setattr(linear, "_COUNTED", [])
+    layer, op = {"_ws": {}, "_device": DEVICE}, type("Op", (), {"need": 4096})
+    own = {}
+    for slot in (0, 1, 0, 1):
+        monkeypatch.setattr(linear, "WORKSPACE_SLOT", slot)
+        for what in ("gu rows", "dn rows", "dn"):
+            ws = moe8._workspace(layer, what, op)
+            assert own.setdefault((slot, what), ws) is ws
+    assert len({ws.data_ptr() for ws in own.values()}) == 6
