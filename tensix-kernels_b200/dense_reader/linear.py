@@ -449,9 +449,7 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
             return out if out is not None else ttnn.Tensor(y, call.out_dtype, ttnn.TILE_LAYOUT, call.device, memory_config)
     y, call = _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0, w_up, max_banks, opts)
     if call_key is not None:
-        if len(first.calls) >= _WEIGHT_CALLS:
-            first.calls.clear()
-        first.calls[call_key] = call
+        _keep(first, call_key, call)
     return y
 
 
@@ -606,9 +604,17 @@ def records_together(x, weights, topk, out):
     for a in launches:
         call.launch(a[2], x.t, out.t, None, _workspace(call.device, need), 0)
     if CACHE:
-        if len(first.calls) >= _WEIGHT_CALLS:
-            first.calls.clear()
-        first.calls[key] = call
+        _keep(first, key, call)
+
+
+def _keep(first, key, call):
+    """Keep a call with its weight. One goes for it where there are too many: the oldest of more than 32 rows (a server's prompts of
+    many lengths leave the decode calls), else the oldest."""
+    calls = first.calls
+    if len(calls) >= _WEIGHT_CALLS:
+        old = list(calls.items())
+        calls.pop(next((k for k, c in old if c.launches[0][1].m > 32), old[0][0]), None)
+    calls[key] = call
 
 
 _PLAIN = {int, bool, str, type(None)}

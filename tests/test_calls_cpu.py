@@ -271,3 +271,21 @@ def test_a_moe_layers_workspaces_go_by_slot(monkeypatch):
             ws = moe8._workspace(layer, what, op)
             assert own.setdefault((slot, what), ws) is ws
     assert len({ws.data_ptr() for ws in own.values()}) == 6
+
+
+def test_prompts_of_many_lengths_leave_the_decode_calls(ran):
+    """A weight keeps so many calls; a new one takes the oldest prompt's place, and the oldest's where there is none."""
+    w = weight(64, 128)
+    xs = [tensor(1, 1, m, 64) for m in (1, 8, *range(33, 133))]
+    for x in xs:
+        linear.matmul(x, w, None)
+    assert len(w.calls) == linear._WEIGHT_CALLS
+    decode = ran[:2]
+    for x in xs[:2]:
+        linear.matmul(x, w, None)
+    assert ran[-2:] == decode and ran[-3].launches[0][1].m == 132
+    linear.matmul(xs[-linear._WEIGHT_CALLS + 2], w, None)
+    assert ran[-1] in ran[:-1]
+    for col0 in range(2 * linear._WEIGHT_CALLS):
+        linear.matmul(xs[0], w, None, out=tensor(1, 1, 1, 32 * (col0 + 4)), col0=col0)
+    assert len(w.calls) == linear._WEIGHT_CALLS and all(c.launches[0][1].m == 1 for c in w.calls.values())
