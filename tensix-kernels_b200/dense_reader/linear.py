@@ -722,6 +722,18 @@ class _Call:
         return a
 
 
+def _ids(v):
+    """What names an argument in a key: numbers by value, a list or tuple by its elements, other objects by identity."""
+    return v if type(v) is int else tuple(map(_ids, v)) if type(v) is list or type(v) is tuple else id(v)
+
+
+def _frozen(v):
+    """An argument as it is now, its lists and dicts copied."""
+    if type(v) is dict:
+        return {k: _frozen(e) for k, e in v.items()}
+    return tuple(map(_frozen, v)) if type(v) is list or type(v) is tuple else v
+
+
 def matmul_host(x_host, out_host, x, w, scale, *, topk=None, out=None, col0=0, w_up=None, max_banks=None, stream=None,
                 **opts):
     """matmul for a caller whose activations and result live in host memory: x_host (pinned torch bf16 [M, K]) is
@@ -730,8 +742,9 @@ def matmul_host(x_host, out_host, x, w, scale, *, topk=None, out=None, col0=0, w
     (tkd_matmul_host) instead of three framework calls. The other arguments are matmul's; up to 32 rows. The first call with a given set of tensors goes
     through matmul itself (which checks everything and also launches once)."""
     assert out is not None and CACHE, "dense_reader.matmul_host: needs out= and the launch cache"
-    key = (ttnn.EPOCH, id(x), id(w), id(scale), id(out), id(w_up), id(topk), col0, max_banks, KS, MAX_CTAS, TOPK_UNIT, WORKSPACE_SLOT,
-           tuple((k, tuple(map(id, v)) if type(v) is tuple else id(v)) for k, v in opts.items()))
+    key = (ttnn.EPOCH, id(x), id(w) if type(w) is ttnn.Weight else _ids(w), id(scale), id(out), id(w_up),
+           None if topk is None else tuple([(k, _ids(v)) for k, v in topk.items()]), col0, max_banks, KS, MAX_CTAS, TOPK_UNIT,
+           WORKSPACE_SLOT, tuple([(k, _ids(v) if type(v) is tuple or type(v) is list else id(v)) for k, v in opts.items()]))
     ws = _WORKSPACE.get(_ws_key(x.device()))
     hit = _CALLS.get(key)
     if hit is None or hit["ws"] is not ws:
@@ -745,9 +758,9 @@ def matmul_host(x_host, out_host, x, w, scale, *, topk=None, out=None, col0=0, w
         res = opts.get("residual")
         hit = _CALLS[key] = {
             "a": call.bound(x.t, out.t, None if res is None else res.t), "ws": _WORKSPACE.get(_ws_key(x.device())), "call": call,
-            # (the arguments stay alive, so their ids stay theirs; ttnn.deallocate starts a new epoch, which retires
-            # every entry made before it)
-            "keep": (x, w, scale, out, w_up, topk, dict(opts)),
+            # (the arguments stay alive, so their ids stay theirs, also what a list or dict held that the caller changes
+            # later; ttnn.deallocate starts a new epoch, which retires every entry made before it)
+            "keep": (x, _frozen(w), scale, out, w_up, _frozen(topk), _frozen(opts)),
         }
     sp = torch.cuda.current_stream().cuda_stream if stream is None else stream.cuda_stream
     rc = _tkd.lib().tkd_matmul_host(ctypes.byref(hit["a"]), x_host.data_ptr(), out_host.data_ptr(), sp)

@@ -1,6 +1,7 @@
 """What linear.matmul describes and keeps, without a GPU: the descriptors' formats and addresses, and which calls a kept one
 serves. Tensors are host ones and no launch is made."""
 
+import contextlib
 import ctypes
 
 import numpy as np
@@ -289,3 +290,39 @@ def test_prompts_of_many_lengths_leave_the_decode_calls(ran):
     for col0 in range(2 * linear._WEIGHT_CALLS):
         linear.matmul(xs[0], w, None, out=tensor(1, 1, 1, 32 * (col0 + 4)), col0=col0)
     assert len(w.calls) == linear._WEIGHT_CALLS and all(c.launches[0][1].m == 1 for c in w.calls.values())
+
+
+def test_matmul_host_sees_a_list_and_a_dict_change(ran, monkeypatch):
+    """matmul_host's calls go by what a block list and a top-k's dict hold, not by the list and the dict."""
+    made = []
+    lib = _tkd.lib()
+    stream = type("Stream", (), {"cuda_stream": 0})
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def tkd_matmul_host(self, a, x, out, sp):
+            made.append(_tkd.TkdMatmul.from_buffer_copy(a._obj))
+            return 0
+
+    monkeypatch.setattr(_tkd, "lib", lambda: Lib())
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(linear, "_CALLS", {})
+    monkeypatch.setattr(linear, "_WORKSPACE", {})
+    x, out, host = tensor(1, 1, 1, 64), tensor(1, 1, 1, 256), torch.zeros(1, 64, dtype=torch.bfloat16)
+    ws = [weight(64, 128) for _ in range(3)]
+    entries = [(ws[0], 0), (ws[1], 4)]
+    topk = {"r": tensor(1, 1, 4, 2, dtype=ttnn.uint32), "k": 1, "rows": 1, "slot0": 0, "base": 0, "n": 128}
+
+    def call(w, **kw):
+        linear.matmul_host(host, host, x, w, None, out=out, stream=stream, **kw)
+        return made[-1]
+
+    assert call(entries).block[1].w == ws[1].t.data_ptr()
+    entries[1] = (ws[2], 4)
+    assert call(entries).block[1].w == ws[2].t.data_ptr()
+    assert call(ws[0], topk=topk).topk_slot0 == 0
+    topk["slot0"] = 3
+    assert call(ws[0], topk=topk).topk_slot0 == 3
+    assert len(linear._CALLS) == 4 and call(entries).block[1].w == ws[2].t.data_ptr() and len(linear._CALLS) == 4
