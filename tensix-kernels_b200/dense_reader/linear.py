@@ -326,7 +326,9 @@ _PLAN_ARGS = set(plan.__code__.co_varnames[: plan.__code__.co_argcount])
 
 
 def choose(device, x, w, full_sync=False, **forced):
-    """[(first row, plan)] for x's rows, cached by shapes and settings. (linear.py:455-495)"""
+    """[(first row, plan)] for x's rows in slices of up to 32, cached by shapes and settings: the launches of a call of up to 32 rows
+    or with fixed_sums (linear.matmul says which others run as slices; the rest go as one launch, planned inside the library).
+    (linear.py:455-495)"""
     blocks = forced.get("blocks")
     shapes = tuple((b.k, b.n, b.dtype, b.fmt) for b in (blocks or (w,)))
     key = (shapes, tuple(x.shape), tuple(sorted((k, v) for k, v in forced.items() if k != "blocks")), KS, MAX_CTAS)
@@ -548,12 +550,19 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     if topk is not None:
         assert M <= 32, "dense_reader: top-k needs one row slice"
         assert 1 <= topk["rows"] <= 16 and topk["rows"] * topk["k"] <= 64 and topk["rows"] <= M, topk
-    slices = choose(device, x, w, full_sync, **opts)
-    if segs:
-        _block_kw_check(device, x, blocks_all, full_sync, opts, slices)
-    launches, need = [], 0
     panels = -(-w.shape[-1] // 128) * (1 if w_up is None else 2)
-    for m0, m in _launch_rows(M, panels, w.fmt, topk, exchange, hadamard, bool(opts.get("fixed_sums"))):
+    parts = _launch_rows(M, panels, w.fmt, topk, exchange, hadamard, bool(opts.get("fixed_sums")))
+    if parts[0][1] > 32:
+        # (tkd_matmul_rows has a plan of its own; the options are checked as plan checks them)
+        plan(device, x, w, full_sync=full_sync, m=32, **{k: v for k, v in opts.items() if k in _PLAN_ARGS})
+        if LOG:
+            print(f"dense_reader: K {w.shape[-2]} N {w.shape[-1]} rows {M}: {len(parts)} launch(es) of up to {parts[0][1]} rows", flush=True)
+    else:
+        slices = choose(device, x, w, full_sync, **opts)
+        if segs:
+            _block_kw_check(device, x, blocks_all, full_sync, opts, slices)
+    launches, need = [], 0
+    for m0, m in parts:
         a, n = _describe_rows(x, blocks_all, scale, col_scales, y, m, topk, act, residual, glu, out32,
                               opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, hadamard)
         launches.append((m0, a))

@@ -326,3 +326,16 @@ def test_matmul_host_sees_a_list_and_a_dict_change(ran, monkeypatch):
     topk["slot0"] = 3
     assert call(ws[0], topk=topk).topk_slot0 == 3
     assert len(linear._CALLS) == 4 and call(entries).block[1].w == ws[2].t.data_ptr() and len(linear._CALLS) == 4
+
+
+def test_the_log_and_the_plans_are_of_what_runs(ran, monkeypatch, capsys):
+    """A call of more than 32 rows in one launch makes no plans of slices and logs none; its options are checked all the same."""
+    w, x = weight(256, 128), tensor(1, 1, 512, 256)
+    monkeypatch.setattr(linear, "LOG", True)
+    monkeypatch.setattr(linear, "_CHOICE", {})
+    linear.matmul(x, w, None)
+    assert not linear._CHOICE and "rows 512: 1 launch(es)" in capsys.readouterr().out
+    with pytest.raises(ValueError):
+        linear.matmul(x, w, None, kb=3)
+    linear.matmul(x, w, None, fixed_sums=True)
+    assert len(linear._CHOICE) == 1 and "ctas" in capsys.readouterr().out
