@@ -7,6 +7,7 @@ Both sit beside their sources (csrc/); the Python layer loads them and refuses t
 cross-compiles: no GPU is needed to build.
 """
 
+import shutil
 import subprocess
 import sys
 import sysconfig
@@ -32,18 +33,39 @@ def stale():
     return _older(LIB, [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *CSRC.glob("*.h"), header])
 
 
+def host_for():
+    """What tkd_host.so is compiled against besides libtkd: another torch or Python needs another module."""
+    import torch
+
+    return f"torch {torch.__version__}, Python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
+def host_stale():
+    return (_older(HOST, [CSRC / "tkd_host.cpp", CSRC.parents[1] / "include" / "tkd.h", LIB])
+            or host_for().encode() not in HOST.read_bytes())
+
+
 def build_host(verbose=False, force=False):
     """tkd_host.so, the extension module over libtkd.so (which it finds beside itself) and torch's C++ libraries."""
-    if not force and not _older(HOST, [CSRC / "tkd_host.cpp", CSRC.parents[1] / "include" / "tkd.h", LIB]):
+    if not force and not host_stale():
         return HOST
     import torch
 
     at = Path(torch.__file__).parent
-    inc = [sysconfig.get_paths()["include"], at / "include", at / "include/torch/csrc/api/include", "/usr/local/cuda/include"]
+    inc = [sysconfig.get_paths()["include"], at / "include", at / "include/torch/csrc/api/include", _cuda_include()]
     _run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          f'-DTKD_HOST_FOR="{host_for()}"',
           *(f"-I{i}" for i in inc), "-o", str(HOST), str(CSRC / "tkd_host.cpp"), f"-L{at / 'lib'}", "-lc10", "-lc10_cuda",
           "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", f"-L{CSRC}", "-l:libtkd.so", "-Wl,-rpath,$ORIGIN"], verbose)
     return HOST
+
+
+def _cuda_include():
+    """The headers of the toolkit whose nvcc compiles the library."""
+    nvcc = shutil.which("nvcc")
+    if nvcc is None:
+        raise RuntimeError("the build needs nvcc on the PATH")
+    return Path(nvcc).resolve().parents[1] / "include"
 
 
 def _run(cmd, verbose):

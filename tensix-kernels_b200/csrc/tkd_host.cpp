@@ -250,4 +250,8 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "tkd_host", nullptr, -1, method
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_tkd_host() { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit_tkd_host() {
+    PyObject* m = PyModule_Create(&module_def);
+    if (m && PyModule_AddStringConstant(m, "built_for", TKD_HOST_FOR) < 0) Py_CLEAR(m);  // (what build.py compiled it against)
+    return m;
+}

@@ -6,6 +6,7 @@ non-zero code raises.
 
 import ctypes
 import importlib.util
+import sys
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parents[1]
@@ -131,9 +132,15 @@ def host():
         lib()  # (checks the library the module links to)
         if not HOST_PATH.exists():
             raise RuntimeError(f"dense_reader: {HOST_PATH} is missing; build it with `python {PKG / 'build.py'}`")
+        import torch  # (the module links to torch's libraries)
+
         spec = importlib.util.spec_from_file_location("tkd_host", HOST_PATH)
-        _host = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(_host)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        here = f"torch {torch.__version__}, Python {sys.version_info[0]}.{sys.version_info[1]}"
+        if mod.built_for != here:
+            raise RuntimeError(f"dense_reader: {HOST_PATH} was built for {mod.built_for}, this is {here}: rebuild")
+        _host = mod
     return _host
 
 

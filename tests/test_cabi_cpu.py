@@ -109,3 +109,20 @@ def test_no_cpu_fallback(tkd):
         pytest.skip("a GPU is present")
     with pytest.raises(RuntimeError):
         ttnn.open_device(0)
+
+
+def test_the_host_module_is_of_this_torch(tkd, monkeypatch):
+    """tkd_host.so is compiled against torch's C++ headers: another torch finds it stale, and is refused if it loads it."""
+    import importlib.util
+
+    import torch
+
+    spec = importlib.util.spec_from_file_location("tkd_build", ROOT / "tensix-kernels_b200" / "build.py")
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    assert not build.host_stale() and tkd.host().built_for == build.host_for()
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    assert build.host_stale()
+    monkeypatch.setattr(tkd, "_host", None)
+    with pytest.raises(RuntimeError, match="rebuild"):
+        tkd.host()
