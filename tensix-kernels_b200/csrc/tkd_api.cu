@@ -396,7 +396,7 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
     const int64_t panels = a->epilogue == TKD_EPI_GLU2 ? npad / 64 : npad / TKD_PANEL_COLS;
     const int chunk_k = tkd_chunk_k(a->fmt);
     p.chunks = (p.K + chunk_k - 1) / chunk_k;
-    if (a->ks % chunk_k) return TKD_ERR_BAD_ARG;
+    if (a->ks < 0 || a->ks % chunk_k) return TKD_ERR_BAD_ARG;
     if (sms <= 0) sms = sm_count();
     if (sms <= 0) sms = 148;
     if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;

@@ -126,3 +126,21 @@ def test_the_host_module_is_of_this_torch(tkd, monkeypatch):
     monkeypatch.setattr(tkd, "_host", None)
     with pytest.raises(RuntimeError, match="rebuild"):
         tkd.host()
+
+
+def test_rows_requests_that_are_refused(tkd):
+    """tkd_matmul_rows' plan refuses what it cannot lay out, before any size is made of it."""
+    def need(**kw):
+        a, bytes_ = tkd.TkdMatmul(), ctypes.c_uint64(0)
+        a.fmt, a.m, a.k, a.nblocks, a.epilogue, a.out_dtype = tkd.FMT_BFP8, 64, 4096, 1, tkd.EPI_PLAIN, tkd.DT_BF16
+        a.block[0].n = 512
+        for k, v in kw.items():
+            setattr(a, k, v)
+        return tkd.lib().tkd_matmul_rows_workspace(ctypes.byref(a), ctypes.byref(bytes_)), bytes_.value
+
+    rc, size = need()
+    assert rc == 0 and size > 0
+    assert need(ks=1024)[0] == 0
+    for bad in ({"ks": -1024}, {"ks": 100}, {"m": 32}, {"m": 4097}, {"k": 4016}, {"out_dtype": tkd.DT_F32}, {"topk_k": 1}):
+        assert need(**bad)[0] == 1, bad
+    assert need(fmt=tkd.FMT_INT4)[0] == 2 and need(nranks=2)[0] == 2
