@@ -165,7 +165,11 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
         // Items of 32 columns over all of K (tkd_narrow.cuh) where the call is a plain one and K makes four slices of nearly
         // the same length: a streaming warp stays with one slice, and where the last is short, its warps wait for the others'.
         // (Three stages are enough there: 100 KB of loads in flight on an SM, of the 60 that its share of the memory's rate
-        // needs, and eight rows of K 5632 in bf16 would not fit beside four.)
+        // needs.) Measured, launches in a graph over weights larger than L2, us with this kernel / the other: bfloat4_b
+        // [3648, 4096] one row 4.4 / 6.2, eight 5.3 / 9.7; bf16 [5632, 2048] eight rows, three stages, 8.1 / 10.5. Both limits
+        // lie on the safe side: beyond them, at a last slice of a third to a half (bfloat4_b [5120, 4096] 5.2 / 7.0, bfloat8_b
+        // [3584, 18944] 14.5 / 14.7, its eight rows 15.1 / 14.9) and two stages (bfloat8_b [7168, 4096], eight rows, 10.2 / 12.5),
+        // it is still the faster one nearly everywhere; they have not been moved.
         const int64_t narrow_xt = p.off_pbuf + 2 * 8 * 32 * (a->m > 1 ? 8 : 1) * 4;
         if (!counted && p.nslices == 4 && 4 * p.ks - p.K < p.ks / 2 && !a->topk_k && a->nranks <= 1 &&
             narrow_xt + a->m * x_row + 3 * (int64_t)p.stage_bytes + 128 <= kMaxSmem) {
@@ -400,8 +404,9 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
     if (sms <= 0) sms = sm_count();
     if (sms <= 0) sms = 148;
     if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
-    // The rows of a tile and the blocks it is cut into, by what the kernel measured (B200, us; K 4096, bfloat8_b): a unit of 128
-    // k takes 0.55 + nt / 600 (the decode, then the traffic of x from L2); a tile's output nt / 29; a cut tile's partial sums
+    // The rows of a tile and the blocks it is cut into, by what the kernel measured (B200, us; K 4096, bfloat8_b; the other
+    // formats, whose decode is other work, go by the same figures, which were not fitted to them): a unit of 128 k takes
+    // 0.55 + nt / 600 (the decode, then the traffic of x from L2); a tile's output nt / 29; a cut tile's partial sums
     // 2 + nt / 60 to store, and nt / 26 for each part that its last CTA adds up.
     double best = 0;
     for (int nrt = (p.M + 255) / 256, nrt1 = (p.M + 31) / 32; nrt <= nrt1; ++nrt) {

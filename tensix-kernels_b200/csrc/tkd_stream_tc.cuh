@@ -4,8 +4,8 @@
 // dense_compute.cpp:95-143, matmul_block): more rows cost it no more weight traffic and hardly more time. With
 // mma.sync the same holds for the traffic but not for the time: 32 rows of accumulators leave room for two streaming
 // warps per scheduler, which wait on their own shared-memory loads and mma chains. Here the weights of a panel are
-// decoded into bf16 tiles in shared memory once, whatever the row count, and one thread issues tcgen05.mma on them with
-// the accumulators in tensor memory:
+// decoded into bf16 tiles in tensor memory once, whatever the row count, and tcgen05.mma multiplies them with the
+// accumulators in tensor memory too:
 //
 //   warps 3-18     decode warps, in two groups of eight; a unit of two tiles of 64 k is one group's work (units in turn:
 //                  while one group waits for its stores to land, the other decodes). A warp turns its 16 columns' share
@@ -31,9 +31,10 @@
 // A slice's sum is accumulated from zero in tensor memory, in two accumulators of 32 columns (the slice's even units
 // in d0, its odd units in d1; the slice's sum is d0 + d1). Two such sets, so that the MMAs of the next slice run while
 // the output warps drain this one. A column's sum is the ascending sum of its slices' sums in plain fp32 adds, as in
-// tkd_stream_kernel, so it depends on K, the format and ks only. No cluster, no multicast, no
-// second CTA: cta_group::1 throughout. Every wait is bounded; the kernel always reaches its end, where the warp that
-// allocated the tensor memory frees it.
+// tkd_stream_kernel, so it depends on K, the format and ks only. cta_group::1 throughout, no
+// multicast; plain calls of four slices may run as clusters of four CTAs, a slice each, whose sums meet in shared memory
+// (CL, below). Every wait is bounded (the output warps, who meet at barriers, go on after one that gave up: mbar_wait); the
+// kernel always reaches its end, where the warp that allocated the tensor memory frees it.
 #pragma once
 #include "tkd_stream_kernel.cuh"
 

@@ -289,7 +289,8 @@ def plan(device, x, w, cores_per_bank=3, full_sync=False, kb=None, kw=None, sbw=
     where they mean something here (MT, KT, NT, KW, SEGS, glu, glu2, out32, noscale, work, l1) and the kernel's own
     (KS: k per slice, SLICES, PANELS of 128 columns, ITEMS = PANELS x SLICES, GRID: CTAs, STAGES of the shared-memory
     ring, BYTES: the weight stream read). work: [(cta, (first item, items))], the contiguous run of items each CTA
-    takes. (linear.py:187-382; the Tensix options are accepted and ignored)"""
+    takes (of the kernels that count panels in; plain calls of four slices may deal the same bytes out as 32 columns over
+    all of K, or to clusters of four CTAs). (linear.py:187-382; the Tensix options are accepted and ignored)"""
     blocks = tuple(blocks) if blocks else (w,)
     if len(blocks) > 1:
         assert 2 <= len(blocks) <= 4, f"dense_reader: {len(blocks)} blocks (at most 4)"

@@ -12,8 +12,8 @@ stream kernel (TKD_FMT_INT4, include/tkd.h; int4/w4a16.py): the packed stream ho
 scale of their group (a group of G = 32 * j inputs repeats its scale j times, which changes no sum). The reference's
 three storage forms ("bfp2", "bfp2c", "bfp4": tiles() makes each, ternary_weight keeps it as the weight's visible
 tensor) therefore run the same stream and give the same bits; the stream is 4.5 bits a weight like the reference's
-"bfp4" form. The kernel is bound by instruction issue per weight, not by bytes (profiles/), so a 2-bit stream would
-save HBM space, not time. Many rows run the ordinary stream kernels on the weight's values q * s held as bf16 (exact:
+"bfp4" form. The kernel is bound by instruction issue per weight before bytes, so a 2-bit stream would save HBM
+space first. Many rows run the ordinary stream kernels on the weight's values q * s held as bf16 (exact:
 a trit times a bf16 scale), as the reference's multi-row kernel dequantizes each tile by its scale row. The Hadamard
 is one small kernel (tkd_hadamard: a fast Walsh-Hadamard transform in fp32) for one row or many; with hadamard=
 t2_linear has the stream kernel do the same transform on its own copy of x (the same additions in the same order, so
