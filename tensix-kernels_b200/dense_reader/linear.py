@@ -22,6 +22,7 @@ What differs from the reference, by necessity or on purpose:
 
 import ctypes
 import itertools
+import operator
 import sys
 import weakref
 from pathlib import Path
@@ -463,18 +464,15 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     if unknown:
         raise TypeError(f"dense_reader.matmul: unknown options {sorted(unknown)}")
     opts = dict(opts)
+    own = [w, w_up]  # the caller's weights (what is launched may be a twin of one: see _one_stream_format)
     if not isinstance(w, (list, tuple)):
         check_banks(w, max_banks)
     elif is_block_list(w):
-        for wt, _ in w:
-            for u in wt if isinstance(wt, (list, tuple)) else (wt,):
-                check_banks(u, max_banks)
+        own = [u for wt, _ in w for u in (wt if isinstance(wt, (list, tuple)) else (wt,))]
+        for u in own:
+            check_banks(u, max_banks)
     check_banks(w_up, max_banks)
     assert fidelity in FIDELITY, fidelity
-    # the caller's weights (what is launched may be a twin of one: see _one_stream_format)
-    own = [w, w_up]
-    if not isinstance(w, ttnn.Weight) and is_block_list(w):
-        own = [u for wt, _ in w for u in (wt if isinstance(wt, (list, tuple)) else (wt,))]
     segs = ()
     if isinstance(w, (list, tuple)):
         assert is_block_list(w), "dense_reader: w is one weight or a block list [(w | (gate, up), col0_tiles), ...]"
@@ -554,8 +552,10 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     panels = -(-w.shape[-1] // 128) * (1 if w_up is None else 2)
     parts = _launch_rows(M, panels, w.fmt, topk, exchange, hadamard, bool(opts.get("fixed_sums")))
     if parts[0][1] > 32:
-        # (tkd_matmul_rows has a plan of its own; the options are checked as plan checks them)
-        plan(device, x, w, full_sync=full_sync, m=32, **{k: v for k, v in opts.items() if k in _PLAN_ARGS})
+        # (tkd_matmul_rows has a plan of its own; the options are checked as plan checks them, once for a kind of call)
+        key = ("rows", x.shape[-1], w.shape[-2], w.n, w.dtype, w.fmt, tuple(sorted(opts.items())), KS, MAX_CTAS)
+        if key not in _CHOICE:
+            _CHOICE[key] = plan(device, x, w, full_sync=full_sync, m=32, **{k: v for k, v in opts.items() if k in _PLAN_ARGS})
         if LOG:
             print(f"dense_reader: K {w.shape[-2]} N {w.shape[-1]} rows {M}: {len(parts)} launch(es) of up to {parts[0][1]} rows", flush=True)
     else:
@@ -569,9 +569,9 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
         launches.append((m0, a))
         need = max(need, n)
     scales = col_scales if isinstance(col_scales, (tuple, list)) else (col_scales,)
-    others = [t for g, u, _ in blocks_all for t in (g, u)][1:]
-    held = {id(t): t for t in (scale, col_scales, *scales, hadamard, topk and topk["r"], *others, *own[1:])}
-    keep = [t for t in held.values() if t is not None and t is not own[0]]
+    launched = [t for g, u, _ in blocks_all for t in (g, u) if t is not None]
+    twins = [] if all(map(operator.is_, launched, own)) else launched
+    keep = [t for t in (scale, col_scales, *scales, hadamard, topk and topk["r"], *own[1:], *twins) if t is not None and t is not own[0]]
     call = _Call(device, launches, need, keep, y.dtype, exchange)
     call.run(x, y, residual)
     return y, call
