@@ -1013,9 +1013,9 @@ def finish(world):
         os._exit(0)
 
 
-# DRAM bytes per launch of tkd_stream_kernel from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum), per
-# workload at M = 1 (the summaries under profiles/); None where no capture of the workload is summarised there.
-TRAFFIC = {"c2": 66_769_408, "c3": 62_681_600, "c5": 667_036_928, "w4": 66_386_432, "moe": 21_298_944}
+# DRAM bytes of one call from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum), per workload at M = 1
+# (profiles/); None where no capture of the workload is summarised there.
+TRAFFIC = {"c2": 66_372_352, "c3": 62_505_984, "c5": 668_029_696, "w4": 66_300_416, "moe": 21_290_496}
 
 if __name__ == "__main__":
     sys.exit(main())
