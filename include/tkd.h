@@ -38,6 +38,8 @@ extern "C" {
 #define TKD_EPI_GLU2 2      /* the same over two weights (w the gate's, w_up), N wide    :200-257, GLU2 */
 #define TKD_EPI_RESIDUAL 3  /* y = bf16(acc + bf16 residual)                             :100-120, 258-301 */
 #define TKD_EPI_OUT32 4     /* y = acc in float32 (+ a float32 residual, an extension)   :302-332 */
+#define TKD_EPI_SILU 5      /* y = bf16(silu(acc * scale)) (scale optional; one weight, no records, no exchange): linear's
+                               activation="silu", dense_reader/linear.py:1073-1124 */
 
 #define TKD_DT_NONE 0
 #define TKD_DT_BF16 1

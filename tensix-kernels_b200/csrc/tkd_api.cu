@@ -70,11 +70,12 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     // bfloat8_b form, as there: int4/w4a16.py dequantize)
     if (a->fmt == TKD_INT4 && a->m > 8) return TKD_ERR_UNSUPPORTED;
     if (a->nblocks < 1 || a->nblocks > 4) return TKD_ERR_BAD_ARG;
-    if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_OUT32) return TKD_ERR_BAD_ARG;
+    if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_SILU) return TKD_ERR_BAD_ARG;
     const bool glu = a->epilogue == TKD_EPI_GLU_IL || a->epilogue == TKD_EPI_GLU2;
     if (a->nblocks > 1 && !(a->epilogue == TKD_EPI_PLAIN || a->epilogue == TKD_EPI_GLU2)) return TKD_ERR_BAD_ARG;
     if (a->nblocks > 1 && (a->scale_dtype != TKD_DT_NONE || (a->topk_k && a->epilogue != TKD_EPI_PLAIN))) return TKD_ERR_BAD_ARG;
-    if (a->topk_k && (glu || a->epilogue == TKD_EPI_OUT32 || a->epilogue == TKD_EPI_RESIDUAL)) return TKD_ERR_BAD_ARG;
+    if (a->topk_k && (glu || a->epilogue >= TKD_EPI_RESIDUAL)) return TKD_ERR_BAD_ARG;
+    if (a->epilogue == TKD_EPI_SILU && a->nranks > 1) return TKD_ERR_BAD_ARG;
     if ((a->epilogue == TKD_EPI_OUT32) != (a->out_dtype == TKD_DT_F32)) return TKD_ERR_BAD_ARG;
     if (a->out_dtype != TKD_DT_F32 && a->out_dtype != TKD_DT_BF16) return TKD_ERR_BAD_ARG;
     if (a->nranks < 0 || a->nranks > TKD_MAX_RANKS || (a->nranks > 1 && (a->rank < 0 || a->rank >= a->nranks)))
@@ -387,7 +388,7 @@ static int check_pointers(const TkdMatmul* a) {
 // The launch of such a call, without the pointers into the workspace. sms 0: ask the device.
 static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_bytes, int sms) {
     if (!a || !fmt_ok(a->fmt) || a->m < 33 || a->m > TKD_ROWS_MAX || a->k < 32 || a->k % 32 || a->k > (1 << 24)) return TKD_ERR_BAD_ARG;
-    if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_OUT32 || a->nblocks != 1 || a->topk_k) return TKD_ERR_BAD_ARG;
+    if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_SILU || a->nblocks != 1 || a->topk_k) return TKD_ERR_BAD_ARG;
     if ((a->epilogue == TKD_EPI_OUT32) != (a->out_dtype == TKD_DT_F32)) return TKD_ERR_BAD_ARG;
     if (a->fmt == TKD_INT4 || a->hadamard || a->nranks > 1) return TKD_ERR_UNSUPPORTED;
     const TkdBlock& b = a->block[0];

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
     const int i0 = (int)((uint64_t)T * blockIdx.x / gridDim.x), i1 = (int)((uint64_t)T * (blockIdx.x + 1) / gridDim.x);
     const int nst = p.nstages, M = ONE ? 1 : p.M, K = p.K, cps = p.ks / CK, nch = (K + CK - 1) / CK;
     const int nsa_total = (K + F::KSA - 1) / F::KSA;
-    const bool glu = p.epi == TKD_EPI_GLU2 || p.epi == TKD_EPI_GLU_IL;
+    const bool glu = p.epi == TKD_EPI_GLU2 || p.epi == TKD_EPI_GLU_IL, silu = p.epi == TKD_EPI_SILU;
     auto seg_of = [&](int it) {
         int s = 0;
 #pragma unroll
@@ -253,11 +253,11 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
 #pragma unroll
                 for (int m = 0; m < MR; ++m) v[m] *= sc;
             }
-            if (glu) {
+            if (glu || silu) {  // (one copy of the activation's code for both: a GLU's other factor, or 1)
 #pragma unroll
                 for (int m = 0; m < MR; ++m) {
                     const float u = __shfl_xor_sync(0xFFFFFFFFu, v[m], 16);
-                    v[m] = act_gate(v[m], p.act) * u;
+                    v[m] = act_gate(v[m], p.act) * (glu ? u : 1.f);
                 }
             }
             if (p.res_dt != TKD_DT_NONE) {

@@ -234,6 +234,7 @@ int for_epilogue(int epi, F f) {
         case TKD_EPI_GLU_IL: return f(std::integral_constant<int, TKD_EPI_GLU2>{});
         case TKD_EPI_RESIDUAL: return f(std::integral_constant<int, TKD_EPI_RESIDUAL>{});
         case TKD_EPI_OUT32: return f(std::integral_constant<int, TKD_EPI_OUT32>{});
+        case TKD_EPI_SILU: return f(std::integral_constant<int, TKD_EPI_SILU>{});
         default: return f(std::integral_constant<int, TKD_EPI_PLAIN>{});
     }
 }
@@ -1105,6 +1106,10 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
                 if (p.scale_dt != TKD_DT_NONE && in_w) {
     #pragma unroll
                     for (int m = 0; m < R; ++m) tot[m] *= sc;
+                }
+                if (PLAIN && p.epi == TKD_EPI_SILU) {
+    #pragma unroll
+                    for (int m = 0; m < R; ++m) tot[m] = act_gate(tot[m], 0);
                 }
                 int ocol = -1;  // the output column this thread writes, if any
                 if (p.epi == TKD_EPI_GLU_IL || glu2) {

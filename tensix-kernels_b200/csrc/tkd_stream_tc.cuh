@@ -615,6 +615,10 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 if (left <= 0) continue;
 #pragma unroll
                 for (int m = 0; m < 8; ++m) v[m] = v[m] * f1 * f2 * sc;
+                if (epi == TKD_EPI_SILU) {
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) v[m] = act_gate(v[m], 0);
+                }
                 if (glu) {
 #pragma unroll
                     for (int m = 0; m < 8; ++m) {
@@ -865,6 +869,10 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                             }
 #pragma unroll
                             for (int m = 0; m < 16; ++m) v[m] = v[m] * colf * colg * cols;
+                            if (epi == TKD_EPI_SILU) {
+#pragma unroll
+                                for (int m = 0; m < 16; ++m) v[m] = act_gate(v[m], 0);
+                            }
                             if (glu) {
 #pragma unroll
                                 for (int m = 0; m < 16; m += 4) {

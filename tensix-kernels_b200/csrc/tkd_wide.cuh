@@ -288,6 +288,10 @@ __device__ __forceinline__ void wide_segment(const TkdWide& p, const WideSeg& sg
             }
 #pragma unroll
             for (int m = 0; m < 16; ++m) v[m] = v[m] * colf * colg;
+            if (EK == TKD_EPI_SILU) {
+#pragma unroll
+                for (int m = 0; m < 16; ++m) v[m] = act_gate(v[m], 0);
+            }
             if (glu) {
                 bar_worker();  // (the batch before has been read)
                 if (!gate)

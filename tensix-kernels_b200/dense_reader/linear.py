@@ -78,6 +78,8 @@ MAX_CTAS = None
 _TENSIX_OPTS = {"cores_per_bank", "split", "rows", "xs", "kb", "kw", "sbw", "noscale", "glu2", "budget", "mt"}
 _OPTS = _TENSIX_OPTS | {"glu", "glu_act", "residual", "residual_mode", "out32", "blocks", "max_banks", "col_scales", "ks",
                         "max_ctas", "exchange", "hadamard", "fixed_sums"}
+_SILU_OPTS = _TENSIX_OPTS | {"max_banks", "ks", "max_ctas", "hadamard", "fixed_sums", "fidelity", "full_sync"}
+_SILU = "linear's silu"  # linear's way of asking matmul for the activation in the kernel's output stage: no option of matmul's
 
 _CALLS = {}      # matmul_host's calls by the identity of their arguments (a hit goes straight to the library)
 _CALLS_MAX = 256
@@ -460,10 +462,11 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
 def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0, w_up, max_banks, opts):
     """matmul's call checked, described and run once: (its output, the _Call that runs it again)."""
     device = x.device()
+    opts = dict(opts)
+    silu = opts.pop(_SILU, False)  # (linear's, which has looked at what goes with it)
     unknown = set(opts) - _OPTS
     if unknown:
         raise TypeError(f"dense_reader.matmul: unknown options {sorted(unknown)}")
-    opts = dict(opts)
     own = [w, w_up]  # the caller's weights (what is launched may be a twin of one: see _one_stream_format)
     if not isinstance(w, (list, tuple)):
         check_banks(w, max_banks)
@@ -565,7 +568,7 @@ def _described(x, w, scale, memory_config, fidelity, full_sync, topk, out, col0,
     launches, need = [], 0
     for m0, m in parts:
         a, n = _describe_rows(x, blocks_all, scale, col_scales, y, m, topk, act, residual, glu, out32,
-                              opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, hadamard)
+                              opts.get("ks") or KS or 0, opts.get("max_ctas") or MAX_CTAS or 0, hadamard, silu=silu)
         launches.append((m0, a))
         need = max(need, n)
     scales = col_scales if isinstance(col_scales, (tuple, list)) else (col_scales,)
@@ -780,7 +783,7 @@ def matmul_host(x_host, out_host, x, w, scale, *, topk=None, out=None, col0=0, w
 
 
 def _describe_rows(x, entries, scale, col_scales, y, m, topk, act, residual, glu, out32, ks=0, max_ctas=0, hadamard=None,
-                   repeats=0):
+                   repeats=0, silu=False):
     """(the descriptor of one launch over m rows of x, without its tensors' addresses; the workspace it needs).
     (linear.py:828-1070)"""
     device = x.device()
@@ -791,7 +794,7 @@ def _describe_rows(x, entries, scale, col_scales, y, m, topk, act, residual, glu
     elif residual is not None and not out32:
         epi = _tkd.EPI_RESIDUAL
     else:
-        epi = _tkd.EPI_OUT32 if out32 else _tkd.EPI_PLAIN
+        epi = _tkd.EPI_OUT32 if out32 else _tkd.EPI_SILU if silu else _tkd.EPI_PLAIN
     sc = sc_up = None
     scale_dt = _tkd.DT_NONE
     if scale is not None:
@@ -913,8 +916,11 @@ def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **o
     x4 = x if len(shape) == 4 else ttnn.reshape(x, [1, 1, shape[-2], shape[-1]])
     if x4.memory_config().memory_layout != ttnn.TensorMemoryLayout.INTERLEAVED:
         x4 = ttnn.sharded_to_interleaved(x4, ttnn.L1_MEMORY_CONFIG)
-    y = matmul(x4, w, scale, memory_config=memory_config, **opts)
-    if activation is not None and activation not in ("swiglu", "geglu"):
+    # silu of a plain product into a new tensor: the kernel's output stage, on the float32 sums (as three elementwise kernels behind
+    # the matmul it took 14 of a call's 26 us; a given out holds the product itself, and a residual is added before the activation)
+    fused = activation == "silu" and not opts.keys() - _SILU_OPTS and type(w) is ttnn.Weight
+    y = matmul(x4, w, scale, memory_config=memory_config, **opts, **({_SILU: True} if fused else {}))
+    if activation is not None and activation not in ("swiglu", "geglu") and not fused:
         assert activation == "silu", f"dense_reader.linear: activation {activation!r}"
         y = ttnn.silu(y)
     if len(shape) != 4 and opts.get("out") is None:

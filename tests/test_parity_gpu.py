@@ -753,3 +753,32 @@ def test_column_shards_give_the_whole_weights_bits(device, fmt, m):
         got = [host(linear.matmul(x, linear.native_weight(device, w[i * cols : (i + 1) * cols], DT[fmt])[0], None, **opts)) for i in range(parts)]
         assert torch.equal(torch.cat(got, dim=1), whole), parts
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
+@pytest.mark.parametrize("m,k,n", [(1, 4096, 1072), (5, 544, 176), (8, 32, 16), (9, 1056, 144), (32, 4096, 208), (33, 96, 320), (300, 1056, 144)])
+def test_linear_silu_in_the_output_stage(device, fmt, m, k, n):
+    """linear(activation="silu") against the oracle for every kernel that has the output stage, with and without column scales:
+    within a rounding to bf16 of the float64 value and float32's sums. With an out the product stays in it and the activation is a
+    tensor of its own; a residual is added before the activation."""
+    g = torch.Generator().manual_seed(m + k + n)
+    w, x = torch.randn(n, k, generator=g) * 0.06, torch.randn(m, k, generator=g)
+    tx, silu = dev_x(device, x), torch.nn.functional.silu
+    for scaled in (False, True):
+        tw, ts = linear.native_weight(device, w, DT[fmt], col_scale=scaled)
+        plain = x.to(torch.bfloat16).double() @ torch.from_numpy(orc.native_values(w, fmt, col_scale=scaled)[0]).double()
+        if scaled:
+            plain = plain * ttnn.to_torch(ts).double().reshape(-1)
+        y = linear.linear(tx, tw, ts if scaled else None, activation="silu")
+        assert y.dtype == ttnn.bfloat16 and tuple(y.shape) == (1, 1, m, n)
+        close_bf16(host(y), silu(plain).numpy())
+    out = ttnn.allocate_tensor_on_device([1, 1, m, n], ttnn.bfloat16, ttnn.TILE_LAYOUT, device)
+    y = linear.linear(tx, tw, ts, activation="silu", out=out)
+    close_bf16(host(out), plain.numpy())
+    close_bf16(host(y), silu(host(out).double()).numpy())
+    unit, _ = linear.native_weight(device, w, DT[fmt])
+    plain = x.to(torch.bfloat16).double() @ torch.from_numpy(orc.native_values(w, fmt)[0]).double()
+    res = torch.randn(m, n, generator=g).to(torch.bfloat16)
+    tr = ttnn.from_torch(res.reshape(1, 1, m, n), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
+    close_bf16(host(linear.linear(tx, unit, None, activation="silu", residual=tr)), silu(plain + res.double()).numpy())
+    linear.check_status(device)
