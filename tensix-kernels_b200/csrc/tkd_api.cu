@@ -163,17 +163,18 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
             p.x_stride = (int)x_row;
             xt_bytes = a->m * x_row;
         }
-        // Items of 32 columns over all of K (tkd_narrow.cuh) where the call is a plain one and K makes four slices of nearly
-        // the same length: a streaming warp stays with one slice, and where the last is short, its warps wait for the others'.
-        // (Three stages are enough there: 100 KB of loads in flight on an SM, of the 60 that its share of the memory's rate
-        // needs.) Measured, launches in a graph over weights larger than L2, us with this kernel / the other: bfloat4_b
-        // [3648, 4096] one row 4.4 / 6.2, eight 5.3 / 9.7; bf16 [5632, 2048] eight rows, three stages, 8.1 / 10.5. Both limits
-        // lie on the safe side: beyond them, at a last slice of a third to a half (bfloat4_b [5120, 4096] 5.2 / 7.0, bfloat8_b
-        // [3584, 18944] 14.5 / 14.7, its eight rows 15.1 / 14.9) and two stages (bfloat8_b [7168, 4096], eight rows, 10.2 / 12.5),
-        // it is still the faster one nearly everywhere; they have not been moved.
+        // Items of 32 columns over all of K (tkd_narrow.cuh) where the call is a plain one of one to four slices, and two stages of
+        // the ring fit beside x (a stage has a chunk of every slice, 35 KB at four; bf16, whose loads need the most in flight, three).
+        // A streaming warp stays with one slice, so those of a short last slice wait, and with fewer slices some have none; still
+        // that is the faster form everywhere, since no sums go through L2. Measured, launches in a graph over weights larger than
+        // L2, us with this kernel / the counting one: bfloat8_b one row, [1280, 4096] (three slices) 3.7 / 4.9, [2080, 4096] (a
+        // third of the last) 4.7 / 5.9; eight rows, [1280, 4096] 4.2 / 5.9, bfloat4_b [5120, 4096] 6.0 / 10.6, [8192, 11008] (two
+        // stages) 17.2 / 21.9; bfloat8_b [8192, 11008] (two stages) 25.7 / 25.8. Two stages of bf16: [8192, 1024] 12.6 / 11.5.
         const int64_t narrow_xt = p.off_pbuf + 2 * 8 * 32 * (a->m > 1 ? 8 : 1) * 4;
-        if (!counted && p.nslices == 4 && 4 * p.ks - p.K < p.ks / 2 && !a->topk_k && a->nranks <= 1 &&
-            narrow_xt + a->m * x_row + 3 * (int64_t)p.stage_bytes + 128 <= kMaxSmem) {
+        const int narrow_stage = p.nslices * 2 * tkd_subsa(a->fmt) * sab;
+        if (!counted && p.nslices <= 4 && !a->topk_k && a->nranks <= 1 &&
+            narrow_xt + a->m * x_row + (a->fmt == TKD_BF16 ? 3 : 2) * (int64_t)narrow_stage + 128 <= kMaxSmem) {
+            p.stage_bytes = narrow_stage;
             p.narrow = p.x_smem = 1;
             p.off_xt = (int)narrow_xt;
             p.x_stride = (int)x_row;

@@ -5,8 +5,9 @@
 // a launch of one row and 2.5 of one of eight, where one token through [4096, 2048] takes 5.5 us. Here a CTA takes two groups
 // of 16 columns over all of K, the same bytes, and its sixteen streaming warps are (slice, half of a chunk's super-atoms,
 // group): the sums are the same sums in the same order (T_h ascending over the slices, then T0 + T1: see there, the two kernels
-// give the same bits), but they meet in shared memory, and no CTA waits for another. The plain calls of four
-// slices whose rows of x fit in shared memory run this kernel (make_layout). Measured, a launch of a sequence in a graph:
+// give the same bits), but they meet in shared memory, and no CTA waits for another. The plain calls of one to four
+// slices whose rows of x fit in shared memory run this kernel (make_layout); FOUR: of four, an instance of its own, because what
+// fewer need (a count instead of a constant here and there) cost the calls of four 0.15 us. Measured, a launch of a sequence in a graph:
 // one row, [4096, 4096] of bfloat8_b 8.3 us before, 6.2 now (2.8 at the memory's rate), [2048, 3072] 5.3 and 3.5; eight rows of
 // bf16, [2048, 2048] 7.2 and 4.2 (1.3). Where an SM has several items the decode of the weights bounds both kernels.
 //
@@ -39,7 +40,7 @@ __device__ __forceinline__ NarrowItem narrow_item(const TkdParams& p, int pl) {
     return {pl >> 2, 2 * (pl & 3), 2 * (pl & 3) + 1};
 }
 
-template <int FMT, bool ONE, bool KWHOLE>
+template <int FMT, bool ONE, bool KWHOLE, bool FOUR>
 __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const __grid_constant__ TkdParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
                 ok = __all_sync(0xFFFFFFFFu, mbar_wait_parked(empty0 + 8 * q, ((st / nst) & 1) ^ 1, p.status));
                 if (!ok) break;
                 const int c = s * cps + i;  // this lane's chunk, if there is one
-                const bool mine = lane < 8 && c < nch && (glu || !g);
+                const bool mine = s < (FOUR ? 4 : p.nslices) && c < nch && (glu || !g);
                 const uint32_t gb = mine ? (uint32_t)min(F::SUBSA, nsa_total - c * F::SUBSA) * F::SAB : 0u, bytes = glu ? gb : 2 * gb;
                 const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, bytes);
                 if (lane == 0) mbar_expect_tx(full0 + 8 * q, all);
@@ -131,6 +132,8 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
         if constexpr (FMT == TKD_INT4)
             rows_for_int4<ONE>(p, xt0, cw, lane, M);
         const int c0 = sl * cps, mine = min(cps, nch - c0);  // (the last slice may have fewer chunks)
+        // (the sums of a slice that K does not have: -0, which changes no float32 that it is added to)
+        const float zero = FOUR || sl < p.nslices ? 0.f : -0.f;
         const uint32_t xs0 = xs_lane + c0 * CK * 2;
         const uint32_t ring_end = ring_a + nst * p.stage_bytes;
         uint32_t at = ring_a, bar = full0, phase = 0;  // the stage, its barrier, its parity
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
         int other = 8 * 32 * MR * 4;
         for (int j = 0; ok && j < i1 - i0; ++j) {
 #pragma unroll
-            for (int a = 0; a < 2; ++a) acc[a][0][0] = acc[a][0][1] = acc[a][0][2] = acc[a][0][3] = 0.f;
+            for (int a = 0; a < 2; ++a) acc[a][0][0] = acc[a][0][1] = acc[a][0][2] = acc[a][0][3] = zero;
             uint32_t xs = xs0;
 #pragma unroll 1
             for (int i = 0; i < cps; ++i, xs += CK * 2) {
@@ -278,9 +281,9 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, 1) tkd_narrow_kernel(const 
     }
 }
 
-template <int FMT, bool ONE, bool KWHOLE>
+template <int FMT, bool ONE, bool KWHOLE, bool FOUR>
 int launch_narrow_one(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
-    auto kern = tkd_narrow_kernel<FMT, ONE, KWHOLE>;
+    auto kern = tkd_narrow_kernel<FMT, ONE, KWHOLE, FOUR>;
     static bool allowed[64] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -299,11 +302,15 @@ int launch_narrow_one(const TkdParams& p, int grid, size_t smem, cudaStream_t st
     cfg.attrs = attr, cfg.numAttrs = p.no_pdl ? 0 : 1;
     return (int)cudaLaunchKernelEx(&cfg, kern, p);
 }
+template <int FMT, bool ONE, bool KWHOLE>
+int launch_narrow_k(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
+    return p.nslices == 4 ? launch_narrow_one<FMT, ONE, KWHOLE, true>(p, grid, smem, st) : launch_narrow_one<FMT, ONE, KWHOLE, false>(p, grid, smem, st);
+}
 template <int FMT>
 int launch_narrow(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     const bool whole = p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0;
-    if (p.M == 1) return whole ? launch_narrow_one<FMT, true, true>(p, grid, smem, st) : launch_narrow_one<FMT, true, false>(p, grid, smem, st);
-    return whole ? launch_narrow_one<FMT, false, true>(p, grid, smem, st) : launch_narrow_one<FMT, false, false>(p, grid, smem, st);
+    if (p.M == 1) return whole ? launch_narrow_k<FMT, true, true>(p, grid, smem, st) : launch_narrow_k<FMT, true, false>(p, grid, smem, st);
+    return whole ? launch_narrow_k<FMT, false, true>(p, grid, smem, st) : launch_narrow_k<FMT, false, false>(p, grid, smem, st);
 }
 
 }  // namespace

@@ -782,3 +782,11 @@ def test_linear_silu_in_the_output_stage(device, fmt, m, k, n):
     tr = ttnn.from_torch(res.reshape(1, 1, m, n), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
     close_bf16(host(linear.linear(tx, unit, None, activation="silu", residual=tr)), silu(plain + res.double()).numpy())
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("dtype,k", [(ttnn.bfloat8_b, 32), (ttnn.bfloat8_b, 288), (ttnn.bfloat8_b, 544), (ttnn.bfloat8_b, 2080), (ttnn.bfloat8_b, 4128),
+                                     (ttnn.bfloat4_b, 480), (ttnn.bfloat4_b, 1056), (ttnn.bfloat4_b, 5120), (ttnn.bfloat16, 160), (ttnn.bfloat16, 1280)])
+@pytest.mark.parametrize("m", [1, 2, 8])
+def test_items_of_one_to_four_slices_equal_the_counted_kernel(device, dtype, k, m):
+    """The same for one to three slices, and for four whose last is short: every K of up to 16384 runs as items of 32 columns."""
+    test_plain_calls_equal_the_counted_kernels(device, dtype, k, m)
