@@ -32,6 +32,7 @@ int tkd_launch_unpack(int fmt, int64_t K, int64_t npad, const void* stream, cons
 #define TKD_PANEL_COLS 128     // columns one work item covers
 #define TKD_MAX_STAGES 16
 #define TKD_SMEM_HEAD 1024     // barriers, the stage headers, flags
+#define TKD_ROWS_PITCH 36      // tkd_rows_kernel: floats from a row of an item's sums to the next (36: no bank conflicts either way)
 #define TKD_TC_SLOTS 6         // tensor-memory kernel: operand slots (a unit of two 64-k tiles: 64 columns of A, 8 KB of x)
 
 struct TkdSegDev {
@@ -93,6 +94,7 @@ struct TkdParams {
     int exchange_wait;
     int tc;              // 9 to 32 rows: the tensor-memory kernel (tkd_stream_tc.cuh); off_xt is where its operand tiles go
     int tc_cluster;      // ... in clusters of four CTAs, a slice each
+    int rows_chunks;     // 9 to 24 rows: chunks of a stage of tkd_rows_kernel (tkd_rows.cuh); 0: the tensor-memory kernel
     int x_smem;          // 1 to 8 rows, and all of x (K rounded up to a chunk) fits in shared memory at off_xt
     int narrow;          // ... and the call runs tkd_narrow_kernel (tkd_narrow.cuh)
     int x_stride;        // ... bytes from one row of it to the next
