@@ -416,7 +416,7 @@ static int check_pointers(const TkdMatmul* a) {
 // ---- more than 32 rows -----------------------------------------------------------------------------------------------
 
 // The launch of such a call, without the pointers into the workspace. sms 0: ask the device.
-static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_bytes, int sms) {
+static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_bytes, int sms, double* us_out = nullptr) {
     if (!a || !fmt_ok(a->fmt) || a->m < 33 || a->m > TKD_ROWS_MAX || a->k < 32 || a->k % 32 || a->k > (1 << 24)) return TKD_ERR_BAD_ARG;
     if (a->epilogue < TKD_EPI_PLAIN || a->epilogue > TKD_EPI_SILU || a->nblocks != 1 || a->topk_k) return TKD_ERR_BAD_ARG;
     if ((a->epilogue == TKD_EPI_OUT32) != (a->out_dtype == TKD_DT_F32)) return TKD_ERR_BAD_ARG;
@@ -461,6 +461,7 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
         }
     }
     if (best == 0) return TKD_ERR_UNSUPPORTED;
+    if (us_out) *us_out = best;
     // (an MMA of up to 128 rows is shorter than its issue: two warps, an accumulator each)
     p.nmma = p.nt <= 128 ? 2 : 1;
     p.nset = p.nmma * p.nt * 2 <= 256 ? 2 : 1;
@@ -493,16 +494,68 @@ int tkd_matmul_rows_workspace(const TkdMatmul* a, uint64_t* bytes) {
     return make_wide(a, &w, &smem, bytes, sms);
 }
 
+// Whether a call of more than 32 rows runs tkd_rows_kernel in tiles of rows (of sixteen, less where x is too long for that), its
+// launch in L without the tensors. wide_us: what make_wide's model expects of tkd_wide_kernel's units and outputs.
+// Both expectations are fitted to launches in a graph over weights larger than L2 (B200; 450 shapes of 33 to 512 rows, K 576 to 3136, N
+// 544 to 10240, three formats): a launch of this kernel by the items of its longest CTA, one of tkd_wide_kernel, with the one that lays x
+// out, by that model, within 5 to 6 % on average, at most 23 %. At nine tenths no shape got slower, and 1.28 times faster is all but the
+// 1.29 that the better of the two would always give: bfloat8_b 33 rows [2048, 544] 12.7 to 4.9 us, [1056, 4096] 9.8 to 7.4; 128 rows
+// [2048, 1024] 13.5 to 7.0; 256 rows [576, 544] 7.3 to 6.2. A weight is taken apart anew for every tile here: with N or rows
+// beyond that the other is the faster one (64 rows of [1056, 10240] 15.7 against 11.2).
+static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
+    int sms = sm_count();
+    if (sms <= 0) sms = 148;
+    if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
+    if (a->ks || a->m > 16 * sms) return false;
+    TkdMatmul one = *a;
+    TkdParams& p = L->p;
+    for (one.m = 16; one.m >= 12; one.m -= 4) {
+        if (make_layout(&one, L, sms)) return false;
+        if (p.rows_chunks) break;
+    }
+    if (!p.rows_chunks) return false;
+    const int tiles = (a->m + one.m - 1) / one.m, items = 4 * p.total_panels;
+    if (tiles > sms) return false;
+    p.rows_team = sms / tiles < items ? sms / tiles : items;
+    p.rows_tile = one.m, p.M = a->m;
+    L->grid = tiles * p.rows_team;
+    const double k = p.K / 1000., most = (items + p.rows_team - 1) / p.rows_team;
+    return 3.2 + 0.2 * k + most * (0.65 + (p.fmt == TKD_BF16 ? 0.8 : 0.65) * k) < 0.9 * (3.4 + 0.62 * wide_us + 1.85 * k);
+}
+
+// A call's tensors in the parameters of its launch (but for the workspace).
+static void bind(const TkdMatmul* a, TkdParams* p) {
+    p->x = static_cast<const uint16_t*>(a->x);
+    p->ldx = a->ldx;
+    p->scale = a->scale;
+    p->scale2 = a->scale_up;
+    p->scale_dt = a->scale_dtype;
+    p->res = a->residual;
+    p->res_dt = a->residual ? a->residual_dtype : TKD_DT_NONE;
+    p->ldr = a->ldr;
+    p->out = a->out;
+    p->out_dt = a->out_dtype;
+    p->ldo = a->ldo;
+    p->status = a->status;
+    p->no_pdl = a->weights_fresh != 0;
+}
+
 int tkd_matmul_rows(const TkdMatmul* a, void* stream) {
     TkdWide p;
     size_t smem;
     uint64_t need;
-    const int rc = make_wide(a, &p, &smem, &need, 0);
+    double us;
+    const int rc = make_wide(a, &p, &smem, &need, 0, &us);
     if (rc) return rc;
     const int ra = check_pointers(a);
     if (ra) return ra;
     if (!a->workspace || a->workspace_bytes < need) return TKD_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(a->workspace) & 255) return TKD_ERR_BAD_ARG;
+    Layout L;
+    if (rows_tiles(a, &L, us)) {
+        bind(a, &L.p);
+        return launch_err(tkd_launch_stream(L.p, L.grid, L.smem, static_cast<cudaStream_t>(stream)));
+    }
     const TkdBlock& b = a->block[0];
     p.w = static_cast<const uint8_t*>(b.w), p.w2 = static_cast<const uint8_t*>(b.w_up), p.emax = b.emax, p.emax2 = b.emax_up;
     p.n_valid = (int)b.n, p.out_col0 = (int)b.out_col0;
@@ -531,25 +584,13 @@ static int run_matmul(const TkdMatmul* a, void* workspace, uint64_t workspace_by
     if (!workspace || workspace_bytes < (uint64_t)L.ws_bytes) return TKD_ERR_WORKSPACE;
     if (workspace && (reinterpret_cast<uintptr_t>(workspace) & 255)) return TKD_ERR_BAD_ARG;
 
-    p.x = static_cast<const uint16_t*>(a->x);
-    p.ldx = a->ldx;
-    p.scale = a->scale;
-    p.scale2 = a->scale_up;
-    p.scale_dt = a->scale_dtype;
-    p.res = a->residual;
-    p.res_dt = a->residual ? a->residual_dtype : TKD_DT_NONE;
-    p.ldr = a->ldr;
-    p.out = a->out;
-    p.out_dt = a->out_dtype;
-    p.ldo = a->ldo;
+    bind(a, &p);
     p.records = static_cast<uint32_t*>(a->records);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     p.counters = reinterpret_cast<int*>(ws + L.off_counters);
     p.unit_counters = reinterpret_cast<int*>(ws + L.off_units);
     p.scratch = reinterpret_cast<float*>(ws + L.off_scratch);
     p.ytmp = reinterpret_cast<uint16_t*>(ws + L.off_ytmp);
-    p.status = a->status;
-    p.no_pdl = a->weights_fresh != 0;
     if (a->hadamard) {
         if (a->fmt != TKD_INT4 || a->k % 1024 || !p.x_smem) return TKD_ERR_UNSUPPORTED;
         if (reinterpret_cast<uintptr_t>(a->hadamard) & 15) return TKD_ERR_BAD_ARG;

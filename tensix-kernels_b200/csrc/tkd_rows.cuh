@@ -128,8 +128,11 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
     }
     __syncthreads();
     const uint32_t T = 4u * (uint32_t)p.total_panels;  // items
-    const int i0 = (int)((uint64_t)T * blockIdx.x / gridDim.x), i1 = (int)((uint64_t)T * (blockIdx.x + 1) / gridDim.x);
-    const int nst = p.nstages, M = p.M, K = p.K, nch = (K + CK - 1) / CK, nsa_total = (K + F::KSA - 1) / F::KSA;
+    // (more than 32 rows: tiles of rows, a team of CTAs each)
+    const uint32_t team = p.rows_team ? p.rows_team : gridDim.x, tile = blockIdx.x / team, cta = blockIdx.x - tile * team;
+    const int i0 = (int)((uint64_t)T * cta / team), i1 = (int)((uint64_t)T * (cta + 1) / team);
+    const int row0 = (int)tile * p.rows_tile, M = p.rows_tile ? min(p.rows_tile, p.M - row0) : p.M;
+    const int nst = p.nstages, K = p.K, nch = (K + CK - 1) / CK, nsa_total = (K + F::KSA - 1) / F::KSA;
     const int spi = (nch + SC - 1) / SC;  // stages of an item
     const int epi = p.epi;
     const bool glu = epi == TKD_EPI_GLU2 || epi == TKD_EPI_GLU_IL;
@@ -185,7 +188,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
         for (int s = 0; s < kRowsSegs; ++s) {  // (the last part: all that is left)
             const int e0 = min(s * SC * CK, K) / 8, e1 = s == kRowsSegs - 1 ? K / 8 : min((s + 1) * SC * CK, K) / 8;
             for (int r = cw; r < M; r += SW) {
-                const uint16_t* src = p.x + (int64_t)r * p.ldx;
+                const uint16_t* src = p.x + (int64_t)(row0 + r) * p.ldx;
                 const uint32_t dst = xt0 + r * p.x_stride;
 #pragma unroll 4
                 for (int e = e0 + lane; e < e1; e += 32)
@@ -322,7 +325,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
             uint32_t q[RW] = {};
             if (p.res_dt != TKD_DT_NONE && oc >= 0 && left > 0) {
                 const int rsz = p.res_dt == TKD_DT_F32 ? 4 : 2;
-                const char* rp = static_cast<const char*>(p.res) + ((int64_t)(RW * ow) * p.ldr + oc) * rsz;
+                const char* rp = static_cast<const char*>(p.res) + ((int64_t)(row0 + RW * ow) * p.ldr + oc) * rsz;
 #pragma unroll
                 for (int m = 0; m < RW; ++m) {
                     q[m] = rsz == 4 ? *reinterpret_cast<const uint32_t*>(rp) : (uint32_t)*reinterpret_cast<const uint16_t*>(rp) << 16;
@@ -357,7 +360,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
 #pragma unroll
                 for (int m = 0; m < RW; ++m) v[m] += __uint_as_float(q[m]);
             }
-            char* yp = static_cast<char*>(p.out) + ((int64_t)(RW * ow) * p.ldo + oc) * (f32out ? 4 : 2);
+            char* yp = static_cast<char*>(p.out) + ((int64_t)(row0 + RW * ow) * p.ldo + oc) * (f32out ? 4 : 2);
             const int rows = oc >= 0 && (topk_k == 0 || p.write_y) ? left : 0;
 #pragma unroll
             for (int m = 0; m < RW; ++m, yp += p.ldo * (f32out ? 4 : 2)) {
@@ -419,14 +422,15 @@ int launch_rows_kernel(const TkdParams& p, int grid, size_t smem, cudaStream_t s
         constexpr int MT = decltype(mt)::value, SC = decltype(sc)::value;
         return p.topk_k || p.npeers ? launch_rows_one<FMT, MT, SC, false>(p, grid, smem, st) : launch_rows_one<FMT, MT, SC, true>(p, grid, smem, st);
     };
+    const int rows = p.rows_tile ? p.rows_tile : p.M;
     auto chunks = [&](auto mt) {
         if constexpr (FMT != TKD_BF16)
             if (p.rows_chunks == 2) return go(mt, std::integral_constant<int, 2>{});
         return go(mt, std::integral_constant<int, 4>{});
     };
     if constexpr (FMT == TKD_BF16)
-        if (p.M > 24) return chunks(std::integral_constant<int, 4>{});
-    return p.M <= 16 ? chunks(std::integral_constant<int, 2>{}) : chunks(std::integral_constant<int, 3>{});
+        if (rows > 24) return chunks(std::integral_constant<int, 4>{});
+    return rows <= 16 ? chunks(std::integral_constant<int, 2>{}) : chunks(std::integral_constant<int, 3>{});
 }
 
 }  // namespace

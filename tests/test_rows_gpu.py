@@ -105,3 +105,18 @@ def test_exchanged_calls_give_the_plain_calls_bits(device, m, out32):
         assert torch.equal(ttnn.to_torch(outs[r]), full), r
         assert bufs[r][: 4 * world].view(torch.int32).tolist() == [1] * world
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
+@pytest.mark.parametrize("m,k,n", [(33, 96, 16), (47, 544, 320), (64, 2080, 144), (97, 1056, 512), (100, 4096, 80), (250, 288, 64)])
+def test_tiles_of_rows(device, fmt, m, k, n):
+    """More than 32 rows of a small weight, tiles of sixteen rows (twelve at K 4096) with a team of CTAs each: every output stage, a
+    last tile in part, a team of one CTA, more items than CTAs."""
+    test_outputs_against_oracle(device, fmt, m, k, n)
+    g = torch.Generator().manual_seed(m)
+    w, x = torch.randn(n, k, generator=g) * 0.05, torch.randn(m, k, generator=g)
+    tw, _ = linear.native_weight(device, w, DT[fmt])
+    plain = x.to(torch.bfloat16).double() @ torch.from_numpy(orc.native_values(w, fmt)[0]).double()
+    for ctas in (None, 17):
+        close_bf16(host(linear.linear(dev_x(device, x), tw, None, activation="silu", max_ctas=ctas)), torch.nn.functional.silu(plain).numpy())
+    linear.check_status(device)
