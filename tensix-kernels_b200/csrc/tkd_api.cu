@@ -59,23 +59,28 @@ int tc_cluster_count(int fmt, size_t smem) {
 // 10.9 / 12.5, [3328, 14336] with 16 rows, the worst, 16.6 / 16.0; bfloat4_b [2816, 4096] 5.9 / 9.2; less of a ring: bfloat8_b [4096, 14336]
 // with 16 rows 21.1 / 17.7. 17 to 24 rows, three MMAs a fragment: of four slices, where that kernel runs in clusters, up to K 1536
 // (bfloat8_b [1024, 4096] 5.2 / 7.1, [2048, 14336] 14.7 / 13.5); of other numbers of slices always (bfloat4_b [2816, 4096] 7.4 / 10.0). 25 to
-// 32 rows: bf16 of other numbers of slices ([1056, 14336] 12.8 / 17.1); a block-float decode beside four MMAs is longer than
-// the tensor memory's way (bfloat8_b [1056, 14336] 19.5 / 16.2).
+// 32 rows of other numbers of slices: bf16 with four MMAs a fragment ([1056, 14336] 12.8 / 17.1); block-float decodes beside four MMAs
+// take longer than the tensor memory's way ([1056, 14336] 19.5 / 16.2), and so run as two tiles of sixteen rows, a team of CTAs each
+// (13.0 / 16.2; bfloat4_b [1056, 4096] 6.1 / 8.6), as do 17 and more rows whose x does not fit, up to K 2816 (bfloat4_b [2816, 14336]
+// 19.9 / 21.4; [3072, 14336] 20.4 / 18.7).
 int rows_layout(TkdParams& p, int sab) {
-    const int ck = tkd_chunk_k(p.fmt), nch = (p.K + ck - 1) / ck, mt = (p.M + 7) / 8;
-    if (mt == 3 && p.nslices == 4 && p.K > 1536) return 0;
-    if (mt == 4 && (p.nslices == 4 || p.fmt != TKD_BF16)) return 0;
-    const int64_t x_row = (int64_t)nch * ck * 2 + 64, tbuf = TKD_SMEM_HEAD + 8 * 8 * mt * TKD_ROWS_PITCH * 4;
-    const int64_t xt = tbuf + 1024, ring = align_up(xt + p.M * x_row, 128);  // (1 KB: the lists of top-k records)
-    for (int chunks = 4; chunks >= (p.fmt == TKD_BF16 ? 4 : 2); chunks -= 2) {
-        const int stage = (nch < chunks ? nch : chunks) * 2 * tkd_subsa(p.fmt) * sab;
-        const int64_t stages = (kMaxSmem - ring) / stage;
-        if (ring > kMaxSmem || stages < 3 || kMaxSmem - ring < 80 * 1024) continue;
-        p.off_pbuf = TKD_SMEM_HEAD, p.off_tbuf = (int)tbuf, p.off_xt = (int)xt, p.off_ring = (int)ring;
-        p.x_stride = (int)x_row, p.stage_bytes = stage, p.nstages = (int)(stages < TKD_MAX_STAGES ? stages : TKD_MAX_STAGES);
-        return chunks;
+    const int ck = tkd_chunk_k(p.fmt), nch = (p.K + ck - 1) / ck;
+    if (p.M > 16 && p.nslices == 4 && (p.M > 24 || p.K > 1536)) return 0;
+    for (int rows = p.M > 24 && p.fmt != TKD_BF16 && p.K <= 2816 ? 16 : p.M;; rows = 16) {
+        const int mt = (rows + 7) / 8;
+        const int64_t x_row = (int64_t)nch * ck * 2 + 64, tbuf = TKD_SMEM_HEAD + 8 * 8 * mt * TKD_ROWS_PITCH * 4;
+        const int64_t xt = tbuf + 1024, ring = align_up(xt + rows * x_row, 128);  // (1 KB: the lists of top-k records)
+        for (int chunks = 4; chunks >= (p.fmt == TKD_BF16 ? 4 : 2); chunks -= 2) {
+            const int stage = (nch < chunks ? nch : chunks) * 2 * tkd_subsa(p.fmt) * sab;
+            const int64_t stages = (kMaxSmem - ring) / stage;
+            if (stages < 3 || kMaxSmem - ring < 80 * 1024) continue;
+            p.off_pbuf = TKD_SMEM_HEAD, p.off_tbuf = (int)tbuf, p.off_xt = (int)xt, p.off_ring = (int)ring;
+            p.x_stride = (int)x_row, p.stage_bytes = stage, p.nstages = (int)(stages < TKD_MAX_STAGES ? stages : TKD_MAX_STAGES);
+            p.rows_tile = rows < p.M ? rows : 0;
+            return chunks;
+        }
+        if (rows <= 16 || p.K > 2816) return 0;
     }
-    return 0;
 }
 
 struct Layout {
@@ -220,7 +225,9 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     if (p.tc && !a->ks) p.rows_chunks = rows_layout(p, sab);
     if (p.rows_chunks) p.tc = 0, L->smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
     const int64_t items = p.narrow || p.rows_chunks ? 4 * (int64_t)panels : p.total_items;
-    L->grid = (int)(items < sms ? items : sms);
+    const int tiles = p.rows_tile ? (p.M + p.rows_tile - 1) / p.rows_tile : 1, team = sms / tiles > 0 ? sms / tiles : 1;
+    L->grid = tiles * (int)(items < team ? items : team);
+    if (p.rows_tile) p.rows_team = L->grid / tiles;
     // 9 to 32 rows: clusters of four CTAs, one to a slice (tkd_stream_tc.cuh), for a plain call of four slices. They take whole
     // panels and leave some SMs idle (a GPC's number of SMs is not a multiple of four: 132 of 148 CTAs on a B200), so they are
     // taken where no CTA gets more items for it; from four items on the other form's SMs that have one less leave theirs to the rest.

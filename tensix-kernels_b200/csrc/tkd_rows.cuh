@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
         // ---------------------------------------------------------------- output warps
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const int ow = warp, left = M - RW * ow;  // rows from this warp's first on
-        const int topk_k = PLAIN ? 0 : p.topk_k, npeers = PLAIN ? 0 : p.npeers;
+        const int topk_k = PLAIN || tile ? 0 : p.topk_k, npeers = PLAIN ? 0 : p.npeers;
         const bool up = glu && lane >= 16, f32out = epi == TKD_EPI_OUT32;
         bool met = true;
         for (int j = 0; j < i1 - i0; ++j) {
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
                 for (int m = 0; m < RW; ++m) v[m] += __uint_as_float(q[m]);
             }
             char* yp = static_cast<char*>(p.out) + ((int64_t)(row0 + RW * ow) * p.ldo + oc) * (f32out ? 4 : 2);
-            const int rows = oc >= 0 && (topk_k == 0 || p.write_y) ? left : 0;
+            const int rows = oc >= 0 && (PLAIN || p.topk_k == 0 || p.write_y) ? left : 0;
 #pragma unroll
             for (int m = 0; m < RW; ++m, yp += p.ldo * (f32out ? 4 : 2)) {
                 if (f32out)
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
 #pragma unroll
                 for (int m = 0; m < RW; ++m) {
                     const int r = RW * ow + m;
-                    const size_t to = (size_t)r * p.ldo + oc;
+                    const size_t to = (size_t)(row0 + r) * p.ldo + oc;
                     const uint16_t b = f32_to_bf16_bits(v[m]);
 #pragma unroll 1
                     for (int pq = 0; m < rows && pq < npeers; ++pq) {

@@ -15,7 +15,7 @@ from test_parity_gpu import DT, close_bf16, dev_x, host  # noqa: E402
 
 @pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
 @pytest.mark.parametrize("m,k,n", [(9, 32, 16), (9, 4096, 208), (12, 288, 144), (16, 544, 320), (16, 3360, 1056), (17, 1024, 64),
-                                   (24, 1184, 5008), (25, 160, 144), (32, 1056, 272)])
+                                   (24, 1184, 5008), (25, 160, 144), (32, 1056, 272), (20, 3136, 144)])
 def test_outputs_against_oracle(device, fmt, m, k, n):
     """Every output stage, K inside a super-atom, a chunk and a stage, N inside a panel and past one item a CTA, few CTAs and all.
     bf16 results within a rounding and the float32 sums' error; float32 ones within K products of relative error 2^-24, added at
@@ -45,7 +45,7 @@ def test_outputs_against_oracle(device, fmt, m, k, n):
     linear.check_status(device)
 
 
-@pytest.mark.parametrize("m,k", [(9, 1024), (16, 288), (24, 1056)])
+@pytest.mark.parametrize("m,k", [(9, 1024), (16, 288), (24, 1056), (30, 1056)])
 def test_records_of_the_plain_calls_outputs(device, m, k):
     """Records are the canonical top-k of the outputs that a plain call gives, with and without y written, of one weight and of a
     block list, with ties and a last unit in part."""
@@ -79,7 +79,7 @@ def check_records(rec, y, n, base):
             assert np.array_equal(rec[u, 0, t], keys) and np.array_equal(rec[u, 1, t], idx), (u, t)
 
 
-@pytest.mark.parametrize("m,out32", [(9, False), (16, True), (20, False)])
+@pytest.mark.parametrize("m,out32", [(9, False), (16, True), (20, False), (31, False)])
 def test_exchanged_calls_give_the_plain_calls_bits(device, m, out32):
     """Column shards of 9 and more rows, their outputs stored into every rank's buffer: the whole weight's bits, and the flags."""
     world, k = 3, 1056
