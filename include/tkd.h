@@ -287,7 +287,7 @@ typedef struct {
                                 layout, moe8.py:507-527 kblock: shared exponents along K), kept exactly at 2 bytes a weight;
                                 emax is then unused */
     int32_t out_rows;        /* by_union: rows of out; those from `rows` on are written with zeros (0: none) */
-    int32_t* status;         /* by_union: one int32 (or NULL): TKD_ERR_TIMEOUT is written here if a wait gives up */
+    int32_t* status;         /* one int32 (or NULL): TKD_ERR_TIMEOUT is written here if a wait gives up */
 } TkdMoe;
 
 int tkd_moe_workspace(const TkdMoe* a, uint64_t* bytes);

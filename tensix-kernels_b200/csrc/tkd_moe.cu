@@ -5,28 +5,23 @@
 //
 // Every expert's weight is a bfloat4_b stream of tkd_layout.h (tkd_pack), all experts back to back, so the kernel
 // finds a chosen expert by its id alone: the ids are read on the device and nothing goes to the host. What a call reads
-// is small (k experts of a few MB) and scattered, so instead of the persistent ring of tkd_stream_kernel.cuh this is
-// a plain grid: a CTA owns (32 columns of one slot's expert, all of its K), its 4 warps are 2 groups of 16 columns x 2
-// runs of super-atoms, and a lane loads its own 16 bytes of codes and 16 bytes of exponents of a super-atom straight
-// from global memory into the mma.sync A fragment's registers (the stream is laid out lane by lane, so a warp's load
-// is one contiguous 512 bytes), four super-atoms at a time. The decode is the stream kernel's (block_mma), and like it
-// the kernel is bound by instruction issue, not by HBM: units this small (384 and 512 CTAs of 128 threads for a layer
-// of 8 experts of 2048 x 1536) are what spreads that work evenly over the SMs.
-//   gate_up: a unit is 16 columns of a gate tile and the same 16 of its up tile: the CTA finishes 16 outputs,
-//            h = routing weight * act(x G + b) * (x U + b), rounded to bf16 once.
-//   down:    a CTA writes its slot's partial sums of 32 columns of y to the workspace; the CTA that arrives last at
-//            the unit's counter adds the slots up in slot order and writes y (no CTA waits for another).
+// is small (k experts of a few MB) and scattered, so instead of the persistent ring of tkd_stream_kernel.cuh this is a plain grid of
+// warps that each take a run of super-atoms of one group of 16 columns: the run's weights and its inputs come into the warp's own
+// shared memory by bulk copies, all asked for as soon as the expert's id is known, and the decode is the stream kernel's (block_mma).
+// The layer is a chain of latencies (the ids, the weights from DRAM, the sums, the launch): as loads into registers, four super-atoms
+// at a time behind a block's copy of the inputs, gate_up took 7.9 us of a layer of 8 experts of 2048 x 1536, and down, whose slots met
+// through L2 by an atomic, 6.8.
+//   gate_up: a CTA is 16 columns of a gate tile and the same 16 of its up tile of one slot's expert, two runs each: it finishes 16
+//            outputs, h = routing weight * act(x G + b) * (x U + b), rounded to bf16 once.
+//   down:    a CTA is 16 columns of y, two runs of every slot's expert: the slots' sums are added in slot order in shared memory.
 // Several rows (by_union): tkd_moe_rows.cuh.
 #include "tkd_moe_rows.cuh"
 
 namespace {
 
-constexpr int kMoeGroups = 2;  // groups of 16 columns a CTA covers at a time (gate_up: 16 gate columns and their 16 up columns)
-// warps along K per group: 4 warps a CTA, four CTAs an SM (with 4 a warp had too few super-atoms to spread its set-up over: the
-// layer of the benchmark 16.9 us, 16.35 with down at 2, 16.8 with gate_up at 2; down at 1: 17.6)
-constexpr int kMoeSplit = 2, kMoeThreads = kMoeGroups * kMoeSplit * 32;
-constexpr int kMoeBatch = 4;  // super-atoms whose loads are issued before the first is used (8: spills, slower)
-constexpr int kMoeCols = kMoeGroups * 16;
+constexpr int kMoeSplit = 2;  // runs of K a group
+constexpr int kMoeHalf = 8;   // super-atoms of a half of a warp's buffer
+constexpr int kMoeCols = 32;  // columns a counter of the workspace stands for
 
 struct MoeParams {
     const uint8_t* w;
@@ -40,18 +35,10 @@ struct MoeParams {
     int slots, act;
     const uint16_t* bias;
     uint16_t* out;
-    float* part;    // down: [slot][npad] partial sums
-    int* counters;  // down: one per block of 64 columns; back to zero when the call ends
+    int* status;
     uint32_t mul16, mul128;
 };
 
-__device__ __forceinline__ uint4 ldg_stream(const uint8_t* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
-}
 __device__ __forceinline__ uint32_t moe_id(const MoeParams& p, int64_t i) {
     return p.ids32 ? static_cast<const uint32_t*>(p.ids)[i] : static_cast<const uint16_t*>(p.ids)[i];
 }
@@ -60,146 +47,159 @@ __device__ __forceinline__ float moe_scale(float v, int ebyte) {
     const int e = tkd_out_exp(TKD_BFP4, ebyte), e1 = e / 2, e2 = e - e1;
     return v * __uint_as_float((uint32_t)(e1 + 127) << 23) * __uint_as_float((uint32_t)(e2 + 127) << 23);
 }
+// Bytes of a warp's buffer: two halves of weights and of the inputs for them.
+template <int FMT>
+constexpr int kMoeHalfBytes = kMoeHalf * (Fmt<FMT>::SAB + Fmt<FMT>::KSA * 2);
+
+// A warp's run of super-atoms of a group, through its buffer `buf` and its two barriers: the sums in acc. st: halves before this run.
+// xs: the inputs at k = 0. false: a wait gave up.
+template <int FMT>
+__device__ __forceinline__ bool moe_run(const MoeParams& p, float (&acc)[2][1][4], const uint8_t* wb, int group, int sa0, int sa1,
+                                        const uint16_t* xs, uint32_t buf, uint32_t bars, uint32_t& st, const uint2 sh) {
+    using F = Fmt<FMT>;
+    constexpr int XB = F::KSA * 2;  // bytes of x a super-atom
+    const int lane = threadIdx.x & 31, t = lane & 3;
+    const int halves = (sa1 - sa0 + kMoeHalf - 1) / kMoeHalf;
+    auto issue = [&](int h) {
+        const uint32_t q = (st + h) & 1, to = buf + q * kMoeHalfBytes<FMT>, bar = bars + 8 * q;
+        const int a = sa0 + h * kMoeHalf, b = min(sa1, a + kMoeHalf);
+        const uint32_t xbytes = (uint32_t)(min(b * F::KSA, p.K) - a * F::KSA) * 2;
+        mbar_expect_tx(bar, (b - a) * F::SAB + xbytes);
+        for (int sa = a; sa < b;) {  // (a group's super-atoms lie back to back inside a chunk)
+            const int end = min(b, (sa | (F::SUBSA - 1)) + 1);
+            bulk_g2s(to + (sa - a) * F::SAB, wb + tkd_sa_offset(FMT, p.K, group, sa), (end - sa) * F::SAB, bar);
+            sa = end;
+        }
+        bulk_g2s(to + kMoeHalf * F::SAB, xs + a * F::KSA, xbytes, bar);
+    };
+    if (lane == 0) {
+        issue(0);
+        if (halves > 1) issue(1);
+    }
+    __syncwarp();
+    for (int h = 0; h < halves; ++h) {
+        const uint32_t q = (st + h) & 1, from = buf + q * kMoeHalfBytes<FMT>, x0 = from + kMoeHalf * F::SAB + 16 * t;
+        if (!mbar_wait(bars + 8 * q, ((st + h) >> 1) & 1, p.status)) {
+            for (uint32_t i = 0; h + 1 < halves && i < 64; ++i)  // (the copies in flight land before the warp goes)
+                if (mbar_try_wait(bars + 8 * (q ^ 1), ((st + h + 1) >> 1) & 1)) break;
+            return false;
+        }
+        const int a = sa0 + h * kMoeHalf, n = min(sa1 - a, kMoeHalf);
+        if (FMT == TKD_BFP4 && (a + n) * F::KSA > p.K) {  // (a K that ends inside a super-atom: zeros after it)
+            if (lane < 4) asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(x0 + n * XB - 64), "r"(0u) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (before the next run's copies)
+            __syncwarp();
+        }
+        auto one = [&](int b) {
+            const uint32_t s = from + b * F::SAB, x = x0 + b * XB;
+            if constexpr (FMT == TKD_BFP4) {
+                const uint4 ev = lds128(s + t * 16), cv = lds128(s + 64 + lane * 16);
+#pragma unroll
+                for (int qq = 0; qq < 2; ++qq) {
+                    const uint32_t cw[4] = {qq ? cv.z : cv.x, qq ? cv.w : cv.y, 0u, 0u}, ew[2] = {qq ? ev.z : ev.x, qq ? ev.w : ev.y};
+                    const uint4 xv[1] = {lds128(x + 64 * qq)};
+                    block_mma<TKD_BFP4, 1, 2>(acc, cw, ew, xv, sh);
+                }
+            } else {  // (bf16: the A fragments of the super-atom's two mmas as they are)
+                const uint4 wa = lds128(s + lane * 16), wc = lds128(s + 512 + lane * 16), xv = lds128(x);
+                mma_bf16(acc[0][0], wa.x, wa.y, wa.z, wa.w, xv.x, xv.y);
+                mma_bf16(acc[1][0], wc.x, wc.y, wc.z, wc.w, xv.z, xv.w);
+            }
+        };
+        if (n == kMoeHalf) {
+#pragma unroll
+            for (int b = 0; b < kMoeHalf; ++b) one(b);
+        } else {
+#pragma unroll 2
+            for (int b = 0; b < n; ++b) one(b);
+        }
+        __syncwarp();
+        if (lane == 0 && h + 2 < halves) issue(h + 2);
+    }
+    st += halves;
+    return true;
+}
+
 // One row. FMT: the experts' stream format (bfloat4_b, or bf16 for a pack held exactly). DOWN: the down matmul.
 template <int FMT, bool DOWN>
-__global__ void __launch_bounds__(kMoeThreads, 4) tkd_moe_kernel(const MoeParams p) {
+__global__ void __launch_bounds__(DOWN ? 512 : 128, DOWN ? 1 : 4) tkd_moe_kernel(const MoeParams p) {
     using F = Fmt<FMT>;  // (k and bytes of a super-atom, super-atoms of a group in a chunk)
-    extern __shared__ __align__(16) uint8_t moe_dsm[];
-    __shared__ int s_last;
+    extern __shared__ __align__(128) uint8_t moe_dsm[];
+    __shared__ uint64_t s_bars[2 * 16];
+    __shared__ int s_e[DOWN ? 17 : 1];  // down: a slot's exponent byte, -1 without an expert
+    __shared__ float red[DOWN ? 17 : 1][kMoeSplit][DOWN ? 16 : 32];  // [slot][run][column]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int gi = warp & (kMoeGroups - 1), ksp = warp / kMoeGroups;
-    const int q = blockIdx.y;
-    const int Kpad = (p.K + 63) & ~63;
-    uint8_t* xs = moe_dsm;
-    float* red = reinterpret_cast<float*>(moe_dsm + Kpad * 2);  // [ksp][column]
-
-    // (launched as a programmatic dependent: nothing the kernels before wrote is read above this line, and the kernel
-    // after may bring its CTAs in while this one runs: it waits at the same place)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t buf = smem_u32(moe_dsm) + warp * 2 * kMoeHalfBytes<FMT>, bars = smem_u32(s_bars) + warp * 16;
+    if (lane == 0) {
+        mbar_init(bars, 1), mbar_init(bars + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    // (launched as a programmatic dependent: nothing the kernels before wrote is read above the wait, and the kernel after may bring
+    // its CTAs in while this one runs: it waits at the same place)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const uint32_t id = moe_id(p, q);
-    const int e = id < (uint32_t)p.E ? (int)id : -1;
-    float w1 = 0.f;  // the slot's routing weight
-    if constexpr (!DOWN)
-        if (e >= 0) w1 = bf16_bits_to_f32(p.rw[q]);
-    // a unit of 32 weight columns. gate_up: unit u is half hf = u & 1 of the tile pair j = u >> 1: columns hf * 16 .. + 15 of
-    // gate tile j (warps gi 0) and of up tile j (gi 1), 16 outputs.
-    const int u = blockIdx.x, group = DOWN ? u * kMoeGroups + gi : (u >> 1) * 4 + 2 * gi + (u & 1);
-    const uint8_t* wb = p.w + (int64_t)max(e, 0) * p.wbytes;
-    const uint8_t* emx = FMT == TKD_BFP4 ? p.emax + (int64_t)max(e, 0) * (p.npad / 16) : nullptr;
-    const int nsa = (p.K + F::KSA - 1) / F::KSA, per = (nsa + kMoeSplit - 1) / kMoeSplit;
-    const int sa0 = ksp * per, sa1 = min(nsa, sa0 + per);
+    const int u = blockIdx.x, nsa = (p.K + F::KSA - 1) / F::KSA, per = (nsa + kMoeSplit - 1) / kMoeSplit;
     const uint2 sh = make_uint2(p.mul16, p.mul128);
-    if (e >= 0) {
-        // This warp's super-atoms are asked into L2 at once (one instruction per run inside a chunk), so that the loads behind
-        // the first batch, which wait for registers, find them there: one trip to HBM, not two.
-        if (lane == 0)
-            for (int sa = sa0; sa < sa1;) {
-                const int end = min(sa1, (sa | (F::SUBSA - 1)) + 1);
-                const uint8_t* s = wb + tkd_sa_offset(FMT, p.K, group, sa);
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s), "r"((end - sa) * F::SAB) : "memory");
-                sa = end;
-            }
-        // the activations: gate_up: x; down: the inputs of slot q. Zeros past K up to a super-atom.
-        const uint16_t* xsrc = p.x + (DOWN ? (int64_t)q * p.K : 0);
-        for (int c = tid; c < Kpad / 8; c += kMoeThreads)
-            reinterpret_cast<uint4*>(xs)[c] = c * 8 < p.K ? __ldg(reinterpret_cast<const uint4*>(xsrc) + c) : make_uint4(0u, 0u, 0u, 0u);
-    }
-    __syncthreads();
-    const uint32_t xa = smem_u32(xs) + 16 * t;
-    if (e >= 0) {
-        // ---- the group's sums over this warp's run of super-atoms
+    uint32_t st = 0;
+    // the sums of group `group` of expert e over run ksp, its inputs from xs on, to d: columns g and g + 8
+    auto run = [&](int e, int group, int ksp, const uint16_t* xs, float* d) {
         float acc[2][1][4] = {};
-        // (the super-atoms of a group lie back to back inside a chunk of 8: the layout is asked at its starts only)
-        const uint8_t* s = wb;
-        for (int sa = sa0; sa < sa1; sa += kMoeBatch) {
-            uint4 cv[kMoeBatch], ev[kMoeBatch];
-#pragma unroll
-            for (int b = 0; b < kMoeBatch; ++b)
-                if (sa + b < sa1) {
-                    s = (b == 0 && sa == sa0) || ((sa + b) & (F::SUBSA - 1)) == 0 ? wb + tkd_sa_offset(FMT, p.K, group, sa + b) : s + F::SAB;
-                    if constexpr (FMT == TKD_BFP4) {
-                        ev[b] = ldg_stream(s + t * 16);
-                        cv[b] = ldg_stream(s + 64 + lane * 16);
-                    } else {  // (bf16: the A fragments of the super-atom's two mmas as they are)
-                        cv[b] = ldg_stream(s + lane * 16);
-                        ev[b] = ldg_stream(s + 512 + lane * 16);
-                    }
-                }
-#pragma unroll
-            for (int b = 0; b < kMoeBatch; ++b)
-                if (sa + b < sa1) {
-                    if constexpr (FMT == TKD_BFP4) {
-#pragma unroll
-                        for (int qq = 0; qq < 2; ++qq) {
-                            const uint32_t cw[4] = {qq ? cv[b].z : cv[b].x, qq ? cv[b].w : cv[b].y, 0u, 0u};
-                            const uint32_t ew[2] = {qq ? ev[b].z : ev[b].x, qq ? ev[b].w : ev[b].y};
-                            const uint4 xv[1] = {lds128(xa + (uint32_t)(sa + b) * 128 + 64 * qq)};
-                            block_mma<TKD_BFP4, 1, 2>(acc, cw, ew, xv, sh);
-                        }
-                    } else {
-                        const uint4 xv = lds128(xa + (uint32_t)(sa + b) * 64);
-                        mma_bf16(acc[0][0], cv[b].x, cv[b].y, cv[b].z, cv[b].w, xv.x, xv.y);
-                        mma_bf16(acc[1][0], ev[b].x, ev[b].y, ev[b].z, ev[b].w, xv.z, xv.w);
-                    }
-                }
-        }
+        const int sa0 = min(ksp * per, nsa), sa1 = min(nsa, sa0 + per);
+        if (e >= 0 && sa0 < sa1) moe_run<FMT>(p, acc, p.w + (int64_t)e * p.wbytes, group, sa0, sa1, xs, buf, bars, st, sh);
         // (every column of D is the one row's; its first is kept: lanes with t = 0 hold columns g and g + 8 of the weight)
-        if (t == 0) {
-            float* d = red + ksp * kMoeCols + gi * 16 + g;
-            d[0] = acc[0][0][0] + acc[1][0][0], d[8] = acc[0][0][2] + acc[1][0][2];
-        }
-    }
-    __syncthreads();
-
-    // column c of the unit (gate_up: 0-15 the gate's, 16-31 the up's): the K sum, in the weight's units
-    auto column_sum = [&](int c, int grp) {
-        float v = 0.f;
-#pragma unroll
-        for (int sp = 0; sp < kMoeSplit; ++sp) v += red[sp * kMoeCols + c];
-        if constexpr (FMT == TKD_BFP4) v = moe_scale(v, emx[grp]);
-        return v;
+        if (t == 0) d[g] = acc[0][0][0] + acc[1][0][0], d[g + 8] = acc[0][0][2] + acc[1][0][2];
+    };
+    auto expert = [&](int q) {
+        const uint32_t id = moe_id(p, q);
+        return id < (uint32_t)p.E ? (int)id : -1;
     };
     if constexpr (!DOWN) {
-        const int j = u >> 1, hf = u & 1;
+        // unit u is half hf = u & 1 of the tile pair j = u >> 1: columns hf * 16 .. + 15 of gate tile j (warps gi 0) and of up tile j
+        // (gi 1), 16 outputs
+        const int q = blockIdx.y, e = expert(q), gi = warp & 1, j = u >> 1, hf = u & 1;
+        int eg = 0, eu = 0;
+        float w1 = 0.f, bg = 0.f, bu = 0.f;
+        if (tid < 16 && e >= 0) {  // (asked for ahead of the weights' wait)
+            w1 = bf16_bits_to_f32(p.rw[q]);  // the slot's routing weight
+            if constexpr (FMT == TKD_BFP4) {
+                const uint8_t* emx = p.emax + (int64_t)e * (p.npad / 16) + j * 4 + hf;
+                eg = emx[0], eu = emx[2];
+            }
+            if (p.bias) {
+                const uint16_t* b = p.bias + (int64_t)e * p.npad + j * 64 + hf * 16 + tid;
+                bg = bf16_bits_to_f32(b[0]), bu = bf16_bits_to_f32(b[32]);
+            }
+        }
+        run(e, j * 4 + 2 * gi + hf, warp >> 1, p.x, &red[0][warp >> 1][gi * 16]);
+        __syncthreads();
         if (tid < 16) {
             float val = 0.f;
             if (e >= 0) {
-                float gt = column_sum(tid, j * 4 + hf), up = column_sum(16 + tid, j * 4 + 2 + hf);
-                if (p.bias) {
-                    const uint16_t* b = p.bias + (int64_t)e * p.npad + j * 64 + hf * 16 + tid;
-                    gt += bf16_bits_to_f32(b[0]), up += bf16_bits_to_f32(b[32]);
-                }
-                val = moe_glu(gt, up, p.act) * w1;
+                float gt = red[0][0][tid] + red[0][1][tid], up = red[0][0][16 + tid] + red[0][1][16 + tid];
+                if constexpr (FMT == TKD_BFP4) gt = moe_scale(gt, eg), up = moe_scale(up, eu);
+                val = moe_glu(gt + bg, up + bu, p.act) * w1;
             }
             p.out[(int64_t)q * (p.N / 2) + j * 32 + hf * 16 + tid] = f32_to_bf16_bits(val);
         }
     } else {
-        // this slot's sums of the unit's columns are written: the CTA that arrives last adds the slots up
-        if (tid < kMoeCols) {
-            if (e >= 0) p.part[(int64_t)q * p.npad + u * kMoeCols + tid] = column_sum(tid, u * kMoeGroups + (tid >> 4));
-            __threadfence();
+        for (int i = warp; i < p.slots * kMoeSplit; i += blockDim.x >> 5) {
+            const int q = i / kMoeSplit, ksp = i - q * kMoeSplit, e = expert(q);
+            int eb = e >= 0 ? 0 : -1;
+            if (FMT == TKD_BFP4 && e >= 0) eb = p.emax[(int64_t)e * (p.npad / 16) + u];
+            run(e, u, ksp, p.x + (int64_t)q * p.K, red[q][ksp]);
+            if (lane == 0 && ksp == 0) s_e[q] = eb;
         }
         __syncthreads();
-        if (tid == 0) s_last = atomicAdd(&p.counters[u], 1) == p.slots - 1;
-        __syncthreads();
-        if (s_last && tid < kMoeCols) {
-            __threadfence();
-            const int col = u * kMoeCols + tid;
-            if (col < p.N) {
-                float v = 0.f;
-                for (int sl = 0; sl < p.slots; sl += 8) {  // (eight loads in flight; added in slot order)
-                    float part[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        part[j] = sl + j < p.slots && moe_id(p, sl + j) < (uint32_t)p.E ? __ldcg(p.part + (int64_t)(sl + j) * p.npad + col) : 0.f;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v += part[j];
-                }
-                p.out[col] = f32_to_bf16_bits(v);
+        if (tid < 16) {
+            float v = 0.f;
+            for (int q = 0; q < p.slots; ++q) {  // (in slot order)
+                float s = red[q][0][tid] + red[q][1][tid];
+                if constexpr (FMT == TKD_BFP4) s = moe_scale(s, max(s_e[q], 0));
+                v += s_e[q] >= 0 ? s : 0.f;
             }
-            if (tid == 0) p.counters[u] = 0;
+            p.out[u * 16 + tid] = f32_to_bf16_bits(v);
         }
     }
 }
@@ -333,15 +333,18 @@ __global__ void __launch_bounds__(32) tkd_moe_route_kernel(const RouteParams p) 
 }
 
 template <int FMT, bool DOWN>
-int moe_launch(const MoeParams& p, dim3 grid, cudaStream_t st) {
+int moe_launch(const MoeParams& p, cudaStream_t st) {
     auto kern = tkd_moe_kernel<FMT, DOWN>;
-    const size_t smem = (size_t)((p.K + 63) & ~63) * 2 + kMoeSplit * kMoeCols * sizeof(float);
+    const int room = 200 * 1024 / (2 * kMoeHalfBytes<FMT>), most = room < 16 ? room : 16;  // warps of down: a run each, if they fit
+    const int warps = DOWN ? (p.slots * kMoeSplit < most ? p.slots * kMoeSplit : most) : 2 * kMoeSplit;
+    const size_t smem = (size_t)warps * 2 * kMoeHalfBytes<FMT>;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid, cfg.blockDim = dim3(kMoeThreads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+    cfg.gridDim = DOWN ? dim3((unsigned)(p.N / 16)) : dim3((unsigned)(p.N / 32), (unsigned)p.slots);
+    cfg.blockDim = dim3(warps * 32), cfg.dynamicSmemBytes = smem, cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -376,6 +379,7 @@ MoeParams moe_params(const TkdMoe* a) {
     p.rw = static_cast<const uint16_t*>(a->route_w);
     p.slots = a->slots, p.act = a->act, p.bias = static_cast<const uint16_t*>(a->bias);
     p.out = static_cast<uint16_t*>(a->out);
+    p.status = a->status;
     p.mul16 = 16, p.mul128 = 128;
     return p;
 }
@@ -436,14 +440,9 @@ int moe_rows(const TkdMoe* a, cudaStream_t st) {
 
 template <bool DOWN>
 int moe_one(const TkdMoe* a, cudaStream_t st) {
-    MoeParams p = moe_params(a);
-    if ((int64_t)((p.K + 63) & ~63) * 2 > 224 * 1024) return TKD_ERR_UNSUPPORTED;  // (the row in shared memory)
-    if (DOWN) {
-        p.counters = static_cast<int*>(a->workspace);
-        p.part = reinterpret_cast<float*>(static_cast<uint8_t*>(a->workspace) + moe_rows_counters(a, true));
-    }
-    const dim3 grid((unsigned)((DOWN ? p.npad : p.N) / kMoeCols), (unsigned)a->slots);
-    const int e = a->fmt == TKD_FMT_BF16 ? moe_launch<TKD_BF16, DOWN>(p, grid, st) : moe_launch<TKD_BFP4, DOWN>(p, grid, st);
+    const MoeParams p = moe_params(a);
+    if (p.K > 112 * 1024) return TKD_ERR_UNSUPPORTED;
+    const int e = a->fmt == TKD_FMT_BF16 ? moe_launch<TKD_BF16, DOWN>(p, st) : moe_launch<TKD_BFP4, DOWN>(p, st);
     return e == 0 ? TKD_OK : TKD_ERR_CUDA + e;
 }
 

@@ -439,8 +439,9 @@ class _Op:
         if gu:
             a.act, a.bias = ACTS[act], P["gu_bias_t"].data_ptr() if P["gu_bias"] else None
         need = ctypes.c_uint64(0)
+        a.status = linear.status_word(P["_device"]).data_ptr()
         if by_union:
-            a.out_rows, a.status = TILE, linear.status_word(P["_device"]).data_ptr()
+            a.out_rows = TILE
             _tkd.check(_tkd.lib().tkd_moe_rows_workspace(ctypes.byref(a), int(not gu), ctypes.byref(need)), "tkd_moe_rows_workspace")
         elif not gu:
             _tkd.check(_tkd.lib().tkd_moe_workspace(ctypes.byref(a), ctypes.byref(need)), "tkd_moe_workspace")

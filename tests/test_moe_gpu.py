@@ -484,3 +484,26 @@ def test_rows_at_the_edges_of_their_tiles(device, e, h, i, k, rows, bad, kblock)
     if u:
         check("h without a workspace", host(bare, th.shape[-1])[:rows, : len(u) * i], want_h, rel=REL)
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("experts,h,i,k", [(4, 64, 32, 1), (8, 96, 32, 3), (12, 1056, 480, 12), (16, 2560, 1216, 16)])
+def test_one_row_runs_of_every_length(device, experts, h, i, k):
+    """One token where a warp's run of super-atoms is short (one, or none for the second half of K), ends inside a super-atom, fills its
+    buffer to the byte or goes through it several times, and with more slots than down has warps: against the oracle, twice the same."""
+    g = torch.Generator().manual_seed(h + i)
+    on_grid = lambda t: torch.from_numpy(  # noqa: E731
+        moe8.bfp4_values(moe8.bfp4_tiles(t)).transpose(0, 2, 1, 3).reshape(t.shape[0], t.shape[1]).copy())
+    gu = torch.stack([on_grid(torch.randn(h, 2 * i, generator=g) * 0.05) for _ in range(experts)])
+    dn = torch.stack([on_grid(torch.randn(i, h, generator=g) * 0.05) for _ in range(experts)])
+    P = moe8.pack(device, gu, dn)
+    x = torch.randn(1, h, generator=g).to(torch.bfloat16)
+    ids = torch.randperm(experts, generator=g)[:k].to(torch.int16)
+    w = torch.rand(k, generator=g).to(torch.bfloat16)
+    put = lambda t, d: ttnn.from_torch(t.reshape(1, 1, *t.shape), dtype=d, layout=ttnn.TILE_LAYOUT, device=device)  # noqa: E731
+    tx, tid, tw = put(x, ttnn.bfloat16), put(ids.reshape(1, k), ttnn.uint16), put(w.reshape(1, k), ttnn.bfloat16)
+    ys = [ttnn.to_torch(moe8.down(moe8.gate_up(tx, P, tid, tw, k), P, tid, k)).double().reshape(1, -1)[:, :h] for _ in range(2)]
+    want, _ = orc.moe_reference(x.float().numpy(), gu.numpy(), dn.numpy(), ids.tolist(), w.float().numpy())
+    want = torch.from_numpy(want).double()
+    assert torch.equal(ys[0], ys[1])
+    assert ((ys[0] - want).norm() / want.norm()).item() < 1e-2
+    linear.check_status(device)
