@@ -421,12 +421,18 @@ __global__ void __launch_bounds__(pack_threads(SCALE)) tkd_pack_weight_kernel(co
                         both[i] = __vmaxu2(w[0], w[1]);
 #pragma unroll
                         for (int o = 4; o < 32; o <<= 1) both[i] = __vmaxu2(both[i], __shfl_xor_sync(0xFFFFFFFFu, both[i], o));
-                        both[i] &= 0x7F807F80u;
                         // an exponent of 1 to 7, or of 255, leaves pack_pair's scale outside the normal numbers; (own scales)
-                        // one below 100 may come of a quotient that was not exact
-                        const uint32_t e0 = both[i] & 0xFFFFu, e1 = both[i] >> 16, low = SCALE == 2 ? 100u << 7 : 8u << 7;
-                        const uint32_t from = SCALE == 2 ? 0u : 1u;
-                        odd |= (e0 - from < low - from) | (e1 - from < low - from) | (e0 == 0x7F80u) | (e1 == 0x7F80u);
+                        // one below 100 may come of a quotient that was not exact, unless the largest upper half is zero: then all
+                        // are zeros by the rule, exact or not. (As they counted among the others, the columns that pad N to a
+                        // panel's 128 took the division for every number: [2912, 1376] to bfloat8_b 20.5 us for 8.9 without scales.)
+                        if constexpr (SCALE == 2) {
+                            const uint32_t z0 = both[i] & 0xFFFFu, z1 = both[i] >> 16, low = 100u << 7;
+                            odd |= (z0 - 1u < low - 1u) | (z1 - 1u < low - 1u);
+                        }
+                        both[i] &= 0x7F807F80u;
+                        const uint32_t e0 = both[i] & 0xFFFFu, e1 = both[i] >> 16, low = 8u << 7;
+                        if constexpr (SCALE != 2) odd |= (e0 - 1u < low - 1u) | (e1 - 1u < low - 1u);
+                        odd |= (e0 == 0x7F80u) | (e1 == 0x7F80u);
                     }
                     return __any_sync(0xFFFFFFFFu, odd) != 0;
                 };

@@ -790,3 +790,23 @@ def test_linear_silu_in_the_output_stage(device, fmt, m, k, n):
 def test_items_of_one_to_four_slices_equal_the_counted_kernel(device, dtype, k, m):
     """The same for one to three slices, and for four whose last is short: every K of up to 16384 runs as items of 32 columns."""
     test_plain_calls_equal_the_counted_kernels(device, dtype, k, m)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("n", [16, 112, 144])
+def test_own_scales_with_zero_and_tiny_inputs(device, fmt, n):
+    """Columns divided by their own scales where inputs are zero, denormal or near it: quotients that are no normal numbers, or come
+    of a shared exponent below 100, are the division's, and zeros are zeros, also in the columns that pad N to a panel. Bit for bit
+    the oracle's."""
+    g = torch.Generator().manual_seed(n)
+    k = 128
+    w = torch.randn(n, k, generator=g) * 0.1
+    for i, size in enumerate((0.0, 1e-45, 3e-42, 2e-39, 1.2e-38, 1e-37, 1e-36, 1e-33, 1e-30, 1e-20, 1e-10)):
+        w[:, 3 * i] = torch.randn(n, generator=g) * size
+    w[:, 40] = torch.where(torch.arange(n) % 16 == 3, torch.randn(n, generator=g) * 1e-39, torch.zeros(n))
+    w[5] = 0.0
+    tw, ts = linear.native_weight(device, w, DT[fmt], col_scale=True)
+    want, scale = orc.native_values(w, fmt, col_scale=True)
+    assert torch.equal(ttnn.to_torch(ts).float().reshape(-1), torch.as_tensor(scale).float().reshape(-1))
+    held = ttnn.to_torch(tw).float().reshape(k, -1)[:, :n]
+    assert torch.equal(held, torch.from_numpy(want))
