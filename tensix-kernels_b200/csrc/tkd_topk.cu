@@ -165,10 +165,65 @@ __device__ __forceinline__ void pick_rounds(const uint32_t (&word)[N], const uin
     }
 }
 
+// The same by counting, for up to kPickSlots slots of up to kPickRecs records: a slot's place among the best is the number of
+// slots before it, and only the `top` records whose best slots are the best of all can hold one of the best. Four threads a record,
+// then a slot, no chain of rounds: as `top` rounds of maxima in every warp and again over the warps' lists the pick of 16
+// from 19 records of 8 took 11.7 us of a launch (2 rows, 37888 columns), 8.2 now; the rest is the rescore, rows of the head at
+// random places in its memory. word: rank << 32 | ~place (0: empty), id: the slots' in shared memory.
+constexpr int kPickSlots = 2048, kPickRecs = 512;
+struct PickCount {
+    unsigned long long word[kPickSlots], most[kPickRecs];
+    uint32_t id[kPickSlots];
+    int kept[32], nkept;
+};
+__device__ __forceinline__ void pick_count(PickCount& s, int nrec, int k, int top, int tid, uint32_t* cid, int* held) {
+    constexpr int T = kPickWarps * 32, G = T / 4;
+    const int sub = tid & 3;
+    auto before = [&](const unsigned long long* w, int n, unsigned long long mine) {  // (by four threads together)
+        int c = 0;
+#pragma unroll 4
+        for (int i = sub; i < n; i += 4) c += w[i] > mine;
+        c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
+        return c + __shfl_xor_sync(0xFFFFFFFFu, c, 2);
+    };
+    for (int b = 0; b < nrec; b += G) {
+        const int rec = b + (tid >> 2);
+        unsigned long long m = 0;
+        for (int q = sub; rec < nrec && q < k; q += 4) m = max(m, s.word[rec * k + q]);
+        m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+        m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
+        if (sub == 0 && rec < nrec) s.most[rec] = m;
+    }
+    if (tid == 0) s.nkept = *held = 0;
+    __syncthreads();
+    for (int b = 0; b < nrec; b += G) {
+        const int rec = b + (tid >> 2);
+        const unsigned long long m = rec < nrec ? s.most[rec] : 0ull;
+        const int c = before(s.most, nrec, m);
+        if (sub == 0 && m && c < top) s.kept[c] = rec, atomicAdd(&s.nkept, 1);
+    }
+    __syncthreads();
+    // (the kept records' slots, in place of the records' maxima)
+    const int n = s.nkept * k;
+    for (int b = 0; b < n; b += G) {
+        const int i = b + (tid >> 2), at = i < n ? s.kept[i / k] * k + i % k : 0;
+        const unsigned long long m = i < n ? s.word[at] : 0ull;
+        int c = 0;
+        for (int j = 0; j < s.nkept; ++j) {
+            const unsigned long long* w = s.word + s.kept[j] * k;
+#pragma unroll 2
+            for (int q = sub; q < k; q += 4) c += w[q] > m;
+        }
+        c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
+        c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
+        if (sub == 0 && m && c < top) cid[c] = s.id[at], atomicAdd(held, 1);
+    }
+}
+
 // One CTA per row r of the step.
 //   1. The best `top` slots of row r over the records in order (record by record, slot by slot), by key (RECORDS: by
-//      rank16, and top is 1); an equal key keeps the earlier slot; a slot with key 0 or an id at or past `vocab` is empty. A
-//      warp takes a run of slots, 256 at a time beside its best so far; one warp merges the warps' lists.
+//      rank16, and top is 1); an equal key keeps the earlier slot; a slot with key 0 or an id at or past `vocab` is empty: by
+//      counting (COUNT: pick_count), or a warp takes a run of slots, 256 at a time beside its best so far; one warp merges the warps' lists.
 //   2. (not RECORDS) Their exact logits: bf16 x row times the candidates' bf16 head rows, float32 sums (a warp per
 //      candidate: every lane sums its 8-element pieces in order, then a shuffle tree), rounded to bf16 with `round`.
 //   3. The pick: the largest logit (order32), the lowest id among equals. Row r of out (32 words):
@@ -176,56 +231,76 @@ __device__ __forceinline__ void pick_rounds(const uint32_t (&word)[N], const uin
 //      valid slots). No valid slot: [0, 0xFFFFFFFF, 0].
 // Bound by latency: as `top` rounds over all slots read anew, with two barriers each, and one candidate after the other, it
 // took a fifth of a vocabulary's call.
-template <bool RECORDS>
+template <bool RECORDS, bool COUNT>
 __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const uint32_t* __restrict__ records, int nrec, int rows,
                                                                         int k, int top, uint32_t vocab,
                                                                         const uint16_t* __restrict__ x, int64_t ldx, int dim,
                                                                         const uint16_t* __restrict__ head, int64_t ld_head,
                                                                         int round, const uint32_t* __restrict__ tmap,
                                                                         uint32_t* __restrict__ out, uint32_t* __restrict__ ids_out) {
-    __shared__ uint32_t srank[kPickWarps][32], sid[kPickWarps][32], cid[32], clogit[32];
+    __shared__ uint32_t srank[COUNT ? 1 : kPickWarps][32], sid[COUNT ? 1 : kPickWarps][32], cid[32], clogit[32];
+    extern __shared__ __align__(16) uint8_t pick_smem[];
     __shared__ int held, nvalid[kPickWarps];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = nrec * k, per = (n + kPickWarps - 1) / kPickWarps, c1 = min(n, (warp + 1) * per);
-    uint32_t rank = 0, id = 0;  // lane t: the t-th so far
+    const int n = nrec * k;
     int mine = 0;
-    for (int c0 = warp * per; c0 < c1; c0 += 32 * kPickOwn) {
-        uint32_t word[kPickOwn + 1], ids[kPickOwn + 1];
+    if constexpr (COUNT) {
+        PickCount& pc = *reinterpret_cast<PickCount*>(pick_smem);
+#pragma unroll 4
+        for (int c = tid; c < n; c += kPickWarps * 32) {
+            const int rec = c / k, q = c - rec * k;
+            const uint32_t* page = records + (size_t)rec * 2 * rows * k;
+            const uint32_t key = __ldg(page + r * k + q) & 0xFFFFu, id = __ldg(page + (rows + r) * k + q);
+            const bool ok = key && id < vocab;
+            mine += ok;
+            pc.id[c] = id;
+            pc.word[c] = ok ? (unsigned long long)(RECORDS ? rank16(key) : key) << 32 | (0xFFFFFFFFu - (uint32_t)c) : 0ull;
+        }
+        mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+        if (lane == 0) nvalid[warp] = mine;
+        __syncthreads();
+        pick_count(pc, nrec, k, top, tid, cid, &held);
+    } else {
+        const int per = (n + kPickWarps - 1) / kPickWarps, c1 = min(n, (warp + 1) * per);
+        uint32_t rank = 0, id = 0;  // lane t: the t-th so far
+        for (int c0 = warp * per; c0 < c1; c0 += 32 * kPickOwn) {
+            uint32_t word[kPickOwn + 1], ids[kPickOwn + 1];
 #pragma unroll
-        for (int j = 0; j < kPickOwn; ++j) {
-            const int c = c0 + 32 * j + lane;
-            word[j] = ids[j] = 0;
-            if (c < c1) {
-                const int rec = c / k, q = c - rec * k;
-                const uint32_t* page = records + (size_t)rec * 2 * rows * k;
-                const uint32_t key = __ldg(page + r * k + q) & 0xFFFFu;
-                ids[j] = __ldg(page + (rows + r) * k + q);
-                if (key && ids[j] < vocab) {
-                    word[j] = (RECORDS ? rank16(key) : key) << 12 | (uint32_t)(4095 - 32 - 32 * j - lane);
-                    ++mine;
+            for (int j = 0; j < kPickOwn; ++j) {
+                const int c = c0 + 32 * j + lane;
+                word[j] = ids[j] = 0;
+                if (c < c1) {
+                    const int rec = c / k, q = c - rec * k;
+                    const uint32_t* page = records + (size_t)rec * 2 * rows * k;
+                    const uint32_t key = __ldg(page + r * k + q) & 0xFFFFu;
+                    ids[j] = __ldg(page + (rows + r) * k + q);
+                    if (key && ids[j] < vocab) {
+                        word[j] = (RECORDS ? rank16(key) : key) << 12 | (uint32_t)(4095 - 32 - 32 * j - lane);
+                        ++mine;
+                    }
                 }
             }
+            word[kPickOwn] = rank ? rank << 12 | (uint32_t)(4095 - lane) : 0u, ids[kPickOwn] = id;
+            pick_rounds(word, ids, top, lane, rank, id);
         }
-        word[kPickOwn] = rank ? rank << 12 | (uint32_t)(4095 - lane) : 0u, ids[kPickOwn] = id;
-        pick_rounds(word, ids, top, lane, rank, id);
-    }
-    srank[warp][lane] = rank, sid[warp][lane] = id;
-    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
-    if (lane == 0) nvalid[warp] = mine;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t word[kPickWarps], ids[kPickWarps];
+        srank[warp][lane] = rank, sid[warp][lane] = id;
+        mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+        if (lane == 0) nvalid[warp] = mine;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t word[kPickWarps], ids[kPickWarps];
 #pragma unroll
-        for (int w = 0; w < kPickWarps; ++w) {
-            const uint32_t rk = srank[w][lane];
-            word[w] = rk ? rk << 12 | (uint32_t)(4095 - 32 * w - lane) : 0u, ids[w] = sid[w][lane];
+            for (int w = 0; w < kPickWarps; ++w) {
+                const uint32_t rk = srank[w][lane];
+                word[w] = rk ? rk << 12 | (uint32_t)(4095 - 32 * w - lane) : 0u, ids[w] = sid[w][lane];
+            }
+            pick_rounds(word, ids, top, lane, rank, id);
+            cid[lane] = id;
+            const uint32_t any = __ballot_sync(0xFFFFFFFFu, rank != 0);
+            if (lane == 0) held = __popc(any);
         }
-        pick_rounds(word, ids, top, lane, rank, id);
-        cid[lane] = id;
-        const uint32_t any = __ballot_sync(0xFFFFFFFFu, rank != 0);
-        if (lane == 0) held = __popc(any);
     }
     __syncthreads();
     const int nc = held;
@@ -234,7 +309,7 @@ __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const ui
         for (int c = warp; c < nc; c += kPickWarps) {
             const uint16_t* wr = head + (size_t)cid[c] * ld_head;
             float acc = 0.f;
-#pragma unroll 8
+#pragma unroll 16
             for (int d = lane * 8; d < dim; d += 256) {
                 const uint4 wv = __ldg(reinterpret_cast<const uint4*>(wr + d));
                 const uint4 xv = __ldg(reinterpret_cast<const uint4*>(xr + d));
@@ -272,8 +347,8 @@ __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const ui
     }
 }
 
-template <bool RECORDS>
-int launch_pick(const uint32_t* records, int nrec, int rows, int k, int top, uint32_t vocab, const uint16_t* x, int64_t ldx,
+template <bool RECORDS, bool COUNT>
+int launch_pick_by(const uint32_t* records, int nrec, int rows, int k, int top, uint32_t vocab, const uint16_t* x, int64_t ldx,
                 int dim, const uint16_t* head, int64_t ld_head, int round, const uint32_t* tmap, uint32_t* out,
                 uint32_t* ids_out, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
@@ -285,8 +360,14 @@ int launch_pick(const uint32_t* records, int nrec, int rows, int k, int top, uin
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, tkd_head_pick_kernel<RECORDS>, records, nrec, rows, k, top, vocab, x, ldx, dim, head,
+    cfg.dynamicSmemBytes = COUNT ? sizeof(PickCount) : 0;
+    return (int)cudaLaunchKernelEx(&cfg, tkd_head_pick_kernel<RECORDS, COUNT>, records, nrec, rows, k, top, vocab, x, ldx, dim, head,
                                    ld_head, round, tmap, out, ids_out);
+}
+template <bool RECORDS, class... A>
+int launch_pick(const uint32_t* records, int nrec, int rows, int k, A... more) {
+    return nrec <= kPickRecs && (int64_t)nrec * k <= kPickSlots ? launch_pick_by<RECORDS, true>(records, nrec, rows, k, more...)
+                                                              : launch_pick_by<RECORDS, false>(records, nrec, rows, k, more...);
 }
 
 }  // namespace

@@ -241,3 +241,32 @@ def test_pick_takes_the_earliest_of_equal_keys(device, nrec, rows, k, top):
         want = cand[z == z.max()].min()
         assert (int(tok[t]), int(best[t]), int(count[t])) == (want, cand[0], len(cand)), t
         assert (int(rtok[t]), int(rcount[t])) == (ids[order][0], len(order)), t
+
+
+@pytest.mark.parametrize("nrec,rows,k,top", [(1, 1, 4, 1), (3, 2, 4, 32), (75, 1, 8, 16), (300, 3, 4, 9), (512, 1, 4, 32), (513, 2, 2, 16), (300, 2, 8, 32)])
+def test_picks_from_records_with_ties_and_holes(device, nrec, rows, k, top):
+    """The best slots of arbitrary records (few distinct keys, empty slots, ids past the vocabulary, a record's slots in no order), by
+    counting and, past 2048 slots or 512 records, in rounds: the first candidate and how many are held, and the pick among their
+    exact logits, as numpy finds them."""
+    g = np.random.default_rng(nrec + k)
+    dim, vocab = 64, 4000
+    keys = g.integers(0x8000, 0x8000 + 60, (nrec, rows, k)).astype(np.uint32)
+    keys[g.random(keys.shape) < 0.2] = 0
+    ids = g.integers(0, vocab + 400, (nrec, rows, k)).astype(np.uint32)
+    rec = np.stack([keys, ids], axis=1).reshape(1, 1, nrec, 2 * rows * k)
+    tr = ttnn.from_torch(torch.from_numpy(rec.view(np.int32)), dtype=ttnn.uint32, layout=ttnn.ROW_MAJOR_LAYOUT, device=device)
+    head = torch.from_numpy(g.standard_normal((vocab, dim))).float().bfloat16()
+    x = torch.from_numpy(g.standard_normal((rows, dim))).float().bfloat16()
+    tx = ttnn.from_torch(x.reshape(1, 1, rows, dim), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
+    exact = x.double() @ head.double().T
+    tok, first, count = head_pick.tokens(head_pick.pick(tr, tx, head_pick.head_rows(device, head), rows, k, top=top, logits="float32"), rows)
+    best, own, valid = head_pick.tokens(head_pick.pick_records(tr, rows, k, vocab), rows)
+    for r in range(rows):
+        kk, ii = keys[:, r].reshape(-1).astype(np.int64), ids[:, r].reshape(-1).astype(np.int64)
+        ok = (kk > 0) & (ii < vocab)
+        order = np.lexsort((np.arange(kk.size), -kk, ~ok))[: min(top, int(ok.sum()))]
+        assert int(count[r]) == len(order) and int(valid[r]) == int(ok.sum())
+        if len(order):
+            assert int(first[r]) == ii[order[0]] == int(own[r]) == int(best[r])
+            logits = exact[r, torch.from_numpy(ii[order])]
+            assert int(tok[r]) in ii[order] and float(exact[r, int(tok[r])]) >= float(logits.max()) - 1e-4
