@@ -176,6 +176,7 @@ class Weight(Tensor):
         self.wide = self.fmt != FMT[dtype]
         self.serial = next(Weight._serials)
         self.calls = {}  # dense_reader.linear's described calls on this weight
+        self.short = {}  # ... those of linear.linear without options, by its own arguments
         sp = memory_config.shard_spec
         self._npad = sp.shape[1] * sp.banks if sp else _pad(n)
 
@@ -333,6 +334,7 @@ def deallocate(t):
         t.emax = None
         t._bf16_twin = None
         t.calls.clear()
+        t.short.clear()
 
 
 def reshape(t, shape):

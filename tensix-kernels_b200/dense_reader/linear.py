@@ -705,7 +705,10 @@ class _Call:
         """Launch: the output's torch tensor (a new one where out is None)."""
         res = None if residual is None else residual.t
         if self.single is not None:
-            return self.launch(self.single, x.t, None if out is None else out.t, res, _workspace(self.device, self.need), 0)
+            ws = _WORKSPACE.get((self.device.id, WORKSPACE_SLOT))
+            if ws is None or ws.numel() < self.need:
+                ws = _workspace(self.device, self.need)
+            return self.launch(self.single, x.t, None if out is None else out.t, res, ws, 0)
         device = self.device
         if out is None:
             a = self.launches[0][1]
@@ -884,10 +887,14 @@ def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **o
     (applied after the matmul), "swiglu" or "geglu" (w is interleave_glu's weight with scale None, the output N / 2
     wide; or w is (gate, up), the output N wide). out_dtype ttnn.float32: out32. A block list for w: plain weights with
     activation None, (gate, up) pairs with "swiglu" or "geglu". opts go to matmul. (linear.py:1073-1124)"""
-    if (activation is None and out_dtype is None and type(w) is ttnn.Weight and x.t.dim() == 4
-            and x._mc.memory_layout is ttnn.TensorMemoryLayout.INTERLEAVED):
-        return matmul(x, w, scale, memory_config=memory_config, **opts)
-    shape = list(x.shape)
+    key = None
+    if type(w) is ttnn.Weight and not opts and CACHE and x.t.dim() == 4 and (activation is None or type(activation) is str):
+        # (a call without options that this weight keeps, found by linear's own arguments: what matmul would find, without its way there)
+        key = (x.t.shape, id(scale), activation, out_dtype, KS, MAX_CTAS, dev.MAX_BANKS)
+        call = w.short.get(key)
+        if call is not None and call.fits(x, None):
+            return ttnn.Tensor(call.run(x, None, None), call.out_dtype, ttnn.TILE_LAYOUT, call.device, memory_config)
+    weight, shape = w, list(x.shape)
     glu_kinds = {"swiglu": 0, "geglu": 1}
     if out_dtype not in (None, ttnn.bfloat16):
         assert out_dtype == ttnn.float32, f"dense_reader.linear: out_dtype {out_dtype}"
@@ -919,7 +926,15 @@ def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **o
     # silu of a plain product into a new tensor: the kernel's output stage, on the float32 sums (as three elementwise kernels behind
     # the matmul it took 14 of a call's 26 us; a given out holds the product itself, and a residual is added before the activation)
     fused = activation == "silu" and not opts.keys() - _SILU_OPTS and type(w) is ttnn.Weight
-    y = matmul(x4, w, scale, memory_config=memory_config, **opts, **({_SILU: True} if fused else {}))
+    if fused:
+        opts = {**opts, _SILU: True}
+    y = matmul(x4, w, scale, memory_config=memory_config, **opts)
+    if key is not None and x4 is x:
+        call = weight.calls.get(_call_key(x, w, scale, None, None, 0, None, None, "hifi2", opts)[1])
+        if call is not None:
+            if len(weight.short) >= _WEIGHT_CALLS:
+                weight.short.clear()
+            weight.short[key] = call
     if activation is not None and activation not in ("swiglu", "geglu") and not fused:
         assert activation == "silu", f"dense_reader.linear: activation {activation!r}"
         y = ttnn.silu(y)

@@ -339,3 +339,37 @@ def test_the_log_and_the_plans_are_of_what_runs(ran, monkeypatch, capsys):
         linear.matmul(x, w, None, kb=3)
     linear.matmul(x, w, None, fixed_sums=True)
     assert len(linear._CHOICE) == 2 and "ctas" in capsys.readouterr().out
+
+
+def test_linears_own_arguments_find_the_kept_call(ran, monkeypatch):
+    """linear.linear without options goes straight to the call its weight keeps: the same one for the same arguments, another for
+    another scale, activation, output type, shape or setting, none of a freed or moved tensor's; the described calls stay 64."""
+    w, x = weight(64, 128), tensor(1, 1, 3, 64)
+    scales = [ttnn.Tensor(torch.ones(1, 1, 1, 128, dtype=torch.bfloat16), ttnn.bfloat16, ttnn.TILE_LAYOUT, DEVICE, None) for _ in range(2)]
+    seen = []
+    for args in ({"scale": None}, {"scale": scales[0]}, {"scale": scales[1]}, {"scale": None, "activation": "silu"},
+                 {"scale": None, "activation": "swiglu"}, {"scale": None, "out_dtype": ttnn.float32}, {"scale": scales[0], "activation": "silu"}):
+        for _ in range(3):
+            linear.linear(x, w, **args)
+        assert ran[-1] is ran[-2] is ran[-3] and ran[-1] not in seen
+        seen.append(ran[-1])
+    assert ran[-1].launches[0][1].epilogue == _tkd.EPI_SILU and len(w.calls) == len(w.short) == len(seen)
+    linear.linear(tensor(1, 1, 4, 64), w, None)
+    assert ran[-1] not in seen
+    monkeypatch.setattr(linear, "MAX_CTAS", 5)
+    linear.linear(x, w, None)
+    assert ran[-1] not in seen and ran[-1].launches[0][1].max_ctas == 5
+    monkeypatch.setattr(linear, "MAX_CTAS", None)
+    linear.linear(x, w, scales[0])
+    assert ran[-1] is seen[1]
+    scales[0].t = torch.ones(1, 1, 1, 256, dtype=torch.bfloat16)[..., :128]  # (moved; some tensor freed)
+    monkeypatch.setattr(ttnn, "EPOCH", ttnn.EPOCH + 1)
+    linear.linear(x, w, scales[0])
+    assert ran[-1] not in seen and ran[-1].launches[0][1].scale == scales[0].t.data_ptr()
+    with pytest.raises(AssertionError):
+        linear.linear(x, w, None, activation="relu")
+    with pytest.raises(AssertionError):
+        linear.linear(x, w, None, out_dtype=ttnn.uint32)
+    for m in range(1, 2 * linear._WEIGHT_CALLS):
+        linear.linear(tensor(1, 1, m, 64), w, None)
+    assert len(w.calls) <= linear._WEIGHT_CALLS and len(w.short) <= linear._WEIGHT_CALLS
