@@ -507,3 +507,50 @@ def test_one_row_runs_of_every_length(device, experts, h, i, k):
     assert torch.equal(ys[0], ys[1])
     assert ((ys[0] - want).norm() / want.norm()).item() < 1e-2
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("rows,k", [(9, 2), (16, 3), (24, 3), (32, 3)])
+def test_rows_of_experts_few_and_many_chose(device, rows, k):
+    """gate_up_rows where an expert is chosen by one row, by eight, by nine and by all of them (up to eight are multiplied alone), the
+    rows anywhere: h against float64 within bf16's rounding of float32 sums, exact zeros where a row did not choose, and nothing of a row
+    of NaNs in the others."""
+    E, H, I = 8, 1056, 96
+    g = torch.Generator().manual_seed(rows)
+    on_grid = lambda t: torch.from_numpy(  # noqa: E731
+        moe8.bfp4_values(moe8.bfp4_tiles(t)).transpose(0, 2, 1, 3).reshape(t.shape[0], t.shape[1]).copy())
+    gu = torch.stack([on_grid(torch.randn(H, 2 * I, generator=g) * 0.05) for _ in range(E)])
+    dn = torch.stack([on_grid(torch.randn(I, H, generator=g) * 0.05) for _ in range(E)])
+    P = moe8.pack(device, gu, dn)
+    order = torch.randperm(rows, generator=g)
+    ids = torch.zeros(rows, k, dtype=torch.int64)
+    ids[:, 0] = 5                                # all rows
+    ids[:, 1] = 1
+    ids[order[:8], 1] = 3                        # eight rows; the others expert 1
+    if k > 2:
+        ids[:, 2] = 6
+        ids[order[-9:], 2] = 0                   # nine rows
+        ids[order[0], 2] = 7                     # one row
+    w = (0.5 + torch.rand(rows, k, generator=g)).to(torch.bfloat16)
+    x = torch.randn(rows, H, generator=g).to(torch.bfloat16)
+    bad = int(order[3])
+    x[bad] = float("nan")
+    put = lambda t, d: ttnn.from_torch(t.reshape(1, 1, *t.shape), dtype=d, layout=ttnn.TILE_LAYOUT, device=device)  # noqa: E731
+    tid = put(ids.to(torch.int16), ttnn.uint16)
+    h = ttnn.to_torch(moe8.gate_up_rows(put(x, ttnn.bfloat16), P, tid, put(w, ttnn.bfloat16), k, rows)).double().reshape(32, -1)
+    union = sorted(set(ids.reshape(-1).tolist()))
+    for q, e in enumerate(union):
+        for r in range(rows):
+            got = h[r, q * I : (q + 1) * I]
+            at = (ids[r] == e).nonzero().reshape(-1)
+            if not len(at):
+                assert r == bad or not got.any(), (q, r)
+                continue
+            if r == bad:
+                assert got.isnan().all()
+                continue
+            xr = x[r].double()
+            up, gate = gu[e].double()[:, :I], gu[e].double()[:, I:]
+            want = torch.nn.functional.silu(xr @ gate) * (xr @ up) * float(w[r, at[0]])
+            assert ((got - want).norm() / want.norm()).item() < 6e-3, (q, r)
+    assert not h[rows:].any()
+    linear.check_status(device)
