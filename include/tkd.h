@@ -278,8 +278,8 @@ typedef struct {
     void* out;               /* bf16 [rows, ldo]. gate_up: slot q's I values at q * I, each routing weight * act(x G +
                                 b) * (x U + b); down: the n columns of y = sum over the slots of h_q @ D_q */
     int64_t ldo;
-    void* workspace;         /* down: tkd_moe_workspace bytes, zeroed once by the caller before the first use (the kernel
-                                returns its counters to zero); calls that share one must be ordered on one stream. by_union:
+    void* workspace;         /* down: tkd_moe_workspace bytes, zeroed once by the caller before the first use (one row: asked
+                                for, not used); calls that share one must be ordered on one stream. by_union:
                                 tkd_moe_rows_workspace bytes, for gate_up too (one of its own; with none, or too little, its
                                 work is spread over the SMs less evenly; down then runs fewer CTAs) */
     uint64_t workspace_bytes;
@@ -293,7 +293,7 @@ typedef struct {
 int tkd_moe_workspace(const TkdMoe* a, uint64_t* bytes);
 /* The workspace of a by_union call of gate_up (down 0) or down, whatever its slots: for a->experts, n and rows. */
 int tkd_moe_rows_workspace(const TkdMoe* a, int down, uint64_t* bytes);
-/* TKD_ERR_UNSUPPORTED: one row of k_in inputs does not fit in shared memory (by_union: never). */
+/* TKD_ERR_UNSUPPORTED: one row of more than 114688 inputs (by_union: never). */
 int tkd_moe_gate_up(const TkdMoe* a, void* stream);
 int tkd_moe_down(const TkdMoe* a, void* stream);
 /* The router's top k and their weights, into the ids and weights the ops above read: stands in for moe8.route

@@ -246,7 +246,7 @@ __global__ void tkd_unpack_kernel(int fmt, int64_t K, int64_t npad, const uint8_
 // col_scale), found by a first walk over the CTA's 16 columns, whose second reading then comes from L2, and written out.
 // Bound: HBM. [14336, 4096] float32 to bfloat4_b (235 MB in, 33 MB out): tkd_quantise, the emax and the permute pass 410 us
 // together (1 byte a weight of codes written and read back, uncoalesced loads of the [N, K] matrix); here 54 us without
-// column scales (5.0 TB/s), 88 with its own.
+// column scales (5.0 TB/s), 84 with its own.
 // threads of a CTA: with the columns' own scales two large CTAs an SM (77 MB of the matrix between the two readings: it stays
 // in the 126 MB L2), else as many as fit
 __host__ __device__ constexpr int pack_threads(int scale) { return scale == 2 ? 512 : 256; }

@@ -4,7 +4,7 @@
 // over an MMA warp to output warps, and unless K makes four slices a panel's sums through L2; and it brings every tile of x for every
 // panel anew. Where x fits in shared memory, mma.sync on weights in registers does without all of that: 16 rows of bfloat8_b,
 // [2048, 4096] 7.8 us before, 5.5 now (1.4 at the memory's rate), bfloat4_b [1280, 4096] 7.6 and 5.0. What bounds it on large weights is
-// instruction issue: some 30 warp instructions for 256 weights and 16 rows. rows_layout (tkd_api.cu) says where which kernel runs.
+// instruction issue: 39 warp instructions for 256 weights and 16 rows, issue active in 0.56 of the cycles (bfloat8_b [2048, 28672]). rows_layout (tkd_api.cu) says where which kernel runs.
 //
 //   warps 0-3      output: a quarter of the rows each, a lane a column (GLU: 16 gate columns and their 16 up columns). The first
 //                  warps: the schedulers favour older ones, and beside four streaming warps that are always ready these took 1.4 us an

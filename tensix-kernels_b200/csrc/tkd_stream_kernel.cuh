@@ -1,9 +1,9 @@
 // tkd_stream_kernel.cuh: the weight-streaming decode matmul for sm_100a (the kernel template; tkd_stream_bfp8.cu,
 // tkd_stream_bfp4.cu and tkd_stream_bf16.cu each compile one format's instantiations of it).
-// Plain calls of four slices run tkd_narrow_kernel instead (tkd_narrow.cuh, which shares this file's helpers and sums).
+// Plain calls of one to four slices run tkd_narrow_kernel instead (tkd_narrow.cuh, which shares this file's helpers and sums).
 //
-// y[m, n] = sum_k x[m, k] * w[k, n] with its fused output stage, M <= 8 activation rows (9 to 32 rows:
-// tkd_stream_tc.cuh, which shares this file's helpers), the weight a packed HBM stream (tkd_layout.h). It takes the place of the reference's three Tensix kernels (dense_reader/kernels/
+// y[m, n] = sum_k x[m, k] * w[k, n] with its fused output stage, M <= 8 activation rows (more:
+// tkd_rows.cuh and tkd_stream_tc.cuh, which share this file's helpers), the weight a packed HBM stream (tkd_layout.h). It takes the place of the reference's three Tensix kernels (dense_reader/kernels/
 // dense_reader.cpp: the DRAM loads; dense_compute.cpp: matmul_block accumulation and the output stages;
 // dense_writer.cpp: output writes and the running top-k) and of the work split linear.plan makes for them
 // (dense_reader/linear.py:187-382).
@@ -681,7 +681,7 @@ __device__ __forceinline__ void rows_for_int4(const TkdParams& p, uint32_t xt0, 
     asm volatile("bar.sync 2, %0;" ::"n"(kStreamWarps * 32) : "memory");
 }
 
-// The kernel for 1 to 8 rows (9 to 32 run tkd_stream_tc_kernel). Sixteen streaming warps: a warp per column group and half
+// The kernel for 1 to 8 rows (more run tkd_rows_kernel or tkd_stream_tc_kernel). Sixteen streaming warps: a warp per column group and half
 // of each chunk's super-atoms.
 // ONE: the call has one row (the decode case): the row count is a constant 1 and everything that serves more rows falls
 // away at compile time. (The length of this kernel's code matters beyond the parts that run: adding two more instances
@@ -1226,7 +1226,7 @@ int launch_rows(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     // (p.x_smem: x fits beside the ring in shared memory, which the one-row instantiations rely on)
     if (p.M == 1 && p.x_smem && !p.topk_k && !p.npeers) return launch_one<FMT, true, true, KWHOLE, true>(p, grid, smem, st);
     if (p.M == 1 && p.x_smem) return launch_one<FMT, true, false, KWHOLE, true>(p, grid, smem, st);
-    // (9 to 32 rows run tkd_stream_tc_kernel: the caller never gets here with them)
+    // (9 and more rows run other kernels: the caller never gets here with them)
     if (p.x_smem && !p.topk_k && !p.npeers) return launch_one<FMT, false, true, KWHOLE, true>(p, grid, smem, st);
     if (p.x_smem) return launch_one<FMT, false, false, KWHOLE, true>(p, grid, smem, st);
     return launch_one<FMT, false, false, KWHOLE, false>(p, grid, smem, st);

@@ -1,4 +1,5 @@
-// tkd_stream_tc.cuh: the stream kernel for 9 to 32 activation rows, on the fifth-generation tensor cores (tcgen05).
+// tkd_stream_tc.cuh: the stream kernel for 9 to 32 activation rows, on the fifth-generation tensor cores (tcgen05). (Where the rows fit
+// in shared memory tkd_rows_kernel is the faster one, tkd_rows.cuh; the rule is rows_layout in tkd_api.cu.)
 //
 // The reference multiplies a tile of up to 32 activation rows by each weight tile it has read (dense_reader/kernels/
 // dense_compute.cpp:95-143, matmul_block): more rows cost it no more weight traffic and hardly more time. With

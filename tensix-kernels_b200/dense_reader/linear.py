@@ -884,7 +884,7 @@ def topk_units(n):
 
 def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **opts):
     """matmul for x of any rank: x [..., rows, K] bf16, the output's rank the input's. activation: None, "silu"
-    (applied after the matmul), "swiglu" or "geglu" (w is interleave_glu's weight with scale None, the output N / 2
+    (in the kernel's output stage, on the float32 sums; after the matmul with a given out, a residual, out32 or a top-k), "swiglu" or "geglu" (w is interleave_glu's weight with scale None, the output N / 2
     wide; or w is (gate, up), the output N wide). out_dtype ttnn.float32: out32. A block list for w: plain weights with
     activation None, (gate, up) pairs with "swiglu" or "geglu". opts go to matmul. (linear.py:1073-1124)"""
     key = None
