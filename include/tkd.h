@@ -91,6 +91,10 @@ int tkd_pack(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* cod
  * calls). */
 int tkd_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, const float* col_div, void* col_scale,
                     void* packed, uint8_t* emax, int32_t* info, void* stream);
+/* tkd_pack_weight without scales, and a bf16 one for each column into ones [n]: what a caller that always has a scale tensor
+ * (native_weight) would fill by a launch of its own. */
+int tkd_pack_weight_unit(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, void* ones, void* packed, uint8_t* emax,
+                         int32_t* info, void* stream);
 /* tkd_quantise's block-float numbers (TKD_FMT_BFP8 or BFP4) as bf16 bits [K, npad] (uint16), the canonical form
  * tkd_pack takes for TKD_FMT_BF16: every such number is a bf16 value exactly, subnormals included. */
 int tkd_dequantise_bf16(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* codes, void* out_bf16, void* stream);

@@ -197,13 +197,18 @@ def pack_weight(device, wt, dtype, orient, col_div=None, memory_config=None, int
     """A float matrix (orient 0: [N, K] as torch's [out, in]; 1: [K, N]) -> Weight, on the GPU in one launch
     (tkd_pack_weight). col_div: divisors of the columns. into: byte tensors for the stream and its exponents (a weight too
     wide for its format's stream has its own all the same)."""
-    return _packed(device, wt, dtype, orient, col_div, memory_config, False, into)[0]
+    return _packed(device, wt, dtype, orient, col_div, memory_config, 0, into)[0]
+
+
+def pack_weight_unit(device, wt, dtype, memory_config=None):
+    """(Weight, bf16 [1, 1, 1, N] ones) of a [N, K] matrix."""
+    return _packed(device, wt, dtype, 0, None, memory_config, 2)
 
 
 def pack_weight_scaled(device, wt, dtype, memory_config=None):
     """(Weight, bf16 [1, 1, 1, N]) of a [N, K] matrix whose columns are first divided by their own scales, their largest
     magnitudes rounded up."""
-    return _packed(device, wt, dtype, 0, None, memory_config, True)
+    return _packed(device, wt, dtype, 0, None, memory_config, 1)
 
 
 def _packed(device, wt, dtype, orient, col_div, memory_config, own, into=(None, None)):
@@ -219,7 +224,10 @@ def _packed(device, wt, dtype, orient, col_div, memory_config, own, into=(None, 
     if state:
         # (a wide weight, or a K past what one pass takes)
         with torch.cuda.device(device.torch):
-            if own:
+            if own == 2:
+                if state == 2:
+                    scale = torch.ones(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch)
+            elif own:
                 if state == 2:
                     top = src.abs().amax(dim=1).clamp(min=1e-8)
                     down = top.to(torch.bfloat16).float()

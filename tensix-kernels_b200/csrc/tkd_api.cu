@@ -332,16 +332,26 @@ int tkd_pack(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* cod
                                          static_cast<cudaStream_t>(stream)));
 }
 
-int tkd_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, const float* col_div, void* col_scale,
-                    void* packed, uint8_t* emax, int32_t* info, void* stream) {
+static int pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, const float* col_div, void* col_scale, bool unit,
+                       void* packed, uint8_t* emax, int32_t* info, void* stream) {
     if (!fmt_ok(fmt) || fmt == TKD_INT4 || !src || !packed || k < 32 || k % 32 || n < 1 || (orient != 0 && orient != 1) ||
         ld < (orient ? n : k) || (col_div && col_scale) || (has_emax(fmt) && (!emax || !info)))
         return TKD_ERR_BAD_ARG;
     if (orient == 0 && (ld % 4 || reinterpret_cast<uintptr_t>(src) & 15)) return TKD_ERR_BAD_ARG;
     if (reinterpret_cast<uintptr_t>(packed) & 15) return TKD_ERR_BAD_ARG;
     if (k > 100 * 1024) return TKD_ERR_UNSUPPORTED;  // (two bytes a k in shared memory)
-    return launch_err(tkd_launch_pack_weight(fmt, src, orient, ld, k, n, tkd_padded_cols(n), col_div, static_cast<uint16_t*>(col_scale),
+    return launch_err(tkd_launch_pack_weight(fmt, src, orient, ld, k, n, tkd_padded_cols(n), col_div, static_cast<uint16_t*>(col_scale), unit,
                                              packed, emax, info, static_cast<cudaStream_t>(stream)));
+}
+
+int tkd_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, const float* col_div, void* col_scale,
+                    void* packed, uint8_t* emax, int32_t* info, void* stream) {
+    return pack_weight(fmt, src, orient, ld, k, n, col_div, col_scale, false, packed, emax, info, stream);
+}
+
+int tkd_pack_weight_unit(int fmt, const float* src, int orient, int64_t ld, int64_t k, int64_t n, void* ones, void* packed, uint8_t* emax,
+                         int32_t* info, void* stream) {
+    return ones ? pack_weight(fmt, src, orient, ld, k, n, nullptr, ones, true, packed, emax, info, stream) : TKD_ERR_BAD_ARG;
 }
 
 int tkd_dequantise_bf16(int fmt, int64_t k, int64_t n, const uint8_t* exps, const void* codes, void* out_bf16, void* stream) {

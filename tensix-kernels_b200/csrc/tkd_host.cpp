@@ -187,12 +187,12 @@ struct WideWord {
     }
 };
 
-// pack(format, float32 matrix, orientation, divisors or None, own scales, stream or None, emax or None) -> (stream, emax or None,
+// pack(format, float32 matrix, orientation, divisors or None, scales (0: none, 1: own, 2: ones), stream or None, emax or None) -> (stream, emax or None,
 // scales or None, state): tkd_pack_weight into the tensors given or into new ones, waited for (launches read weights ahead of stream order). state 0: done; 1: the weight
 // is wide; 2: this K is not taken (then nothing was packed).
 PyObject* host_pack(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 7 || !all_tensors(args, {1}, {3, 5, 6})) return type_error("tkd_host.pack: format, matrix, orientation, divisors, own scales, stream, emax");
-    const int fmt = (int)PyLong_AsLong(args[0]), orient = (int)PyLong_AsLong(args[2]), own = PyObject_IsTrue(args[4]);
+    if (n != 7 || !all_tensors(args, {1}, {3, 5, 6})) return type_error("tkd_host.pack: format, matrix, orientation, divisors, scales, stream, emax");
+    const int fmt = (int)PyLong_AsLong(args[0]), orient = (int)PyLong_AsLong(args[2]), own = (int)PyLong_AsLong(args[4]);
     if (PyErr_Occurred()) return nullptr;
     static thread_local WideWord word;
     try {
@@ -217,9 +217,13 @@ PyObject* host_pack(PyObject*, PyObject* const* args, Py_ssize_t n) {
         cudaStream_t st = c10::cuda::getCurrentCUDAStream(src.get_device()).stream();
         int rc;
         cudaError_t e = cudaSuccess;
-        Py_BEGIN_ALLOW_THREADS rc = tkd_pack_weight(fmt, static_cast<const float*>(src.data_ptr()), orient, src.stride(0), k, cols,
-                                                    div ? static_cast<const float*>(div->data_ptr()) : nullptr, own ? scales.data_ptr() : nullptr,
-                                                    stream.data_ptr(), emax.defined() ? static_cast<uint8_t*>(emax.data_ptr()) : nullptr, wide, st);
+        Py_BEGIN_ALLOW_THREADS {
+            const auto* sp = static_cast<const float*>(src.data_ptr());
+            uint8_t* ep = emax.defined() ? static_cast<uint8_t*>(emax.data_ptr()) : nullptr;
+            rc = own == 2 ? tkd_pack_weight_unit(fmt, sp, orient, src.stride(0), k, cols, scales.data_ptr(), stream.data_ptr(), ep, wide, st)
+                          : tkd_pack_weight(fmt, sp, orient, src.stride(0), k, cols, div ? static_cast<const float*>(div->data_ptr()) : nullptr,
+                                            own ? scales.data_ptr() : nullptr, stream.data_ptr(), ep, wide, st);
+        }
         if (!rc) e = cudaStreamSynchronize(st);
         Py_END_ALLOW_THREADS if (rc && rc != TKD_ERR_UNSUPPORTED) return tkd_error(rc, "tkd_pack_weight");
         if (e != cudaSuccess) return tkd_error(TKD_ERR_CUDA + (int)e, "tkd_pack_weight");

@@ -11,7 +11,7 @@ int tkd_launch_quantise(int fmt, const float* src, int orient, int64_t K, int64_
 int tkd_launch_permute(int fmt, int64_t K, int64_t npad, const uint8_t* exps, const void* codes, uint8_t* emax,
                        int* info, void* stream, cudaStream_t st);
 int tkd_launch_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t K, int64_t N, int64_t npad, const float* col_div,
-                           uint16_t* scale_out, void* packed, uint8_t* emax, int* info, cudaStream_t st);
+                           uint16_t* scale_out, bool unit, void* packed, uint8_t* emax, int* info, cudaStream_t st);  // unit: scales of one
 int tkd_launch_dequantise_bf16(int fmt, int64_t K, int64_t npad, const uint8_t* exps, const void* codes, void* out,
                                cudaStream_t st);
 int tkd_launch_unpack(int fmt, int64_t K, int64_t npad, const void* stream, const uint8_t* emax, float* out,

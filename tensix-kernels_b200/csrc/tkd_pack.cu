@@ -331,6 +331,8 @@ __global__ void __launch_bounds__(pack_threads(SCALE)) tkd_pack_weight_kernel(co
     };
     float d0 = 1.f, d1 = 1.f, r0 = 1.f, r1 = 1.f;
     bool slow = SCALE == 1;  // divide by the division
+    // (scales of one, for a caller that wants some beside undivided columns)
+    if (SCALE == 0 && scale_out && tid < 16 && grp * 16 + tid < N) scale_out[grp * 16 + tid] = 0x3F80;
     if constexpr (SCALE == 1) {
         if (in0) d0 = col_div[n0];
         if (in1) d1 = col_div[n1];
@@ -510,26 +512,26 @@ __global__ void __launch_bounds__(pack_threads(SCALE)) tkd_pack_weight_kernel(co
 
 template <int FMT, int ORIENT>
 int launch_pack_weight(const float* src, int64_t ld, int64_t K, int64_t N, int64_t npad, const float* col_div, uint16_t* scale_out,
-                       void* packed, uint8_t* emax, int* info, cudaStream_t st) {
+                       bool unit, void* packed, uint8_t* emax, int* info, cudaStream_t st) {
     const size_t smem = FMT == TKD_BF16 ? 0 : (size_t)(K + 63) / 64 * 128;
-    auto kern = scale_out ? tkd_pack_weight_kernel<FMT, ORIENT, 2>
+    auto kern = scale_out && !unit ? tkd_pack_weight_kernel<FMT, ORIENT, 2>
                           : col_div ? tkd_pack_weight_kernel<FMT, ORIENT, 1> : tkd_pack_weight_kernel<FMT, ORIENT, 0>;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    kern<<<(unsigned)(npad / 16), pack_threads(scale_out ? 2 : 0), smem, st>>>(src, ld, (int)K, N, col_div, scale_out, static_cast<uint8_t*>(packed), emax, info);
+    kern<<<(unsigned)(npad / 16), pack_threads(scale_out && !unit ? 2 : 0), smem, st>>>(src, ld, (int)K, N, col_div, scale_out, static_cast<uint8_t*>(packed), emax, info);
     return (int)cudaGetLastError();
 }
 
 }  // namespace
 
 int tkd_launch_pack_weight(int fmt, const float* src, int orient, int64_t ld, int64_t K, int64_t N, int64_t npad, const float* col_div,
-                           uint16_t* scale_out, void* packed, uint8_t* emax, int* info, cudaStream_t st) {
+                           uint16_t* scale_out, bool unit, void* packed, uint8_t* emax, int* info, cudaStream_t st) {
     auto go = [&](auto f) {
         constexpr int F = decltype(f)::value;
-        return orient == 0 ? launch_pack_weight<F, 0>(src, ld, K, N, npad, col_div, scale_out, packed, emax, info, st)
-                           : launch_pack_weight<F, 1>(src, ld, K, N, npad, col_div, scale_out, packed, emax, info, st);
+        return orient == 0 ? launch_pack_weight<F, 0>(src, ld, K, N, npad, col_div, scale_out, unit, packed, emax, info, st)
+                           : launch_pack_weight<F, 1>(src, ld, K, N, npad, col_div, scale_out, unit, packed, emax, info, st);
     };
     return fmt == TKD_BFP8 ? go(std::integral_constant<int, TKD_BFP8>{}) : fmt == TKD_BFP4 ? go(std::integral_constant<int, TKD_BFP4>{})
                                                                                            : go(std::integral_constant<int, TKD_BF16>{});

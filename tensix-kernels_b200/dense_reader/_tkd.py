@@ -67,6 +67,7 @@ SYMBOLS = {
     "tkd_quantise": (c_i32, [c_i32, c_vp, c_i32, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp]),
     "tkd_pack": (c_i32, [c_i32, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "tkd_pack_weight": (c_i32, [c_i32, c_vp, c_i32, c_i64, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "tkd_pack_weight_unit": (c_i32, [c_i32, c_vp, c_i32, c_i64, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "tkd_layout_version": (c_i32, []),
     "tkd_dequantise_bf16": (c_i32, [c_i32, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp]),
     "tkd_unpack": (c_i32, [c_i32, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp]),

@@ -135,8 +135,7 @@ def native_weight(device, t, dtype, col_scale=False, sharded=True, max_banks=Non
     if col_scale:
         w, c = ttnn.pack_weight_scaled(device, t, dtype, memory_config=mc)
     else:
-        w = ttnn.pack_weight(device, t, dtype, 0, memory_config=mc)
-        c = torch.ones(1, 1, 1, n, dtype=torch.bfloat16, device=device.torch)
+        w, c = ttnn.pack_weight_unit(device, t, dtype, memory_config=mc)
     return w, ttnn.Tensor(c, ttnn.bfloat16, ttnn.TILE_LAYOUT, device, ttnn.DRAM_MEMORY_CONFIG)
 
 

@@ -810,3 +810,19 @@ def test_own_scales_with_zero_and_tiny_inputs(device, fmt, n):
     assert torch.equal(ttnn.to_torch(ts).float().reshape(-1), torch.as_tensor(scale).float().reshape(-1))
     held = ttnn.to_torch(tw).float().reshape(k, -1)[:, :n]
     assert torch.equal(held, torch.from_numpy(want))
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
+@pytest.mark.parametrize("n,k", [(1, 32), (40, 96), (130, 544), (4096, 1024)])
+def test_unit_scales_come_with_the_pack(device, fmt, n, k):
+    """native_weight without column scales: the same weight as the packer's alone, and a one for every column, of a wide weight too."""
+    g = torch.Generator().manual_seed(n)
+    w = torch.randn(n, k, generator=g) * 0.1
+    for wide in (False, True):
+        if wide:
+            w[:, 1] = 1e-30
+        tw, ts = linear.native_weight(device, w, DT[fmt])
+        alone = ttnn.pack_weight(device, w, DT[fmt], 0)
+        assert tw.fmt == alone.fmt and torch.equal(tw.t, alone.t) and (tw.emax is None) == (alone.emax is None)
+        assert tw.emax is None or torch.equal(tw.emax, alone.emax)
+        assert ts.t.dtype == torch.bfloat16 and tuple(ts.t.shape) == (1, 1, 1, n) and bool((ts.t == 1).all())
