@@ -919,6 +919,7 @@ def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **o
             opts = {**opts, "glu": True, **({"glu_act": 1} if glu_kinds[activation] else {})}
             if opts.get("w_up") is None:
                 n //= 2
+    assert activation in (None, "silu", *glu_kinds), f"dense_reader.linear: activation {activation!r}"
     x4 = x if len(shape) == 4 else ttnn.reshape(x, [1, 1, shape[-2], shape[-1]])
     if x4.memory_config().memory_layout != ttnn.TensorMemoryLayout.INTERLEAVED:
         x4 = ttnn.sharded_to_interleaved(x4, ttnn.L1_MEMORY_CONFIG)
@@ -928,14 +929,14 @@ def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **o
     if fused:
         opts = {**opts, _SILU: True}
     y = matmul(x4, w, scale, memory_config=memory_config, **opts)
-    if key is not None and x4 is x:
+    after = activation == "silu" and not fused
+    if key is not None and x4 is x and not after:  # (a kept call's output is returned as it is: nothing may follow it)
         call = weight.calls.get(_call_key(x, w, scale, None, None, 0, None, None, "hifi2", opts)[1])
         if call is not None:
             if len(weight.short) >= _WEIGHT_CALLS:
                 weight.short.clear()
             weight.short[key] = call
-    if activation is not None and activation not in ("swiglu", "geglu") and not fused:
-        assert activation == "silu", f"dense_reader.linear: activation {activation!r}"
+    if after:
         y = ttnn.silu(y)
     if len(shape) != 4 and opts.get("out") is None:
         y = ttnn.reshape(y, [*shape[:-1], n])

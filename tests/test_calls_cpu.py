@@ -373,3 +373,41 @@ def test_linears_own_arguments_find_the_kept_call(ran, monkeypatch):
     for m in range(1, 2 * linear._WEIGHT_CALLS):
         linear.linear(tensor(1, 1, m, 64), w, None)
     assert len(w.calls) <= linear._WEIGHT_CALLS and len(w.short) <= linear._WEIGHT_CALLS
+
+
+@pytest.mark.parametrize("out_dtype", [None, ttnn.bfloat16, ttnn.float32])
+@pytest.mark.parametrize("activation", [None, "silu", "swiglu", "geglu", "relu", ""])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_a_repeated_linear_gives_what_the_first_gave(ran, monkeypatch, activation, out_dtype, scaled):
+    """linear.linear three times with the same arguments, for every activation and output type: equal outputs, the activation among
+    them, or a refusal each time. The launch is stood in for by the product 2 with what its output stage adds."""
+    act = lambda v, which: torch.nn.functional.silu(v) if which == 0 else torch.nn.functional.gelu(v, approximate="tanh")  # noqa: E731
+
+    def run(call, x, out, residual):
+        ran.append(call)
+        a = call.launches[0][1]
+        v = torch.full((1, 1, x.t.shape[-2], a.ldo), 2.0)
+        return act(v, 0) if a.epilogue == _tkd.EPI_SILU else act(v, a.act) * 2.0 if a.epilogue == _tkd.EPI_GLU_IL else v
+
+    monkeypatch.setattr(linear._Call, "run", run)
+    # (the first call's launch writes into a tensor made before it: described calls return that one)
+    described = linear._described
+
+    def with_output(*args):
+        y, call = described(*args)
+        return ttnn.Tensor(run(call, args[0], None, None), y.dtype, y.layout, y._device, y._mc), call
+
+    monkeypatch.setattr(linear, "_described", with_output)
+    w, x = weight(64, 128), tensor(1, 1, 3, 64)
+    scale = ttnn.Tensor(torch.ones(1, 1, 1, 128, dtype=torch.bfloat16), ttnn.bfloat16, ttnn.TILE_LAYOUT, DEVICE, None) if scaled else None
+    two = torch.tensor(2.0)
+    want = {None: two, "silu": act(two, 0), "swiglu": act(two, 0) * 2, "geglu": act(two, 1) * 2}.get(activation)
+    if want is None or (scaled and activation in ("swiglu", "geglu")) or (out_dtype == ttnn.float32 and (scaled or activation in ("swiglu", "geglu"))):
+        for _ in range(3):
+            with pytest.raises(AssertionError):
+                linear.linear(x, w, scale, activation=activation, out_dtype=out_dtype)
+        return
+    for _ in range(3):
+        y = linear.linear(x, w, scale, activation=activation, out_dtype=out_dtype)
+        assert y.dtype == (out_dtype or ttnn.bfloat16)
+        assert torch.equal(y.t, torch.full_like(y.t, float(want))), (activation, out_dtype)

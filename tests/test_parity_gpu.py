@@ -826,3 +826,19 @@ def test_unit_scales_come_with_the_pack(device, fmt, n, k):
         assert tw.fmt == alone.fmt and torch.equal(tw.t, alone.t) and (tw.emax is None) == (alone.emax is None)
         assert tw.emax is None or torch.equal(tw.emax, alone.emax)
         assert ts.t.dtype == torch.bfloat16 and tuple(ts.t.shape) == (1, 1, 1, n) and bool((ts.t == 1).all())
+
+
+@pytest.mark.parametrize("m", [1, 16, 64])
+def test_silu_behind_a_float32_product(device, m):
+    """linear(activation="silu") into float32 applies the activation to the float32 product, each time it is called alike."""
+    g = torch.Generator().manual_seed(m)
+    tw, ts = linear.native_weight(device, torch.randn(144, 544, generator=g) * 0.06, ttnn.bfloat8_b)
+    tx = dev_x(device, torch.randn(m, 544, generator=g))
+    want = torch.nn.functional.silu(host(linear.matmul(tx, tw, None, out32=True)))
+    for _ in range(3):
+        y = linear.linear(tx, tw, None, activation="silu", out_dtype=ttnn.float32)
+        # (exponentials of the CPU and the GPU: a few units in the last place)
+        assert y.dtype == ttnn.float32 and torch.allclose(host(y), want, rtol=1e-6, atol=1e-7)
+        with pytest.raises(AssertionError):
+            linear.linear(tx, tw, None, activation="relu")
+    linear.check_status(device)
