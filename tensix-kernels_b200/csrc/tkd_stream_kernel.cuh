@@ -1108,7 +1108,7 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
     #pragma unroll
                     for (int m = 0; m < R; ++m) tot[m] *= sc;
                 }
-                if (PLAIN && p.epi == TKD_EPI_SILU) {
+                if ((PLAIN || !XSM) && p.epi == TKD_EPI_SILU) {  // (without x in shared memory one instance serves plain calls and others)
     #pragma unroll
                     for (int m = 0; m < R; ++m) tot[m] = act_gate(tot[m], 0);
                 }

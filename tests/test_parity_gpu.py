@@ -842,3 +842,20 @@ def test_silu_behind_a_float32_product(device, m):
         with pytest.raises(AssertionError):
             linear.linear(tx, tw, None, activation="relu")
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("fmt,m,k", [("bf16", 8, 7168), ("bf16", 8, 7200), ("bf16", 8, 8192), ("bfp8", 8, 8960), ("bfp8", 8, 8992), ("bfp8", 6, 14336),
+                                     ("bfp4", 8, 8704), ("bfp4", 8, 8736), ("bfp4", 7, 14336), ("bfp8", 8, 9632), ("bfp4", 8, 9632), ("bf16", 6, 9632),
+                                     ("bfp8", 1, 114688), ("bfp8", 32, 20480), ("bfp4", 20, 20512), ("bf16", 12, 20480), ("bfp8", 40, 9632)])
+def test_linear_silu_of_long_rows(device, fmt, m, k):
+    """linear(activation="silu") of long rows: where x leaves tkd_narrow_kernel's ring no room, and then tkd_stream_kernel's (on both
+    sides of that limit, and a K that ends inside a chunk), slices past four, more than 32 rows."""
+    g = torch.Generator().manual_seed(m + k)
+    w, x = torch.randn(80, k, generator=g) * 0.02, torch.randn(m, k, generator=g)
+    for scaled in (False, True):
+        tw, ts = linear.native_weight(device, w, DT[fmt], col_scale=scaled)
+        plain = x.to(torch.bfloat16).double() @ torch.from_numpy(orc.native_values(w, fmt, col_scale=scaled)[0]).double()
+        if scaled:
+            plain = plain * ttnn.to_torch(ts).double().reshape(-1)
+        close_bf16(host(linear.linear(dev_x(device, x), tw, ts if scaled else None, activation="silu")), torch.nn.functional.silu(plain).numpy())
+    linear.check_status(device)
