@@ -79,7 +79,7 @@ int rows_layout(TkdParams& p, int sab) {
             p.rows_tile = rows < p.M ? rows : 0;
             return chunks;
         }
-        if (rows <= 16 || p.K > 2816) return 0;
+        if (rows <= 16 || p.K > 2816 || p.fmt == TKD_BF16) return 0;  // (bf16: the rows of such a K fit)
     }
 }
 
@@ -225,9 +225,11 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     if (p.tc && !a->ks) p.rows_chunks = rows_layout(p, sab);
     if (p.rows_chunks) p.tc = 0, L->smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
     const int64_t items = p.narrow || p.rows_chunks ? 4 * (int64_t)panels : p.total_items;
-    const int tiles = p.rows_tile ? (p.M + p.rows_tile - 1) / p.rows_tile : 1, team = sms / tiles > 0 ? sms / tiles : 1;
-    L->grid = tiles * (int)(items < team ? items : team);
-    if (p.rows_tile) p.rows_team = L->grid / tiles;
+    // (tiles of rows: a team of CTAs each; where max_ctas leaves fewer than the tiles, one for several)
+    const int tiles = p.rows_tile ? (p.M + p.rows_tile - 1) / p.rows_tile : 1, teams = sms < tiles ? sms : tiles, team = sms / teams;
+    L->grid = teams * (int)(items < team ? items : team);
+    if (p.rows_tile) p.rows_team = L->grid / teams;
+    p.rows_turns = teams < tiles;
     // 9 to 32 rows: clusters of four CTAs, one to a slice (tkd_stream_tc.cuh), for a plain call of four slices. They take whole
     // panels and leave some SMs idle (a GPC's number of SMs is not a multiple of four: 132 of 148 CTAs on a B200), so they are
     // taken where no CTA gets more items for it; from four items on the other form's SMs that have one less leave theirs to the rest.

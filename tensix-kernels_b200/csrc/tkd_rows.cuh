@@ -102,8 +102,10 @@ __device__ __forceinline__ void rows_block(float (&acc)[2][MT][4], uint32_t ca, 
     }
 }
 
-// SC: chunks of a stage (TkdParams.rows_chunks). PLAIN: no top-k records and no exchange with other GPUs.
-template <int FMT, int MT, int SC, bool PLAIN>
+// SC: chunks of a stage (TkdParams.rows_chunks). PLAIN: no top-k records and no exchange with other GPUs. TURNS: fewer CTAs than
+// tiles of rows (two tiles, and max_ctas leaves one CTA), which take their tiles in turn, the ring and the hand-over of sums running on;
+// an instance of its own, so that the others keep their code.
+template <int FMT, int MT, int SC, bool PLAIN, bool TURNS>
 __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __grid_constant__ TkdParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
@@ -129,9 +131,12 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
     __syncthreads();
     const uint32_t T = 4u * (uint32_t)p.total_panels;  // items
     // (more than 32 rows: tiles of rows, a team of CTAs each)
-    const uint32_t team = p.rows_team ? p.rows_team : gridDim.x, tile = blockIdx.x / team, cta = blockIdx.x - tile * team;
-    const int i0 = (int)((uint64_t)T * cta / team), i1 = (int)((uint64_t)T * (cta + 1) / team);
-    const int row0 = (int)tile * p.rows_tile, M = p.rows_tile ? min(p.rows_tile, p.M - row0) : p.M;
+    const uint32_t team = p.rows_team ? p.rows_team : gridDim.x, tile0 = blockIdx.x / team, cta = blockIdx.x - tile0 * team;
+    const int i0 = (int)((uint64_t)T * cta / team), i1 = (int)((uint64_t)T * (cta + 1) / team), ni = i1 - i0;
+    const int step = TURNS ? gridDim.x / team : 1, turns = TURNS ? ((p.M - 1) / p.rows_tile - (int)tile0) / step + 1 : 1;
+    // the rows of this CTA's tile number `turn`: the first, and how many
+    auto first_row = [&](int turn) { return ((int)tile0 + turn * step) * p.rows_tile; };
+    auto rows_of = [&](int turn) { return p.rows_tile ? min(p.rows_tile, p.M - first_row(turn)) : p.M; };
     const int nst = p.nstages, K = p.K, nch = (K + CK - 1) / CK, nsa_total = (K + F::KSA - 1) / F::KSA;
     const int spi = (nch + SC - 1) / SC;  // stages of an item
     const int epi = p.epi;
@@ -150,7 +155,8 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
         uint32_t st = 0;
         bool ok = true;
         const int s = lane >> 1, g = lane & 1;
-        for (int it = i0; ok && it < i1; ++it) {
+        for (int j = 0; ok && j < turns * ni; ++j) {
+            const int it = i0 + (TURNS ? j % ni : j);
             const TkdSegDev& sg = p.seg[seg_of(it)];
             const NarrowItem n = narrow_item(p, it - 4 * sg.panel0);
             const uint8_t* src = (g && epi == TKD_EPI_GLU2 ? sg.w2 : sg.w) + (int64_t)n.panel * p.panel_bytes;
@@ -178,123 +184,130 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
         const int cw = warp - kRowsOut - 1, g = lane >> 2, t = lane & 3;
         if (nch * CK > K) {
             // the rows of x end in zeros up to a whole chunk
-            for (int r = cw; r < M; r += SW)
+            for (int r = cw; r < rows_of(0); r += SW)  // (no later tile has more)
                 for (int e = K / 8 + lane; e < nch * (CK / 8); e += 32)
                     asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(xt0 + r * p.x_stride + e * 16), "r"(0u) : "memory");
             asm volatile("bar.sync 2, %0;" ::"n"(SW * 32) : "memory");
         }
         // (x and the outputs may belong to the kernel before this one: wait for it to complete)
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        for (int s = 0; s < kRowsSegs; ++s) {  // (the last part: all that is left)
-            const int e0 = min(s * SC * CK, K) / 8, e1 = s == kRowsSegs - 1 ? K / 8 : min((s + 1) * SC * CK, K) / 8;
-            for (int r = cw; r < M; r += SW) {
-                const uint16_t* src = p.x + (int64_t)(row0 + r) * p.ldx;
-                const uint32_t dst = xt0 + r * p.x_stride;
-#pragma unroll 4
-                for (int e = e0 + lane; e < e1; e += 32)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + e * 16), "l"(src + e * 8) : "memory");
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(xbar0 + 8 * s) : "memory");
-        }
-        const uint2 sh = make_uint2(p.mul16, p.mul128);
-        // (a lane whose row lies beyond M reads row M - 1: a column of B only feeds its own column of D)
-        uint32_t xrow[MT];
-#pragma unroll
-        for (int m = 0; m < MT; ++m) xrow[m] = xt0 + min(8 * m + g, M - 1) * p.x_stride + t * 16;
-        const int cc = cw / F::SUBSA, si = cw % F::SUBSA;  // this warp's (first) super-atom of a stage
-        constexpr int NU = SC * F::SUBSA / SW, CSTEP = SW / F::SUBSA;
-        const uint32_t gbl = (nsa_total - (nch - 1) * F::SUBSA) * F::SAB;  // a group's share of K's last chunk
-        const int cwhole = nsa_total / F::SUBSA;                           // whole chunks
-        const uint32_t exp_lane = cc * 2 * GB + si * F::SAB + t * (EXPB / 4), code_lane = cc * 2 * GB + si * F::SAB + EXPB + lane * 16;
-        const uint32_t xk0 = (cc * CK + si * F::KSA) * 2;
-        const uint32_t ring_end = ring0 + nst * p.stage_bytes;
-        const uint32_t slot = pbuf + (cw & 7) * SLOT + ((2 * t) * PP + g) * 4;  // (where this lane's sums go)
-        float acc[2][MT][4];
         uint32_t at = ring0, bar = full0, phase = 0;
         bool ok = true;
-        for (int j = 0; ok && j < i1 - i0; ++j) {
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int m = 0; m < MT; ++m) acc[a][m][0] = acc[a][m][1] = acc[a][m][2] = acc[a][m][3] = 0.f;
-            uint32_t xk = xk0;
-            int c = 0;
-#pragma unroll 1
-            for (int i = 0; i < spi; ++i, xk += SC * CK * 2, c += SC) {
-                if (j == 0) ok = mbar_wait(xbar0 + 8 * min(i, kRowsSegs - 1), 0, p.status);
-                ok = ok && mbar_wait(bar, phase, p.status);
-                if (!ok) break;
-                const uint32_t ca = at + code_lane, ea = at + exp_lane;
-                uint32_t xa[MT];
-#pragma unroll
-                for (int m = 0; m < MT; ++m) xa[m] = xrow[m] + xk;
-                if (c + SC <= cwhole && MT == 2) {
-                    unrolled(std::make_integer_sequence<int, NU>{}, [&](auto uc) {
-                        constexpr int u = decltype(uc)::value;
-                        rows_block<FMT, MT, u * CSTEP * 2 * GB, u * CSTEP * CK * 2, GB>(acc, ca, ea, 0u, xa, sh);
-                    });
-                } else if (c + SC <= cwhole) {
-                    // (one after the other: side by side they spill)
-#pragma unroll 1
-                    for (int u = 0; u < NU; ++u) {
-                        const uint32_t by = u * CSTEP * 2 * GB;
-                        uint32_t xu[MT];
-#pragma unroll
-                        for (int m = 0; m < MT; ++m) xu[m] = xa[m] + u * CSTEP * CK * 2;
-                        rows_block<FMT, MT, 0, 0, GB>(acc, ca + by, ea + by, 0u, xu, sh);
-                    }
-                } else {
-                    // (K's last chunk may have fewer super-atoms: its groups lie closer together)
-#pragma unroll 1
-                    for (int u = 0; u < NU; ++u) {
-                        const int ch = c + cc + u * CSTEP;
-                        if (ch >= nch || ch * F::SUBSA + si >= nsa_total) break;
-                        const uint32_t by = u * CSTEP * 2 * GB;
-                        uint32_t xu[MT];
-#pragma unroll
-                        for (int m = 0; m < MT; ++m) xu[m] = xa[m] + u * CSTEP * CK * 2;
-                        rows_block<FMT, MT, 0, 0, 0>(acc, ca + by, ea + by, ch == nch - 1 ? gbl : (uint32_t)GB, xu, sh);
-                    }
+        for (int turn = 0; turn < turns; ++turn) {
+            const int row0 = first_row(turn), M = rows_of(turn);
+            // (the rows of the tile before have been read by every warp: one whose wait gave up comes here too)
+            if (TURNS && turn) asm volatile("bar.sync 2, %0;" ::"n"(SW * 32) : "memory");
+            for (int s = 0; s < kRowsSegs; ++s) {  // (the last part: all that is left)
+                const int e0 = min(s * SC * CK, K) / 8, e1 = s == kRowsSegs - 1 ? K / 8 : min((s + 1) * SC * CK, K) / 8;
+                for (int r = cw; r < M; r += SW) {
+                    const uint16_t* src = p.x + (int64_t)(row0 + r) * p.ldx;
+                    const uint32_t dst = xt0 + r * p.x_stride;
+#pragma unroll 4
+                    for (int e = e0 + lane; e < e1; e += 32)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + e * 16), "l"(src + e * 8) : "memory");
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar + 8 * TKD_MAX_STAGES);
-                at += p.stage_bytes, bar += 8;
-                if (at == ring_end) at = ring0, bar = full0, phase ^= 1;
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(xbar0 + 8 * s) : "memory");
             }
-            if (!ok) break;
-            // ---- the item's sums: the upper eight warps' through shared memory to the lower eight, theirs to the output warps
-            if (cw >= 8) {
-                ok = mbar_wait(pempty, (j & 1) ^ 1, p.status);
+            const uint2 sh = make_uint2(p.mul16, p.mul128);
+            // (a lane whose row lies beyond M reads row M - 1: a column of B only feeds its own column of D)
+            uint32_t xrow[MT];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) xrow[m] = xt0 + min(8 * m + g, M - 1) * p.x_stride + t * 16;
+            const int cc = cw / F::SUBSA, si = cw % F::SUBSA;  // this warp's (first) super-atom of a stage
+            constexpr int NU = SC * F::SUBSA / SW, CSTEP = SW / F::SUBSA;
+            const uint32_t gbl = (nsa_total - (nch - 1) * F::SUBSA) * F::SAB;  // a group's share of K's last chunk
+            const int cwhole = nsa_total / F::SUBSA;                           // whole chunks
+            const uint32_t exp_lane = cc * 2 * GB + si * F::SAB + t * (EXPB / 4), code_lane = cc * 2 * GB + si * F::SAB + EXPB + lane * 16;
+            const uint32_t xk0 = (cc * CK + si * F::KSA) * 2;
+            const uint32_t ring_end = ring0 + nst * p.stage_bytes;
+            const uint32_t slot = pbuf + (cw & 7) * SLOT + ((2 * t) * PP + g) * 4;  // (where this lane's sums go)
+            float acc[2][MT][4];
+            for (int j0 = 0; ok && j0 < ni; ++j0) {
+                const int j = turn * ni + j0;
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) acc[a][m][0] = acc[a][m][1] = acc[a][m][2] = acc[a][m][3] = 0.f;
+                uint32_t xk = xk0;
+                int c = 0;
+#pragma unroll 1
+                for (int i = 0; i < spi; ++i, xk += SC * CK * 2, c += SC) {
+                    if (j0 == 0) ok = mbar_wait(xbar0 + 8 * min(i, kRowsSegs - 1), turn & 1, p.status);
+                    ok = ok && mbar_wait(bar, phase, p.status);
+                    if (!ok) break;
+                    const uint32_t ca = at + code_lane, ea = at + exp_lane;
+                    uint32_t xa[MT];
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) xa[m] = xrow[m] + xk;
+                    if (c + SC <= cwhole && MT == 2) {
+                        unrolled(std::make_integer_sequence<int, NU>{}, [&](auto uc) {
+                            constexpr int u = decltype(uc)::value;
+                            rows_block<FMT, MT, u * CSTEP * 2 * GB, u * CSTEP * CK * 2, GB>(acc, ca, ea, 0u, xa, sh);
+                        });
+                    } else if (c + SC <= cwhole) {
+                        // (one after the other: side by side they spill)
+#pragma unroll 1
+                        for (int u = 0; u < NU; ++u) {
+                            const uint32_t by = u * CSTEP * 2 * GB;
+                            uint32_t xu[MT];
+#pragma unroll
+                            for (int m = 0; m < MT; ++m) xu[m] = xa[m] + u * CSTEP * CK * 2;
+                            rows_block<FMT, MT, 0, 0, GB>(acc, ca + by, ea + by, 0u, xu, sh);
+                        }
+                    } else {
+                        // (K's last chunk may have fewer super-atoms: its groups lie closer together)
+#pragma unroll 1
+                        for (int u = 0; u < NU; ++u) {
+                            const int ch = c + cc + u * CSTEP;
+                            if (ch >= nch || ch * F::SUBSA + si >= nsa_total) break;
+                            const uint32_t by = u * CSTEP * 2 * GB;
+                            uint32_t xu[MT];
+#pragma unroll
+                            for (int m = 0; m < MT; ++m) xu[m] = xa[m] + u * CSTEP * CK * 2;
+                            rows_block<FMT, MT, 0, 0, 0>(acc, ca + by, ea + by, ch == nch - 1 ? gbl : (uint32_t)GB, xu, sh);
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar + 8 * TKD_MAX_STAGES);
+                    at += p.stage_bytes, bar += 8;
+                    if (at == ring_end) at = ring0, bar = full0, phase ^= 1;
+                }
                 if (!ok) break;
-            } else {
-                ok = mbar_wait(half0 + 8 * cw, j & 1, p.status);
-                if (!ok) break;
+                // ---- the item's sums: the upper eight warps' through shared memory to the lower eight, theirs to the output warps
+                if (cw >= 8) {
+                    ok = mbar_wait(pempty, (j & 1) ^ 1, p.status);
+                    if (!ok) break;
+                } else {
+                    ok = mbar_wait(half0 + 8 * cw, j & 1, p.status);
+                    if (!ok) break;
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+#pragma unroll
+                        for (int m = 0; m < MT; ++m)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[a][m][e] += lds32f(slot + ((8 * m + (e & 1)) * PP + a * 16 + (e >> 1) * 8) * 4);
+                }
 #pragma unroll
                 for (int a = 0; a < 2; ++a)
 #pragma unroll
                     for (int m = 0; m < MT; ++m)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) acc[a][m][e] += lds32f(slot + ((8 * m + (e & 1)) * PP + a * 16 + (e >> 1) * 8) * 4);
+                        for (int e = 0; e < 4; ++e) sts32(slot + ((8 * m + (e & 1)) * PP + a * 16 + (e >> 1) * 8) * 4, acc[a][m][e]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(cw >= 8 ? half0 + 8 * (cw - 8) : pfull);
             }
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int m = 0; m < MT; ++m)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) sts32(slot + ((8 * m + (e & 1)) * PP + a * 16 + (e >> 1) * 8) * 4, acc[a][m][e]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cw >= 8 ? half0 + 8 * (cw - 8) : pfull);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // ---------------------------------------------------------------- output warps
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        const int ow = warp, left = M - RW * ow;  // rows from this warp's first on
-        const int topk_k = PLAIN || tile ? 0 : p.topk_k, npeers = PLAIN ? 0 : p.npeers;
+        const int ow = warp, npeers = PLAIN ? 0 : p.npeers;
         const bool up = glu && lane >= 16, f32out = epi == TKD_EPI_OUT32;
         bool met = true;
-        for (int j = 0; j < i1 - i0; ++j) {
-            const int it = i0 + j, seg = seg_of(it);
+        for (int j = 0; j < turns * ni; ++j) {
+            const int turn = TURNS ? j / ni : 0, row0 = first_row(turn), left = rows_of(turn) - RW * ow;  // rows from this warp's first on
+            const int topk_k = PLAIN || row0 ? 0 : p.topk_k;
+            const int it = i0 + (TURNS ? j % ni : j), seg = seg_of(it);
             const TkdSegDev& sg = p.seg[seg];
             const int pl = it - 4 * sg.panel0;
             const int plw = !PLAIN && p.rep_panels ? pl % (4 * p.rep_panels) : pl;  // (the item's number in its weight)
@@ -395,9 +408,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
     }
 }
 
-template <int FMT, int MT, int SC, bool PLAIN>
+template <int FMT, int MT, int SC, bool PLAIN, bool TURNS = false>
 int launch_rows_one(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
-    auto kern = tkd_rows_kernel<FMT, MT, SC, PLAIN>;
+    auto kern = tkd_rows_kernel<FMT, MT, SC, PLAIN, TURNS>;
     static bool allowed[64] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -420,6 +433,10 @@ template <int FMT>
 int launch_rows_kernel(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     auto go = [&](auto mt, auto sc) {
         constexpr int MT = decltype(mt)::value, SC = decltype(sc)::value;
+        if constexpr (FMT != TKD_BF16 && MT == 2)  // (two tiles of 17 to 32 rows are a block-float weight's: rows_layout)
+            if (p.rows_turns)
+                return p.topk_k || p.npeers ? launch_rows_one<FMT, MT, SC, false, true>(p, grid, smem, st)
+                                            : launch_rows_one<FMT, MT, SC, true, true>(p, grid, smem, st);
         return p.topk_k || p.npeers ? launch_rows_one<FMT, MT, SC, false>(p, grid, smem, st) : launch_rows_one<FMT, MT, SC, true>(p, grid, smem, st);
     };
     const int rows = p.rows_tile ? p.rows_tile : p.M;

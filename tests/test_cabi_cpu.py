@@ -144,3 +144,13 @@ def test_rows_requests_that_are_refused(tkd):
     for bad in ({"ks": -1024}, {"ks": 100}, {"m": 32}, {"m": 4097}, {"k": 4016}, {"out_dtype": tkd.DT_F32}, {"topk_k": 1}):
         assert need(**bad)[0] == 1, bad
     assert need(fmt=tkd.FMT_INT4)[0] == 2 and need(nranks=2)[0] == 2
+
+
+def test_no_plan_takes_more_ctas_than_it_may(tkd):
+    """A call's grid stays within max_ctas at every row count, where the rows run as tiles with a team of CTAs each too."""
+    for fmt in (tkd.FMT_BFP8, tkd.FMT_BFP4, tkd.FMT_BF16):
+        for m in (1, 8, 9, 16, 17, 24, 25, 32):
+            for k in (96, 1056, 2304, 2816, 4096):
+                for ctas in (1, 2, 3, 5, 147):
+                    rc, p = plan(tkd, fmt=fmt, m=m, k=k, ns=[2224], max_ctas=ctas)
+                    assert rc == 0 and 1 <= p.grid <= ctas, (fmt, m, k, ctas, p.grid)

@@ -120,3 +120,44 @@ def test_tiles_of_rows(device, fmt, m, k, n):
     for ctas in (None, 17):
         close_bf16(host(linear.linear(dev_x(device, x), tw, None, activation="silu", max_ctas=ctas)), torch.nn.functional.silu(plain).numpy())
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("fmt,m,k", [("bfp8", 32, 1056), ("bfp4", 25, 96), ("bfp4", 24, 2816), ("bfp8", 31, 2304)])
+def test_two_tiles_of_rows_on_one_cta(device, fmt, m, k):
+    """17 to 32 rows as two tiles of sixteen where max_ctas leaves one CTA: it takes one tile after the other. The same bits as with
+    two, three and all CTAs, of the outputs, their float32 form, the records and an exchanged call."""
+    g = torch.Generator().manual_seed(m + k)
+    n, rows, kk = 2048 + 176, 9, 7
+    w, x = torch.randn(n, k, generator=g) * 0.05, torch.randn(m, k, generator=g)
+    tw, _ = linear.native_weight(device, w, DT[fmt])
+    tx, res = dev_x(device, x), torch.randn(m, n, generator=g)
+    t32 = ttnn.from_torch(res.reshape(1, 1, m, n), dtype=ttnn.float32, layout=ttnn.TILE_LAYOUT, device=device)
+    plain = x.to(torch.bfloat16).double() @ torch.from_numpy(orc.native_values(w, fmt)[0]).double()
+    whole, whole32 = host(linear.matmul(tx, tw, None)), host(linear.matmul(tx, tw, None, residual=t32, out32=True))
+    close_bf16(whole, plain.numpy())
+    for ctas in (1, 2, 3, 1):
+        assert torch.equal(host(linear.matmul(tx, tw, None, max_ctas=ctas)), whole), ctas
+        assert torch.equal(host(linear.matmul(tx, tw, None, residual=t32, out32=True, max_ctas=ctas)), whole32), ctas
+        for write_y in (True, False):
+            r = linear.topk_result(device, 2, rows, kk)
+            out = ttnn.from_torch(torch.full((1, 1, m, n), -7.0, dtype=torch.bfloat16), dtype=ttnn.bfloat16, layout=ttnn.TILE_LAYOUT, device=device)
+            spec = {"r": r, "k": kk, "rows": rows, "slot0": 0, "base": 0, "n": n, "write_y": write_y}
+            linear.matmul(tx, tw, None, topk=spec, out=out, max_ctas=ctas)
+            assert torch.equal(host(out), whole) if write_y else bool((host(out) == -7.0).all())
+            check_records(ttnn.to_torch(r).reshape(2, 2, rows, kk), whole, n, 0)
+    nbytes = 1 << 20
+    bufs = [torch.zeros(nbytes + 256, dtype=torch.uint8, device=device.torch) for _ in range(2)]
+    ranks = [fake_rank(device, r, 2, bufs, nbytes) for r in range(2)]
+    outs = [ex.tensor([1, 1, m, n], ttnn.bfloat16) for ex in ranks]
+    half = 1024
+    parts = [linear.native_weight(device, w[:half], DT[fmt])[0], linear.native_weight(device, w[half:], DT[fmt])[0]]
+    status = torch.zeros(1, dtype=torch.int32, device=device.torch)
+    for r, ex in enumerate(ranks):
+        linear.matmul(tx, parts[r], None, out=outs[r], col0=r * half // 32, exchange=ex, max_ctas=1)
+    for ex in ranks:
+        ex.wait_all(status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for r in range(2):
+        assert torch.equal(host(outs[r]), whole), r
+    linear.check_status(device)
