@@ -9,8 +9,9 @@
 //                bulk copy, and the rows' activations for those k by the warp's own 16-byte asynchronous copies, both counted
 //                on the stage's barrier
 //   warps 1-16   streaming: warp (g, h) multiplies the 16 columns of group g by every other super-atom with mma.sync, 8 rows an
-//                MMA; from two MMAs on the scales go into the weights instead (exact: a code times a power of two), once for
-//                all rows. An expert's sums, times its group's factor, are added to the tile's in registers
+//                MMA; from nine rows on the scales go into the weights instead (exact: a code times a power of two), once for
+//                all rows, and where an expert's few rows take one MMA too: an activation times the largest scale, 2^64, may be
+//                past bf16's range. An expert's sums, times its group's factor, are added to the tile's in registers
 //   warps 17-20  output (thread = column)
 //
 // A tile is 128 columns of the result: gate_up: of one expert (64 outputs act(x G + b) * (x U + b) * routing weight); down: of
@@ -143,8 +144,9 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
     };
 
     // gate_up: the rows that chose the expert of slot q, a bit each (by a whole warp). Up to eight of them (of 16 rows and 8 of 128 experts
-    // one or two as a rule) are brought and multiplied alone, as rows 0, 1, ..: one MMA a fragment. gate_up of 16 rows, 8 of 128 experts of
-    // 2048 x 1536, 52.8 us before, 48.9 now; of 32 rows 109 and 87.
+    // one or two as a rule) are brought and multiplied alone, as rows 0, 1, ..: one MMA a fragment. (The scales in those rows'
+    // activations: gate_up of 16 rows, 8 of 128 experts of 2048 x 1536, 49.9 us, of 32 rows 80.6; in the weights 50.6 and 82.7, but
+    // an input's range does not depend on how many rows chose the same expert.)
     constexpr bool PICK = !DOWN && MT > 1 && FMT == TKD_BFP4;
     auto rows_of = [&](int q) {
         const int e = ulist[q];
@@ -255,17 +257,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
 #pragma unroll
                             for (int m = 0; m < (FEW ? 1 : MT); ++m) xv[m] = lds128(sb + (FEW ? xfew : xrow[m]) + (sa * F::KSA + 32 * q) * 2);
                             const uint32_t cwd[4] = {q ? cv.z : cv.x, q ? cv.w : cv.y, 0u, 0u}, ewd[2] = {q ? ev.z : ev.x, q ? ev.w : ev.y};
-                            if constexpr (FEW) {  // (one MMA a fragment: the scales go into the activations, as of up to eight rows)
-#pragma unroll
-                                for (int jj = 0; jj < 2; ++jj) {
-                                    const uint32_t w = cwd[jj], w8 = __funnelshift_r(w, w, 8);
-                                    const uint32_t s0 = and_or(ewd[jj], TKD_EMASK_BFP4, ebase(sh));
-                                    const uint32_t s1 = and_or(shl_fma<7>(ewd[jj], sh.y), TKD_EMASK_BFP4, ebase(sh));
-                                    mma_bf16(acc[jj][0], w & TKD_MASK_BFP4, shl_fma<4>(w, sh.x) & TKD_MASK_BFP4, w8 & TKD_MASK_BFP4,
-                                             shl_fma<4>(w8, sh.x) & TKD_MASK_BFP4, mul_bf16x2(jj ? xv[0].z : xv[0].x, s0),
-                                             mul_bf16x2(jj ? xv[0].w : xv[0].y, s1));
-                                }
-                            } else if constexpr (MT == 1) {
+                            if constexpr (MT == 1) {
                                 block_mma<TKD_BFP4, MT, 2>(acc, cwd, ewd, xv, sh);
                             } else {
 #pragma unroll
@@ -276,7 +268,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
                                     const uint32_t a0 = mul_bf16x2(w & TKD_MASK_BFP4, s0), a1 = mul_bf16x2(shl_fma<4>(w, sh.x) & TKD_MASK_BFP4, s0);
                                     const uint32_t a2 = mul_bf16x2(w8 & TKD_MASK_BFP4, s1), a3 = mul_bf16x2(shl_fma<4>(w8, sh.x) & TKD_MASK_BFP4, s1);
 #pragma unroll
-                                    for (int m = 0; m < MT; ++m)
+                                    for (int m = 0; m < (FEW ? 1 : MT); ++m)
                                         mma_bf16(acc[jj][m], a0, a1, a2, a3, jj ? xv[m].z : xv[m].x, jj ? xv[m].w : xv[m].y);
                                 }
                             }

@@ -554,3 +554,36 @@ def test_rows_of_experts_few_and_many_chose(device, rows, k):
             assert ((got - want).norm() / want.norm()).item() < 6e-3, (q, r)
     assert not h[rows:].any()
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("rows,chosen", [(9, 1), (16, 8), (16, 9), (32, 8)])
+def test_rows_of_large_inputs_stay_finite(device, rows, chosen):
+    """gate_up_rows of nine and more rows with inputs of 2^66: finite products and sums stay finite, however many rows chose the
+    expert (an activation times the largest scale, 2^64, is past bf16's range). h against float64: within three times its own rounding
+    to bf16, 2^-9."""
+    E, H, I = 4, 96, 32
+    g = torch.Generator().manual_seed(rows + chosen)
+    on_grid = lambda t: torch.from_numpy(  # noqa: E731
+        moe8.bfp4_values(moe8.bfp4_tiles(t)).transpose(0, 2, 1, 3).reshape(t.shape[0], t.shape[1]).copy())
+    gu = torch.stack([on_grid(torch.randn(H, 2 * I, generator=g) * 2.0**-70) for _ in range(E)])
+    dn = torch.stack([on_grid(torch.randn(I, H, generator=g) * 0.05) for _ in range(E)])
+    P = moe8.pack(device, gu, dn)
+    ids = torch.full((rows, 1), 2)
+    ids[torch.randperm(rows, generator=g)[:chosen], 0] = 1
+    w = (0.5 + torch.rand(rows, 1, generator=g)).to(torch.bfloat16)
+    x = (torch.randn(rows, H, generator=g) * 2.0**66).to(torch.bfloat16)
+    put = lambda t, d: ttnn.from_torch(t.reshape(1, 1, *t.shape), dtype=d, layout=ttnn.TILE_LAYOUT, device=device)  # noqa: E731
+    h = ttnn.to_torch(moe8.gate_up_rows(put(x, ttnn.bfloat16), P, put(ids.to(torch.int16), ttnn.uint16), put(w, ttnn.bfloat16), 1, rows))
+    h = h.double().reshape(32, -1)
+    assert h.isfinite().all()
+    union = sorted(set(ids.reshape(-1).tolist()))
+    for q, e in enumerate(union):
+        for r in range(rows):
+            got = h[r, q * I : (q + 1) * I]
+            if ids[r, 0] != e:
+                assert not got.any()
+                continue
+            up, gate = (x[r].double() @ m for m in (gu[e].double()[:, :I], gu[e].double()[:, I:]))
+            want = torch.nn.functional.silu(gate) * up * float(w[r, 0])
+            assert ((got - want).norm() / want.norm()).item() < 6e-3, (q, r)
+    linear.check_status(device)
