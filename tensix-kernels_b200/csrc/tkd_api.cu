@@ -124,7 +124,7 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     p.K = (int)a->k;
     p.nseg = a->nblocks;
     p.epi = a->epilogue;
-    p.act = a->act;
+    p.act = a->epilogue == TKD_EPI_SILU ? 0 : a->act;  // (silu is no GLU's choice)
     p.mul16 = 16, p.mul128 = 128;
     const int mt = a->m <= 8 ? 1 : (a->m <= 16 ? 2 : 4);
     const int sab = tkd_sab(a->fmt);

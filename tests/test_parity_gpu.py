@@ -859,3 +859,17 @@ def test_linear_silu_of_long_rows(device, fmt, m, k):
             plain = plain * ttnn.to_torch(ts).double().reshape(-1)
         close_bf16(host(linear.linear(dev_x(device, x), tw, ts if scaled else None, activation="silu")), torch.nn.functional.silu(plain).numpy())
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("m,k", [(1, 1024), (5, 544), (8, 14336), (16, 1056), (32, 1056), (32, 4096), (40, 1056), (300, 4096)])
+def test_the_silu_output_stage_has_no_other_activation(device, m, k):
+    """TKD_EPI_SILU is silu whatever `act` (a GLU's) says, in every kernel: the same bits with act 1."""
+    g = torch.Generator().manual_seed(m + k)
+    tw, _ = linear.native_weight(device, torch.randn(144, k, generator=g) * 0.06, ttnn.bfloat8_b)
+    tx = dev_x(device, torch.randn(m, k, generator=g))
+    first = host(linear.linear(tx, tw, None, activation="silu"))
+    (call,) = tw.calls.values()
+    for _, a in call.launches:
+        a.act = 1
+    assert torch.equal(host(linear.linear(tx, tw, None, activation="silu")), first)
+    linear.check_status(device)
