@@ -144,9 +144,11 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
     };
 
     // gate_up: the rows that chose the expert of slot q, a bit each (by a whole warp). Up to eight of them (of 16 rows and 8 of 128 experts
-    // one or two as a rule) are brought and multiplied alone, as rows 0, 1, ..: one MMA a fragment. (The scales in those rows'
-    // activations: gate_up of 16 rows, 8 of 128 experts of 2048 x 1536, 49.9 us, of 32 rows 80.6; in the weights 50.6 and 82.7, but
-    // an input's range does not depend on how many rows chose the same expert.)
+    // one or two as a rule) are multiplied alone, one MMA a fragment: a lane's column of it is its row among them. Us of gate_up with all
+    // rows multiplied / so: 8 of 128 experts of 2048 x 1536, 16 rows 51.9 / 46.1, 24 rows 79.9 / 73.5, 32 rows 108.8 / 83.1; 2 of 8 of
+    // 4096 x 4096, 16 rows 30.8 / 27.5, 24 rows 38.8 / 39.1, 32 rows 46.5 / 46.7. All rows are brought: a producer that picks is one warp
+    // with a row after the other, and took the latter's 16 rows to 34. (With the scales in the activations instead of the weights 32
+    // rows of the former take 2 us less, but then an input's range depends on how many rows chose the expert.)
     constexpr bool PICK = !DOWN && MT > 1 && FMT == TKD_BFP4;
     auto rows_of = [&](int q) {
         const int e = ulist[q];
@@ -158,8 +160,6 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
-        int qm = -1;
-        uint32_t mask = 0;
         uint32_t st = 0;
         bool ok = true;
         if (i0 < i1) {
@@ -178,14 +178,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
                 // the rows' inputs, 8 k a piece
                 const uint16_t* xq = p.x + (DOWN ? (int64_t)a.q * K : 0) + a.c * CK;
                 const int pieces = min(CK, K - a.c * CK) / 8;
-                if (PICK && a.q != qm) qm = a.q, mask = rows_of(qm);
-                const bool few = PICK && __popc(mask) <= 8;
-                for (int e = lane; few && e < pieces; e += 32) {
-                    uint32_t xd = dst + p.w_bytes + e * 16;
-                    for (uint32_t left = mask; left; left &= left - 1, xd += p.x_stride)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(xd), "l"(xq + (__ffs(left) - 1) * p.ldx + e * 8) : "memory");
-                }
-                for (int e = lane; !few && e < pieces; e += 32) {
+                for (int e = lane; e < pieces; e += 32) {
                     const uint16_t* xr = xq + e * 8;
                     uint32_t xd = dst + p.w_bytes + e * 16;
 #pragma unroll 8
@@ -229,8 +222,10 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
             const int c = a.c;
             if (PICK && a.q != qm) {
                 qm = a.q;
-                const int n = __popc(rows_of(qm));
-                few = n <= 8, xfew = p.w_bytes + max(min(g, n - 1), 0) * p.x_stride + 16 * t;
+                const uint32_t mask = rows_of(qm);
+                const int n = __popc(mask);
+                few = n <= 8;
+                xfew = p.w_bytes + (uint32_t)(n ? __fns(mask, 0, min(g, n - 1) + 1) : 0) * p.x_stride + 16 * t;
             }
             // (the expert's last block here: its group's largest exponent is asked for before the stage is waited for)
             const bool fold = c == nch - 1 || it == i1 - 1, deliver = a.j == nb - 1 || it == i1 - 1;
@@ -440,21 +435,23 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
                 for (int m = 0; m < RW; m += 4) *reinterpret_cast<float4*>(col + m) = make_float4(v[m], v[m + 1], v[m + 2], v[m + 3]);
                 bar_output_warps();
                 const float *gp = pbuf + gc * MP + r0, *up = gp + 32 * MP;
-                const bool few = PICK && __popc(mask) <= 8;
                 uint16_t* op = p.out + (int64_t)r0 * p.ldo + (int64_t)q * (p.N / 2) + panel * 64 + o;
                 const int left = panel * 64 + o < p.N / 2 ? R - r0 : 0;
-                if (few) {
+                auto value = [&](int at, int m) { return f32_to_bf16_bits(moe_glu(gp[at] + bg, up[at] + bu, p.act) * wrow[r0 + m]); };
+                if (PICK && __popc(mask) <= 8) {
+                    // (the rows multiplied lie together, in order; the others' outputs are zeros)
+                    const uint32_t mine = mask >> r0 & ((1u << 4 * MT) - 1u);
+                    int at = __popc(mask & ((1u << r0) - 1u)) - r0;
+#pragma unroll
+                    for (int m = 0; m < 4 * MT; ++m) st16_if(m < left && !(mine >> m & 1u), op + m * p.ldo, (uint16_t)0);
 #pragma unroll 1
-                    for (int m = 0; m < 4 * MT; ++m, op += p.ldo) {
-                        const uint32_t bit = mask >> (r0 + m) & 1u;
-                        const int at = __popc(mask & ((1u << (r0 + m)) - 1u)) - r0;  // (the row's place among those multiplied)
-                        const float v = bit ? moe_glu(gp[at] + bg, up[at] + bu, p.act) * wrow[r0 + m] : 0.f;
-                        st16_if(m < left, op, f32_to_bf16_bits(v));
+                    for (uint32_t b = left > 0 ? mine : 0u; b; b &= b - 1, ++at) {
+                        const int m = __ffs(b) - 1;
+                        op[m * p.ldo] = value(at, m);
                     }
                 } else {
 #pragma unroll
-                    for (int m = 0; m < 4 * MT; ++m, op += p.ldo)
-                        st16_if(m < left, op, f32_to_bf16_bits(moe_glu(gp[m] + bg, up[m] + bu, p.act) * wrow[r0 + m]));
+                    for (int m = 0; m < 4 * MT; ++m, op += p.ldo) st16_if(m < left, op, value(m, m));
                 }
             }
             bar_output_warps();  // (the sums, wrow and sflag are read)
