@@ -199,7 +199,7 @@ int tkd_matmul(const TkdMatmul* a, void* stream);
 
 /* tkd_matmul for more rows than 32 (m from 33 to TKD_ROWS_MAX; the reference's row slices, linear.py:179-184): one weight or
  * pair, every output stage, no records, exchange, rotation or TKD_FMT_INT4 (TKD_ERR_UNSUPPORTED). A weight is read once for
- * every 256 rows. The workspace is as tkd_matmul's and may be the same one; its size is tkd_matmul_rows_workspace's. A
+ * every 256 rows. The output may share memory with x (which is then copied before anything is written). The workspace is as tkd_matmul's and may be the same one; its size is tkd_matmul_rows_workspace's. A
  * column's sum depends on K, the format and where a tile of columns is cut between CTAs: on the row count, N, max_ctas and the
  * number of SMs, not on the rows' values. A caller whose columns have to give the same bits alone and beside others (a weight
  * sharded over GPUs) takes slices of 32 rows by tkd_matmul, whose sums depend on K, the format and ks alone. */

@@ -542,6 +542,15 @@ static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     return 3.2 + 0.2 * k + most * (0.65 + (p.fmt == TKD_BF16 ? 0.8 : 0.65) * k) < 0.9 * (3.4 + 0.62 * wide_us + 1.85 * k);
 }
 
+// Whether a call's output shares memory with x. (More than 32 rows may: tkd_wide_kernel reads a copy of x.)
+static bool out_meets_x(const TkdMatmul* a) {
+    const TkdBlock& b = a->block[0];
+    const int64_t width = a->epilogue == TKD_EPI_GLU_IL ? b.n / 2 : b.n, esz = a->out_dtype == TKD_DT_F32 ? 4 : 2;
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(a->x), x1 = x0 + ((a->m - 1) * a->ldx + a->k) * 2;
+    const uintptr_t y0 = reinterpret_cast<uintptr_t>(a->out) + b.out_col0 * esz, y1 = y0 + ((a->m - 1) * a->ldo + width) * esz;
+    return x0 < y1 && y0 < x1;
+}
+
 // A call's tensors in the parameters of its launch (but for the workspace).
 static void bind(const TkdMatmul* a, TkdParams* p) {
     p->x = static_cast<const uint16_t*>(a->x);
@@ -571,7 +580,7 @@ int tkd_matmul_rows(const TkdMatmul* a, void* stream) {
     if (!a->workspace || a->workspace_bytes < need) return TKD_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(a->workspace) & 255) return TKD_ERR_BAD_ARG;
     Layout L;
-    if (rows_tiles(a, &L, us)) {
+    if (!out_meets_x(a) && rows_tiles(a, &L, us)) {  // (that kernel reads x while other CTAs write their outputs)
         bind(a, &L.p);
         return launch_err(tkd_launch_stream(L.p, L.grid, L.smem, static_cast<cudaStream_t>(stream)));
     }

@@ -873,3 +873,28 @@ def test_the_silu_output_stage_has_no_other_activation(device, m, k):
         a.act = 1
     assert torch.equal(host(linear.linear(tx, tw, None, activation="silu")), first)
     linear.check_status(device)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bf16"])
+@pytest.mark.parametrize("m", [33, 64, 300])
+def test_more_rows_in_place(device, fmt, m):
+    """More than 32 rows whose output is x's own memory, or overlaps it: what an output of its own gets, within the rounding of other
+    sums (such a call runs the kernel that reads a copy of x)."""
+    g = torch.Generator().manual_seed(m)
+    k = n = 288
+    tw, _ = linear.native_weight(device, torch.randn(n, k, generator=g) * 0.06, DT[fmt])
+    x = torch.randn(m, k, generator=g)
+    want = host(linear.matmul(dev_x(device, x), tw, None))
+    tx = dev_x(device, x)
+    for _ in range(2):
+        linear.matmul(tx, tw, None, out=tx)
+        close_bf16(host(tx), want)
+        tx.t.copy_(x.reshape(1, 1, m, k))
+    # (the output's first row is x's last)
+    both = torch.empty(1, 1, 2 * m - 1, k, dtype=torch.bfloat16, device=device.torch)
+    both[..., :m, :] = x.to(device.torch)
+    view = lambda t: ttnn.Tensor(t, ttnn.bfloat16, ttnn.TILE_LAYOUT, device, ttnn.DRAM_MEMORY_CONFIG)  # noqa: E731
+    out = view(both[..., m - 1 :, :])
+    linear.matmul(view(both[..., :m, :]), tw, None, out=out)
+    close_bf16(host(out), want)
+    linear.check_status(device)
