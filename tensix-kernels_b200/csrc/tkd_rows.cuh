@@ -131,12 +131,15 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
     __syncthreads();
     const uint32_t T = 4u * (uint32_t)p.total_panels;  // items
     // (more than 32 rows: tiles of rows, a team of CTAs each)
-    const uint32_t team = p.rows_team ? p.rows_team : gridDim.x, tile0 = blockIdx.x / team, cta = blockIdx.x - tile0 * team;
-    const int i0 = (int)((uint64_t)T * cta / team), i1 = (int)((uint64_t)T * (cta + 1) / team), ni = i1 - i0;
-    const int step = TURNS ? gridDim.x / team : 1, turns = TURNS ? ((p.M - 1) / p.rows_tile - (int)tile0) / step + 1 : 1;
-    // the rows of this CTA's tile number `turn`: the first, and how many
-    auto first_row = [&](int turn) { return ((int)tile0 + turn * step) * p.rows_tile; };
-    auto rows_of = [&](int turn) { return p.rows_tile ? min(p.rows_tile, p.M - first_row(turn)) : p.M; };
+    const uint32_t team = p.rows_team ? p.rows_team : gridDim.x, tile = blockIdx.x / team, cta = blockIdx.x - tile * team;
+    const int i0 = (int)((uint64_t)T * cta / team), i1 = (int)((uint64_t)T * (cta + 1) / team);
+    int row0 = (int)tile * p.rows_tile, M = p.rows_tile ? min(p.rows_tile, p.M - row0) : p.M;
+    // (TURNS: the first row and the number of rows of the tile after this one, `step` tiles on; false: there is none)
+    const int step = TURNS ? gridDim.x / team * p.rows_tile : 0;
+    auto next_tile = [&]() {
+        row0 += step, M = min(p.rows_tile, p.M - row0);
+        return TURNS && row0 < p.M;
+    };
     const int nst = p.nstages, K = p.K, nch = (K + CK - 1) / CK, nsa_total = (K + F::KSA - 1) / F::KSA;
     const int spi = (nch + SC - 1) / SC;  // stages of an item
     const int epi = p.epi;
@@ -155,26 +158,27 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
         uint32_t st = 0;
         bool ok = true;
         const int s = lane >> 1, g = lane & 1;
-        for (int j = 0; ok && j < turns * ni; ++j) {
-            const int it = i0 + (TURNS ? j % ni : j);
-            const TkdSegDev& sg = p.seg[seg_of(it)];
-            const NarrowItem n = narrow_item(p, it - 4 * sg.panel0);
-            const uint8_t* src = (g && epi == TKD_EPI_GLU2 ? sg.w2 : sg.w) + (int64_t)n.panel * p.panel_bytes;
-            for (int i = 0; i < spi; ++i, ++st) {
-                const uint32_t q = st % nst;
-                ok = __all_sync(0xFFFFFFFFu, mbar_wait_parked(empty0 + 8 * q, ((st / nst) & 1) ^ 1, p.status));
-                if (!ok) break;
-                const int c = i * SC + s;  // this lane's chunk, if there is one
-                const bool mine = s < SC && c < nch && (glu || !g);
-                const uint32_t gb = mine ? (uint32_t)min(F::SUBSA, nsa_total - c * F::SUBSA) * F::SAB : 0u, bytes = glu ? gb : 2 * gb;
-                const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, bytes);
-                if (lane == 0) mbar_expect_tx(full0 + 8 * q, all);
-                __syncwarp();
-                if (mine)
-                    bulk_g2s(ring0 + q * p.stage_bytes + s * 2 * GB + g * gb, src + (int64_t)c * (GB * 8) + (int64_t)(g ? n.gb : n.ga) * gb, bytes,
-                             full0 + 8 * q);
+        do {
+            for (int it = i0; ok && it < i1; ++it) {
+                const TkdSegDev& sg = p.seg[seg_of(it)];
+                const NarrowItem n = narrow_item(p, it - 4 * sg.panel0);
+                const uint8_t* src = (g && epi == TKD_EPI_GLU2 ? sg.w2 : sg.w) + (int64_t)n.panel * p.panel_bytes;
+                for (int i = 0; i < spi; ++i, ++st) {
+                    const uint32_t q = st % nst;
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_parked(empty0 + 8 * q, ((st / nst) & 1) ^ 1, p.status));
+                    if (!ok) break;
+                    const int c = i * SC + s;  // this lane's chunk, if there is one
+                    const bool mine = s < SC && c < nch && (glu || !g);
+                    const uint32_t gb = mine ? (uint32_t)min(F::SUBSA, nsa_total - c * F::SUBSA) * F::SAB : 0u, bytes = glu ? gb : 2 * gb;
+                    const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, bytes);
+                    if (lane == 0) mbar_expect_tx(full0 + 8 * q, all);
+                    __syncwarp();
+                    if (mine)
+                        bulk_g2s(ring0 + q * p.stage_bytes + s * 2 * GB + g * gb, src + (int64_t)c * (GB * 8) + (int64_t)(g ? n.gb : n.ga) * gb, bytes,
+                                 full0 + 8 * q);
+                }
             }
-        }
+        } while (TURNS && next_tile());
         if (!ok)  // (the copies in flight land before the CTA goes)
             for (uint32_t back = 1; back <= (uint32_t)nst && back <= st; ++back)
                 for (uint32_t i = 0; i < 64; ++i)
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
         const int cw = warp - kRowsOut - 1, g = lane >> 2, t = lane & 3;
         if (nch * CK > K) {
             // the rows of x end in zeros up to a whole chunk
-            for (int r = cw; r < rows_of(0); r += SW)  // (no later tile has more)
+            for (int r = cw; r < M; r += SW)  // (no later tile has more)
                 for (int e = K / 8 + lane; e < nch * (CK / 8); e += 32)
                     asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(xt0 + r * p.x_stride + e * 16), "r"(0u) : "memory");
             asm volatile("bar.sync 2, %0;" ::"n"(SW * 32) : "memory");
@@ -193,10 +197,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
         asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t at = ring0, bar = full0, phase = 0;
         bool ok = true;
-        for (int turn = 0; turn < turns; ++turn) {
-            const int row0 = first_row(turn), M = rows_of(turn);
-            // (the rows of the tile before have been read by every warp: one whose wait gave up comes here too)
-            if (TURNS && turn) asm volatile("bar.sync 2, %0;" ::"n"(SW * 32) : "memory");
+        int n = 0;              // items of the tiles before this one
+        uint32_t xphase = 0;
+        do {
             for (int s = 0; s < kRowsSegs; ++s) {  // (the last part: all that is left)
                 const int e0 = min(s * SC * CK, K) / 8, e1 = s == kRowsSegs - 1 ? K / 8 : min((s + 1) * SC * CK, K) / 8;
                 for (int r = cw; r < M; r += SW) {
@@ -222,8 +225,8 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
             const uint32_t ring_end = ring0 + nst * p.stage_bytes;
             const uint32_t slot = pbuf + (cw & 7) * SLOT + ((2 * t) * PP + g) * 4;  // (where this lane's sums go)
             float acc[2][MT][4];
-            for (int j0 = 0; ok && j0 < ni; ++j0) {
-                const int j = turn * ni + j0;
+            for (int j0 = 0; ok && j0 < i1 - i0; ++j0) {
+                const int j = n + j0;
 #pragma unroll
                 for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
                 int c = 0;
 #pragma unroll 1
                 for (int i = 0; i < spi; ++i, xk += SC * CK * 2, c += SC) {
-                    if (j0 == 0) ok = mbar_wait(xbar0 + 8 * min(i, kRowsSegs - 1), turn & 1, p.status);
+                    if (j0 == 0) ok = mbar_wait(xbar0 + 8 * min(i, kRowsSegs - 1), xphase, p.status);
                     ok = ok && mbar_wait(bar, phase, p.status);
                     if (!ok) break;
                     const uint32_t ca = at + code_lane, ea = at + exp_lane;
@@ -296,18 +299,26 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
                 __syncwarp();
                 if (lane == 0) mbar_arrive(cw >= 8 ? half0 + 8 * (cw - 8) : pfull);
             }
-        }
+            if (!TURNS || !next_tile()) break;
+            // (every warp has read this tile's rows: one whose wait gave up comes here too)
+            asm volatile("bar.sync 2, %0;" ::"n"(SW * 32) : "memory");
+            n += i1 - i0, xphase ^= 1;
+        } while (true);
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // ---------------------------------------------------------------- output warps
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const int ow = warp, npeers = PLAIN ? 0 : p.npeers;
+        int left = M - RW * ow;  // rows from this warp's first on
+        int topk_k = PLAIN || tile ? 0 : p.topk_k;
         const bool up = glu && lane >= 16, f32out = epi == TKD_EPI_OUT32;
         bool met = true;
-        for (int j = 0; j < turns * ni; ++j) {
-            const int turn = TURNS ? j / ni : 0, row0 = first_row(turn), left = rows_of(turn) - RW * ow;  // rows from this warp's first on
-            const int topk_k = PLAIN || row0 ? 0 : p.topk_k;
-            const int it = i0 + (TURNS ? j % ni : j), seg = seg_of(it);
+        for (int j = 0, it = i0;; ++j, ++it) {
+            if (it == i1) {
+                if (!TURNS || !next_tile()) break;
+                it = i0, left = M - RW * ow, topk_k = 0;
+            }
+            const int seg = seg_of(it);
             const TkdSegDev& sg = p.seg[seg];
             const int pl = it - 4 * sg.panel0;
             const int plw = !PLAIN && p.rep_panels ? pl % (4 * p.rep_panels) : pl;  // (the item's number in its weight)
