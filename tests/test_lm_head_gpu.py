@@ -243,10 +243,11 @@ def test_pick_takes_the_earliest_of_equal_keys(device, nrec, rows, k, top):
         assert (int(rtok[t]), int(rcount[t])) == (ids[order][0], len(order)), t
 
 
-@pytest.mark.parametrize("nrec,rows,k,top", [(1, 1, 4, 1), (3, 2, 4, 32), (75, 1, 8, 16), (300, 3, 4, 9), (512, 1, 4, 32), (513, 2, 2, 16), (300, 2, 8, 32)])
+@pytest.mark.parametrize("nrec,rows,k,top", [(1, 1, 4, 1), (3, 2, 4, 32), (75, 1, 8, 16), (300, 3, 4, 9), (512, 1, 4, 32), (513, 2, 2, 16), (300, 2, 8, 32),
+                                            (180, 2, 4, 9), (181, 2, 4, 9)])
 def test_picks_from_records_with_ties_and_holes(device, nrec, rows, k, top):
     """The best slots of arbitrary records (few distinct keys, empty slots, ids past the vocabulary, a record's slots in no order), by
-    counting and, past 2048 slots or 512 records, in rounds: the first candidate and how many are held, and the pick among their
+    counting and, past 2048 slots, 512 records or twenty records for each of the top, in rounds: the first candidate and how many are held, and the pick among their
     exact logits, as numpy finds them."""
     g = np.random.default_rng(nrec + k)
     dim, vocab = 64, 4000
