@@ -53,7 +53,7 @@ int tc_cluster_count(int fmt, size_t smem) {
 }
 
 // 9 to 32 rows: tkd_rows_kernel's chunks of a stage, with its shared-memory map in p; 0: the tensor-memory kernel. A rule on K, the
-// format and the rows in eights only, because the two kernels' sums are different ones and a column's must not depend on more; it
+// format and the number of rows only, because the two kernels' sums are different ones and a column's must not depend on more; it
 // goes for records and exchanged calls as well. Measured, launches in a graph over weights larger than L2, us with tkd_rows_kernel /
 // the tensor-memory kernel: 9 to 16 rows, wherever x leaves 80 KB of the 227 to the ring: bfloat8_b [1280, 4096] 4.8 / 6.8, [2048, 14336]
 // 10.9 / 12.5, [3328, 14336] with 16 rows, the worst, 16.6 / 16.0; bfloat4_b [2816, 4096] 5.9 / 9.2; less of a ring: bfloat8_b [4096, 14336]
@@ -93,8 +93,9 @@ struct Layout {
 };
 
 // Everything a launch needs except the device pointers into the workspace. sms 0: ask the device.
-// counted: the kernel with the counters and slice sums of the workspace, even where tkd_narrow_kernel could run.
-int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
+// counted: the kernel with the counters and slice sums of the workspace, even where tkd_narrow_kernel could run. tile: a is a tile of the
+// rows of a call of more than 32.
+int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false, bool tile = false) {
     if (!a || !fmt_ok(a->fmt)) return TKD_ERR_BAD_ARG;
     if (a->m < 1 || a->m > 32 || a->k < 32 || a->k % 32 || a->k > (1 << 24)) return TKD_ERR_BAD_ARG;
     // (the int4 weight with group scales is the reference's one-token op; more rows go through its dequantised
@@ -167,6 +168,10 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     }
     p.total_panels = panels;
     p.total_items = (int64_t)panels * p.nslices;
+    const bool on_device = sms <= 0;
+    if (sms <= 0) sms = sm_count();
+    if (sms <= 0) sms = 148;
+    if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
 
     // shared-memory map: barriers, the hand-over buffers of the streaming warps, the GLU exchange buffer, the ring
     const int mp = mt == 1 ? 8 : (mt == 2 ? 24 : 40);
@@ -197,13 +202,20 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
         // Items of 32 columns over all of K (tkd_narrow.cuh) where the call is a plain one of one to four slices, and two stages of
         // the ring fit beside x (a stage has a chunk of every slice, 35 KB at four; bf16, whose loads need the most in flight, three).
         // A streaming warp stays with one slice, so those of a short last slice wait, and with fewer slices some have none; still
-        // that is the faster form everywhere, since no sums go through L2. Measured, launches in a graph over weights larger than
-        // L2, us with this kernel / the counting one: bfloat8_b one row, [1280, 4096] (three slices) 3.7 / 4.9, [2080, 4096] (a
+        // that is the faster form, since no sums go through L2, but for a K of one slice, whose sums need not: there only up to an item
+        // for every other CTA; and of two or three slices at one row, or of bf16, only up to six items a CTA. Measured, launches in a
+        // graph over weights larger than L2, us with this kernel / the counting one: bfloat8_b one row, [256, 2048] 1.9 / 2.3, [256, 5392]
+        // 3.2 / 2.3, [256, 20480] 5.0 / 4.5, with w_up [1536, 20480] 15.3 / 13.6; bf16 one row, [128, 5392] 3.5 / 2.1, with w_up
+        // [384, 20480] 11.0 / 8.9; bfloat8_b one row, [1280, 4096] (three slices) 3.7 / 4.9, [2080, 4096] (a
         // third of the last) 4.7 / 5.9; eight rows, [1280, 4096] 4.2 / 5.9, bfloat4_b [5120, 4096] 6.0 / 10.6, [8192, 11008] (two
         // stages) 17.2 / 21.9; bfloat8_b [8192, 11008] (two stages) 25.7 / 25.8. Two stages of bf16: [8192, 1024] 12.6 / 11.5.
         const int64_t narrow_xt = p.off_pbuf + 2 * 8 * 32 * (a->m > 1 ? 8 : 1) * 4;
         const int narrow_stage = p.nslices * 2 * tkd_subsa(a->fmt) * sab;
-        if (!counted && p.nslices <= 4 && !a->topk_k && a->nranks <= 1 &&
+        const int64_t items = 4 * (int64_t)panels;
+        const bool faster = p.nslices == 1   ? 2 * items <= sms
+                            : p.nslices < 4 ? items <= 6 * (int64_t)sms || (a->m > 1 && a->fmt != TKD_BF16)
+                                            : p.nslices == 4;
+        if (!counted && faster && !a->topk_k && a->nranks <= 1 &&
             narrow_xt + a->m * x_row + (a->fmt == TKD_BF16 ? 3 : 2) * (int64_t)narrow_stage + 128 <= kMaxSmem) {
             p.stage_bytes = narrow_stage;
             p.narrow = p.x_smem = 1;
@@ -218,11 +230,9 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false) {
     if (p.nstages < 2) return TKD_ERR_UNSUPPORTED;
     L->smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
 
-    const bool on_device = sms <= 0;
-    if (sms <= 0) sms = sm_count();
-    if (sms <= 0) sms = 148;
-    if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
-    if (p.tc && !a->ks) p.rows_chunks = rows_layout(p, sab);
+    // (a K of one slice: the tensor-memory kernel, a panel an item, no sums through L2. Us with tkd_rows_kernel / with that: bfloat4_b
+    // [512, 11008] 24 rows 10.2 / 5.3; bfloat8_b [256, 11008] 32 rows 7.7 / 4.6, [256, 5392] 9 rows 4.8 / 3.5, with w_up [256, 2048] 4.0 / 4.4)
+    if (p.tc && !a->ks && (p.nslices > 1 || tile)) p.rows_chunks = rows_layout(p, sab);
     if (p.rows_chunks) p.tc = 0, L->smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
     const int64_t items = p.narrow || p.rows_chunks ? 4 * (int64_t)panels : p.total_items;
     // (tiles of rows: a team of CTAs each; where max_ctas leaves fewer than the tiles, one for several)
@@ -529,7 +539,7 @@ static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     TkdMatmul one = *a;
     TkdParams& p = L->p;
     for (one.m = 16; one.m >= 12; one.m -= 4) {
-        if (make_layout(&one, L, sms)) return false;
+        if (make_layout(&one, L, sms, false, true)) return false;
         if (p.rows_chunks) break;
     }
     if (!p.rows_chunks) return false;
