@@ -66,7 +66,8 @@ int tc_cluster_count(int fmt, size_t smem) {
 int rows_layout(TkdParams& p, int sab) {
     const int ck = tkd_chunk_k(p.fmt), nch = (p.K + ck - 1) / ck;
     if (p.M > 16 && p.nslices == 4 && (p.M > 24 || p.K > 1536)) return 0;
-    for (int rows = p.M > 24 && p.fmt != TKD_BF16 && p.K <= 2816 ? 16 : p.M;; rows = 16) {
+    if (p.M > 24 && p.fmt != TKD_BF16 && p.K > 2816) return 0;  // (no tiles, and no instance of four MMAs a block-float fragment)
+    for (int rows = p.M > 24 && p.fmt != TKD_BF16 ? 16 : p.M;; rows = 16) {
         const int mt = (rows + 7) / 8;
         const int64_t x_row = (int64_t)nch * ck * 2 + 64, tbuf = TKD_SMEM_HEAD + 8 * 8 * mt * TKD_ROWS_PITCH * 4;
         const int64_t xt = tbuf + 1024, ring = align_up(xt + rows * x_row, 128);  // (1 KB: the lists of top-k records)

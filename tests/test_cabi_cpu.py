@@ -154,3 +154,13 @@ def test_no_plan_takes_more_ctas_than_it_may(tkd):
                 for ctas in (1, 2, 3, 5, 147):
                     rc, p = plan(tkd, fmt=fmt, m=m, k=k, ns=[2224], max_ctas=ctas)
                     assert rc == 0 and 1 <= p.grid <= ctas, (fmt, m, k, ctas, p.grid)
+
+
+def test_25_to_32_rows_past_the_tiles_run_the_tensor_memory_kernel(tkd):
+    """tkd_rows_kernel has no instance of four MMAs a block-float fragment: where K is too long for two tiles of sixteen rows, an item is a
+    slice of a panel, of which one CTA takes one (and not 32 columns, of which four CTAs would take a panel)."""
+    for k in range(2848, 4097, 32):
+        for m in (25, 32):
+            for fmt in (tkd.FMT_BFP8, tkd.FMT_BFP4):
+                rc, p = plan(tkd, fmt=fmt, m=m, k=k, ns=[128])
+                assert rc == 0 and p.grid == p.items == p.nslices and (p.nslices == 4 or p.grid < 4), (fmt, m, k)
