@@ -122,7 +122,7 @@ typedef struct {
     int32_t nblocks;        /* 1, or 2..4 for a block list (linear.py:615-624) */
     int32_t epilogue;       /* TKD_EPI_* */
     TkdBlock block[4];
-    int32_t act;            /* GLU: 0 silu, 1 gelu_tanh (common/kernels/dense_ops.h:44-59) */
+    int32_t act;            /* GLU: 0 silu, 1 gelu_tanh (common/kernels/dense_ops.h:44-59); TKD_EPI_SILU: not looked at */
     int32_t scale_dtype;    /* TKD_DT_NONE | BF16 (the reference's scale tensor) | F32 (extension) */
     const void* scale;      /* [n] per output column of w */
     const void* scale_up;   /* [n] of w_up (an extension: scales with a GLU) */
@@ -199,10 +199,11 @@ int tkd_matmul(const TkdMatmul* a, void* stream);
 
 /* tkd_matmul for more rows than 32 (m from 33 to TKD_ROWS_MAX; the reference's row slices, linear.py:179-184): one weight or
  * pair, every output stage, no records, exchange, rotation or TKD_FMT_INT4 (TKD_ERR_UNSUPPORTED). A weight is read once for
- * every 256 rows. The output may share memory with x (which is then copied before anything is written). The workspace is as tkd_matmul's and may be the same one; its size is tkd_matmul_rows_workspace's. A
- * column's sum depends on K, the format and where a tile of columns is cut between CTAs: on the row count, N, max_ctas and the
- * number of SMs, not on the rows' values. A caller whose columns have to give the same bits alone and beside others (a weight
- * sharded over GPUs) takes slices of 32 rows by tkd_matmul, whose sums depend on K, the format and ks alone. */
+ * every 256 rows, a small one for every 16. The output may share memory with x (which is then copied before anything is written).
+ * The workspace is as tkd_matmul's and may be the same one; its size is tkd_matmul_rows_workspace's. A column's sum depends on K,
+ * the format, the kernel and where a tile of columns is cut between CTAs: on the row count, N, max_ctas and the number of SMs, not
+ * on the rows' values. A caller whose columns have to give the same bits alone and beside others (a weight sharded over GPUs) takes
+ * slices of 32 rows by tkd_matmul, whose sums depend on K, the format, ks and the slice's rows alone. */
 #define TKD_ROWS_MAX 4096
 int tkd_matmul_rows_workspace(const TkdMatmul* a, uint64_t* bytes);
 int tkd_matmul_rows(const TkdMatmul* a, void* stream);

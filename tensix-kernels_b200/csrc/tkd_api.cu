@@ -62,7 +62,10 @@ int tc_cluster_count(int fmt, size_t smem) {
 // 32 rows of other numbers of slices: bf16 with four MMAs a fragment ([1056, 14336] 12.8 / 17.1); block-float decodes beside four MMAs
 // take longer than the tensor memory's way ([1056, 14336] 19.5 / 16.2), and so run as two tiles of sixteen rows, a team of CTAs each
 // (13.0 / 16.2; bfloat4_b [1056, 4096] 6.1 / 8.6), as do 17 and more rows whose x does not fit, up to K 2816 (bfloat4_b [2816, 14336]
-// 19.9 / 21.4; [3072, 14336] 20.4 / 18.7).
+// 19.9 / 21.4; [3072, 14336] 20.4 / 18.7). N may not enter, and the gain of 17 and more rows of a block-float weight ends at some 12000
+// to 20000 columns (with w_up both weights' count): 32 rows of bfloat8_b with w_up, [1536, 4608] 0.64 of the other's time, [1536, 6144]
+// 1.03, [1536, 20480] 1.37; 24 rows of bfloat4_b, [1024, 4096] 0.85, [1024, 20480] 1.24; K 2560 of bfloat4_b is the worst
+// ([2560, 5120] 32 rows 1.09, 17 rows 1.26).
 int rows_layout(TkdParams& p, int sab) {
     const int ck = tkd_chunk_k(p.fmt), nch = (p.K + ck - 1) / ck;
     if (p.M > 16 && p.nslices == 4 && (p.M > 24 || p.K > 1536)) return 0;

@@ -94,8 +94,8 @@ struct TkdParams {
     int exchange_wait;
     int tc;              // 9 to 32 rows: the tensor-memory kernel (tkd_stream_tc.cuh); off_xt is where its operand tiles go
     int tc_cluster;      // ... in clusters of four CTAs, a slice each
-    int rows_chunks;     // 9 to 24 rows: chunks of a stage of tkd_rows_kernel (tkd_rows.cuh); 0: the tensor-memory kernel
-    int rows_tile, rows_team;  // ... in tiles of rows: rows of a tile, CTAs of each tile (0: all rows, all CTAs)
+    int rows_chunks;     // 9 and more rows: chunks of a stage of tkd_rows_kernel (tkd_rows.cuh); 0: another kernel
+    int rows_tile, rows_team;  // ... in tiles of rows (17 and more): rows of a tile, CTAs of each tile (0: all rows, all CTAs)
     int rows_turns;            // ... and the CTAs are fewer than the tiles, which they take in turn
     int x_smem;          // 1 to 8 rows, and all of x (K rounded up to a chunk) fits in shared memory at off_xt
     int narrow;          // ... and the call runs tkd_narrow_kernel (tkd_narrow.cuh)

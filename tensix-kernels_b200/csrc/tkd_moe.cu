@@ -441,7 +441,7 @@ int moe_rows(const TkdMoe* a, cudaStream_t st) {
 template <bool DOWN>
 int moe_one(const TkdMoe* a, cudaStream_t st) {
     const MoeParams p = moe_params(a);
-    if (p.K > 112 * 1024) return TKD_ERR_UNSUPPORTED;
+    if (p.K > 112 * 1024) return TKD_ERR_UNSUPPORTED;  // (no limit of this kernel: what tkd_moe_gate_up and _down always refused)
     const int e = a->fmt == TKD_FMT_BF16 ? moe_launch<TKD_BF16, DOWN>(p, st) : moe_launch<TKD_BFP4, DOWN>(p, st);
     return e == 0 ? TKD_OK : TKD_ERR_CUDA + e;
 }

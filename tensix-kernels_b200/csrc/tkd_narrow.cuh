@@ -5,8 +5,8 @@
 // a launch of one row and 2.5 of one of eight, where one token through [4096, 2048] takes 5.5 us. Here a CTA takes two groups
 // of 16 columns over all of K, the same bytes, and its sixteen streaming warps are (slice, half of a chunk's super-atoms,
 // group): the sums are the same sums in the same order (T_h ascending over the slices, then T0 + T1: see there, the two kernels
-// give the same bits), but they meet in shared memory, and no CTA waits for another. The plain calls of one to four
-// slices whose rows of x fit in shared memory run this kernel (make_layout); FOUR: of four, an instance of its own, because what
+// give the same bits), but they meet in shared memory, and no CTA waits for another. Plain calls of one to four
+// slices whose rows of x fit in shared memory run this kernel, but for large weights of one to three (make_layout has the limits); FOUR: of four, an instance of its own, because what
 // fewer need (a count instead of a constant here and there) cost the calls of four 0.15 us. Measured, a launch of a sequence in a graph:
 // one row, [4096, 4096] of bfloat8_b 8.3 us before, 6.2 now (2.8 at the memory's rate), [2048, 3072] 5.3 and 3.5; eight rows of
 // bf16, [2048, 2048] 7.2 and 4.2 (1.3). Where an SM has several items the decode of the weights bounds both kernels.

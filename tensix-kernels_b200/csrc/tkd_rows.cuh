@@ -16,7 +16,7 @@
 //                  share. They bring x as well, 16 bytes a lane, a stage's part of K after the other
 //
 // A column's sum: streaming warp w's sums T_w over all its super-atoms, U_i = T_i + T_{i + 8}, then U_0 + U_1 + .. + U_7 in order. It
-// depends on K, the format and the number of rows in eights only.
+// depends on K and the format only; where this kernel runs goes by the number of rows as well (rows_layout).
 #pragma once
 #include "tkd_narrow.cuh"
 
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
     }
     __syncthreads();
     const uint32_t T = 4u * (uint32_t)p.total_panels;  // items
-    // (more than 32 rows: tiles of rows, a team of CTAs each)
+    // (tiles of rows: a team of CTAs each)
     const uint32_t team = p.rows_team ? p.rows_team : gridDim.x, tile = blockIdx.x / team, cta = blockIdx.x - tile * team;
     const int i0 = (int)((uint64_t)T * cta / team), i1 = (int)((uint64_t)T * (cta + 1) / team);
     int row0 = (int)tile * p.rows_tile, M = p.rows_tile ? min(p.rows_tile, p.M - row0) : p.M;

@@ -1,6 +1,6 @@
 // tkd_stream_kernel.cuh: the weight-streaming decode matmul for sm_100a (the kernel template; tkd_stream_bfp8.cu,
 // tkd_stream_bfp4.cu and tkd_stream_bf16.cu each compile one format's instantiations of it).
-// Plain calls of one to four slices run tkd_narrow_kernel instead (tkd_narrow.cuh, which shares this file's helpers and sums).
+// Most plain calls of one to four slices run tkd_narrow_kernel instead (tkd_narrow.cuh, which shares this file's helpers and sums).
 //
 // y[m, n] = sum_k x[m, k] * w[k, n] with its fused output stage, M <= 8 activation rows (more:
 // tkd_rows.cuh and tkd_stream_tc.cuh, which share this file's helpers), the weight a packed HBM stream (tkd_layout.h). It takes the place of the reference's three Tensix kernels (dense_reader/kernels/

@@ -291,8 +291,8 @@ def plan(device, x, w, cores_per_bank=3, full_sync=False, kb=None, kw=None, sbw=
     where they mean something here (MT, KT, NT, KW, SEGS, glu, glu2, out32, noscale, work, l1) and the kernel's own
     (KS: k per slice, SLICES, PANELS of 128 columns, ITEMS = PANELS x SLICES, GRID: CTAs, STAGES of the shared-memory
     ring, BYTES: the weight stream read). work: [(cta, (first item, items))], the contiguous run of items each CTA
-    takes (of the kernels that count panels in; plain calls of four slices may deal the same bytes out as 32 columns over
-    all of K, or to clusters of four CTAs). (linear.py:187-382; the Tensix options are accepted and ignored)"""
+    takes (of the kernels that count panels in; the others deal the same bytes out as items of 32 columns over all of K,
+    or to clusters of four CTAs). (linear.py:187-382; the Tensix options are accepted and ignored)"""
     blocks = tuple(blocks) if blocks else (w,)
     if len(blocks) > 1:
         assert 2 <= len(blocks) <= 4, f"dense_reader: {len(blocks)} blocks (at most 4)"
@@ -435,9 +435,9 @@ def matmul(x, w, scale, *, memory_config=None, fidelity="hifi2", full_sync=False
     buffer, are also written to every other rank's buffer, and the call completes when all ranks' have arrived.
     col_scales=(gate scales, up scales) float32 [N] each with w_up (or one float32 vector in the
     interleaved weight's column order with glu); a float32 residual with out32 (y = x @ w + residual in float32);
-    fixed_sums=True: more than 32 rows run as slices of 32 as well, whose sums depend on K, the format and ks alone; those of one
-    launch depend on where its tiles are cut, which goes by N, the rows and the number of CTAs (a weight's columns, or a part of
-    them on each GPU, may then differ in a rounding).
+    fixed_sums=True: more than 32 rows run as slices of 32 as well, whose sums depend on K, the format, ks and a slice's rows alone;
+    those of one launch depend on its kernel and where its tiles are cut, which go by N, the rows and the number of CTAs (a weight's
+    columns, or a part of them on each GPU, may then differ in a rounding).
     hadamard= (the sign words of ternary_matmul.t2.hadamard_signs; int4-stream weights only): x is rotated by the block
     Hadamard inside the kernel first.
 
@@ -883,8 +883,9 @@ def topk_units(n):
 
 def linear(x, w, scale, memory_config=None, activation=None, out_dtype=None, **opts):
     """matmul for x of any rank: x [..., rows, K] bf16, the output's rank the input's. activation: None, "silu"
-    (in the kernel's output stage, on the float32 sums; after the matmul with a given out, a residual, out32 or a top-k), "swiglu" or "geglu" (w is interleave_glu's weight with scale None, the output N / 2
-    wide; or w is (gate, up), the output N wide). out_dtype ttnn.float32: out32. A block list for w: plain weights with
+    (of the float32 sums, in the kernel's output stage, rounded once; with a given out, a residual or a top-k of the product as it is
+    stored, rounded to bf16 before and after; with out32 of the float32 product), "swiglu" or "geglu" (w is interleave_glu's weight with
+    scale None, the output N / 2 wide; or w is (gate, up), the output N wide). out_dtype ttnn.float32: out32. A block list for w: plain weights with
     activation None, (gate, up) pairs with "swiglu" or "geglu". opts go to matmul. (linear.py:1073-1124)"""
     key = None
     if type(w) is ttnn.Weight and not opts and CACHE and x.t.dim() == 4 and (activation is None or type(activation) is str):

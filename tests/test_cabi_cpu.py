@@ -164,3 +164,16 @@ def test_25_to_32_rows_past_the_tiles_run_the_tensor_memory_kernel(tkd):
             for fmt in (tkd.FMT_BFP8, tkd.FMT_BFP4):
                 rc, p = plan(tkd, fmt=fmt, m=m, k=k, ns=[128])
                 assert rc == 0 and p.grid == p.items == p.nslices and (p.nslices == 4 or p.grid < 4), (fmt, m, k)
+
+
+def test_which_plain_calls_of_a_short_k_run_as_items_of_32_columns(tkd):
+    """One slice of K: up to an item for every other CTA (148), else a panel an item. Two and three slices: as items of 32 columns, but for
+    more than six a CTA at one row or of bf16, where an item is a slice of a panel."""
+    items = lambda n, m, k, fmt, epi=tkd.EPI_PLAIN: plan(tkd, fmt=fmt, m=m, k=k, ns=[n], epilogue=epi)[1].grid  # noqa: E731
+    for fmt, k in ((tkd.FMT_BFP8, 256), (tkd.FMT_BFP4, 512), (tkd.FMT_BF16, 128)):
+        for m in (1, 8):
+            assert items(2304, m, k, fmt) == 72 and items(2432, m, k, fmt) == 19 and items(1152, m, k, fmt, tkd.EPI_GLU2) == 72
+            assert items(20480, m, k, fmt) == 148 and items(3072, m, k, fmt) == 24
+    for fmt, k in ((tkd.FMT_BFP8, 384), (tkd.FMT_BFP4, 1024), (tkd.FMT_BF16, 384)):
+        stages = lambda n, m: plan(tkd, fmt=fmt, m=m, k=k, ns=[n])[1].stages  # noqa: E731
+        assert stages(28416, 1) != stages(28544, 1) and (stages(28416, 8) != stages(28544, 8)) == (fmt == tkd.FMT_BF16)

@@ -247,8 +247,8 @@ def test_pick_takes_the_earliest_of_equal_keys(device, nrec, rows, k, top):
                                             (180, 2, 4, 9), (181, 2, 4, 9)])
 def test_picks_from_records_with_ties_and_holes(device, nrec, rows, k, top):
     """The best slots of arbitrary records (few distinct keys, empty slots, ids past the vocabulary, a record's slots in no order), by
-    counting and, past 2048 slots, 512 records or twenty records for each of the top, in rounds: the first candidate and how many are held, and the pick among their
-    exact logits, as numpy finds them."""
+    counting and, past 2048 slots, 512 records or twenty records for each of the top, in rounds: the first candidate and how many are
+    held, and the pick among their exact logits, as numpy finds them."""
     g = np.random.default_rng(nrec + k)
     dim, vocab = 64, 4000
     keys = g.integers(0x8000, 0x8000 + 60, (nrec, rows, k)).astype(np.uint32)

@@ -758,7 +758,7 @@ def test_column_shards_give_the_whole_weights_bits(device, fmt, m):
 @pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
 @pytest.mark.parametrize("m,k,n", [(1, 4096, 1072), (5, 544, 176), (8, 32, 16), (9, 1056, 144), (32, 4096, 208), (33, 96, 320), (300, 1056, 144)])
 def test_linear_silu_in_the_output_stage(device, fmt, m, k, n):
-    """linear(activation="silu") against the oracle for every kernel that has the output stage, with and without column scales:
+    """linear(activation="silu") against the oracle for the kernels that have the output stage (long rows: the test of that name), with and without column scales:
     within a rounding to bf16 of the float64 value and float32's sums. With an out the product stays in it and the activation is a
     tensor of its own; a residual is added before the activation."""
     g = torch.Generator().manual_seed(m + k + n)
@@ -785,10 +785,13 @@ def test_linear_silu_in_the_output_stage(device, fmt, m, k, n):
 
 
 @pytest.mark.parametrize("dtype,k", [(ttnn.bfloat8_b, 32), (ttnn.bfloat8_b, 288), (ttnn.bfloat8_b, 544), (ttnn.bfloat8_b, 2080), (ttnn.bfloat8_b, 4128),
-                                     (ttnn.bfloat4_b, 480), (ttnn.bfloat4_b, 1056), (ttnn.bfloat4_b, 5120), (ttnn.bfloat16, 160), (ttnn.bfloat16, 1280)])
+                                     (ttnn.bfloat4_b, 480), (ttnn.bfloat4_b, 1056), (ttnn.bfloat4_b, 5120), (ttnn.bfloat16, 160), (ttnn.bfloat16, 1280),
+                                     (ttnn.bfloat8_b, 8960), (ttnn.bfloat8_b, 8992), (ttnn.bfloat4_b, 8704), (ttnn.bfloat4_b, 8736),
+                                     (ttnn.bfloat16, 7168), (ttnn.bfloat16, 7200)])
 @pytest.mark.parametrize("m", [1, 2, 8])
 def test_items_of_one_to_four_slices_equal_the_counted_kernel(device, dtype, k, m):
-    """The same for one to three slices, and for four whose last is short: every K of up to 16384 runs as items of 32 columns."""
+    """The same for one to three slices (of one, the smallest weights only), for four whose last is short, and at both sides of the
+    longest eight rows that fit beside the ring, where the plain call is the counting kernel too."""
     test_plain_calls_equal_the_counted_kernels(device, dtype, k, m)
 
 
