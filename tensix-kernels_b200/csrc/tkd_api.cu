@@ -65,7 +65,8 @@ int tc_cluster_count(int fmt, size_t smem) {
 // 19.9 / 21.4; [3072, 14336] 20.4 / 18.7). N may not enter, and the gain of 17 and more rows of a block-float weight ends at some 12000
 // to 20000 columns (with w_up both weights' count): 32 rows of bfloat8_b with w_up, [1536, 4608] 0.64 of the other's time, [1536, 6144]
 // 1.03, [1536, 20480] 1.37; 24 rows of bfloat4_b, [1024, 4096] 0.85, [1024, 20480] 1.24; K 2560 of bfloat4_b is the worst
-// ([2560, 5120] 32 rows 1.09, 17 rows 1.26).
+// ([2560, 5120] 32 rows 1.09, 17 rows 1.26). A head of 75968 columns takes up to twice the other's time (bfloat4_b, 24 rows, K 2560,
+// 77 / 38 us; bfloat8_b, 32 rows, K 1536, 56 / 33), which the projections of a model's layers outweigh.
 int rows_layout(TkdParams& p, int sab) {
     const int ck = tkd_chunk_k(p.fmt), nch = (p.K + ck - 1) / ck;
     if (p.M > 16 && p.nslices == 4 && (p.M > 24 || p.K > 1536)) return 0;

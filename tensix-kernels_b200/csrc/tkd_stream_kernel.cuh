@@ -489,8 +489,8 @@ __device__ __forceinline__ uint32_t topk_best(const uint32_t (&cand)[N], uint32_
 // quarter of the unit (16 columns a lane; a round is one warp-wide maximum in hardware, and only the lane that gave it looks
 // through its candidates again), a row after the other, then a warp merges a row's four lists. (Every round's maximum over
 // the four warps through shared memory, with two barriers a round, took 8 rows of 8 some 5 us a unit.)
-// parts: calls a panel.
-__device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c, const TkdSegDev& sg, int parts, int et, int ow, int lane,
+// parts: what a panel counts for; add: what this call does.
+__device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c, const TkdSegDev& sg, int parts, int add, int et, int ow, int lane,
                                              float* tbuf, volatile int* sflag, uint16_t* y16, int topk_k, int npeers) {
     // (the weight's number in the call, by block or by repeat, its panels, and the panel's number in it)
     const int upanels = p.topk_unit / TKD_PANEL_COLS, wpanels = p.rep_panels ? p.rep_panels : p.total_panels / p.nseg;
@@ -500,8 +500,8 @@ __device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c
     __threadfence();
     bar_output_warps();
     if (et == 0) {
-        const int old = atomicAdd(p.unit_counters + slot, 1);
-        const int last = old + 1 == in_unit * parts;
+        const int old = atomicAdd(p.unit_counters + slot, add);
+        const int last = old + add == in_unit * parts;
         if (last) p.unit_counters[slot] = 0;
         sflag[0] = last;
     }
@@ -1184,7 +1184,7 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
             }
             if (topk_k == 0) continue;
 
-            topk_records(p, c, sg, 1, et, ow, lane, tbuf, sflag, y16, topk_k, npeers);
+            topk_records(p, c, sg, 1, 1, et, ow, lane, tbuf, sflag, y16, topk_k, npeers);
         
         }
         if (npeers) exchange_done(p, lane, npeers, sflag);

@@ -1116,7 +1116,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 if (glu) bar_output_warps();  // tbuf is free again
             }
             if (topk_k == 0) continue;
-            topk_records(p, c, sg, 1, et, ow, lane, tbuf, sflag, y16, topk_k, npeers);
+            topk_records(p, c, sg, 1, 1, et, ow, lane, tbuf, sflag, y16, topk_k, npeers);
         }
         if (npeers) exchange_done(p, lane, npeers, sflag);
     }
