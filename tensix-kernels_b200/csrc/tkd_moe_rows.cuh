@@ -144,11 +144,11 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
     };
 
     // gate_up: the rows that chose the expert of slot q, a bit each (by a whole warp). Up to eight of them (of 16 rows and 8 of 128 experts
-    // one or two as a rule) are multiplied alone, one MMA a fragment: a lane's column of it is its row among them. Us of gate_up with all
-    // rows multiplied / so: 8 of 128 experts of 2048 x 1536, 16 rows 51.9 / 46.1, 24 rows 79.9 / 73.5, 32 rows 108.8 / 83.1; 2 of 8 of
-    // 4096 x 4096, 16 rows 30.8 / 27.5, 24 rows 38.8 / 39.1, 32 rows 46.5 / 46.7. All rows are brought: a producer that picks is one warp
-    // with a row after the other, and took the latter's 16 rows to 34. (With the scales in the activations instead of the weights 32
-    // rows of the former take 2 us less, but then an input's range depends on how many rows chose the expert.)
+    // one or two as a rule) are brought and multiplied alone, as rows 0, 1, ..: one MMA a fragment. Us of gate_up with all rows multiplied /
+    // so: 8 of 128 experts of 2048 x 1536, 16 rows 54.1 / 47.6, 24 rows 80.9 / 72.7, 32 rows 106.3 / 78.1; 2 of 8 of 4096 x 4096, 16
+    // rows 30.5 / 29.3, 24 rows 38.7 / 40.2, 32 rows 46.5 / 47.9. (A producer that walks the bits, a row after the other, took the
+    // latter's 16 rows to 33.5; one that brings all rows the former's 15 rows from 44.2 to 48.5. With the scales in the activations
+    // instead of the weights 16 rows of the former take 0.7 us less, but then an input's range depends on how many rows chose the expert.)
     constexpr bool PICK = !DOWN && MT > 1 && FMT == TKD_BFP4;
     auto rows_of = [&](int q) {
         const int e = ulist[q];
@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
+        int qm = -1, row = 0, nfew = 0;
         uint32_t st = 0;
         bool ok = true;
         if (i0 < i1) {
@@ -178,7 +179,28 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
                 // the rows' inputs, 8 k a piece
                 const uint16_t* xq = p.x + (DOWN ? (int64_t)a.q * K : 0) + a.c * CK;
                 const int pieces = min(CK, K - a.c * CK) / 8;
-                for (int e = lane; e < pieces; e += 32) {
+                if (PICK && a.q != qm) {  // (lane i < 8: the i-th of the rows that chose the expert)
+                    qm = a.q;
+                    const uint32_t mask = rows_of(qm);
+                    nfew = __popc(mask);
+                    row = nfew <= 8 && lane < nfew ? (int)__fns(mask, 0, lane + 1) : 0;
+                }
+                const bool few = PICK && nfew <= 8;
+                if (few) {
+                    const uint16_t* xl = xq + lane * 8;
+                    const uint32_t xd = dst + p.w_bytes + lane * 16;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int64_t off = (int64_t)__shfl_sync(0xFFFFFFFFu, row, i) * p.ldx;
+                        if (i < nfew) {
+#pragma unroll
+                            for (int e = 0; e < CK / 8; e += 32)
+                                if (lane + e < pieces)
+                                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(xd + i * p.x_stride + e * 16), "l"(xl + off + e * 8) : "memory");
+                        }
+                    }
+                }
+                for (int e = lane; !few && e < pieces; e += 32) {
                     const uint16_t* xr = xq + e * 8;
                     uint32_t xd = dst + p.w_bytes + e * 16;
 #pragma unroll 8
@@ -212,7 +234,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
 #pragma unroll
             for (int m = 0; m < MT; ++m) tot[m][0] = tot[m][1] = tot[m][2] = tot[m][3] = 0.f;
         };
-        uint32_t slot = 0, phase = 0, np = 0, xfew = 0;
+        uint32_t slot = 0, phase = 0, np = 0;
         int qm = -1;
         bool few = false;
         clear(), clear_tot();
@@ -222,10 +244,9 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
             const int c = a.c;
             if (PICK && a.q != qm) {
                 qm = a.q;
-                const uint32_t mask = rows_of(qm);
-                const int n = __popc(mask);
-                few = n <= 8;
-                xfew = p.w_bytes + (uint32_t)(n ? __fns(mask, 0, min(g, n - 1) + 1) : 0) * p.x_stride + 16 * t;
+                const int n = __popc(rows_of(qm));
+                few = n <= 8;  // (then this lane's one row is in xrow[0]: another register for it spilled at 17 to 24 rows)
+                xrow[0] = p.w_bytes + (uint32_t)max(min(g, (few ? n : R) - 1), 0) * p.x_stride + 16 * t;
             }
             // (the expert's last block here: its group's largest exponent is asked for before the stage is waited for)
             const bool fold = c == nch - 1 || it == i1 - 1, deliver = a.j == nb - 1 || it == i1 - 1;
@@ -250,7 +271,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 1) tkd_moe_rows_kernel(const __
                             if (!FULL && c * CK + sa * F::KSA + 32 * q >= K) break;  // (a K that ends inside the super-atom)
                             uint4 xv[MT];
 #pragma unroll
-                            for (int m = 0; m < (FEW ? 1 : MT); ++m) xv[m] = lds128(sb + (FEW ? xfew : xrow[m]) + (sa * F::KSA + 32 * q) * 2);
+                            for (int m = 0; m < (FEW ? 1 : MT); ++m) xv[m] = lds128(sb + xrow[m] + (sa * F::KSA + 32 * q) * 2);
                             const uint32_t cwd[4] = {q ? cv.z : cv.x, q ? cv.w : cv.y, 0u, 0u}, ewd[2] = {q ? ev.z : ev.x, q ? ev.w : ev.y};
                             if constexpr (MT == 1) {
                                 block_mma<TKD_BFP4, MT, 2>(acc, cwd, ewd, xv, sh);
