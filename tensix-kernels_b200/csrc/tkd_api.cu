@@ -469,10 +469,11 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
     if (sms <= 0) sms = sm_count();
     if (sms <= 0) sms = 148;
     if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
-    // The rows of a tile and the blocks it is cut into, by what the kernel measured (B200, us; K 4096, bfloat8_b; the other
-    // formats, whose decode is other work, go by the same figures, which were not fitted to them): a unit of 128 k takes
-    // 0.55 + nt / 600 (the decode, then the traffic of x from L2); a tile's output nt / 29; a cut tile's partial sums
-    // 2 + nt / 60 to store, and nt / 26 for each part that its last CTA adds up.
+    // The rows of a tile and the blocks it is cut into, by what the kernel measured (B200, us; a fit to 350 launches in a graph of 40 to
+    // 512 rows, K 1024 to 4096, N 2048 to 14336, three formats, 7 % on average): besides 2.6 + K / 3000 a launch, a unit of 128 k takes
+    // 0.4 + nt / 2250 (the decode, then the MMAs; bf16, whose weights are twice the traffic, nt / 750), a tile's output nt / 37, a cut
+    // tile 2.2 and nt / 31 for each part that its last CTA adds up.
+    const double per_row = a->fmt == TKD_BF16 ? 1 / 750. : 1 / 2250.;
     double best = 0;
     for (int nrt = (p.M + 255) / 256, nrt1 = (p.M + 31) / 32; nrt <= nrt1; ++nrt) {
         const int nt = ((p.M + nrt - 1) / nrt + 15) / 16 * 16;
@@ -485,8 +486,8 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
             const double units = (double)(run * q * chunk_k) / 128;
             // parts of a tile: one whenever runs are whole tiles
             const int parts = total % grid == 0 && run % blocks == 0 ? 1 : (int)((blocks + run - 2) / run) + 1;
-            const double us = units * (0.55 + nt / 600.) + (double)((run + blocks - 1) / blocks) * nt / 29. +
-                              (parts > 1 ? 2 + nt / 60. + (parts - 1) * nt / 26. : 0);
+            const double us = units * (0.4 + nt * per_row) + (double)((run + blocks - 1) / blocks) * nt / 37. +
+                              (parts > 1 ? 2.2 + (parts - 1) * nt / 31. : 0);
             if (best == 0 || us < best) {
                 best = us;
                 p.nrt = nrt, p.nt = nt, p.q = q, p.blocks = blocks, p.total = (int)total, p.grid = (int)grid;
@@ -530,12 +531,11 @@ int tkd_matmul_rows_workspace(const TkdMatmul* a, uint64_t* bytes) {
 
 // Whether a call of more than 32 rows runs tkd_rows_kernel in tiles of rows (of sixteen, less where x is too long for that), its
 // launch in L without the tensors. wide_us: what make_wide's model expects of tkd_wide_kernel's units and outputs.
-// Both expectations are fitted to launches in a graph over weights larger than L2 (B200; 450 shapes of 33 to 512 rows, K 576 to 3136, N
-// 544 to 10240, three formats): a launch of this kernel by the items of its longest CTA, one of tkd_wide_kernel, with the one that lays x
-// out, by that model, within 5 to 6 % on average, at most 23 %. At nine tenths no shape got slower, and 1.28 times faster is all but the
-// 1.29 that the better of the two would always give: bfloat8_b 33 rows [2048, 544] 12.7 to 4.9 us, [1056, 4096] 9.8 to 7.4; 128 rows
-// [2048, 1024] 13.5 to 7.0; 256 rows [576, 544] 7.3 to 6.2. A weight is taken apart anew for every tile here: with N or rows
-// beyond that the other is the faster one (64 rows of [1056, 10240] 15.7 against 11.2).
+// Both expectations are fitted to launches in a graph (B200; 33 to 512 rows, K 576 to 3136, N 544 to 10240, three formats): a launch of
+// this kernel by the items of its longest CTA, which for block-float weights comes out about a tenth high, hence the 1.1; one of
+// tkd_wide_kernel, with the one that lays x out, by make_wide's model. bfloat8_b, this kernel / the other, us: 40 rows [3072, 6144] with a
+// residual 13.3 / 15.8, 128 rows [2048, 2048] 10.4 / 11.3, 320 rows [640, 608] 6.3 / 6.7. A weight is taken apart anew for every tile
+// here: with N or rows beyond that the other is the faster one (64 rows [3072, 6144] with a residual 22.2 / 15.3).
 static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     int sms = sm_count();
     if (sms <= 0) sms = 148;
@@ -554,7 +554,7 @@ static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     p.rows_tile = one.m, p.M = a->m;
     L->grid = tiles * p.rows_team;
     const double k = p.K / 1000., most = (items + p.rows_team - 1) / p.rows_team;
-    return 3.2 + 0.2 * k + most * (0.65 + (p.fmt == TKD_BF16 ? 0.8 : 0.65) * k) < 0.9 * (3.4 + 0.62 * wide_us + 1.85 * k);
+    return 3.2 + 0.2 * k + most * (0.65 + (p.fmt == TKD_BF16 ? 0.8 : 0.65) * k) < 1.1 * (2.6 + wide_us + 0.34 * k);
 }
 
 // Whether a call's output shares memory with x. (More than 32 rows may: tkd_wide_kernel reads a copy of x.)

@@ -375,7 +375,9 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
     const uint32_t xs0 = (smem_u32(smem + p.off_x) + 1023u) & ~1023u;  // (the swizzle is a function of the address)
     const uint32_t ring0 = smem_u32(smem + p.off_ring);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (the warp's number by a shuffle: what follows from it is then known to be the same in all lanes, as the operands of an MMA have
+    // to be; else each is taken from a lane before it is issued. 512 rows of [14336, 4096] bfloat8_b, launches in a graph: 67.2 to 58.7 us)
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
         for (int s = 0; s < p.nstages; ++s) mbar_init(full0 + 8 * s, 1), mbar_init(empty0 + 8 * s, SW);
@@ -435,20 +437,20 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
         // ---------------------------------------------------------------- producer of the x tiles, two a unit
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint32_t bytes = (uint32_t)NT * 128;
-        uint32_t st = 0;
+        uint32_t st = 0, s = 0, phase = 1;
         bool ok = true;
         for (int it = i0; ok && wide_next(p, it, i1, sg);) {
             const uint8_t* src = p.xt + (int64_t)(sg.tile % p.nrt) * p.nkb * bytes;
             const int kb1 = 2 * ((min(K, sg.c1 * CK) + 127) / 128);
             for (int kb = sg.c0 * (CK / 64); kb < kb1; ++kb, ++st) {
-                const uint32_t s = st % nx;
-                ok = mbar_wait_parked(xempty0 + 8 * s, ((st / nx) & 1) ^ 1, p.status);
+                ok = mbar_wait(xempty0 + 8 * s, phase, p.status);
                 if (!ok) break;
                 if (lane == 0) {
                     mbar_expect_tx(xfull0 + 8 * s, bytes);
                     bulk_g2s(xs0 + s * bytes, src + (int64_t)kb * bytes, bytes, xfull0 + 8 * s);
                 }
                 __syncwarp();
+                if (++s == (uint32_t)nx) s = 0, phase ^= 1;
             }
         }
         if (!ok)
@@ -458,48 +460,53 @@ __global__ void __launch_bounds__(kWideWarps * 32, 1) tkd_wide_kernel(const __gr
     } else if (warp == 0 || warp == 2) {
         // ---------------------------------------------------------------- MMA issue. A unit belongs to the warp of its number's
         // parity in the CTA's sequence (so a slot's barriers are one warp's and it sees every phase of them), an accumulator
-        // to the parity within the segment.
+        // to the parity within the segment. The loop is on every unit's way from decoded to multiplied, a warp alone: slots and their
+        // parities are counted, not divided out of the unit's number (the x tiles' number is no constant), and a whole unit's MMAs
+        // stand without a test between them. With divisions a unit took the warp 1540 cycles at 256 rows, where its eight MMAs run
+        // 1050: 384 rows of [14336, 4096] bfloat8_b 63.4 us, 45.4 so (with the shuffle above).
         const int mw = warp >> 1, nm = p.nmma;
         if (mw < nm) {
             const uint64_t bd0 = tc_desc(xs0);
             const uint32_t dhi = (uint32_t)(bd0 >> 32), blo0 = (uint32_t)bd0, xstep = (uint32_t)NT * 128 >> 4;
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)NT >> 3) << 17) | ((128u >> 4) << 24);
             uint32_t us = 0, j = 0;
+            uint32_t ps = mw, aphase = 0, xs = 2 * mw, xphase = 0;  // this warp's next slots and their parities
             bool ok = true;
             for (int it = i0; ok && wide_next(p, it, i1, sg); ++j) {
                 const int kv = min(K, sg.c1 * CK) - sg.c0 * CK, nu = (kv + 127) >> 7;
-                const uint32_t set = j % p.nset;
-                ok = mbar_wait(accempty0 + 8 * set, ((j / p.nset) & 1) ^ 1, p.status);
+                const uint32_t set = p.nset == 2 ? j & 1 : 0;
+                ok = mbar_wait(accempty0 + 8 * set, ((p.nset == 2 ? j >> 1 : j) & 1) ^ 1, p.status);
                 if (!ok) break;
                 tc_fence_after();
                 for (int ui = nm == 2 ? (int)((mw - us) & 1u) : 0; ui < nu; ui += nm) {
-                    const uint32_t g = us + ui, ps = g % kWideASlots;
-                    ok = mbar_wait(afull0 + 8 * ps, (g / kWideASlots) & 1, p.status);
+                    ok = mbar_wait(afull0 + 8 * ps, aphase, p.status);
                     if (!ok) break;
-                    const int kleft = kv - 128 * ui, nb = kleft >= 128 ? 8 : kleft >> 4;
-                    const uint32_t d = tmem0 + (set * nm + (ui & (nm - 1))) * NT;
-                    uint32_t acc = ui >= nm;
+                    const int kleft = kv - 128 * ui;
+                    const uint32_t d = tmem0 + (set * nm + (ui & (nm - 1))) * NT, acc = ui >= nm;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const uint32_t xq = 2 * g + h, s = xq % nx;
-                        ok = ok && mbar_wait(xfull0 + 8 * s, (xq / nx) & 1, p.status);
+                        ok = ok && mbar_wait(xfull0 + 8 * (xs + h), xphase, p.status);
                         if (!ok) break;
                         tc_fence_after();
                         if (tc_elect()) {
-                            const uint32_t al = tmem0 + kWideA0 + ps * 64 + h * 32, bl = blo0 + s * xstep;
+                            const uint32_t al = tmem0 + kWideA0 + ps * 64 + h * 32, bl = blo0 + (xs + h) * xstep;
+                            auto issue = [&](int nb) {
 #pragma unroll
-                            for (int b = 0; b < 4; ++b) {
-                                if (4 * h + b >= nb) break;
-                                wide_mma(d, al + 8 * b, bl + 2 * b, dhi, idesc, acc);
-                                acc = 1;
-                            }
-                            tc_commit(xempty0 + 8 * s);
+                                for (int b = 0; b < 4; ++b)
+                                    if (b < nb) wide_mma(d, al + 8 * b, bl + 2 * b, dhi, idesc, h || b ? 1u : acc);
+                            };
+                            if (kleft >= 128)
+                                issue(4);
+                            else
+                                issue((kleft >> 4) - 4 * h);
+                            tc_commit(xempty0 + 8 * (xs + h));
                             if (h == 1) tc_commit(aempty0 + 8 * ps);
                         }
-                        acc = 1;
                         __syncwarp();
                     }
                     if (!ok) break;
+                    if ((ps += nm) >= kWideASlots) ps -= kWideASlots, aphase ^= 1;
+                    if ((xs += 2 * nm) >= (uint32_t)nx) xs -= nx, xphase ^= 1;
                 }
                 us += nu;
                 if (ok && tc_elect()) tc_commit(accfull0 + 8 * set);
