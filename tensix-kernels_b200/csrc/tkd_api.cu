@@ -179,18 +179,19 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false, bo
     if (a->max_ctas > 0 && a->max_ctas < sms) sms = a->max_ctas;
 
     // shared-memory map: barriers, the hand-over buffers of the streaming warps, the GLU exchange buffer, the ring
+    const int xslots = a->fmt == TKD_BF16 ? TKD_TC_XSLOTS : TKD_TC_SLOTS;
     const int mp = mt == 1 ? 8 : (mt == 2 ? 24 : 40);
     p.stage_bytes = 8 * tkd_subsa(a->fmt) * sab;
     p.off_pbuf = TKD_SMEM_HEAD;
     if (a->m > 8) {
         // 9 to 32 rows, the tensor-memory kernel: the running sums [128][40] floats, then (from the next 1024-byte
-        // boundary of the window, hence the slack) TKD_TC_SLOTS slots of two x tiles (4 KB each), then the ring. (The kernel
+        // boundary of the window, hence the slack) `xslots` slots of two x tiles (4 KB each), then the ring. (The kernel
         // addresses x by 32-bit element offsets.)
         if (a->ldx > (1 << 26)) return TKD_ERR_BAD_ARG;
         p.tc = 1;
         p.off_tbuf = TKD_SMEM_HEAD;
         p.off_xt = p.off_tbuf + TKD_PANEL_COLS * 40 * 4;
-        p.off_ring = (int)align_up(p.off_xt + 1024 + TKD_TC_SLOTS * 2 * 4096, 128);
+        p.off_ring = (int)align_up(p.off_xt + 1024 + xslots * 2 * 4096, 128);
     } else {
         // (one to eight rows: two hand-over buffers; all of x in shared memory, K rounded up to a chunk, if that leaves
         // the ring at least four stages; rows 64 bytes further apart than their length, so that the eight rows a warp
@@ -249,7 +250,7 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false, bo
     // panels and leave some SMs idle (a GPC's number of SMs is not a multiple of four: 132 of 148 CTAs on a B200), so they are
     // taken where no CTA gets more items for it; from four items on the other form's SMs that have one less leave theirs to the rest.
     if (p.tc && !counted && on_device && p.nslices == 4 && !a->topk_k && a->nranks <= 1) {
-        const int off_xt = p.off_tbuf + 2 * 4 * 8 * 32 * 16, off_ring = (int)align_up(off_xt + 1024 + TKD_TC_SLOTS * 2 * 4096, 128);
+        const int off_xt = p.off_tbuf + 2 * 4 * 8 * 32 * 16, off_ring = (int)align_up(off_xt + 1024 + xslots * 2 * 4096, 128);
         const int stages = (int)((kMaxSmem - off_ring) / p.stage_bytes < TKD_MAX_STAGES ? (kMaxSmem - off_ring) / p.stage_bytes : TKD_MAX_STAGES);
         const size_t smem = (size_t)off_ring + (size_t)stages * p.stage_bytes;
         int clusters = tc_cluster_count(a->fmt, smem);

@@ -33,7 +33,8 @@ int tkd_launch_unpack(int fmt, int64_t K, int64_t npad, const void* stream, cons
 #define TKD_MAX_STAGES 16
 #define TKD_SMEM_HEAD 1024     // barriers, the stage headers, flags
 #define TKD_ROWS_PITCH 36      // tkd_rows_kernel: floats from a row of an item's sums to the next (36: no bank conflicts either way)
-#define TKD_TC_SLOTS 6         // tensor-memory kernel: operand slots (a unit of two 64-k tiles: 64 columns of A, 8 KB of x)
+#define TKD_TC_SLOTS 6         // tensor-memory kernel: slots of weights in tensor memory (a unit of two 64-k tiles: 64 columns)
+#define TKD_TC_XSLOTS 8        // ... of activations in shared memory (8 KB a unit), bf16; block float: as many as of weights
 
 struct TkdSegDev {
     const uint8_t* w;     // packed stream (the gate's with a separate up weight)

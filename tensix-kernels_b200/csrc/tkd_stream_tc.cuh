@@ -22,7 +22,7 @@
 //                  The same warps write the tile of activations a unit is multiplied by (32 rows x 64 k, rows past M
 //                  zero, K-major with the 128-byte swizzle, in that order of k) into shared memory: each lane loads
 //                  its 16 bytes of the NEXT chunk's tiles into registers while it decodes this chunk (they come from
-//                  L2, a microsecond away).
+//                  L2, a microsecond away). bf16 weights: warps 23-26 do, by asynchronous copies of 8 bytes.
 //   warps 19-22    output warps (thread = panel column = tensor-memory lane): read a slice's sums with tcgen05.ld, keep
 //                  the running sums in shared memory, and from there on do what tkd_stream_kernel's output warps do
 //   warp 1         producer (one lane issues): the same ring of packed-weight chunks as tkd_stream_kernel
@@ -48,11 +48,20 @@ constexpr int kTcSlot = 2 * kTcXTile;  // ... of a slot's two x tiles
 constexpr int kTcACols = 32;         // tensor-memory columns of an A tile: 128 lanes x 64 k of bf16, two to a column
 constexpr int kTcAcc0 = 0, kTcA0 = 128;  // tensor-memory columns: two sets of two accumulators of 32, then the A slots
 static_assert(kTcA0 + kTcSlots * 2 * kTcACols <= 512, "the A slots must fit the tensor memory");
-// Warps: 0 and 2 the MMA issuers, 1 the producer, 3-18 decode, 19-22 output (23 warps: 736 threads may use 88
-// registers each, 768 only 80, two fewer than the kernel needs without spilling). The MMA issuer is the warp with the
+// Warps: 0 and 2 the MMA issuers, 1 the producer, 3-18 decode, 19-22 output (23 warps: six on an SM's quarter at most, 80
+// registers a thread). The MMA issuer is the warp with the
 // lowest number on purpose: the schedulers favour older warps, and as the last warp of the CTA it got an issue slot
 // every twenty cycles beside four decode warps that are always ready (its unit of eight MMAs took 770 ns).
-constexpr int kTcWarps = 23, kTcMmaWarp = 0, kTcProducerWarp = 1, kTcDecodeWarp0 = 3, kTcOutputWarp0 = 19, kTcMmaWarps = 2;
+constexpr int kTcMmaWarp = 0, kTcProducerWarp = 1, kTcDecodeWarp0 = 3, kTcOutputWarp0 = 19, kTcXWarp0 = 23, kTcMmaWarps = 2;
+// bf16 weights need no arithmetic, and the activations have four warps of their own (warps 23-26, at 72 registers a thread; they write
+// as far ahead as kTcXSlots units): launches in a graph, 32 rows, us with the decode warps bringing x / so: [2048, 2048] 5.6 / 4.6,
+// [4096, 6144] 15.3 / 13.5, [4096, 28672] 42.9 / 40.9. Block-float weights keep the decode warps busy, and x costs them less than four
+// more warps do: bfloat4_b, 32 rows, [4096, 57344] 39.0 / 46.1, [4096, 14336] 15.9 / 17.6 (bfloat8_b 47.0 / 49.7, 17.3 / 17.7).
+template <int FMT>
+constexpr bool kTcXw = FMT == TKD_BF16;
+constexpr int kTcXWarps = 4, kTcXSlots = TKD_TC_XSLOTS;
+template <int FMT>
+constexpr int kTcWarps = kTcXWarp0 + (kTcXw<FMT> ? kTcXWarps : 0);
 // the MMA warp number (0, 1) of a warp, or -1: warps 0 and 2
 __device__ __forceinline__ int tc_mma_warp(int warp) { return warp == 0 ? 0 : warp == 2 ? 1 : -1; }
 constexpr int kTcMP = 40;            // floats per column in tbuf (32 rows, padded)
@@ -137,10 +146,11 @@ constexpr int kTcExchange = 4 * 8 * 32 * 16;  // bytes: [slice][4 rows][32 colum
 // sums and their order are those of the other form, whose panels end in a chain of trips through L2 by one CTA alone: sums
 // stored 0.6 us, counted in 0.9, added up 2.4, put out 1.0 (32 rows, [4096, 4096] of bfloat8_b, 11.5 us from start to end).
 template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false, int EK = EK_ANY>
-__global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const __grid_constant__ TkdParams p) {
+__global__ void __launch_bounds__(kTcWarps<FMT> * 32, 1) tkd_stream_tc_kernel(const __grid_constant__ TkdParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
     constexpr int SW = 16, MP = kTcMP;
+    constexpr bool XW = kTcXw<FMT>;
     constexpr int CK = F::SUBSA * F::KSA;
     // A unit of two tiles is written (and its "full" barrier arrived on) by the warps of one group of decode warps.
     constexpr int NWT = 16 / kTcGroups;  // the warps of a group
@@ -149,6 +159,9 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     const uint32_t afull0 = smem_u32(bars + 2 * TKD_MAX_STAGES), aempty0 = afull0 + 8 * kTcSlots;
     const uint32_t accfull0 = aempty0 + 8 * kTcSlots, accempty0 = accfull0 + 16;
     const uint32_t xfull0 = accempty0 + 16, xempty0 = xfull0 + 16;  // CL: of the exchange buffers
+    const uint32_t bfull0 = smem_u32(smem + 768), bempty0 = bfull0 + 8 * kTcXSlots;  // XW: of the units of activations
+    static_assert(8 * (2 * TKD_MAX_STAGES + 2 * kTcSlots + 8) <= 512 && 16 * TKD_MAX_STAGES <= 256 && 768 + 16 * kTcXSlots <= TKD_SMEM_HEAD - 32,
+                  "barriers, the stages' headers, barriers again");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + TKD_SMEM_HEAD - 32);
     volatile int* sflag = reinterpret_cast<volatile int*>(smem + TKD_SMEM_HEAD - 16);
     uint4* hdr = reinterpret_cast<uint4*>(smem + 512);
@@ -157,7 +170,10 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     // the operand tiles start on a 1024-byte boundary of the shared-memory window (the swizzle is a function of the address)
     const uint32_t ops0 = (smem_u32(smem + p.off_xt) + 1023u) & ~1023u;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (the warp's number by a shuffle: what follows from it is then known to be the same in all lanes, as the operands of an MMA have to
+    // be; else each is taken from a lane before it is issued. A unit's eight MMAs and their commit take an issuing warp 350 to 420 cycles
+    // so, 650 before.)
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
         for (int s = 0; s < p.nstages; ++s) {
@@ -167,6 +183,10 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
         for (int s = 0; s < kTcSlots; ++s) {
             mbar_init(afull0 + 8 * s, NWT);
             mbar_init(aempty0 + 8 * s, 1);
+        }
+        for (int s = 0; XW && s < kTcXSlots; ++s) {
+            mbar_init(bfull0 + 8 * s, 32 * kTcXWarps);
+            mbar_init(bempty0 + 8 * s, 1);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(accfull0 + 8 * s, kTcMmaWarps);
@@ -200,6 +220,15 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     const int64_t lead = i1 - tail0;
     const int64_t nitems = CL ? pan1 - pan0 : i1 - i0;
     auto item_at = [&](int64_t j) { return CL ? i0 + j * p.nslices : j < lead ? tail0 + j : i0 + (j - lead); };
+    // the slice of item j, after that of the item before
+    auto next_slice = [&](int slice, int64_t j) {
+        if (CL) return rank;
+        if (j == 0 || j == lead) {
+            const int64_t it = item_at(j);
+            return (int)(it - idiv(p, it, p.nslices) * p.nslices);
+        }
+        return slice + 1 == p.nslices ? 0 : slice + 1;
+    };
 
     // tensor memory: all 512 columns (two sets of two accumulators of 32, then the A slots of 64), allocated and freed by
     // the MMA warp.
@@ -270,7 +299,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
         }
     } else if (warp >= kTcDecodeWarp0 && warp < kTcDecodeWarp0 + SW) {
         // ---------------------------------------------------------------- decode warps
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // (x may be the output of the kernel before this one)
+        if constexpr (!XW) asm volatile("griddepcontrol.wait;" ::: "memory");  // (x may be the output of the kernel before this one)
         // The warps form G groups, and a unit (by its number in this CTA's sequence, mod G) is one group's work from its
         // slot's "empty" to its "full": while a group waits for its stores to land (tcgen05.wait::st, the proxy fence),
         // the others decode. A slot is always the same group's (kTcSlots is a multiple of G), so the group's warps see
@@ -294,7 +323,8 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
         // the tensor-memory address of this warp's first 16 lanes (panel columns 16 rg0 .. + 15) at the first A column
         const uint32_t alane = tmem0 + ((uint32_t)(16 * rg0) << 16) + kTcA0;
         uint32_t slot = 0, phase = 0, useq = 0;
-        // This lane's pieces of an x tile (PP of the 256: piece = (row, 16 bytes of the row)). A piece's 16 bytes (8 k of
+        uint32_t ps = (uint32_t)grp, aphase = 1;  // the group's next operand slot, the parity its "empty" is waited for with
+        // (not XW) This lane's pieces of an x tile (PP of the 256: piece = (row, 16 bytes of the row)). A piece's 16 bytes (8 k of
         // one row) go to two places of the row's 128 bytes, 8 bytes each: k 0-3 to the block of 16 k with jj = 0 of its
         // block of 32 k, k 4-7 to the one with jj = 1, both at position 4 t (t = the piece's number within the block of
         // 32 k); then the swizzle (16-byte piece ^ row).
@@ -324,7 +354,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                     }
         };
         uint4 xcur[XT], xnext[XT];
-        {
+        if constexpr (!XW) {
             const int64_t first_it = lead > 0 ? tail0 : i0;
             load_x(xcur, (int)(first_it - idiv(p, first_it, p.nslices) * p.nslices) * p.ks, grp);
         }
@@ -401,19 +431,18 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
             const int ntiles = (nsa * F::KSA + 63) / 64;
             const int nunits = (ntiles + 1) >> 1;
             const int u0 = (int)((uint32_t)grp - useq) & (G - 1);  // the group's first unit of this chunk
-            load_x(xnext, (int)hd.z, (int)((uint32_t)grp - (useq + nunits)) & (G - 1));  // (used a whole chunk from now)
+            if constexpr (!XW) load_x(xnext, (int)hd.z, (int)((uint32_t)grp - (useq + nunits)) & (G - 1));  // (used a whole chunk from now)
             const uint32_t gb = ring_a + slot * p.stage_bytes + rg0 * nsa * F::SAB;
             bool ok = true;
             // The group's units of the chunk (unrolled: the x pieces are indexed at compile time): the slot is waited
-            // for, both tiles decoded and stored, then one proxy fence and one arrival.
+            // for, both tiles decoded and stored, then one arrival.
 #pragma unroll
             for (int i = 0; i < MU; ++i) {
                 const int u = u0 + G * i;
                 if (u >= nunits) break;
-                const uint32_t us = useq + u, ps = us % kTcSlots;
-                ok = mbar_wait(aempty0 + 8 * ps, ((us / kTcSlots) & 1) ^ 1, p.status);
+                ok = mbar_wait(aempty0 + 8 * ps, aphase, p.status);
                 if (!ok) break;
-                const uint32_t sb = ops0 + ps * kTcSlot, ta = alane + ps * 2 * kTcACols;
+                const uint32_t sb = XW ? 0 : ops0 + ps * kTcSlot, ta = alane + ps * 2 * kTcACols;
 #pragma unroll
                 for (int sub = 0; sub < 2; ++sub) {
                     const int ti = 2 * u + sub;  // the tile of the chunk
@@ -430,7 +459,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                         }
                     }
 #pragma unroll
-                    for (int pp = 0; pp < PP; ++pp) {
+                    for (int pp = 0; !XW && pp < PP; ++pp) {
                         const uint4 v = xcur[(2 * i + sub) * PP + pp];
                         const uint32_t xb = sb + sub * kTcXTile;
                         asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(xb + xdst0[pp]), "r"(v.x), "r"(v.y) : "memory");
@@ -439,46 +468,80 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");  // this warp's tensor-memory stores are done
                 tc_fence_before();
-                fence_proxy_async();  // this lane's shared-memory stores, for the tensor core's reads
                 __syncwarp();
                 if (lane == 0) mbar_arrive(afull0 + 8 * ps);
+                if ((ps += G) >= kTcSlots) ps -= kTcSlots, aphase ^= 1;
             }
             if (!ok) break;
 #pragma unroll
-            for (int i = 0; i < XT; ++i) xcur[i] = xnext[i];
+            for (int i = 0; !XW && i < XT; ++i) xcur[i] = xnext[i];
             useq += nunits;
             __syncwarp();
             if (lane == 0) mbar_arrive(empty0 + 8 * slot);
             if (++slot == (uint32_t)nst) slot = 0, phase ^= 1;
             if (at_end) break;
         }
+    } else if (XW && warp >= kTcXWarp0) {
+        // ---------------------------------------------------------------- activations: the tiles a unit is multiplied by (32 rows x
+        // 64 k, K-major with the 128-byte swizzle), copied straight into the unit's slot as soon as that is free, half a dozen
+        // units ahead (they come from L2, most of a microsecond away). The 16 bytes (8 k) a lane of an mma owns go to two places
+        // of the row's 128 bytes: k 0-3 to the block of 16 k with jj = 0 of its block of 32 k, k 4-7 to the one with jj = 1, both
+        // at position 4 t (t = the piece's number within the block of 32 k); then the swizzle (16-byte piece ^ row). So the copies
+        // are of 8 bytes; a lane has the same 8 bytes of every RS-th row. What lies in rows past M only feeds columns of D that
+        // nothing reads.
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // (x may be the output of the kernel before this one)
+        constexpr int RS = 2 * kTcXWarps, NR = 32 / RS;
+        const int gl = (warp - kTcXWarp0) * 32 + lane, r0 = gl >> 4, ke = 4 * (gl & 15);  // this lane's first row, its k of a tile
+        const uint32_t o = 64 * (ke >> 5) + 32 * ((ke >> 2) & 1) + 8 * ((ke >> 3) & 3);
+        const uint32_t d0 = ops0 + r0 * 128 + (o & 15), c0 = ((o >> 4) ^ (r0 & 7)) << 4;
+        uint32_t xoff[NR];  // (an element offset into x: x is at most 32 rows)
+#pragma unroll
+        for (int i = 0; i < NR; ++i) xoff[i] = (uint32_t)(min(r0 + RS * i, M - 1) * p.ldx) + ke;
+        uint32_t ps = 0, aphase = 1;
+        int slice = 0;
+        bool ok = true;
+        for (int64_t j = 0; ok && j < nitems; ++j) {
+            slice = next_slice(slice, j);
+            const int k0 = slice * p.ks, kend = min(k0 + p.ks, K);
+            for (int k = k0; k < kend; k += 128) {
+                ok = mbar_wait(bempty0 + 8 * ps, aphase, p.status);
+                if (!ok) break;
+                const uint32_t at = d0 + ps * kTcSlot;
+                const bool in0 = k + ke < K, in1 = k + ke + 64 < K;
+#pragma unroll
+                for (int i = 0; i < NR; ++i) {
+                    if (RS * i >= M) break;
+                    const uint16_t* src = p.x + (xoff[i] + (uint32_t)k);
+                    const uint32_t dst = at + (c0 ^ (uint32_t)(((RS * i) & 7) << 4)) + RS * i * 128;
+                    if (in0) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+                    if (in1) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + kTcXTile), "l"(src + 64) : "memory");
+                }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bfull0 + 8 * ps) : "memory");
+                if (++ps == kTcXSlots) ps = 0, aphase ^= 1;
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");  // (also after a wait that gave up: none is in flight when the CTA goes)
     } else if (tc_mma_warp(warp) >= 0) {
         // ---------------------------------------------------------------- the MMA issuers (a warp walks the loop, one
-        // lane issues). Issuing a unit's eight MMAs costs a warp ~450 ns beside the decode warps (60 cycles an MMA on an
-        // idle SM, about 115 here) and its loop as much again, more than the decode of a unit takes: two warps share the
-        // units by their number in the CTA's sequence (even: the first warp; odd: the second), so that a slot's
-        // barriers are always the same warp's and it sees every phase of them (a parity wait tells phase n from n + 2
-        // only then). The accumulator is chosen by the unit's number within its SLICE (even: d0, odd: d1), so that a
+        // lane issues). A unit's eight MMAs and their commits cost a warp some 400 cycles (a micro-benchmark of MMAs of 32
+        // rows: 32 cycles each from one warp on an idle SM, 42 beside busy warps, half of both from two warps), its waits and the
+        // proxy fence as much again, and a decode group takes a unit in some 900: two warps share the units by their number
+        // in the CTA's sequence (even: the first warp; odd: the second), so that a slot's barriers are always the same
+        // warp's and it sees every phase of them (a parity wait tells phase n from n + 2 only then). The accumulator is chosen by the unit's number within its SLICE (even: d0, odd: d1), so that a
         // slice's sums do not depend on where in the sequence it starts; the two warps are on opposite parities at
         // any time, hence on different accumulators.
         {
             const int mw = tc_mma_warp(warp);
             int slice = 0;    // the item's slice of its panel: all this role needs to know of it
-            uint32_t us = 0;  // units before this slice
+            uint32_t us = 0;  // units before this slice (mod 2)
             bool ok = true;
             // the descriptor of slot 0's first x tile as 32-bit halves (a slot further on is kTcSlot / 16 more in the low
             // half, a tile kTcXTile / 16, a block of 16 k 2 more); the A operand: tensor-memory columns, 8 a block
             const uint64_t bd0 = tc_desc(ops0);
             const uint32_t dhi = (uint32_t)(bd0 >> 32), blo0 = (uint32_t)bd0, alo0 = tmem0 + kTcA0;
+            uint32_t ps = mw, aphase = 0, xs = mw, bphase = 0;  // this warp's next slots, every other one, and their parities
             for (int64_t j = 0; j < nitems && ok; ++j) {
-                if (CL) {
-                    slice = rank;
-                } else if (j == 0 || j == lead) {
-                    const int64_t it = item_at(j);
-                    slice = (int)(it - idiv(p, it, p.nslices) * p.nslices);
-                } else if (++slice == p.nslices) {
-                    slice = 0;
-                }
+                slice = next_slice(slice, j);
                 const int kv = min(p.ks, K - slice * p.ks);
                 const int nu = (kv + 127) >> 7;  // units of the slice (a chunk is a whole number of units but for K's end)
                 const uint32_t buf = (uint32_t)j & 1;
@@ -487,27 +550,35 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t dbase = tmem0 + kTcAcc0 + buf * 64;
-                for (int ui = (int)(((uint32_t)mw - us) & 1u); ui < nu; ui += 2) {
-                    const uint32_t g = us + ui, ps = g % kTcSlots;
-                    ok = mbar_wait(afull0 + 8 * ps, (g / kTcSlots) & 1, p.status);
+                for (int ui = (int)(((uint32_t)mw ^ us) & 1u); ui < nu; ui += 2) {
+                    ok = (!XW || mbar_wait(bfull0 + 8 * xs, bphase, p.status)) && mbar_wait(afull0 + 8 * ps, aphase, p.status);
                     if (!ok) break;
+                    // (the activations' stores or copies, for the tensor core's reads: fenced here, since a fence waits for its own
+                    // warp's loads and copies in flight, and those of the warps that bring x are under way at any time)
+                    fence_proxy_async();
                     tc_fence_after();  // (the decode warps' tensor-memory stores, completed before they arrived)
                     if (tc_elect()) {
                         const uint32_t d = dbase + (ui & 1) * 32, acc = ui >= 2;
-                        uint32_t al = alo0 + ps * 2 * kTcACols, bl = blo0 + ps * (kTcSlot >> 4);
+                        const uint32_t al = alo0 + ps * 2 * kTcACols, bl = blo0 + (XW ? xs : ps) * (kTcSlot >> 4);
                         // (the unit's blocks of 16 k, eight if it is whole: two tiles of four)
-                        const int kleft = kv - 128 * ui;
-                        const int nb = kleft >= 128 ? 8 : (kleft + 15) >> 4;
+                        auto issue = [&](int nb) {
 #pragma unroll
-                        for (int b = 0; b < 8; ++b) {
-                            if (b >= nb) break;
-                            if (b == 4) al += kTcACols - 32, bl += (kTcXTile >> 4) - 8;
-                            tc_mma(d, al + 8 * b, bl + 2 * b, dhi, b ? 1u : acc);
-                        }
+                            for (int b = 0; b < 8; ++b)
+                                if (b < nb) tc_mma(d, al + 8 * b, bl + 2 * (b & 3) + (b >> 2) * (kTcXTile >> 4), dhi, b ? 1u : acc);
+                        };
+                        const int kleft = kv - 128 * ui;
+                        if (kleft >= 128)
+                            issue(8);
+                        else
+                            issue((kleft + 15) >> 4);
                         tc_commit(aempty0 + 8 * ps);
+                        if (XW) tc_commit(bempty0 + 8 * xs);
                     }
                     __syncwarp();
+                    if ((ps += 2) >= kTcSlots) ps -= kTcSlots, aphase ^= 1;
+                    if (XW && (xs += 2) >= kTcXSlots) xs -= kTcXSlots, bphase ^= 1;
                 }
+                if (!ok) break;
                 us += nu;
                 // (a warp without a unit in this slice commits all the same: the barrier counts both)
                 if (ok && lane == 0) tc_commit(accfull0 + 8 * buf);
@@ -1125,7 +1196,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
     tc_fence_before();
     if constexpr (CL) {
         // (no CTA goes while another may still store or arrive in its shared memory)
-        if (warp < kTcOutputWarp0) cl_barrier_wait();
+        if (warp < kTcOutputWarp0 || warp >= kTcXWarp0) cl_barrier_wait();
         __syncwarp();
         cl_barrier_arrive();
         cl_barrier_wait();
@@ -1138,10 +1209,10 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1) tkd_stream_tc_kernel(const _
 }
 
 template <bool CL>
-cudaLaunchConfig_t tc_config(int grid, size_t smem, cudaStream_t st, bool pdl, cudaLaunchAttribute (&attr)[2]) {
+cudaLaunchConfig_t tc_config(int grid, int threads, size_t smem, cudaStream_t st, bool pdl, cudaLaunchAttribute (&attr)[2]) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kTcWarps * 32);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     int n = 0;
@@ -1164,7 +1235,7 @@ int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
         if (dev >= 0 && dev < 64) allowed[dev] = true;
     }
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = tc_config<CL>(grid, smem, st, !p.no_pdl, attr);
+    const cudaLaunchConfig_t cfg = tc_config<CL>(grid, kTcWarps<FMT> * 32, smem, st, !p.no_pdl, attr);
     return (int)cudaLaunchKernelEx(&cfg, kern, p);
 }
 // Clusters of four that the device runs at a time (a CTA takes an SM; a cluster's SMs lie in one GPC), 0 if it cannot tell.
@@ -1173,7 +1244,7 @@ int tc_clusters(size_t smem) {
     auto kern = tkd_stream_tc_kernel<FMT, true, true, true, TKD_EPI_PLAIN>;
     int n = 0;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = tc_config<true>(4, smem, nullptr, false, attr);
+    const cudaLaunchConfig_t cfg = tc_config<true>(4, kTcWarps<FMT> * 32, smem, nullptr, false, attr);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
