@@ -468,11 +468,6 @@ __device__ __forceinline__ void chunk_mma(float (&acc)[NA][MT][4], uint32_t code
     });
 }
 
-// bf16 output as the top-k records order it: a monotone 16-bit key, 0 below every value (dense_writer.cpp:215).
-__device__ __forceinline__ uint32_t topk_key(uint16_t b) {
-    return (uint32_t)(b ^ (0x8000u | (0x7FFFu & (0u - (uint32_t)(b >> 15))))) & 0xFFFFu;
-}
-
 // The largest of a lane's candidates below `bound` (all of them: bound ~0).
 template <int N>
 __device__ __forceinline__ uint32_t topk_best(const uint32_t (&cand)[N], uint32_t bound) {
@@ -483,12 +478,24 @@ __device__ __forceinline__ uint32_t topk_best(const uint32_t (&cand)[N], uint32_
     return best;
 }
 
+// A lane's two largest candidates below `bound`.
+__device__ __forceinline__ void topk_two(const uint32_t (&cand)[16], uint32_t bound, uint32_t& b1, uint32_t& b2) {
+    b1 = b2 = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const uint32_t c = cand[j] < bound ? cand[j] : 0u;
+        b2 = max(b2, min(b1, c)), b1 = max(b1, c);
+    }
+}
+
 // The top-k records of the unit of columns that panel c.pl belongs to, made by the CTA whose output warps complete the
 // unit's last panel, from the bf16 outputs themselves (all four output warps call this after a panel's output stage). A
 // candidate is key << 16 | 0xFFFF - its column in the unit: key descending, column ascending. Each warp finds the best k of its
-// quarter of the unit (16 columns a lane; a round is one warp-wide maximum in hardware, and only the lane that gave it looks
-// through its candidates again), a row after the other, then a warp merges a row's four lists. (Every round's maximum over
-// the four warps through shared memory, with two barriers a round, took 8 rows of 8 some 5 us a unit.)
+// quarter of the unit (16 columns a lane; a round is one warp-wide maximum in hardware, and the lane that gave it puts up its
+// second; it looks through its candidates again only when that one has gone too), a row after the other, then a warp merges a row's
+// four lists. Lane q keeps the q-th. (Every round's maximum over the four warps through shared memory, with two barriers a round,
+// took 8 rows of 8 some 5 us a unit; with the winner's next looked for among its sixteen every round a head of 118656 columns
+// of 3328, bfloat4_b, took 75.9 us for 8 rows, 70.1 so.)
 // parts: what a panel counts for; add: what this call does.
 __device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c, const TkdSegDev& sg, int parts, int add, int et, int ow, int lane,
                                              float* tbuf, volatile int* sflag, uint16_t* y16, int topk_k, int npeers) {
@@ -538,41 +545,65 @@ __device__ __forceinline__ void topk_records(const TkdParams& p, const Cursor& c
         uint32_t cand[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            const uint32_t key = topk_key((uint16_t)(next[j >> 1] >> (16 * (j & 1))));
-            cand[j] = j < have && key ? (key << 16) | (0xFFFFu - (uint32_t)(c0 + j)) : 0u;
+            // (a bf16 output as the records order it: a monotone 16-bit key, 0 below every value, dense_writer.cpp:215; two a word)
+            const uint32_t w = next[j >> 1], keys = w ^ (((w >> 15) & 0x00010001u) * 0x7FFFu | 0x80008000u);
+            const uint32_t key = j & 1 ? keys & 0xFFFF0000u : keys << 16;
+            cand[j] = j < have && key ? key | (0xFFFFu - (uint32_t)(c0 + j)) : 0u;
         }
         if (r + 1 < p.topk_rows) load(r + 1, next);
-        uint32_t best = topk_best(cand, 0xFFFFFFFFu);
+        uint32_t b1, b2, mine = 0, mine2 = 0;  // (mine2: k past 32)
+        topk_two(cand, 0xFFFFFFFFu, b1, b2);
+        bool gone = false;  // the lane's second is its best already
         for (int q = 0; q < topk_k; ++q) {
-            const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, best);
-            if (lane == 0) red[(r * 4 + ow) * topk_k + q] = m;  // (0: nothing left)
-            if (best == m) best = topk_best(cand, m);
+            const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, b1);  // (0: nothing left)
+            if (lane == q) mine = m;
+            if (lane + 32 == q) mine2 = m;
+            if (b1 == m) {
+                if (gone)
+                    topk_two(cand, m, b1, b2), gone = false;
+                else
+                    b1 = b2, gone = true;
+            }
         }
+        if (lane < topk_k) red[(r * 4 + ow) * topk_k + lane] = mine;
+        if (lane + 32 < topk_k) red[(r * 4 + ow) * topk_k + lane + 32] = mine2;
     }
     bar_output_warps();
     const size_t rec_at = (size_t)(p.topk_slot0 + slot) * 2 * p.topk_rows * topk_k;
     uint32_t* rec = p.records + rec_at;
     const uint32_t base = p.topk_base + (uint32_t)wi * (uint32_t)sg.n_valid + (uint32_t)col0;
     for (int r = ow; r < p.topk_rows; r += 4) {
-        uint32_t cand[8];  // (4 k candidates, k at most 64)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) cand[j] = lane + 32 * j < 4 * topk_k ? red[r * 4 * topk_k + lane + 32 * j] : 0u;
-        uint32_t best = topk_best(cand, 0xFFFFFFFFu);
-        for (int q = 0; q < topk_k; ++q) {
-            const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, best);
-            if (best == m) best = topk_best(cand, m);
-            if (lane == 0) {
-                const uint32_t key = m >> 16, idx = m ? base + (0xFFFFu - (m & 0xFFFFu)) : 0xFFFFFFFFu;
-                const int at_k = r * topk_k + q, at_i = (p.topk_rows + r) * topk_k + q;
-                rec[at_k] = key;
-                rec[at_i] = idx;
-#pragma unroll 1
-                for (int pq = 0; pq < npeers; ++pq)
-                    if (p.peer_records[pq]) {
-                        p.peer_records[pq][rec_at + at_k] = key;
-                        p.peer_records[pq][rec_at + at_i] = idx;
-                    }
+        uint32_t mine = 0, mine2 = 0;
+        if (4 * topk_k <= 32) {  // a candidate a lane
+            uint32_t best = lane < 4 * topk_k ? red[r * 4 * topk_k + lane] : 0u;
+            for (int q = 0; q < topk_k; ++q) {
+                const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, best);
+                if (lane == q) mine = m;
+                if (best == m) best = 0;
             }
+        } else {
+            uint32_t cand[8];  // (4 k candidates, k at most 64)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) cand[j] = lane + 32 * j < 4 * topk_k ? red[r * 4 * topk_k + lane + 32 * j] : 0u;
+            uint32_t best = topk_best(cand, 0xFFFFFFFFu);
+            for (int q = 0; q < topk_k; ++q) {
+                const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, best);
+                if (lane == q) mine = m;
+                if (lane + 32 == q) mine2 = m;
+                if (best == m) best = topk_best(cand, m);
+            }
+        }
+        for (int q = lane; q < topk_k; q += 32) {
+            const uint32_t m = q < 32 ? mine : mine2, key = m >> 16, idx = m ? base + (0xFFFFu - (m & 0xFFFFu)) : 0xFFFFFFFFu;
+            const int at_k = r * topk_k + q, at_i = (p.topk_rows + r) * topk_k + q;
+            rec[at_k] = key;
+            rec[at_i] = idx;
+#pragma unroll 1
+            for (int pq = 0; pq < npeers; ++pq)
+                if (p.peer_records[pq]) {
+                    p.peer_records[pq][rec_at + at_k] = key;
+                    p.peer_records[pq][rec_at + at_i] = idx;
+                }
         }
     }
     bar_output_warps();  // (the lists have been read)
