@@ -118,7 +118,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) tkd_rows_kernel(const __gr
     const uint32_t half0 = xbar0 + 8 * kRowsSegs, pfull = half0 + 64, pempty = pfull + 8;
     const uint32_t pbuf = smem_u32(smem + p.off_pbuf), ring0 = smem_u32(smem + p.off_ring), xt0 = smem_u32(smem + p.off_xt);
     volatile int* sflag = reinterpret_cast<volatile int*>(smem + TKD_SMEM_HEAD - 16);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (the warp's number by a shuffle, as in tkd_narrow_kernel: 9 rows of bfloat4_b [4096, 57344] 41.2 us without, 37.3 so; bfloat8_b 48.7
+    // and 47.6; 17 rows of bfloat4_b [1152, 4288], two tiles, 6.5 and 5.1)
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
         for (int s = 0; s < p.nstages; ++s) mbar_init(full0 + 8 * s, 1), mbar_init(empty0 + 8 * s, SW);
