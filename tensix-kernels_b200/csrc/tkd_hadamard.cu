@@ -21,6 +21,8 @@ __global__ void __launch_bounds__(kThreads) tkd_hadamard_kernel(const uint16_t* 
                                                                 const uint32_t* __restrict__ signs, int K,
                                                                 uint16_t* __restrict__ out, int64_t ldo) {
     __shared__ float v[kBlock];
+    // (the matmul behind this one streams its weights meanwhile)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");  // (x may be the output of the kernel before this one)
     const int row = blockIdx.y, b = blockIdx.x, t = threadIdx.x;
     const uint16_t* xr = x + (int64_t)row * ldx + (int64_t)b * kBlock;

@@ -174,6 +174,29 @@ PyObject* host_pick(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
 }
 
+// hadamard(x [rows, K], sign words) -> x' [1, 1, rows, K] bf16: tkd_hadamard.
+PyObject* host_hadamard(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2 || !all_tensors(args, {0, 1}, {})) return type_error("tkd_host.hadamard: x, signs");
+    try {
+        const at::Tensor &x = THPVariable_Unpack(args[0]), &signs = THPVariable_Unpack(args[1]);
+        if (x.dim() != 2 || !x.is_cuda()) return type_error("tkd_host.hadamard: x is [rows, K] on the device");
+        c10::cuda::OptionalCUDAGuard guard;
+        if (c10::cuda::current_device() != x.get_device()) guard.set_index(x.get_device());
+        const int64_t rows = x.size(0), k = x.size(1), shape[4] = {1, 1, rows, k}, ldx = x.stride(0);
+        at::Tensor out = at::detail::empty_cuda(shape, at::kBFloat16, x.device(), std::nullopt);
+        void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
+        const void *xp = x.data_ptr(), *sp = signs.data_ptr();
+        void* op = out.data_ptr();
+        int rc;
+        Py_BEGIN_ALLOW_THREADS rc = tkd_hadamard(xp, ldx, static_cast<const uint32_t*>(sp), (int)rows, (int)k, op, k, stream);
+        Py_END_ALLOW_THREADS if (rc) return tkd_error(rc, "tkd_hadamard");
+        return THPVariable_Wrap(std::move(out));
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
 // This thread's int in pinned host memory, which a packing kernel sets when its weight is wide: read after the stream has been
 // waited for, with nothing copied back.
 struct WideWord {
@@ -248,6 +271,7 @@ PyMethodDef methods[] = {
     fast<host_route>("route"),
     fast<host_pack>("pack"),
     fast<host_pick>("pick"),
+    fast<host_hadamard>("hadamard"),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "tkd_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -123,12 +123,8 @@ def _rotated(x, mask, memory_config):
     device = x.device()
     m, k = x.shape[-2], x.shape[-1]
     assert x.dtype == ttnn.bfloat16 and k % HADAMARD == 0 and mask.t.numel() == k // TILE * 64, (x.shape, mask.shape)
-    y = ttnn.allocate_tensor_on_device([1, 1, m, k], ttnn.bfloat16, ttnn.TILE_LAYOUT, device, memory_config)
-    xt = x.t.reshape(m, k)
-    with torch.cuda.device(device.torch):
-        _tkd.check(_tkd.lib().tkd_hadamard(xt.data_ptr(), xt.stride(0), mask.t.data_ptr(), m, k, y.t.data_ptr(), k,
-                                           torch.cuda.current_stream().cuda_stream), "tkd_hadamard")
-    return y
+    y = _tkd.host().hadamard(x.t.reshape(m, k), mask.t)
+    return ttnn.Tensor(y, ttnn.bfloat16, ttnn.TILE_LAYOUT, device, memory_config)
 
 
 def rotate_rows(x, hadamard):
