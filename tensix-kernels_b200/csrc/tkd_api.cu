@@ -67,6 +67,7 @@ int tc_cluster_count(int fmt, size_t smem) {
 // 1.03, [1536, 20480] 1.37; 24 rows of bfloat4_b, [1024, 4096] 0.85, [1024, 20480] 1.24; K 2560 of bfloat4_b is the worst
 // ([2560, 5120] 32 rows 1.09, 17 rows 1.26). A head of 75968 columns takes up to twice the other's time (bfloat4_b, 24 rows, K 2560,
 // 77 / 38 us; bfloat8_b, 32 rows, K 1536, 56 / 33), which the projections of a model's layers outweigh.
+// (Measured with the warps' numbers not yet shuffled: both kernels have taken 0.9 to 0.95 of these times since.)
 int rows_layout(TkdParams& p, int sab) {
     const int ck = tkd_chunk_k(p.fmt), nch = (p.K + ck - 1) / ck;
     if (p.M > 16 && p.nslices == 4 && (p.M > 24 || p.K > 1536)) return 0;
