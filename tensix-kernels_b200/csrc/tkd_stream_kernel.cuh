@@ -742,7 +742,7 @@ __global__ void __launch_bounds__((1 + kStreamWarps + 4) * 32, 1) tkd_stream_ker
     float* tbuf = reinterpret_cast<float*>(smem + p.off_tbuf);  // [128 columns][MP]
     uint8_t* ring = smem + p.off_ring;
 
-    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // let the kernel after this one in the stream start its CTAs as SMs become free
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
