@@ -138,7 +138,7 @@ __device__ __forceinline__ uint32_t rank16(uint32_t kk) {
     return kk == 0x7FFFu ? 0x8000u : kk;
 }
 
-constexpr int kPickWarps = 16, kPickOwn = 8;
+constexpr int kPickWarps = 16, kPickOwn = 8, kPickCluster = 4;
 
 // The best `top` (at most 32) of a warp's candidates, lane t the t-th: (rank, id), rank 0 where there are none. A candidate's
 // word is rank << 12 | 4095 - its place, so that an equal rank keeps the earlier place; a round is one warp-wide maximum in
@@ -230,8 +230,12 @@ __device__ __forceinline__ void pick_count(PickCount& s, int nrec, int k, int to
 //      [token, the first candidate by the device's own logit, count, 0 ...]; count is the candidates held (RECORDS: all
 //      valid slots). No valid slot: [0, 0xFFFFFFFF, 0].
 // Bound by latency: as `top` rounds over all slots read anew, with two barriers each, and one candidate after the other, it
-// took a fifth of a vocabulary's call.
-template <bool RECORDS, bool COUNT>
+// took a fifth of a vocabulary's call. CL, of three and more rows: a row is a cluster of CL CTAs; each finds the same
+// candidates and takes its share of their rows, whose exact logits meet in the first one's shared memory. The candidates lie anywhere in
+// the head, each in a page of its own as a rule, and sixteen such rows at a time were more than an SM has under way beside other CTAs
+// that ask for theirs: records and pick of 8 rows of a head of 118656 columns of 3328 90.5 us with a CTA a row, 87.6 so; 4 rows of 34304
+// columns of 3712 44.7 and 41.5; one row 65.5 and 66.0, so one and two rows keep a CTA each.
+template <bool RECORDS, bool COUNT, int CL>
 __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const uint32_t* __restrict__ records, int nrec, int rows,
                                                                         int k, int top, uint32_t vocab,
                                                                         const uint16_t* __restrict__ x, int64_t ldx, int dim,
@@ -242,8 +246,9 @@ __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const ui
     extern __shared__ __align__(16) uint8_t pick_smem[];
     __shared__ int held, nvalid[kPickWarps];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (CL > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");  // (waited for before the first store to another CTA)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = blockIdx.x / CL, part = blockIdx.x % CL, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = nrec * k;
     int mine = 0;
     if constexpr (COUNT) {
@@ -306,7 +311,8 @@ __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const ui
     const int nc = held;
     if constexpr (!RECORDS) {
         const uint16_t* xr = x + (size_t)r * ldx;
-        for (int c = warp; c < nc; c += kPickWarps) {
+        if constexpr (CL > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        for (int c = warp * CL + part; c < nc; c += kPickWarps * CL) {
             const uint16_t* wr = head + (size_t)cid[c] * ld_head;
             float acc = 0.f;
 #pragma unroll 16
@@ -325,10 +331,21 @@ __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const ui
             if (lane == 0) {
                 uint32_t bits = __float_as_uint(acc);
                 if (round) bits = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(acc)) << 16;
-                clogit[c] = order32(bits);
+                if constexpr (CL > 1) {
+                    uint32_t to;  // (clogit[c] of the cluster's first CTA)
+                    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"((uint32_t)__cvta_generic_to_shared(&clogit[c])));
+                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to), "r"(order32(bits)) : "memory");
+                } else {
+                    clogit[c] = order32(bits);
+                }
             }
         }
-        __syncthreads();
+        if constexpr (CL > 1) {
+            asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+            if (part) return;
+        } else {
+            __syncthreads();
+        }
     }
     if (warp == 0) {
         const bool have = lane < nc;
@@ -347,21 +364,22 @@ __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const ui
     }
 }
 
-template <bool RECORDS, bool COUNT>
+template <bool RECORDS, bool COUNT, int CL>
 int launch_pick_by(const uint32_t* records, int nrec, int rows, int k, int top, uint32_t vocab, const uint16_t* x, int64_t ldx,
                 int dim, const uint16_t* head, int64_t ld_head, int round, const uint32_t* tmap, uint32_t* out,
                 uint32_t* ids_out, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)rows);
+    cfg.gridDim = dim3((unsigned)(rows * CL));
     cfg.blockDim = dim3(kPickWarps * 32);
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (CL > 1) attr[1].id = cudaLaunchAttributeClusterDimension, attr[1].val.clusterDim = {CL, 1, 1}, cfg.numAttrs = 2;
     cfg.dynamicSmemBytes = COUNT ? sizeof(PickCount) : 0;
-    return (int)cudaLaunchKernelEx(&cfg, tkd_head_pick_kernel<RECORDS, COUNT>, records, nrec, rows, k, top, vocab, x, ldx, dim, head,
+    return (int)cudaLaunchKernelEx(&cfg, tkd_head_pick_kernel<RECORDS, COUNT, CL>, records, nrec, rows, k, top, vocab, x, ldx, dim, head,
                                    ld_head, round, tmap, out, ids_out);
 }
 // Counting compares every record with every other, rounds take `top` turns: counting up to twenty records for each of the top. Measured,
@@ -372,8 +390,11 @@ template <bool RECORDS, class... A>
 int launch_pick(const uint32_t* records, int nrec, int rows, int k, int top, A... more) {
     if constexpr (!RECORDS)
         if (nrec <= 20 * top && nrec <= kPickRecs && (int64_t)nrec * k <= kPickSlots)
-            return launch_pick_by<RECORDS, true>(records, nrec, rows, k, top, more...);
-    return launch_pick_by<RECORDS, false>(records, nrec, rows, k, top, more...);
+            return rows > 2 ? launch_pick_by<RECORDS, true, kPickCluster>(records, nrec, rows, k, top, more...)
+                            : launch_pick_by<RECORDS, true, 1>(records, nrec, rows, k, top, more...);
+    if constexpr (!RECORDS)
+        if (rows > 2) return launch_pick_by<RECORDS, false, kPickCluster>(records, nrec, rows, k, top, more...);
+    return launch_pick_by<RECORDS, false, 1>(records, nrec, rows, k, top, more...);
 }
 
 }  // namespace
