@@ -442,6 +442,7 @@ __global__ void __launch_bounds__(kTcWarps<FMT> * 32, 1) tkd_stream_tc_kernel(co
                 if (u >= nunits) break;
                 ok = mbar_wait(aempty0 + 8 * ps, aphase, p.status);
                 if (!ok) break;
+                tc_fence_after();  // (the MMAs that read the slot before have completed: tcgen05.commit's arrival)
                 const uint32_t sb = XW ? 0 : ops0 + ps * kTcSlot, ta = alane + ps * 2 * kTcACols;
 #pragma unroll
                 for (int sub = 0; sub < 2; ++sub) {
