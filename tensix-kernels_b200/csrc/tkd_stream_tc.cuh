@@ -22,7 +22,7 @@
 //                  The same warps write the tile of activations a unit is multiplied by (32 rows x 64 k, rows past M
 //                  zero, K-major with the 128-byte swizzle, in that order of k) into shared memory: each lane loads
 //                  its 16 bytes of the NEXT chunk's tiles into registers while it decodes this chunk (they come from
-//                  L2, a microsecond away). bf16 weights: warps 23-26 do, by asynchronous copies of 8 bytes.
+//                  L2, a microsecond away). bf16 weights: the warps from 23 on do, by asynchronous copies of 8 bytes.
 //   warps 19-22    output warps (thread = panel column = tensor-memory lane): read a slice's sums with tcgen05.ld, keep
 //                  the running sums in shared memory, and from there on do what tkd_stream_kernel's output warps do
 //   warp 1         producer (one lane issues): the same ring of packed-weight chunks as tkd_stream_kernel
@@ -53,15 +53,20 @@ static_assert(kTcA0 + kTcSlots * 2 * kTcACols <= 512, "the A slots must fit the 
 // lowest number on purpose: the schedulers favour older warps, and as the last warp of the CTA it got an issue slot
 // every twenty cycles beside four decode warps that are always ready (its unit of eight MMAs took 770 ns).
 constexpr int kTcMmaWarp = 0, kTcProducerWarp = 1, kTcDecodeWarp0 = 3, kTcOutputWarp0 = 19, kTcXWarp0 = 23, kTcMmaWarps = 2;
-// bf16 weights need no arithmetic, and the activations have four warps of their own (warps 23-26, at 72 registers a thread; they write
-// as far ahead as kTcXSlots units): launches in a graph, 32 rows, us with the decode warps bringing x / so: [2048, 2048] 5.6 / 4.6,
-// [4096, 6144] 15.3 / 13.5, [4096, 28672] 42.9 / 40.9. Block-float weights keep the decode warps busy, and x costs them less than four
+// bf16 weights need no arithmetic, and the activations have warps of their own (at 72 registers a thread; they write as far ahead as
+// kTcXSlots units): launches in a graph, 32 rows, us with the decode warps bringing x / so: [2048, 2048] 5.6 / 4.6, [4096, 6144] 15.3 /
+// 13.5, [4096, 28672] 44.4 / 39.7. In clusters four (warps 23-26): a launch is short, and x is what its first units wait for ([2080, 2048]
+// with two 5.4, with four 5.0; [4128, 2048] 6.9 / 6.4). Elsewhere two: as fast, and the compiler keeps more of the output stage's values
+// in registers ([2080, 14336] with four 19.5, with two 16.1; gate and up [4128, 14336] 53.9 / 43.6, [4096, 14336] 47.3 / 44.5).
+// Block-float weights keep the decode warps busy, and x costs them less than four
 // more warps do: bfloat4_b, 32 rows, [4096, 57344] 39.0 / 46.1, [4096, 14336] 15.9 / 17.6 (bfloat8_b 47.0 / 49.7, 17.3 / 17.7).
 template <int FMT>
 constexpr bool kTcXw = FMT == TKD_BF16;
-constexpr int kTcXWarps = 4, kTcXSlots = TKD_TC_XSLOTS;
-template <int FMT>
-constexpr int kTcWarps = kTcXWarp0 + (kTcXw<FMT> ? kTcXWarps : 0);
+constexpr int kTcXSlots = TKD_TC_XSLOTS;
+template <bool CL>
+constexpr int kTcXWarps = CL ? 4 : 2;
+template <int FMT, bool CL>
+constexpr int kTcWarps = kTcXWarp0 + (kTcXw<FMT> ? kTcXWarps<CL> : 0);
 // the MMA warp number (0, 1) of a warp, or -1: warps 0 and 2
 __device__ __forceinline__ int tc_mma_warp(int warp) { return warp == 0 ? 0 : warp == 2 ? 1 : -1; }
 constexpr int kTcMP = 40;            // floats per column in tbuf (32 rows, padded)
@@ -146,7 +151,7 @@ constexpr int kTcExchange = 4 * 8 * 32 * 16;  // bytes: [slice][4 rows][32 colum
 // sums and their order are those of the other form, whose panels end in a chain of trips through L2 by one CTA alone: sums
 // stored 0.6 us, counted in 0.9, added up 2.4, put out 1.0 (32 rows, [4096, 4096] of bfloat8_b, 11.5 us from start to end).
 template <int FMT, bool KWHOLE, bool PLAIN, bool CL = false, int EK = EK_ANY>
-__global__ void __launch_bounds__(kTcWarps<FMT> * 32, 1) tkd_stream_tc_kernel(const __grid_constant__ TkdParams p) {
+__global__ void __launch_bounds__(kTcWarps<FMT, CL> * 32, 1) tkd_stream_tc_kernel(const __grid_constant__ TkdParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     using F = Fmt<FMT>;
     constexpr int SW = 16, MP = kTcMP;
@@ -185,7 +190,7 @@ __global__ void __launch_bounds__(kTcWarps<FMT> * 32, 1) tkd_stream_tc_kernel(co
             mbar_init(aempty0 + 8 * s, 1);
         }
         for (int s = 0; XW && s < kTcXSlots; ++s) {
-            mbar_init(bfull0 + 8 * s, 32 * kTcXWarps);
+            mbar_init(bfull0 + 8 * s, 32 * kTcXWarps<CL>);
             mbar_init(bempty0 + 8 * s, 1);
         }
         for (int s = 0; s < 2; ++s) {
@@ -491,7 +496,7 @@ __global__ void __launch_bounds__(kTcWarps<FMT> * 32, 1) tkd_stream_tc_kernel(co
         // are of 8 bytes; a lane has the same 8 bytes of every RS-th row. What lies in rows past M only feeds columns of D that
         // nothing reads.
         asm volatile("griddepcontrol.wait;" ::: "memory");  // (x may be the output of the kernel before this one)
-        constexpr int RS = 2 * kTcXWarps, NR = 32 / RS;
+        constexpr int RS = 2 * kTcXWarps<CL>, NR = 32 / RS;
         const int gl = (warp - kTcXWarp0) * 32 + lane, r0 = gl >> 4, ke = 4 * (gl & 15);  // this lane's first row, its k of a tile
         const uint32_t o = 64 * (ke >> 5) + 32 * ((ke >> 2) & 1) + 8 * ((ke >> 3) & 3);
         const uint32_t d0 = ops0 + r0 * 128 + (o & 15), c0 = ((o >> 4) ^ (r0 & 7)) << 4;
@@ -1236,7 +1241,7 @@ int launch_tc(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
         if (dev >= 0 && dev < 64) allowed[dev] = true;
     }
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = tc_config<CL>(grid, kTcWarps<FMT> * 32, smem, st, !p.no_pdl, attr);
+    const cudaLaunchConfig_t cfg = tc_config<CL>(grid, kTcWarps<FMT, CL> * 32, smem, st, !p.no_pdl, attr);
     return (int)cudaLaunchKernelEx(&cfg, kern, p);
 }
 // Clusters of four that the device runs at a time (a CTA takes an SM; a cluster's SMs lie in one GPC), 0 if it cannot tell.
@@ -1245,7 +1250,7 @@ int tc_clusters(size_t smem) {
     auto kern = tkd_stream_tc_kernel<FMT, true, true, true, TKD_EPI_PLAIN>;
     int n = 0;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = tc_config<true>(4, kTcWarps<FMT> * 32, smem, nullptr, false, attr);
+    const cudaLaunchConfig_t cfg = tc_config<true>(4, kTcWarps<FMT, true> * 32, smem, nullptr, false, attr);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
