@@ -1264,12 +1264,15 @@ int launch_fmt_all(const TkdParams& p, int grid, size_t smem, cudaStream_t st) {
     if (p.tc) {
         const bool whole = p.K % (Fmt<FMT>::SUBSA * Fmt<FMT>::KSA) == 0;
         if (!p.topk_k && !p.npeers) {
-            // (a K that ends inside a chunk, the rare case: one instance for all outputs)
-            // (but silu, whose code in it cost the others up to 1.8 %)
-            if (!whole && p.epi == TKD_EPI_SILU)
-                return p.tc_cluster ? launch_tc<FMT, false, true, true, TKD_EPI_SILU>(p, grid, smem, st)
-                                    : launch_tc<FMT, false, true, false, TKD_EPI_SILU>(p, grid, smem, st);
-            if (!whole) return p.tc_cluster ? launch_tc<FMT, false, true, true>(p, grid, smem, st) : launch_tc<FMT, false, true>(p, grid, smem, st);
+            // A K that ends inside a chunk: in clusters, the shorter launches, one instance for all outputs but silu (whose code in it cost
+            // the others up to 1.8 %); elsewhere an instance for each kind, as for whole chunks: that for all spilled registers (32 rows
+            // of [4128, 14336], us with it / so: bfloat8_b 22.3 / 20.1, gate and up 41.1 / 33.5; bfloat4_b 22.4 / 20.5, 28.1 / 26.4;
+            // bf16 24.6 / 23.9).
+            if (!whole && p.tc_cluster)
+                return p.epi == TKD_EPI_SILU ? launch_tc<FMT, false, true, true, TKD_EPI_SILU>(p, grid, smem, st)
+                                             : launch_tc<FMT, false, true, true>(p, grid, smem, st);
+            if (!whole)
+                return for_epilogue(p.epi, [&](auto ek) { return launch_tc<FMT, false, true, false, decltype(ek)::value>(p, grid, smem, st); });
             return for_epilogue(p.epi, [&](auto ek) {
                 constexpr int EK = decltype(ek)::value;
                 return p.tc_cluster ? launch_tc<FMT, true, true, true, EK>(p, grid, smem, st) : launch_tc<FMT, true, true, false, EK>(p, grid, smem, st);

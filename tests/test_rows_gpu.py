@@ -63,6 +63,20 @@ def test_units_of_the_tensor_memory_kernel(device, fmt, m, k, n):
     linear.check_status(device)
 
 
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
+@pytest.mark.parametrize("m,k,n", [(17, 3104, 192), (32, 4128, 144), (9, 14368, 64)])
+def test_every_output_of_a_k_that_ends_inside_a_chunk(device, fmt, m, k, n):
+    """The tensor-memory kernel has an instance for each kind of output, outside clusters and (for fewer kinds) in them."""
+    test_outputs_against_oracle(device, fmt, m, k, n)
+    g = torch.Generator().manual_seed(m)
+    w, x = torch.randn(n, k, generator=g) * 0.05, torch.randn(m, k, generator=g)
+    tw, _ = linear.native_weight(device, w, DT[fmt])
+    plain = x.to(torch.bfloat16).double() @ torch.from_numpy(orc.native_values(w, fmt)[0]).double()
+    for ctas in (None, 3):
+        close_bf16(host(linear.linear(dev_x(device, x), tw, None, activation="silu", max_ctas=ctas)), torch.nn.functional.silu(plain).numpy())
+    linear.check_status(device)
+
+
 @pytest.mark.parametrize("m,k", [(9, 1024), (16, 288), (24, 1056), (30, 1056)])
 def test_records_of_the_plain_calls_outputs(device, m, k):
     """Records are the canonical top-k of the outputs that a plain call gives, with and without y written, of one weight and of a
