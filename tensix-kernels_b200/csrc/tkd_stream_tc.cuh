@@ -847,40 +847,41 @@ __global__ void __launch_bounds__(kTcWarps<FMT, CL> * 32, 1) tkd_stream_tc_kerne
                         }
                         asm volatile("cp.async.wait_all;" ::: "memory");
                     }
-                    // eight rows of four slices at a time, their loads side by side (a row past M: what lies there)
+                    // eight rows of four slices at a time, their loads side by side (a row past M: what lies there); a loop for each
+                    // place, since one that asks at every load where it reads held both addresses and spilled (112 bytes a thread
+                    // of bf16's gate and up, 140 with records): 32 rows, us with one / so: bf16 gate and up [4096, 14336] 44.7 / 43.9,
+                    // [4096, 4736] 11.4 / 10.7; bfloat4_b with records [4096, 28672] 41.5 / 39.4; bfloat8_b [2048, 14336] 14.1 / 13.3.
                     const float* src0 = part(0);
                     const size_t step = (size_t)2 * M * TKD_PANEL_COLS;
+                    auto add = [&](auto at) {  // at(slice, four rows): the sums there
 #pragma unroll 1
-                    for (int r = 0; r < m4; r += 2) {
-                        float4 th[2] = {};
+                        for (int r = 0; r < m4; r += 2) {
+                            float4 th[2] = {};
 #pragma unroll 1
-                        for (int s4 = 0; s4 < ns; s4 += 4) {
-                            float4 v[4][2];
+                            for (int s = 0; s < ns; s += 4) {
+                                float4 v[4][2];
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                const int si = min(s4 + u, ns - 1);
-                                const float4* src_g = reinterpret_cast<const float4*>(src0 + si * step + r * 512);
-                                const uint32_t src_s = ring_c + (si * m4 + r) * 2048;
+                                for (int u = 0; u < 4; ++u)
 #pragma unroll
-                                for (int q = 0; q < 2; ++q) {
-                                    if (staged) {
-                                        const uint4 w = lds128(src_s + q * 2048);
-                                        v[u][q] = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
-                                    } else {
-                                        v[u][q] = __ldcg(src_g + q * 128);
-                                    }
-                                }
+                                    for (int q = 0; q < 2; ++q) v[u][q] = at(min(s + u, ns - 1), r + q);
+#pragma unroll
+                                for (int u = 0; u < 4; ++u)
+                                    if (s + u < ns)
+#pragma unroll
+                                        for (int q = 0; q < 2; ++q)
+                                            th[q] = make_float4(th[q].x + v[u][q].x, th[q].y + v[u][q].y, th[q].z + v[u][q].z, th[q].w + v[u][q].w);
                             }
 #pragma unroll
-                            for (int u = 0; u < 4; ++u)
-                                if (s4 + u < ns)
-#pragma unroll
-                                    for (int q = 0; q < 2; ++q)
-                                        th[q] = make_float4(th[q].x + v[u][q].x, th[q].y + v[u][q].y, th[q].z + v[u][q].z, th[q].w + v[u][q].w);
+                            for (int q = 0; q < 2; ++q) *reinterpret_cast<float4*>(trow + 4 * (r + q)) = th[q];
                         }
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) *reinterpret_cast<float4*>(trow + 4 * (r + q)) = th[q];
-                    }
+                    };
+                    if (staged)
+                        add([&](int si, int r) {
+                            const uint4 w = lds128(ring_c + (si * m4 + r) * 2048);
+                            return make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+                        });
+                    else
+                        add([&](int si, int r) { return __ldcg(reinterpret_cast<const float4*>(src0 + si * step + r * 512)); });
                 }
                 bar_output_warps();  // sflag may be written again only after everyone has read it
             }
