@@ -533,11 +533,14 @@ int tkd_matmul_rows_workspace(const TkdMatmul* a, uint64_t* bytes) {
 
 // Whether a call of more than 32 rows runs tkd_rows_kernel in tiles of rows (of sixteen, less where x is too long for that), its
 // launch in L without the tensors. wide_us: what make_wide's model expects of tkd_wide_kernel's units and outputs.
-// Both expectations are fitted to launches in a graph (B200; 33 to 512 rows, K 576 to 3136, N 544 to 10240, three formats): a launch of
-// this kernel by the items of its longest CTA, which for block-float weights comes out about a tenth high, hence the 1.1; one of
-// tkd_wide_kernel, with the one that lays x out, by make_wide's model. bfloat8_b, this kernel / the other, us: 40 rows [3072, 6144] with a
-// residual 13.3 / 15.8, 128 rows [2048, 2048] 10.4 / 11.3, 320 rows [640, 608] 6.3 / 6.7. A weight is taken apart anew for every tile
-// here: with N or rows beyond that the other is the faster one (64 rows [3072, 6144] with a residual 22.2 / 15.3).
+// Fitted to launches in a graph (B200, us): 1870 shapes of 33 to 512 rows, K 32 to 3136, N 16 to 8192, three formats, every kind of
+// output, each with both kernels, by those whose two times lie within a factor of 1.5. A launch of this kernel goes by K in whole chunks
+// and the items of its longest CTA (5 % off on average, 18 % at most); one of tkd_wide_kernel, with the one that lays x out, by make_wide's
+// model, x and the kind of output (6 %, 24 %). The rule's time is 1.001 of the better of the two (K below 256 1.003), at worst 1.12; on 260
+// other shapes 1.001 and 1.09. This kernel / the other: bfloat8_b, 40 rows [1056, 4096] 7.1 / 7.3, 128 rows [2048, 2048] 10.2 / 11.3, 64 rows
+// of gate and up [2944, 1728] 14.1 / 17.6, 48 rows [576, 4096] 6.3 / 5.4; bfloat4_b, 64 rows [576, 4096] 7.4 / 5.4, 128 rows [2048, 2048]
+// 9.2 / 11.2; bf16, 40 rows [1056, 4096] 6.9 / 7.2, 256 rows of K 2048, N 1024 10.5 / 11.4, N 4096 31.6 / 12.4. A weight is taken apart
+// anew for every tile here: with N or rows the other is the faster one.
 static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     int sms = sm_count();
     if (sms <= 0) sms = 148;
@@ -555,8 +558,15 @@ static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     p.rows_team = sms / tiles < items ? sms / tiles : items;
     p.rows_tile = one.m, p.M = a->m;
     L->grid = tiles * p.rows_team;
-    const double k = p.K / 1000., most = (items + p.rows_team - 1) / p.rows_team;
-    return 3.2 + 0.2 * k + most * (0.65 + (p.fmt == TKD_BF16 ? 0.8 : 0.65) * k) < 1.1 * (2.6 + wide_us + 0.34 * k);
+    struct Fit { double launch, launch_k, item, item_k, wide, wide_k, wide_us; };
+    const Fit f = p.fmt == TKD_BFP8   ? Fit{2.9, 0.3, 0.56, 0.557, 2.44, 0.56, 0.88}
+                  : p.fmt == TKD_BFP4 ? Fit{2.53, 0.58, 0.69, 0.373, 2.86, 2.03, 0.365}
+                                      : Fit{2.92, 0.165, 0.45, 0.716, 2.92, 0.9, 0.663};
+    const bool glu = p.epi == TKD_EPI_GLU2 || p.epi == TKD_EPI_GLU_IL, silu = p.epi == TKD_EPI_SILU, res = a->residual != nullptr;
+    const int ck = tkd_chunk_k(p.fmt);
+    const double k = p.K / 1000., kc = (p.K + ck - 1) / ck * ck / 1000., most = (items + p.rows_team - 1) / p.rows_team;
+    const double mine = f.launch + f.launch_k * kc + most * (f.item + f.item_k * kc + (glu || silu ? 0.145 : res ? 0.11 : 0));
+    return mine < f.wide + f.wide_k * k + f.wide_us * wide_us + 0.002 * a->m * k + (glu ? 4.7 : silu ? 1.85 : res ? 1.2 : 0);
 }
 
 // Whether a call's output shares memory with x. (More than 32 rows may: tkd_wide_kernel reads a copy of x.)
