@@ -537,10 +537,10 @@ int tkd_matmul_rows_workspace(const TkdMatmul* a, uint64_t* bytes) {
 // output, each with both kernels, by those whose two times lie within a factor of 1.5. A launch of this kernel goes by K in whole chunks
 // and the items of its longest CTA (5 % off on average, 18 % at most); one of tkd_wide_kernel, with the one that lays x out, by make_wide's
 // model, x and the kind of output (6 %, 24 %). The rule's time is 1.001 of the better of the two (K below 256 1.003), at worst 1.12; on 260
-// other shapes 1.001 and 1.09. This kernel / the other: bfloat8_b, 40 rows [1056, 4096] 7.1 / 7.3, 128 rows [2048, 2048] 10.2 / 11.3, 64 rows
-// of gate and up [2944, 1728] 14.1 / 17.6, 48 rows [576, 4096] 6.3 / 5.4; bfloat4_b, 64 rows [576, 4096] 7.4 / 5.4, 128 rows [2048, 2048]
-// 9.2 / 11.2; bf16, 40 rows [1056, 4096] 6.9 / 7.2, 256 rows of K 2048, N 1024 10.5 / 11.4, N 4096 31.6 / 12.4. A weight is taken apart
-// anew for every tile here: with N or rows the other is the faster one.
+// other shapes, and on 360 of K 2688 to 5440, 1.001 and 1.09. This kernel / the other: bfloat8_b, 40 rows [1056, 4096] 7.1 / 7.3, 128 rows
+// [2048, 2048] 10.2 / 11.3, 64 rows of gate and up [2944, 1728] 14.1 / 17.6, 48 rows [576, 4096] 6.3 / 5.4; bfloat4_b, 64 rows [576, 4096]
+// 7.4 / 5.4, 128 rows [2048, 2048] 9.2 / 11.2; bf16, 40 rows [1056, 4096] 6.9 / 7.2, 256 rows of K 2048, N 1024 10.5 / 11.4, N 4096 31.6 /
+// 12.4. A weight is taken apart anew for every tile here: with N or rows the other is the faster one.
 static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     int sms = sm_count();
     if (sms <= 0) sms = 148;
@@ -565,7 +565,10 @@ static bool rows_tiles(const TkdMatmul* a, Layout* L, double wide_us) {
     const bool glu = p.epi == TKD_EPI_GLU2 || p.epi == TKD_EPI_GLU_IL, silu = p.epi == TKD_EPI_SILU, res = a->residual != nullptr;
     const int ck = tkd_chunk_k(p.fmt);
     const double k = p.K / 1000., kc = (p.K + ck - 1) / ck * ck / 1000., most = (items + p.rows_team - 1) / p.rows_team;
-    const double mine = f.launch + f.launch_k * kc + most * (f.item + f.item_k * kc + (glu || silu ? 0.145 : res ? 0.11 : 0));
+    // (bfloat8_b in stages of two chunks, K 3360 to 3840 and from 4384 on: 1.28 times as long an item, 372 rows [4640, 448] 21.5 us where
+    // the other kernel takes 16.2; bfloat4_b 1.06)
+    const double item = (f.item + f.item_k * kc + (glu || silu ? 0.145 : res ? 0.11 : 0)) * (p.fmt == TKD_BFP8 && p.rows_chunks == 2 ? 1.28 : 1);
+    const double mine = f.launch + f.launch_k * kc + most * item;
     return mine < f.wide + f.wide_k * k + f.wide_us * wide_us + 0.002 * a->m * k + (glu ? 4.7 : silu ? 1.85 : res ? 1.2 : 0);
 }
 
