@@ -55,19 +55,21 @@ int tc_cluster_count(int fmt, size_t smem) {
 // 9 to 32 rows: tkd_rows_kernel's chunks of a stage, with its shared-memory map in p; 0: the tensor-memory kernel. A rule on K, the
 // format and the number of rows only, because the two kernels' sums are different ones and a column's must not depend on more; it
 // goes for records and exchanged calls as well. Measured, launches in a graph over weights larger than L2, us with tkd_rows_kernel /
-// the tensor-memory kernel: 9 to 16 rows, wherever x leaves 80 KB of the 227 to the ring: bfloat8_b [1280, 4096] 4.8 / 6.8, [2048, 14336]
-// 10.9 / 12.5, [3328, 14336] with 16 rows, the worst, 16.6 / 16.0; bfloat4_b [2816, 4096] 5.9 / 9.2; less of a ring: bfloat8_b [4096, 14336]
-// with 16 rows 21.1 / 17.7. 17 to 24 rows, three MMAs a fragment: of four slices, where that kernel runs in clusters, up to K 1536
-// (bfloat8_b [1024, 4096] 5.2 / 7.1, [2048, 14336] 14.7 / 13.5); of other numbers of slices always (bfloat4_b [2816, 4096] 7.4 / 10.0). 25 to
-// 32 rows of other numbers of slices: bf16 with four MMAs a fragment ([1056, 14336] 12.8 / 17.1); block-float decodes beside four MMAs
-// take longer than the tensor memory's way ([1056, 14336] 19.5 / 16.2), and so run as two tiles of sixteen rows, a team of CTAs each
-// (13.0 / 16.2; bfloat4_b [1056, 4096] 6.1 / 8.6), as do 17 and more rows whose x does not fit, up to K 2816 (bfloat4_b [2816, 14336]
-// 19.9 / 21.4; [3072, 14336] 20.4 / 18.7). N may not enter, and the gain of 17 and more rows of a block-float weight ends at some 12000
-// to 20000 columns (with w_up both weights' count): 32 rows of bfloat8_b with w_up, [1536, 4608] 0.64 of the other's time, [1536, 6144]
-// 1.03, [1536, 20480] 1.37; 24 rows of bfloat4_b, [1024, 4096] 0.85, [1024, 20480] 1.24; K 2560 of bfloat4_b is the worst
-// ([2560, 5120] 32 rows 1.09, 17 rows 1.26). A head of 75968 columns takes up to twice the other's time (bfloat4_b, 24 rows, K 2560,
-// 77 / 38 us; bfloat8_b, 32 rows, K 1536, 56 / 33), which the projections of a model's layers outweigh.
-// (Measured with the warps' numbers not yet shuffled: both kernels have taken 0.9 to 0.95 of these times since.)
+// the tensor-memory kernel, 900 shapes of 9 to 32 rows, K 544 to 4096, N 1024 to 14336:
+// 9 to 16 rows, wherever x leaves 80 KB of the 227 to the ring: bfloat8_b [1280, 4096] 4.5 / 6.4, [2048, 14336] 10.5 / 11.7, [3584, 14336]
+// with 16 rows, the worst, 17.9 / 15.0 ([3584, 4096] 7.4 / 9.1); bfloat4_b [2816, 4096] 5.4 / 7.7; bf16, 16 rows, [2048, 4096] 5.6 / 7.7,
+// [3072, 4096] 7.1 / 8.7, but [3072, 2048] 6.4 / 4.9 and [3072, 14336] 19.2 / 17.3 (over all N, 16 rows of K 3072 1.06 of the other's time,
+// of K 2048 0.91, 9 rows of K 4096 1.04). Less of a ring: bfloat8_b, 16 rows, [4096, 14336] 20.0 / 16.3, [4096, 4096] 8.0 / 9.2.
+// 17 to 24 rows, three MMAs a fragment: of four slices, where the other runs in clusters, up to K 1536 (bfloat8_b [1056, 4096] 5.3 / 7.2;
+// of K 2048, 24 rows, N 2048 6.1 / 5.3, N 4096 6.5 / 7.3, N 14336 13.6 / 12.7, though 17 rows of K 2048 would take 0.9 of the other's time
+// over all N; bf16 of K 1536, N 2048 5.3 / 4.4, over all N 0.99); of other numbers of slices always (bfloat4_b [2816, 4096] 6.3 / 8.2).
+// 25 to 32 rows of other numbers of slices: bf16 with four MMAs a fragment ([1056, 14336] 11.6 / 11.9, [1056, 4096] 5.9 / 6.8); block-float
+// decodes beside four MMAs took longer than the tensor memory's way ([1056, 14336] 19.5 / 16.2, before either kernel's last speed-up), and
+// so run as two tiles of sixteen rows, a team of CTAs each ([1056, 14336] 12.4 / 14.0; bfloat4_b [1056, 4096] 5.9 / 7.3), as do 17 and
+// more rows whose x does not fit, up to K 2816 (bfloat4_b [2816, 4096] 8.0 / 8.7, [2816, 14336] 18.4 / 17.4; of K 3072, N 2048 5.8 / 8.2, N
+// 8192 12.3 / 14.4, N 14336 18.9 / 17.0).
+// N may not enter, and the gain of 17 and more rows of a block-float weight ends at some 12000 to 20000 columns: 24 rows of bfloat4_b,
+// [1056, 14336] 9.8 / 11.8, 32 rows of bfloat8_b [1536, 4096] 6.5 / 7.4, [1536, 14336] 14.1 / 13.7, of bfloat4_b [2560, 14336] 17.6 / 16.6.
 int rows_layout(TkdParams& p, int sab) {
     const int ck = tkd_chunk_k(p.fmt), nch = (p.K + ck - 1) / ck;
     if (p.M > 16 && p.nslices == 4 && (p.M > 24 || p.K > 1536)) return 0;
@@ -211,11 +213,13 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false, bo
         // A streaming warp stays with one slice, so those of a short last slice wait, and with fewer slices some have none; still
         // that is the faster form, since no sums go through L2, but for a K of one slice, whose sums need not: there only up to an item
         // for every other CTA; and of two or three slices at one row, or of bf16, only up to six items a CTA. Measured, launches in a
-        // graph over weights larger than L2, us with this kernel / the counting one: bfloat8_b one row, [256, 2048] 1.9 / 2.3, [256, 5392]
-        // 3.2 / 2.3, [256, 20480] 5.0 / 4.5, with w_up [1536, 20480] 15.3 / 13.6; bf16 one row, [128, 5392] 3.5 / 2.1, with w_up
-        // [384, 20480] 11.0 / 8.9; bfloat8_b one row, [1280, 4096] (three slices) 3.7 / 4.9, [2080, 4096] (a
-        // third of the last) 4.7 / 5.9; eight rows, [1280, 4096] 4.2 / 5.9, bfloat4_b [5120, 4096] 6.0 / 10.6, [8192, 11008] (two
-        // stages) 17.2 / 21.9; bfloat8_b [8192, 11008] (two stages) 25.7 / 25.8. Two stages of bf16: [8192, 1024] 12.6 / 11.5.
+        // graph over weights larger than L2, us with this kernel / the counting one. One slice: bfloat8_b one row, [256, 2048] 1.8 / 2.3,
+        // [256, 4096] 2.4 / 2.3, [256, 20480] 4.7 / 4.6; bfloat4_b [512, 2048] 1.9 / 2.7, [512, 4096] 2.6 / 2.7, eight rows 3.1 / 3.3; bf16
+        // [128, 2048] 1.8 / 2.1, [128, 4096] 2.4 / 2.1, [256, 20480] 6.0 / 4.4. Two and three: with w_up bfloat8_b [1536, 10240] 9.0 / 9.8,
+        // [1536, 20480] 14.4 / 13.5, bf16 [384, 10240] 6.9 / 7.3, [384, 20480] 10.4 / 8.8 (one row of bfloat8_b [768, 28672] would take 7.1
+        // where the other takes 8.7); bfloat8_b [1280, 4096] 2.95 / 4.6, eight rows 3.5 / 5.9; bfloat4_b, eight rows, [5120, 4096] 5.4 / 10.4, [2560,
+        // 28672] 13.3 / 12.7. Four: bfloat8_b [2080, 4096] (a third of the last) 3.7 / 5.6; two stages of the ring, eight rows: bfloat8_b [8192,
+        // 11008] 25.0 / 25.8, bfloat4_b 16.6 / 22.0. Two stages of bf16, eight rows: [8192, 1024] 12.6 / 11.5 (before this kernel's last speed-up).
         const int64_t narrow_xt = p.off_pbuf + 2 * 8 * 32 * (a->m > 1 ? 8 : 1) * 4;
         const int narrow_stage = p.nslices * 2 * tkd_subsa(a->fmt) * sab;
         const int64_t items = 4 * (int64_t)panels;
@@ -238,7 +242,7 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false, bo
     L->smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
 
     // (a K of one slice: the tensor-memory kernel, a panel an item, no sums through L2. Us with tkd_rows_kernel / with that: bfloat4_b
-    // [512, 11008] 24 rows 10.2 / 5.3; bfloat8_b [256, 11008] 32 rows 7.7 / 4.6, [256, 5392] 9 rows 4.8 / 3.5, with w_up [256, 2048] 4.0 / 4.4)
+    // [512, 11008] 24 rows 7.1 / 5.0; bfloat8_b [256, 11008] 32 rows 7.6 / 4.4, [256, 5392] 9 rows 4.7 / 3.3, with w_up [256, 2048] 4.0 / 4.1)
     if (p.tc && !a->ks && (p.nslices > 1 || tile)) p.rows_chunks = rows_layout(p, sab);
     if (p.rows_chunks) p.tc = 0, L->smem = (size_t)p.off_ring + (size_t)p.nstages * p.stage_bytes;
     const int64_t items = p.narrow || p.rows_chunks ? 4 * (int64_t)panels : p.total_items;
@@ -250,6 +254,10 @@ int make_layout(const TkdMatmul* a, Layout* L, int sms, bool counted = false, bo
     // 9 to 32 rows: clusters of four CTAs, one to a slice (tkd_stream_tc.cuh), for a plain call of four slices. They take whole
     // panels and leave some SMs idle (a GPC's number of SMs is not a multiple of four: 132 of 148 CTAs on a B200), so they are
     // taken where no CTA gets more items for it; from four items on the other form's SMs that have one less leave theirs to the rest.
+    // 32 rows, us in clusters / without: one item, bfloat8_b [4096, 2048] 6.9 / 9.0, [4096, 4224] 9.6 / 10.0, bf16 10.2 / 10.1; two, [4096,
+    // 6144] 12.9 / 14.6, bf16 13.8 / 15.1, where it is one without, [4096, 4736] 13.1 / 10.7; three, [4096, 12672] 17.3 / 17.8, bf16, whose
+    // bytes want every SM, 21.9 / 20.8 (K 8192 34.3 / 36.1); four, [4096, 14336] 21.0 / 17.3, [4096, 16896] 21.3 / 21.0, [8192, 16896] 30.7 /
+    // 33.1, seven, [4096, 28672] 34.1 / 27.9.
     if (p.tc && !counted && on_device && p.nslices == 4 && !a->topk_k && a->nranks <= 1) {
         const int off_xt = p.off_tbuf + 2 * 4 * 8 * 32 * 16, off_ring = (int)align_up(off_xt + 1024 + xslots * 2 * 4096, 128);
         const int stages = (int)((kMaxSmem - off_ring) / p.stage_bytes < TKD_MAX_STAGES ? (kMaxSmem - off_ring) / p.stage_bytes : TKD_MAX_STAGES);
@@ -502,7 +510,7 @@ static int make_wide(const TkdMatmul* a, TkdWide* w, size_t* smem, uint64_t* ws_
     // (an MMA of up to 128 rows is shorter than its issue: two warps, an accumulator each)
     p.nmma = p.nt <= 128 ? 2 : 1;
     p.nset = p.nmma * p.nt * 2 <= 256 ? 2 : 1;
-    p.nx = p.nt <= 128 ? 8 : 4;
+    p.nx = p.nt <= 128 ? 8 : 4;  // (a multiple of two tiles for each MMA warp: a warp's slots wrap with one subtraction, tkd_wide.cuh)
     p.panel_bytes = tkd_panel_bytes(a->fmt, a->k);
     p.stage_bytes = 8 * tkd_subsa(a->fmt) * tkd_sab(a->fmt);
     p.off_stage = TKD_SMEM_HEAD;
