@@ -128,6 +128,8 @@ __global__ void __launch_bounds__(DOWN ? 512 : 128, DOWN ? 1 : 4) tkd_moe_kernel
     __shared__ uint64_t s_bars[2 * 16];
     __shared__ int s_e[DOWN ? 17 : 1];  // down: a slot's exponent byte, -1 without an expert
     __shared__ float red[DOWN ? 17 : 1][kMoeSplit][DOWN ? 16 : 32];  // [slot][run][column]
+    // (the warp's number by a shuffle, as in tkd_narrow_kernel: gate_up of 8 of 128 experts, 2048 -> 2 x 768, 6.3 us without, 6.0 so, down 3.76
+    // and 3.72)
     const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t = lane & 3;
     const uint32_t buf = smem_u32(moe_dsm) + warp * 2 * kMoeHalfBytes<FMT>, bars = smem_u32(s_bars) + warp * 16;
     if (lane == 0) {

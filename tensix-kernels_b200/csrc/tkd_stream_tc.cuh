@@ -22,7 +22,9 @@
 //                  The same warps write the tile of activations a unit is multiplied by (32 rows x 64 k, rows past M
 //                  zero, K-major with the 128-byte swizzle, in that order of k) into shared memory: each lane loads
 //                  its 16 bytes of the NEXT chunk's tiles into registers while it decodes this chunk (they come from
-//                  L2, a microsecond away). bf16 weights: the warps from 23 on do, by asynchronous copies of 8 bytes.
+//                  L2, a microsecond away). bf16 weights: the warps from 23 on do, by asynchronous copies of 8 bytes; their tiles'
+//                  rows past M hold copies of the last row or what lay there, and only columns of D that nothing reads
+//                  depend on them.
 //   warps 19-22    output warps (thread = panel column = tensor-memory lane): read a slice's sums with tcgen05.ld, keep
 //                  the running sums in shared memory, and from there on do what tkd_stream_kernel's output warps do
 //   warp 1         producer (one lane issues): the same ring of packed-weight chunks as tkd_stream_kernel
@@ -63,6 +65,7 @@ constexpr int kTcMmaWarp = 0, kTcProducerWarp = 1, kTcDecodeWarp0 = 3, kTcOutput
 template <int FMT>
 constexpr bool kTcXw = FMT == TKD_BF16;
 constexpr int kTcXSlots = TKD_TC_XSLOTS;
+static_assert(kTcXSlots % kTcMmaWarps == 0, "a slot of x is one MMA warp's: it sees every phase of its barriers");
 template <bool CL>
 constexpr int kTcXWarps = CL ? 4 : 2;
 template <int FMT, bool CL>
@@ -306,8 +309,8 @@ __global__ void __launch_bounds__(kTcWarps<FMT, CL> * 32, 1) tkd_stream_tc_kerne
         // ---------------------------------------------------------------- decode warps
         if constexpr (!XW) asm volatile("griddepcontrol.wait;" ::: "memory");  // (x may be the output of the kernel before this one)
         // The warps form G groups, and a unit (by its number in this CTA's sequence, mod G) is one group's work from its
-        // slot's "empty" to its "full": while a group waits for its stores to land (tcgen05.wait::st, the proxy fence),
-        // the others decode. A slot is always the same group's (kTcSlots is a multiple of G), so the group's warps see
+        // slot's "empty" to its "full": while a group waits for its stores to land (tcgen05.wait::st), the others
+        // decode. A slot is always the same group's (kTcSlots is a multiple of G), so the group's warps see
         // every phase of its barriers. A warp may touch the tensor-memory lanes 32 (warp % 4) .. + 31 only: its RG row
         // groups of 16 panel columns are among them.
         constexpr int G = kTcGroups, RG = G / 2, PP = G / 2;
@@ -497,6 +500,7 @@ __global__ void __launch_bounds__(kTcWarps<FMT, CL> * 32, 1) tkd_stream_tc_kerne
         // nothing reads.
         asm volatile("griddepcontrol.wait;" ::: "memory");  // (x may be the output of the kernel before this one)
         constexpr int RS = 2 * kTcXWarps<CL>, NR = 32 / RS;
+        static_assert(RS == 4 || RS == 8, "a lane's rows r0 + RS i share the low bits of the swizzle, or differ in one that RS i sets");
         const int gl = (warp - kTcXWarp0) * 32 + lane, r0 = gl >> 4, ke = 4 * (gl & 15);  // this lane's first row, its k of a tile
         const uint32_t o = 64 * (ke >> 5) + 32 * ((ke >> 2) & 1) + 8 * ((ke >> 3) & 3);
         const uint32_t d0 = ops0 + r0 * 128 + (o & 15), c0 = ((o >> 4) ^ (r0 & 7)) << 4;

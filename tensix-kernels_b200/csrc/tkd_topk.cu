@@ -220,7 +220,7 @@ __device__ __forceinline__ void pick_count(PickCount& s, int nrec, int k, int to
     }
 }
 
-// One CTA per row r of the step.
+// One CTA, or one cluster of CL CTAs, per row r of the step.
 //   1. The best `top` slots of row r over the records in order (record by record, slot by slot), by key (RECORDS: by
 //      rank16, and top is 1); an equal key keeps the earlier slot; a slot with key 0 or an id at or past `vocab` is empty: by
 //      counting (COUNT: pick_count), or a warp takes a run of slots, 256 at a time beside its best so far; one warp merges the warps' lists.
@@ -233,8 +233,9 @@ __device__ __forceinline__ void pick_count(PickCount& s, int nrec, int k, int to
 // took a fifth of a vocabulary's call. CL, of three and more rows: a row is a cluster of CL CTAs; each finds the same
 // candidates and takes its share of their rows, whose exact logits meet in the first one's shared memory. The candidates lie anywhere in
 // the head, each in a page of its own as a rule, and sixteen such rows at a time were more than an SM has under way beside other CTAs
-// that ask for theirs: records and pick of 8 rows of a head of 118656 columns of 3328 90.5 us with a CTA a row, 87.6 so; 4 rows of 34304
-// columns of 3712 44.7 and 41.5; one row 65.5 and 66.0, so one and two rows keep a CTA each.
+// that ask for theirs: records and pick of 8 rows of a head of 118656 columns of 3328 89.4 us with a CTA a row, 88.3 so, 4 rows 78.3 and
+// 77.3; 4 rows of 34304 columns of 3712 45.2 and 41.6. One and two rows keep a CTA each: 65.9 and 66.4, 72.5 and 72.4 (31.7 and 31.6, 38.8
+// and 38.5).
 template <bool RECORDS, bool COUNT, int CL>
 __global__ void __launch_bounds__(kPickWarps * 32) tkd_head_pick_kernel(const uint32_t* __restrict__ records, int nrec, int rows,
                                                                         int k, int top, uint32_t vocab,
