@@ -1,5 +1,7 @@
 """The kernel that keeps 9 to 32 rows of x in shared memory (csrc/tkd_rows.cuh): its outputs, its records and its exchanged calls."""
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -7,7 +9,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 from common import ttnn_like as ttnn  # noqa: E402
-from dense_reader import linear, sharded  # noqa: E402
+from dense_reader import _tkd, linear, sharded  # noqa: E402
 from oracle import oracle as orc  # noqa: E402
 from test_exchange_gpu import fake_rank  # noqa: E402
 from test_parity_gpu import DT, close_bf16, dev_x, host  # noqa: E402
@@ -45,8 +47,23 @@ def test_outputs_against_oracle(device, fmt, m, k, n):
     linear.check_status(device)
 
 
+def runs_in_tensor_memory(fmt, m, k, n, ctas):
+    """Whether a plain call of 9 to 32 rows runs the tensor-memory kernel: given its slice size, which the other kernel does not serve, it is
+    the same launch."""
+    a, plans = _tkd.TkdMatmul(), []
+    a.fmt, a.m, a.k = {"bfp8": _tkd.FMT_BFP8, "bfp4": _tkd.FMT_BFP4, "bf16": _tkd.FMT_BF16}[fmt], m, k
+    a.nblocks, a.epilogue, a.out_dtype = 1, _tkd.EPI_PLAIN, _tkd.DT_BF16
+    a.block[0].n, a.max_ctas = n, ctas or 0
+    for _ in range(2):
+        p = _tkd.TkdPlan()
+        assert _tkd.lib().tkd_matmul_plan(ctypes.byref(a), ctypes.byref(p)) == 0
+        plans.append((p.smem_bytes, p.stages, p.grid))
+        a.ks = p.ks
+    return plans[0] == plans[1]
+
+
 @pytest.mark.parametrize("fmt", ["bfp8", "bfp4", "bf16"])
-@pytest.mark.parametrize("m,k,n", [(17, 2080, 208), (24, 4128, 144), (31, 6560, 2064), (32, 8224, 272), (9, 14368, 80)])
+@pytest.mark.parametrize("m,k,n", [(17, 3104, 208), (24, 4128, 144), (31, 6560, 2064), (32, 8224, 272), (9, 14368, 80)])
 def test_units_of_the_tensor_memory_kernel(device, fmt, m, k, n):
     """K that ends inside a unit of 128, a tile of 64 and a chunk, more units than there are slots, in clusters and without; the rows
     past the call's, which hold what a call before left in shared memory (here NaN), show nowhere. float32 results within K products
@@ -57,6 +74,8 @@ def test_units_of_the_tensor_memory_kernel(device, fmt, m, k, n):
     tx, nan = dev_x(device, x), dev_x(device, torch.full((32, k), float("nan")))
     want = x.to(torch.bfloat16).double() @ torch.from_numpy(orc.native_values(w, fmt)[0]).double()
     for ctas in (None, 3):
+        for rows in (m, 32):
+            assert runs_in_tensor_memory(fmt, rows, k, n, ctas), (rows, ctas)
         assert bool(host(linear.matmul(nan, tw, None, max_ctas=ctas)).isnan().all())
         y = host(linear.matmul(tx, tw, None, out32=True, max_ctas=ctas)).double()
         assert ((y - want).norm() / want.norm()).item() < 1e-5
@@ -67,6 +86,7 @@ def test_units_of_the_tensor_memory_kernel(device, fmt, m, k, n):
 @pytest.mark.parametrize("m,k,n", [(17, 3104, 192), (32, 4128, 144), (9, 14368, 64)])
 def test_every_output_of_a_k_that_ends_inside_a_chunk(device, fmt, m, k, n):
     """The tensor-memory kernel has an instance for each kind of output, outside clusters and (for fewer kinds) in them."""
+    assert runs_in_tensor_memory(fmt, m, k, n, None) and runs_in_tensor_memory(fmt, m, k, n, 3)
     test_outputs_against_oracle(device, fmt, m, k, n)
     g = torch.Generator().manual_seed(m)
     w, x = torch.randn(n, k, generator=g) * 0.05, torch.randn(m, k, generator=g)
